@@ -6,7 +6,7 @@ import ctypes as C
 import torch
 
 from ..core import native as N
-from .kernels import _dt
+from .kernels import _dt, status_tensor
 
 
 def flash_prefill_available(head_dim: int) -> bool:
@@ -17,6 +17,10 @@ def flash_prefill_available(head_dim: int) -> bool:
 
 
 FLASH_TILE_ROWS = 64
+# Visible keys from which heads of 256 columns take the tcgen05 kernel.  Its set-up (tensor memory, maps) costs 6 us more than the
+# register form, a key a quarter of the time (24 heads on 4: 161 / 193 / 225 / 257 / 385 rows of a new sequence 36 / 37 / 37 / 38 / 40
+# us against 34 / 35 / 39 / 40 / 57; 65 rows after 8192 tokens 165 against 523)
+TC_MIN_KEYS = 224
 
 
 def flash_prefill_segs(q, gate, kv_cache, block_table, seg_start, seg_slot, pos, seg_rows, out, H, Hkv, D, page, scale,
@@ -49,6 +53,16 @@ def flash_prefill(q, gate, kv_cache, block_table, slot: int, pos0: int, out, H, 
     L = N.lib()
     T = q.shape[0]
     bt_row = block_table[slot]
+    aligned = not (q.data_ptr() | kv_cache.data_ptr() | out.data_ptr() | (0 if gate is None else gate.data_ptr())) & 15
+    if (D == 256 and page == 16 and window == 0 and pos0 + T >= TC_MIN_KEYS and scale > 0 and aligned
+            and hasattr(L, "he_flash_prefill_tc")):
+        st = status_tensor(q.device)
+        N.check(L.he_flash_prefill_tc(C.c_void_p(q.data_ptr()), C.c_void_p(None if gate is None else gate.data_ptr()),
+                                      C.c_void_p(kv_cache.data_ptr()), C.c_longlong(kv_cache.shape[0]),
+                                      C.c_void_p(bt_row.data_ptr()), C.c_void_p(out.data_ptr()), C.c_int(T), C.c_int(H),
+                                      C.c_int(Hkv), C.c_int(pos0), C.c_float(scale), C.c_void_p(st.data_ptr()),
+                                      C.c_void_p(torch.cuda.current_stream().cuda_stream)), "he_flash_prefill_tc")
+        return
     N.check(L.he_flash_prefill(C.c_void_p(q.data_ptr()), C.c_void_p(None if gate is None else gate.data_ptr()),
                                C.c_void_p(kv_cache.data_ptr()), C.c_void_p(bt_row.data_ptr()),
                                C.c_void_p(out.data_ptr()), C.c_int(T), C.c_int(H), C.c_int(Hkv), C.c_int(D),
