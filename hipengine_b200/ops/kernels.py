@@ -92,7 +92,8 @@ class _GdnDecodeArgs(C.Structure):
 class _GdnChunkArgs(C.Structure):
     _fields_ = [("qkv", c_vp), ("decay", c_vp), ("beta", c_vp), ("state", c_vp), ("seg_start", c_vp),
                 ("seg_slot", c_vp), ("out", c_vp), ("C", C.c_int), ("G", C.c_int), ("Hv", C.c_int), ("T", C.c_int),
-                ("n_seg", C.c_int), ("write_state", C.c_int)]
+                ("n_seg", C.c_int), ("write_state", C.c_int), ("ws", c_vp), ("ws_floats", c_ll), ("c_lo", C.c_int),
+                ("c_hi", C.c_int)]
 
 
 class _MoeSelArgs(C.Structure):
@@ -490,17 +491,24 @@ def gdn_scan(qkv: torch.Tensor, decay: torch.Tensor, beta: torch.Tensor, state: 
     N.check(N.lib().he_gdn_scan(C.byref(p), _stream()), "he_gdn_scan")
 
 
+def gdn_chunk_ws_floats(T: int, n_seg: int, Hv: int, write_state: bool = True) -> int:
+    L = N.lib()
+    L.he_gdn_chunk_ws_floats.restype = C.c_longlong
+    return int(L.he_gdn_chunk_ws_floats(C.c_int(T), C.c_int(n_seg), C.c_int(Hv), C.c_int(int(write_state))))
+
+
 def gdn_scan_chunked(qkv: torch.Tensor, decay: torch.Tensor, beta: torch.Tensor, state: torch.Tensor,
                      seg_start: torch.Tensor, seg_slot: torch.Tensor, out: torch.Tensor, G: int, Hv: int,
-                     write_state: bool = True) -> None:
-    """Chunked (16-token, WY form) tensor-core scan for prefill segments; same contract as ``gdn_scan`` without the
-    journal.  Products run in TF32 with fp32 accumulation."""
+                     write_state: bool = True, ws: Optional[torch.Tensor] = None) -> None:
+    """Chunked (32-token, WY form) tensor-core scan for prefill segments; same contract as ``gdn_scan`` without the
+    journal.  Products run in TF32 with fp32 accumulation.  ``ws``: fp32 workspace of ``gdn_chunk_ws_floats``."""
     _check_abi()
     p = _GdnChunkArgs()
     p.qkv, p.decay, p.beta, p.state = qkv.data_ptr(), decay.data_ptr(), beta.data_ptr(), state.data_ptr()
     p.seg_start, p.seg_slot, p.out = seg_start.data_ptr(), seg_slot.data_ptr(), out.data_ptr()
-    p.C, p.G, p.Hv, p.T, p.n_seg, p.write_state = qkv.shape[1], G, Hv, qkv.shape[0], seg_slot.numel(), int(write_state)
-    assert qkv.dtype == torch.float32 and qkv.is_contiguous()
+    p.C, p.G, p.Hv, p.T, p.n_seg, p.write_state = qkv.shape[1], G, Hv, T, n_seg, int(write_state)
+    p.ws, p.ws_floats = ws.data_ptr(), ws.numel()
+    assert qkv.dtype == torch.float32 and qkv.is_contiguous() and ws.dtype == torch.float32
     N.check(N.lib().he_gdn_scan_chunked(C.byref(p), _stream()), "he_gdn_scan_chunked")
 
 
@@ -526,6 +534,10 @@ def gdn_decode(x: torch.Tensor, conv_w: torch.Tensor, conv_state: torch.Tensor, 
     p.qkv, p.decay, p.beta, p.state = qkv.data_ptr(), decay.data_ptr(), beta.data_ptr(), state.data_ptr()
     p.z, p.z_dtype, p.z_stride, p.norm_w = z.data_ptr(), _dt(z), z.stride(0), norm_w.data_ptr()
     p.out, p.out_stride, p.eps = out.data_ptr(), out.stride(0), eps
+    T, n_seg = qkv.shape[0], seg_slot.numel()
+    n_ws = gdn_chunk_ws_floats(T, n_seg, Hv, write_state)
+    if ws is None:
+        ws = torch.empty(n_ws, dtype=torch.float32, device=qkv.device)
     p.C, p.G, p.Hv, p.R = qkv.shape[1], G, Hv, x.shape[0]
     assert x.dtype == torch.float32
     N.check(N.lib().he_gdn_decode(C.byref(p), _stream()), "he_gdn_decode")

@@ -4,6 +4,8 @@ import math
 import pytest
 import torch
 
+from hipengine_b200.ref import ops as R
+
 pytestmark = pytest.mark.gpu
 
 
@@ -36,3 +38,30 @@ def test_tensor_memory_attention_matches_64_bit(T, H, Hkv, pos0):
         assert float((out.double() - want).norm() / want.norm()) < 5e-3
         assert float((out.double() - want).abs().max()) < 2e-2 * float(want.abs().max())
     K.check_status()
+
+
+@pytest.mark.parametrize("lens,Hv", [([5500], 1), ([64, 1, 95], 2), ([100, 2600, 33], 2)])
+def test_scan_windows_and_segments(lens, Hv):
+    """More chunks than one window holds, segments of uneven length: the same recurrence as the serial kernel."""
+    from hipengine_b200.ops import kernels as K
+    G, S, T = 1, 128, sum(lens)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    q, k = R.l2norm(rand(T, G, S)) * S ** -0.5, R.l2norm(rand(T, G, S))
+    qkv = torch.cat([q.reshape(T, -1), k.reshape(T, -1), rand(T, Hv * S) * 0.5], 1).contiguous()
+    decay, beta = torch.exp(-0.2 * rand(T, Hv).abs()), torch.sigmoid(rand(T, Hv))
+    start = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+    slot = torch.arange(len(lens), 0, -1, dtype=torch.int32, device="cuda")
+    state0 = rand(len(lens) + 1, Hv, S, S) * 0.1
+    outs, states = [], []
+    for fn in (K.gdn_scan, K.gdn_scan_chunked):
+        st, out = state0.clone(), torch.zeros(T, Hv, S, device="cuda")
+        fn(qkv, decay, beta, st, start, slot, out, G, Hv)
+        outs.append(out)
+        states.append(st)
+    assert torch.equal(states[1][0], state0[0])
+    for a, b in ((outs[1], outs[0]), (states[1], states[0])):
+        assert float((a - b).norm() / b.norm()) < 2e-3          # TF32 products against fp32
+    st, out = state0.clone(), torch.zeros(T, Hv, S, device="cuda")
+    K.gdn_scan_chunked(qkv, decay, beta, st, start, slot, out, G, Hv, write_state=False)
+    assert torch.equal(st, state0) and float((out - outs[1]).norm() / outs[1].norm()) < 1e-6
