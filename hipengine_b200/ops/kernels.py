@@ -504,6 +504,10 @@ def gdn_scan_chunked(qkv: torch.Tensor, decay: torch.Tensor, beta: torch.Tensor,
     journal.  Products run in TF32 with fp32 accumulation.  ``ws``: fp32 workspace of ``gdn_chunk_ws_floats``."""
     _check_abi()
     p = _GdnChunkArgs()
+    T, n_seg = qkv.shape[0], seg_slot.numel()
+    n_ws = gdn_chunk_ws_floats(T, n_seg, Hv, write_state)
+    if ws is None:
+        ws = torch.empty(n_ws, dtype=torch.float32, device=qkv.device)
     p.qkv, p.decay, p.beta, p.state = qkv.data_ptr(), decay.data_ptr(), beta.data_ptr(), state.data_ptr()
     p.seg_start, p.seg_slot, p.out = seg_start.data_ptr(), seg_slot.data_ptr(), out.data_ptr()
     p.C, p.G, p.Hv, p.T, p.n_seg, p.write_state = qkv.shape[1], G, Hv, T, n_seg, int(write_state)
@@ -534,10 +538,6 @@ def gdn_decode(x: torch.Tensor, conv_w: torch.Tensor, conv_state: torch.Tensor, 
     p.qkv, p.decay, p.beta, p.state = qkv.data_ptr(), decay.data_ptr(), beta.data_ptr(), state.data_ptr()
     p.z, p.z_dtype, p.z_stride, p.norm_w = z.data_ptr(), _dt(z), z.stride(0), norm_w.data_ptr()
     p.out, p.out_stride, p.eps = out.data_ptr(), out.stride(0), eps
-    T, n_seg = qkv.shape[0], seg_slot.numel()
-    n_ws = gdn_chunk_ws_floats(T, n_seg, Hv, write_state)
-    if ws is None:
-        ws = torch.empty(n_ws, dtype=torch.float32, device=qkv.device)
     p.C, p.G, p.Hv, p.R = qkv.shape[1], G, Hv, x.shape[0]
     assert x.dtype == torch.float32
     N.check(N.lib().he_gdn_decode(C.byref(p), _stream()), "he_gdn_decode")
