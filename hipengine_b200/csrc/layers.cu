@@ -276,6 +276,95 @@ __global__ void qkv_post_kernel(const QkvArgs a) {
   }
 }
 
+// The same for heads of 256 columns in bf16, one CTA per token: the token's angles are computed once for all its heads
+// (every element of every head did so before: at 4096 tokens x 32 heads 296 us, 84 us now), a warp takes whole heads, eight
+// columns a lane, so all traffic is 16 bytes wide and the norm needs no barrier.  rope_dim: a multiple of 16.
+__global__ void __launch_bounds__(256) qkv_post_rows_kernel(const QkvArgs a) {
+  constexpr int D = 256;
+  __shared__ float2 rot[D / 2];
+  const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, d0 = lane * 8;
+  pdl_wait();
+  pdl_launch();
+  const int p = a.pos[t], half = a.rope_dim >> 1;
+  if ((int)threadIdx.x < half) {
+    const float inv_freq =
+        powf(a.theta, -2.0f * (float)threadIdx.x / (float)(a.rope_denom > 0 ? a.rope_denom : a.rope_dim));
+    float sn, cs;
+    sincosf((float)p * inv_freq, &sn, &cs);
+    rot[threadIdx.x] = make_float2(cs, sn);
+  }
+  __syncthreads();
+  const int s = a.slot[t];
+  const bool in_table = HE_INDEX_OK(p / a.page, a.max_pages, HE_SITE_KV_WRITE_PAGE);
+  const int page_id = in_table ? a.block_table[(size_t)s * a.max_pages + p / a.page] : 0;
+  auto load8 = [&](const void* src, size_t i, float (&v)[8]) {
+    if (a.in_dtype == 0) {
+      const float4* q = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(src) + i);
+      const float4 x = q[0], y = q[1];
+      v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+    } else {
+      const uint4 u = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(src) + i);
+      const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = __bfloat1622float2(h2[e]);
+        v[2 * e] = f.x; v[2 * e + 1] = f.y;
+      }
+    }
+  };
+  auto store8 = [&](__nv_bfloat16* dst, const float (&v)[8]) {
+    uint4 u;
+    __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&u);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) h2[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+    *reinterpret_cast<uint4*>(dst) = u;
+  };
+  for (int hh = warp; hh < a.H + 2 * a.Hkv; hh += 8) {
+    const int kind = hh < a.H ? 0 : (hh < a.H + a.Hkv ? 1 : 2);
+    const int h = kind == 0 ? hh : (kind == 1 ? hh - a.H : hh - a.H - a.Hkv);
+    float v[8];
+    if (kind == 0) load8(a.q, (size_t)t * a.q_stride + (size_t)h * D * (a.gated ? 2 : 1) + d0, v);
+    else if (kind == 1) load8(a.k, (size_t)t * a.k_stride + (size_t)h * D + d0, v);
+    else load8(a.v, (size_t)t * a.v_stride + (size_t)h * D + d0, v);
+    float gt[8];
+    const bool gate = kind == 0 && a.gated && a.gate_out != nullptr;
+    if (gate) load8(a.q, (size_t)t * a.q_stride + (size_t)h * D * 2 + D + d0, gt);
+    const float* nw = kind == 0 ? a.q_norm : (kind == 1 ? a.k_norm : nullptr);
+    if ((kind < 2 && nw != nullptr) || (kind == 2 && a.v_norm)) {
+      float ss = 0.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ss += v[e] * v[e];
+      const float inv = rsqrtf(warp_sum(ss) / (float)D + a.eps);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] *= inv;
+      if (nw != nullptr) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] *= nw[d0 + e];
+      }
+    }
+    if (kind < 2 && half > 0) {
+      const int step = half >> 3;                   // lanes between the two columns of a pair
+      const bool first = d0 < half, turns = d0 < a.rope_dim;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float other = __shfl_sync(0xffffffffu, v[e], (first ? lane + step : lane - step) & 31);
+        if (turns) {
+          const float2 r = rot[first ? d0 + e : d0 - half + e];
+          v[e] = first ? v[e] * r.x - other * r.y : v[e] * r.x + other * r.y;
+        }
+      }
+    }
+    if (kind == 0) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] *= a.q_scale;
+      store8(a.q_out + ((size_t)t * a.H + h) * D + d0, v);
+      if (gate) store8(a.gate_out + ((size_t)t * a.H + h) * D + d0, gt);
+    } else if (in_table) {
+      store8(a.kv_cache + ((((size_t)page_id * 2 + (kind - 1)) * a.Hkv + h) * a.page + (p % a.page)) * D + d0, v);
+    }
+  }
+}
+
 // ---------------------------------------------------------------- causal conv1d (k<=4) + SiLU with rolling state
 struct ConvArgs {
   const void* x;        // [T][x_stride] (first C columns used)
@@ -579,6 +668,15 @@ HE_API int he_qkv_post(const QkvArgs* args, int T, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (a.D % 32 != 0 || a.D > 512 || a.d_in > a.D || a.dv_in > a.D) return -HE_ERR_BAD_ARG;
   if ((a.d_in > 0 && a.d_in < a.D) && (a.gated || a.rope_dim > 0)) return -HE_ERR_BAD_ARG;
+  // whole heads per warp where every access is 16 bytes wide; for a few tokens a CTA per head spreads over more SMs
+  const auto al = [](const void* q, long long stride, int es) {
+    return (reinterpret_cast<uintptr_t>(q) & 15) == 0 && (stride * es) % 16 == 0;
+  };
+  const int es = a.in_dtype == 0 ? 4 : 2;
+  if (T >= 16 && a.D == 256 && (a.d_in == 0 || a.d_in == 256) && (a.dv_in == 0 || a.dv_in == 256) && !a.out_f32 &&
+      a.rope_dim % 16 == 0 && a.rope_dim <= 256 && al(a.q, a.q_stride, es) && al(a.k, a.k_stride, es) &&
+      al(a.v, a.v_stride, es) && al(a.q_out, 0, 2) && al(a.gate_out, 0, 2) && al(a.kv_cache, 0, 2))
+    return (int)launch_pdl(qkv_post_rows_kernel, dim3(T), dim3(256), 0, stream, a);
   dim3 grid(T, a.H + 2 * a.Hkv);
   cudaError_t le = launch_pdl(qkv_post_kernel, grid, dim3(a.D), a.D * sizeof(float), stream, a);
   if (le != cudaSuccess) return (int)le;

@@ -462,10 +462,14 @@ class HybridExecutor:
         cj = journal["conv"][i] if journal is not None else None
         _gdn_stage = self._stage("gdn_core")
         _gdn_stage.__enter__()
-        K.conv1d(qkv, self.F(i, "ssm_conv1d.weight"), self.conv_state[i], b.seg_start, b.seg_slot, b.tok_seg, conv, C,
-                 update_state=journal is None, journal=cj)
-        K.gdn_prepare(conv, a_p, b_p, self.F(i, "ssm_a").reshape(-1), self.F(i, "ssm_dt.bias").reshape(-1), decay, beta,
-                      G, Hv, S)
+        if journal is None and S == 128 and cfg.conv_kernel == 4:
+            K.gdn_front(qkv, self.F(i, "ssm_conv1d.weight"), self.conv_state[i], b.seg_start, b.seg_slot, conv, a_p, b_p,
+                        self.F(i, "ssm_a").reshape(-1), self.F(i, "ssm_dt.bias").reshape(-1), decay, beta, G, Hv)
+        else:
+            K.conv1d(qkv, self.F(i, "ssm_conv1d.weight"), self.conv_state[i], b.seg_start, b.seg_slot, b.tok_seg, conv, C,
+                     update_state=journal is None, journal=cj)
+            K.gdn_prepare(conv, a_p, b_p, self.F(i, "ssm_a").reshape(-1), self.F(i, "ssm_dt.bias").reshape(-1), decay,
+                          beta, G, Hv, S)
         o = sc.get("gdn_o", (T, Hv, S), torch.float32)
         gj = journal["gdn"][i] if journal is not None else None
         if (journal is None and S == 128 and T >= 64 * b.n_seg and os.environ.get("HE_GDN_CHUNKED", "1") != "0"):

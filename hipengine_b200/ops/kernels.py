@@ -89,6 +89,13 @@ class _GdnDecodeArgs(C.Structure):
                 ("C", C.c_int), ("G", C.c_int), ("Hv", C.c_int), ("R", C.c_int)]
 
 
+class _GdnFrontArgs(C.Structure):
+    _fields_ = [("x", c_vp), ("in_dtype", C.c_int), ("x_stride", c_ll), ("w", c_vp), ("conv_state", c_vp),
+                ("seg_start", c_vp), ("seg_slot", c_vp), ("out", c_vp), ("a", c_vp), ("b", c_vp), ("a_stride", c_ll),
+                ("b_stride", c_ll), ("ssm_a", c_vp), ("dt_bias", c_vp), ("decay", c_vp), ("beta", c_vp),
+                ("C", C.c_int), ("G", C.c_int), ("Hv", C.c_int), ("T", C.c_int), ("n_seg", C.c_int)]
+
+
 class _GdnChunkArgs(C.Structure):
     _fields_ = [("qkv", c_vp), ("decay", c_vp), ("beta", c_vp), ("state", c_vp), ("seg_start", c_vp),
                 ("seg_slot", c_vp), ("out", c_vp), ("C", C.c_int), ("G", C.c_int), ("Hv", C.c_int), ("T", C.c_int),
@@ -165,7 +172,7 @@ def _check_abi() -> None:
              ("he_gdn_prep_args_size", _GdnPrepArgs), ("he_gdn_scan_args_size", _GdnScanArgs),
              ("he_attn_dec_args_size", _AttnDecArgs), ("he_moe_sel_args_size", _MoeSelArgs),
              ("he_gdn_decode_args_size", _GdnDecodeArgs), ("he_gdn_chunk_args_size", _GdnChunkArgs),
-             ("he_gemv_comm_size", GemvComm)]
+             ("he_gdn_front_args_size", _GdnFrontArgs), ("he_gemv_comm_size", GemvComm)]
     for fn, st in pairs:
         if not hasattr(L, fn):           # a library built from a subset of the sources
             continue
@@ -489,6 +496,21 @@ def gdn_scan(qkv: torch.Tensor, decay: torch.Tensor, beta: torch.Tensor, state: 
     p.seg_start, p.seg_slot, p.out, p.journal = seg_start.data_ptr(), seg_slot.data_ptr(), out.data_ptr(), _p(journal)
     p.C, p.G, p.Hv, p.T, p.n_seg, p.write_state = qkv.shape[1], G, Hv, qkv.shape[0], seg_slot.numel(), int(write_state)
     N.check(N.lib().he_gdn_scan(C.byref(p), _stream()), "he_gdn_scan")
+
+
+def gdn_front(x: torch.Tensor, conv_w: torch.Tensor, conv_state: torch.Tensor, seg_start: torch.Tensor,
+              seg_slot: torch.Tensor, out: torch.Tensor, a: torch.Tensor, b: torch.Tensor, ssm_a: torch.Tensor,
+              dt_bias: torch.Tensor, decay: torch.Tensor, beta: torch.Tensor, G: int, Hv: int) -> None:
+    """``conv1d`` (four taps, state updated) and ``gdn_prepare`` of heads of 128 in one pass over the projections."""
+    _check_abi()
+    p = _GdnFrontArgs()
+    p.x, p.in_dtype, p.x_stride, p.w, p.conv_state = x.data_ptr(), _dt(x), x.stride(0), conv_w.data_ptr(), conv_state.data_ptr()
+    p.seg_start, p.seg_slot, p.out = seg_start.data_ptr(), seg_slot.data_ptr(), out.data_ptr()
+    p.a, p.b, p.a_stride, p.b_stride = a.data_ptr(), b.data_ptr(), a.stride(0), b.stride(0)
+    p.ssm_a, p.dt_bias, p.decay, p.beta = ssm_a.data_ptr(), dt_bias.data_ptr(), decay.data_ptr(), beta.data_ptr()
+    p.C, p.G, p.Hv, p.T, p.n_seg = out.shape[1], G, Hv, out.shape[0], seg_slot.numel()
+    assert out.dtype == torch.float32 and out.is_contiguous() and conv_w.shape[1] == 4
+    N.check(N.lib().he_gdn_front(C.byref(p), _stream()), "he_gdn_front")
 
 
 def gdn_chunk_ws_floats(T: int, n_seg: int, Hv: int, write_state: bool = True) -> int:

@@ -65,3 +65,71 @@ def test_scan_windows_and_segments(lens, Hv):
     st, out = state0.clone(), torch.zeros(T, Hv, S, device="cuda")
     K.gdn_scan_chunked(qkv, decay, beta, st, start, slot, out, G, Hv, write_state=False)
     assert torch.equal(st, state0) and float((out - outs[1]).norm() / outs[1].norm()) < 1e-6
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("lens", [[1], [2, 3, 40], [17, 1, 16, 100]])
+def test_front_is_convolution_then_preparation(dtype, lens):
+    from hipengine_b200.ops import kernels as K
+    G, Hv, S, T = 2, 6, 128, sum(lens)
+    C = 2 * G * S + Hv * S
+    g = torch.Generator(device="cuda").manual_seed(T)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x, w, ab = rand(T, C + 8).to(dtype)[:, :C], rand(C, 4) * 0.5, rand(T, 2 * Hv + 4)
+    a, b, ssm_a, dt = ab[:, :Hv], ab[:, Hv:2 * Hv], -rand(Hv).abs(), rand(Hv)
+    start = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+    slot = torch.arange(len(lens), 0, -1, dtype=torch.int32, device="cuda")
+    seg = torch.repeat_interleave(torch.arange(len(lens), device="cuda", dtype=torch.int32), torch.tensor(lens, device="cuda"))
+    state0 = rand(len(lens) + 1, C, 3)
+    got, want = [], []
+    for res, front in ((got, True), (want, False)):
+        st, out = state0.clone(), torch.zeros(T, C, device="cuda")
+        decay, beta = torch.zeros(T, Hv, device="cuda"), torch.zeros(T, Hv, device="cuda")
+        if front:
+            K.gdn_front(x, w, st, start, slot, out, a, b, ssm_a, dt, decay, beta, G, Hv)
+        else:
+            K.conv1d(x, w, st, start, slot, seg, out, C)
+            K.gdn_prepare(out, a, b, ssm_a, dt, decay, beta, G, Hv, S)
+        res += [st, out, decay, beta]
+    assert torch.equal(got[0], want[0])
+    for p, q in zip(got[1:], want[1:]):
+        assert torch.allclose(p, q, rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T", [1, 33])
+def test_gated_norm_of_128_columns(dtype, T):
+    from hipengine_b200.ops import kernels as K
+    Hv = 5
+    o, w = torch.randn(T, Hv, 128, device="cuda"), torch.rand(128, device="cuda") + 0.5
+    z = torch.randn(T, Hv * 128 + 8, device="cuda").to(dtype)[:, :Hv * 128]
+    out = torch.zeros(T, Hv * 128 + 4, device="cuda", dtype=torch.bfloat16)[:, :Hv * 128]
+    K.gdn_gated_norm(o, z, w, out, Hv, 128, 1e-6)
+    ref = R.gated_rmsnorm(o, w, z.float().reshape(T, Hv, 128), 1e-6).reshape(T, -1)
+    assert torch.allclose(out.float(), ref, rtol=8e-3, atol=1e-5)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("gated,rope,qk_norm", [(True, 64, True), (False, 256, True), (False, 0, False), (True, 16, False)])
+def test_projection_rows_match_the_per_head_kernel(dtype, gated, rope, qk_norm):
+    """16 tokens and more go a token per CTA; the same rows one by one go a head per CTA."""
+    from hipengine_b200.ops import kernels as K
+    T, H, Hkv, D = 19, 6, 2, 256
+    g = torch.Generator(device="cuda").manual_seed(5)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    q, k, v = (rand(T, n).to(dtype) for n in (H * D * (2 if gated else 1), Hkv * D, Hkv * D))
+    qn, kn = (rand(D).abs() + 0.5, rand(D).abs() + 0.5) if qk_norm else (None, None)
+    table = torch.randperm(8, device="cuda", generator=g).int().reshape(2, 4)
+    slot = torch.ones(T, dtype=torch.int32, device="cuda")
+    pos = torch.arange(11, 11 + T, dtype=torch.int32, device="cuda")
+    res = []
+    for step in (T, 1):
+        qo, go = torch.zeros(T, H, D, device="cuda", dtype=torch.bfloat16), torch.zeros(T, H, D, device="cuda", dtype=torch.bfloat16)
+        kv = torch.zeros(9, 2, Hkv, 16, D, device="cuda", dtype=torch.bfloat16)
+        for r in range(0, T, step):
+            s = slice(r, r + step)
+            K.qkv_post(q[s], k[s], v[s], qn, kn, qo[s], go[s] if gated else None, kv, table, slot[s], pos[s], H, Hkv, D, 16,
+                       gated, rope, 1e7, 1e-6)
+        res.append((qo, go, kv))
+    for a, b in zip(*res):
+        assert torch.allclose(a.float(), b.float(), rtol=8e-3, atol=1e-5)      # one bf16 rounding apart at most
