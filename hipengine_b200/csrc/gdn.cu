@@ -361,12 +361,75 @@ struct GdnDecodeArgs {
   long long out_stride;
   float eps;
   int C, G, Hv, R;
+  // one row, gates from the residual (gate_w non-null; then a and b are not read): alpha and beta rows of all heads
+  // [2 Hv][K] fp32, the residual row [K] fp32 and the norm in front of them
+  const float* gate_w;
+  const float* gate_x;
+  const float* gate_norm;
+  float gate_eps;
+  int K;
 };
 
-// grid (C/128, R), block 128: one channel per thread.  conv(k=4)+SiLU, rolling state shift, L2 norm of q/k heads,
-// and (block 0) the decay / beta gates of the row.
+// Alpha and beta of one head and their gates, in fp32, by a block of 128 threads: the two weight rows are requested ahead
+// of the predecessor's end.  As a product of their own (two 48-row weights, 8-bit) they cost a launch of ~5 us per layer.
+__device__ __forceinline__ void gate_block(const GdnDecodeArgs& p, int h, float* red) {
+  constexpr int KEEP = 12;                     // float4 per thread and row: 6144 columns; the rest is loaded in place
+  const int n4 = p.K >> 2, tid = threadIdx.x;
+  const float4* wa = reinterpret_cast<const float4*>(p.gate_w + (size_t)h * p.K);
+  const float4* wb = reinterpret_cast<const float4*>(p.gate_w + (size_t)(p.Hv + h) * p.K);
+  const float4* nw = reinterpret_cast<const float4*>(p.gate_norm);
+  float4 a[KEEP], b[KEEP];
+#pragma unroll
+  for (int i = 0; i < KEEP; ++i)
+    if (i * 128 + tid < n4) {
+      const float4 m = __ldg(nw + i * 128 + tid);
+      a[i] = __ldg(wa + i * 128 + tid);
+      b[i] = __ldg(wb + i * 128 + tid);
+      a[i] = make_float4(a[i].x * m.x, a[i].y * m.y, a[i].z * m.z, a[i].w * m.w);
+      b[i] = make_float4(b[i].x * m.x, b[i].y * m.y, b[i].z * m.z, b[i].w * m.w);
+    }
+  pdl_wait();
+  pdl_launch();
+  const float4* x = reinterpret_cast<const float4*>(p.gate_x);
+  float ss = 0.f, da = 0.f, db = 0.f;
+  const auto add = [&](const float4& v, const float4& fa, const float4& fb) {
+    ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+    da += v.x * fa.x + v.y * fa.y + v.z * fa.z + v.w * fa.w;
+    db += v.x * fb.x + v.y * fb.y + v.z * fb.z + v.w * fb.w;
+  };
+#pragma unroll
+  for (int i = 0; i < KEEP; ++i)
+    if (i * 128 + tid < n4) add(x[i * 128 + tid], a[i], b[i]);
+  for (int i = KEEP * 128 + tid; i < n4; i += 128) {
+    const float4 m = __ldg(nw + i), fa = __ldg(wa + i), fb = __ldg(wb + i);
+    add(x[i], make_float4(fa.x * m.x, fa.y * m.y, fa.z * m.z, fa.w * m.w),
+        make_float4(fb.x * m.x, fb.y * m.y, fb.z * m.z, fb.w * m.w));
+  }
+  ss = warp_sum(ss);
+  da = warp_sum(da);
+  db = warp_sum(db);
+  if ((tid & 31) == 0) {
+    red[tid >> 5] = ss;
+    red[4 + (tid >> 5)] = da;
+    red[8 + (tid >> 5)] = db;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    const float inv = rsqrtf(((red[0] + red[1]) + (red[2] + red[3])) / (float)p.K + p.gate_eps);
+    const float av = ((red[4] + red[5]) + (red[6] + red[7])) * inv, bv = ((red[8] + red[9]) + (red[10] + red[11])) * inv;
+    p.beta[h] = sigmoid_f(bv);
+    p.decay[h] = __expf(p.ssm_a[h] * softplus20_f(av + p.dt_bias[h]));
+  }
+}
+
+// grid (C/128 [+ Hv], R), block 128: one channel per thread.  conv(k=4)+SiLU, rolling state shift, L2 norm of q/k heads,
+// and (block 0, or Hv blocks of their own) the decay / beta gates of the row.
 __global__ void __launch_bounds__(128) gdn_decode_pre_kernel(const GdnDecodeArgs p) {
   __shared__ float red[32];
+  if ((int)blockIdx.x >= p.C / 128) {
+    gate_block(p, (int)blockIdx.x - p.C / 128, red);
+    return;
+  }
   pdl_wait();
   pdl_launch();
   const int r = blockIdx.y, blk = blockIdx.x, c = blk * 128 + threadIdx.x;
@@ -383,7 +446,7 @@ __global__ void __launch_bounds__(128) gdn_decode_pre_kernel(const GdnDecodeArgs
     y *= inv;
   }
   p.qkv[(size_t)r * p.C + c] = y;
-  if (blk == 0) {
+  if (blk == 0 && p.gate_w == nullptr) {
     for (int h = threadIdx.x; h < p.Hv; h += 128) {
       const float av = p.a[(size_t)r * p.a_stride + h], bv = p.b[(size_t)r * p.b_stride + h];
       p.beta[(size_t)r * p.Hv + h] = sigmoid_f(bv);
@@ -392,68 +455,67 @@ __global__ void __launch_bounds__(128) gdn_decode_pre_kernel(const GdnDecodeArgs
   }
 }
 
-// grid (Hv, R), block 512: thread (col = tid/4, ks = tid%4) owns rows ks*32..+31 of one column of S.
+// grid (Hv, R), block 512: thread (ks = tid / 128, col = tid % 128) owns rows ks*32..+31 of one column of S, so that a
+// warp's access covers whole 128-byte lines of the state; the four partial sums of a column meet in shared memory.
 // One recurrent step, then RMSNorm over the head's 128 outputs * w * SiLU(z) -> bf16.
-__global__ void __launch_bounds__(512) gdn_decode_step_kernel(const GdnDecodeArgs p) {
-  __shared__ __align__(16) float sq[KPAD];
-  __shared__ __align__(16) float sk[KPAD];
-  __shared__ float red[32];
+// Bound by the state (read and written once, 128 KB per head and row).
+__global__ void __launch_bounds__(512, 2) gdn_decode_step_kernel(const GdnDecodeArgs p) {
+  __shared__ __align__(16) float sq[DK];
+  __shared__ __align__(16) float sk[DK];
+  __shared__ float part[2][4][DV];
+  __shared__ float red[4];
   const int h = blockIdx.x, r = blockIdx.y, tid = threadIdx.x;
-  const int col = tid >> 2, ks = tid & 3;
+  const int col = tid & 127, ks = tid >> 7;
   const int kh = h % p.G;
   const float* row = p.qkv + (size_t)r * p.C;
   pdl_wait();
   pdl_launch();
-  if (tid < 128) {
-    const int dst = tid + (tid >> 5) * 4;
-    sq[dst] = row[(size_t)kh * DK + tid];
-    sk[dst] = row[(size_t)p.G * DK + (size_t)kh * DK + tid];
-  }
-  float* Sg = p.state + (((size_t)p.slot[r] * p.Hv + h) * DK) * DV;
+  float* Sg = p.state + (((size_t)p.slot[r] * p.Hv + h) * DK + ks * 32) * DV + col;
   float S[32];
 #pragma unroll
-  for (int i = 0; i < 32; ++i) S[i] = Sg[(size_t)(ks * 32 + i) * DV + col];
+  for (int i = 0; i < 32; ++i) S[i] = Sg[(size_t)i * DV];
+  if (ks == 0) sq[col] = row[(size_t)kh * DK + col];
+  if (ks == 1) sk[col] = row[(size_t)p.G * DK + (size_t)kh * DK + col];
   const float v = row[(size_t)2 * p.G * DK + (size_t)h * DV + col];
   const float dec = p.decay[(size_t)r * p.Hv + h], bet = p.beta[(size_t)r * p.Hv + h];
   __syncthreads();
-  float kr[32];
-#pragma unroll
-  for (int i4 = 0; i4 < 8; ++i4) {
-    const float4 k4 = *reinterpret_cast<const float4*>(&sk[ks * 36 + i4 * 4]);
-    kr[i4 * 4] = k4.x; kr[i4 * 4 + 1] = k4.y; kr[i4 * 4 + 2] = k4.z; kr[i4 * 4 + 3] = k4.w;
-  }
   float kv4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    S[i] *= dec;
-    kv4[i & 3] += kr[i] * S[i];
+  for (int i4 = 0; i4 < 8; ++i4) {
+    const float4 k4 = *reinterpret_cast<const float4*>(&sk[ks * 32 + i4 * 4]);
+    S[i4 * 4] *= dec;     kv4[0] += k4.x * S[i4 * 4];
+    S[i4 * 4 + 1] *= dec; kv4[1] += k4.y * S[i4 * 4 + 1];
+    S[i4 * 4 + 2] *= dec; kv4[2] += k4.z * S[i4 * 4 + 2];
+    S[i4 * 4 + 3] *= dec; kv4[3] += k4.w * S[i4 * 4 + 3];
   }
-  float kv = (kv4[0] + kv4[1]) + (kv4[2] + kv4[3]);
-  kv += __shfl_xor_sync(0xffffffffu, kv, 1);
-  kv += __shfl_xor_sync(0xffffffffu, kv, 2);
+  part[0][ks][col] = (kv4[0] + kv4[1]) + (kv4[2] + kv4[3]);
+  __syncthreads();
+  const float kv = (part[0][0][col] + part[0][1][col]) + (part[0][2][col] + part[0][3][col]);
   const float delta = (v - kv) * bet;
   float o4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
   for (int i4 = 0; i4 < 8; ++i4) {
-    const float4 q4 = *reinterpret_cast<const float4*>(&sq[ks * 36 + i4 * 4]);
-    S[i4 * 4] += kr[i4 * 4] * delta;         o4[0] += q4.x * S[i4 * 4];
-    S[i4 * 4 + 1] += kr[i4 * 4 + 1] * delta; o4[1] += q4.y * S[i4 * 4 + 1];
-    S[i4 * 4 + 2] += kr[i4 * 4 + 2] * delta; o4[2] += q4.z * S[i4 * 4 + 2];
-    S[i4 * 4 + 3] += kr[i4 * 4 + 3] * delta; o4[3] += q4.w * S[i4 * 4 + 3];
+    const float4 k4 = *reinterpret_cast<const float4*>(&sk[ks * 32 + i4 * 4]);
+    const float4 q4 = *reinterpret_cast<const float4*>(&sq[ks * 32 + i4 * 4]);
+    S[i4 * 4] += k4.x * delta;     o4[0] += q4.x * S[i4 * 4];
+    S[i4 * 4 + 1] += k4.y * delta; o4[1] += q4.y * S[i4 * 4 + 1];
+    S[i4 * 4 + 2] += k4.z * delta; o4[2] += q4.z * S[i4 * 4 + 2];
+    S[i4 * 4 + 3] += k4.w * delta; o4[3] += q4.w * S[i4 * 4 + 3];
   }
-  float o = (o4[0] + o4[1]) + (o4[2] + o4[3]);
-  o += __shfl_xor_sync(0xffffffffu, o, 1);
-  o += __shfl_xor_sync(0xffffffffu, o, 2);
+  part[1][ks][col] = (o4[0] + o4[1]) + (o4[2] + o4[3]);
 #pragma unroll
-  for (int i = 0; i < 32; ++i) Sg[(size_t)(ks * 32 + i) * DV + col] = S[i];
-  const float ss = block_sum(ks == 0 ? o * o : 0.f, red);
-  if (ks == 0) {
-    const float inv = rsqrtf(ss / (float)DV + p.eps);
-    const size_t zi = (size_t)r * p.z_stride + (size_t)h * DV + col;
-    const float zv = p.z_dtype == 0 ? reinterpret_cast<const float*>(p.z)[zi]
-                                    : bf16_to_f32(reinterpret_cast<const __nv_bfloat16*>(p.z)[zi]);
-    p.out[(size_t)r * p.out_stride + (size_t)h * DV + col] = f32_to_bf16(o * inv * p.norm_w[col] * silu_f(zv));
-  }
+  for (int i = 0; i < 32; ++i) Sg[(size_t)i * DV] = S[i];
+  __syncthreads();
+  if (ks != 0) return;
+  const float o = (part[1][0][col] + part[1][1][col]) + (part[1][2][col] + part[1][3][col]);
+  const float sw = warp_sum(o * o);
+  if ((tid & 31) == 0) red[tid >> 5] = sw;
+  asm volatile("bar.sync 1, 128;" ::: "memory");
+  const float inv = rsqrtf(((red[0] + red[1]) + (red[2] + red[3])) / (float)DV + p.eps);
+  const size_t zi = (size_t)r * p.z_stride + (size_t)h * DV + col;
+  const float zv = p.z_dtype == 0 ? reinterpret_cast<const float*>(p.z)[zi]
+                                  : bf16_to_f32(reinterpret_cast<const __nv_bfloat16*>(p.z)[zi]);
+  p.out[(size_t)r * p.out_stride + (size_t)h * DV + col] = f32_to_bf16(o * inv * p.norm_w[col] * silu_f(zv));
 }
 
 }  // namespace
@@ -530,7 +592,12 @@ HE_API int he_gdn_decode(const GdnDecodeArgs* args, cudaStream_t stream) {
   const GdnDecodeArgs& a = *args;
   if (a.R <= 0) return 0;
   if (a.C % 128 != 0 || a.C != 2 * a.G * 128 + a.Hv * 128 || a.Hv % a.G != 0) return -HE_ERR_BAD_ARG;
-  cudaError_t e = launch_pdl(gdn_decode_pre_kernel, dim3(a.C / 128, a.R), dim3(128), 0, stream, a);
+  if (a.gate_w != nullptr && (a.R != 1 || a.K <= 0 || a.K % 4 != 0 || a.gate_x == nullptr || a.gate_norm == nullptr ||
+                              ((reinterpret_cast<uintptr_t>(a.gate_w) | reinterpret_cast<uintptr_t>(a.gate_x) |
+                                reinterpret_cast<uintptr_t>(a.gate_norm)) & 15) != 0))
+    return -HE_ERR_BAD_ARG;
+  const int gates = a.gate_w != nullptr ? a.Hv : 0;
+  cudaError_t e = launch_pdl(gdn_decode_pre_kernel, dim3(a.C / 128 + gates, a.R), dim3(128), 0, stream, a);
   if (e != cudaSuccess) return (int)e;
   e = launch_pdl(gdn_decode_step_kernel, dim3(a.Hv, a.R), dim3(512), 0, stream, a);
   if (e != cudaSuccess) return (int)e;

@@ -1,0 +1,462 @@
+// Operands and host helpers of the few-row products (gemm_rows.cu, moe_rows.cu): quantised weight blocks as fp16 MMA
+// operands, the activation image, waits, tensor maps of weight rows.  See gemm_rows.cu for the method.
+#pragma once
+#include "common.cuh"
+#include "sm100.cuh"
+
+namespace herows {
+
+using namespace he;
+
+// Image of one block of one activation row: 16 units [v][c] of 64 bytes (lane t's 16 bytes of two MMAs), the eight sums per
+// 32 columns in two parts, the scale, and padding that puts neighbouring rows half a bank cycle apart.
+constexpr int IMG_COL = 576, SX_OFF = 512, XS_OFF = 544;
+constexpr int MAX_STAGES = 8;
+constexpr int SMEM_TOTAL = 220 * 1024;
+
+__host__ __device__ inline int rows_block_bytes(int qt) { return qt == HE_Q4_K ? 144 : qt == HE_Q6_K ? 224 : 272; }
+__host__ __device__ inline int col_groups(int R) {             // n8 tiles of R rows
+  const int n = (R + 7) / 8;
+  return n == 7 ? 8 : n;
+}
+
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+  return r;
+}
+__device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t d;
+  asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+__device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+__device__ __forceinline__ uint32_t h2_add(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+__device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                    uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// ... and one that starts a sum (`first`) instead of adding to it
+__device__ __forceinline__ void mma_from(bool first, float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                         uint32_t b0, uint32_t b1) {
+  if (!first) {
+    mma(d, a0, a1, a2, a3, b0, b1);
+    return;
+  }
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+
+// fp16 pairs (bit patterns)
+constexpr uint32_t MAGIC = 0x64006400u;       //  1024
+constexpr uint32_t M1024 = 0xE400E400u;       // -1024
+constexpr uint32_t M1056 = 0xE420E420u;       // -1056 = -(1024 + 32)
+constexpr uint32_t M1536 = 0xE600E600u;       // -1536 = -(1024 + 16 * 32)
+constexpr uint32_t M1152 = 0xE480E480u;       // -1152 = -(1024 + 128)
+constexpr uint32_t M64 = 0xD400D400u;         //   -64
+constexpr uint32_t P1_16 = 0x2C002C00u;       //  1/16
+
+// (x & mask) | c as ONE instruction: LOP3 takes a single immediate, so `c` has to be a register the compiler cannot see
+// through (with both constants visible it emits two; the integer pipe is the busiest one here)
+template <uint32_t MASK>
+__device__ __forceinline__ uint32_t and_or(uint32_t x, uint32_t c) {
+  uint32_t r;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(x), "n"(MASK), "r"(c));
+  return r;
+}
+__device__ __forceinline__ uint32_t opaque(uint32_t c) {
+  uint32_t r;
+  asm volatile("mov.b32 %0, %1;" : "=r"(r) : "r"(c));
+  return r;
+}
+
+// byte i of w as the fp16 pair (1024 + byte, 1024 + byte)
+__device__ __forceinline__ uint32_t dup_byte(uint32_t w, uint32_t i) { return prmt(w, 0x64646464u, 0x4040u | i | (i << 8)); }
+
+// One block (256 columns) of the 16 weight rows of a warp: `r0`, `r1` are the shared addresses of rows g and g + 8 in
+// the stage, `img` that of the block's image.  acc[nt] += the block's product in the MMA's C layout (rows g / g + 8,
+// activation rows 8 nt + 2t, + 1); only the first L groups of eight rows are computed.
+template <int NT, int L>
+__device__ __forceinline__ void block_q4k(uint32_t r0, uint32_t r1, uint32_t img, int lane, uint32_t mg,
+                                          float (&acc)[NT][4]) {
+  const int g = lane >> 2, t = lane & 3, h = t >> 1, u = t & 1;
+  const uint4 ma = lds128(r0), mb = lds128(r1);
+  const uint32_t qo = 16 + 64 * h + 16 * u;
+  const uint4 qa[2] = {lds128(r0 + qo), lds128(r0 + qo + 32)}, qb[2] = {lds128(r1 + qo), lds128(r1 + qo + 32)};
+  // 6-bit scales and minima of sub-blocks 4h .. 4h + 3, one per byte: the upper half's are split into four and two bits
+  const uint32_t low_bits = h ? 0x0F0F0F0Fu : 0x3F3F3F3Fu, high_bits = h ? 0x30303030u : 0u;
+  const uint32_t sca = ((h ? ma.w : ma.y) & low_bits) | ((ma.y >> 2) & high_bits);
+  const uint32_t scb = ((h ? mb.w : mb.y) & low_bits) | ((mb.y >> 2) & high_bits);
+  const uint32_t mna = ((h ? ma.w >> 4 : ma.z) & low_bits) | ((ma.z >> 2) & high_bits);
+  const uint32_t mnb = ((h ? mb.w >> 4 : mb.z) & low_bits) | ((mb.z >> 2) & high_bits);
+  float D[L][4], E[L <= 2 ? L : 1][4];      // few columns: two accumulators, half the dependent MMAs in a row
+  const uint32_t xb = img + g * IMG_COL + t * 16;
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {      // chunk 2h + c: low nibbles are group 2c of the half, high nibbles group 2c + 1
+    const uint32_t sla = h2_add(dup_byte(sca, 2 * c), M1024), slb = h2_add(dup_byte(scb, 2 * c), M1024);
+    const uint32_t sha_ = h2_add(dup_byte(sca, 2 * c + 1), M1024), shb_ = h2_add(dup_byte(scb, 2 * c + 1), M1024);
+    const uint32_t cla = h2_mul(sla, M1024), clb = h2_mul(slb, M1024);
+    const uint32_t cha = h2_mul(sha_, M64), chb = h2_mul(shb_, M64);         // high nibbles stay in place: 16 q
+    const uint32_t sha = h2_mul(sha_, P1_16), shb = h2_mul(shb_, P1_16);
+    const uint32_t wa[4] = {qa[c].x, qa[c].y, qa[c].z, qa[c].w}, wb[4] = {qb[c].x, qb[c].y, qb[c].z, qb[c].w};
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const uint32_t a = wa[v], b = wb[v], a8 = a >> 8, b8 = b >> 8;
+      const uint32_t l0 = h2_fma(and_or<0x000F000Fu>(a, mg), sla, cla), l1 = h2_fma(and_or<0x000F000Fu>(b, mg), slb, clb);
+      const uint32_t l2 = h2_fma(and_or<0x000F000Fu>(a8, mg), sla, cla), l3 = h2_fma(and_or<0x000F000Fu>(b8, mg), slb, clb);
+      const uint32_t u0 = h2_fma(and_or<0x00F000F0u>(a, mg), sha, cha), u1 = h2_fma(and_or<0x00F000F0u>(b, mg), shb, chb);
+      const uint32_t u2 = h2_fma(and_or<0x00F000F0u>(a8, mg), sha, cha), u3 = h2_fma(and_or<0x00F000F0u>(b8, mg), shb, chb);
+#pragma unroll
+      for (int n = 0; n < L; ++n) {
+        const uint4 x = lds128(xb + n * 8 * IMG_COL + (v * 2 + c) * 64);
+        mma_from(v + c == 0, D[n], l0, l1, l2, l3, x.x, x.y);
+        mma_from(L <= 2 && v + c == 0, L <= 2 ? E[L <= 2 ? n : 0] : D[n], u0, u1, u2, u3, x.z, x.w);
+      }
+    }
+  }
+  if (L <= 2) {
+#pragma unroll
+    for (int n = 0; n < L; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) D[n][i] += E[L <= 2 ? n : 0][i];
+  }
+  // minima: slots (2t, 2t + 1) meet the high parts of the sums of sub-blocks 2t, 2t + 1, slots + 8 the low parts
+  const uint32_t msel = 0x4040u | (2 * u) | ((2 * u + 1) << 8);
+  const uint32_t na = h2_add(prmt(mna, 0x64646464u, msel), M1024), nb = h2_add(prmt(mnb, 0x64646464u, msel), M1024);
+  const float2 da = __half22float2(*reinterpret_cast<const __half2*>(&ma.x));
+  const float2 db = __half22float2(*reinterpret_cast<const __half2*>(&mb.x));
+  const uint32_t sx = img + g * IMG_COL + SX_OFF + t * 8, xs = img + 2 * t * IMG_COL + XS_OFF;
+#pragma unroll
+  for (int n = 0; n < L; ++n) {
+    float M[4];
+    const uint2 s = lds64(sx + n * 8 * IMG_COL);
+    mma_from(true, M, na, nb, na, nb, s.x, s.y);
+    const float p0 = __uint_as_float(lds32(xs + n * 8 * IMG_COL)), p1 = __uint_as_float(lds32(xs + (n * 8 + 1) * IMG_COL));
+    acc[n][0] += p0 * (da.x * D[n][0] - da.y * M[0]);
+    acc[n][1] += p1 * (da.x * D[n][1] - da.y * M[1]);
+    acc[n][2] += p0 * (db.x * D[n][2] - db.y * M[2]);
+    acc[n][3] += p1 * (db.x * D[n][3] - db.y * M[3]);
+  }
+}
+
+template <int NT, int L>
+__device__ __forceinline__ void block_scale(uint32_t img, int t, float da, float db, const float (&D)[L][4],
+                                            float (&acc)[NT][4]) {
+  const uint32_t xs = img + 2 * t * IMG_COL + XS_OFF;
+#pragma unroll
+  for (int n = 0; n < L; ++n) {
+    const float p0 = __uint_as_float(lds32(xs + n * 8 * IMG_COL)), p1 = __uint_as_float(lds32(xs + (n * 8 + 1) * IMG_COL));
+    acc[n][0] += p0 * da * D[n][0];
+    acc[n][1] += p1 * da * D[n][1];
+    acc[n][2] += p0 * db * D[n][2];
+    acc[n][3] += p1 * db * D[n][3];
+  }
+}
+
+template <int NT, int L>
+__device__ __forceinline__ void block_q6k(uint32_t r0, uint32_t r1, uint32_t img, int lane, uint32_t mg,
+                                          float (&acc)[NT][4]) {
+  const int g = lane >> 2, t = lane & 3, h = t >> 1, u = t & 1;
+  const uint32_t lo = 64 * h + 16 * u, ho = 128 + 32 * h + 16 * u;
+  const uint4 la = lds128(r0 + lo), lb = lds128(r0 + lo + 32), lh = lds128(r0 + ho);
+  const uint4 ka = lds128(r1 + lo), kb = lds128(r1 + lo + 32), kh = lds128(r1 + ho);
+  const uint2 sa = lds64(r0 + 192 + 8 * h), sb = lds64(r1 + 192 + 8 * h);
+  // signed scales of the four groups (byte 2 qt + u), one per byte, as byte + 128
+  const uint32_t ssel = u ? 0x7531u : 0x6420u;
+  const uint32_t sca = prmt(sa.x, sa.y, ssel) ^ 0x80808080u, scb = prmt(sb.x, sb.y, ssel) ^ 0x80808080u;
+  float D[L][4], E[L <= 2 ? L : 1][4];      // few columns: two accumulators, half the dependent MMAs in a row
+  const uint32_t xb = img + g * IMG_COL + t * 16;
+  uint32_t fa[4], fb[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    fa[q] = h2_add(dup_byte(sca, q), M1152);
+    fb[q] = h2_add(dup_byte(scb, q), M1152);
+    if (q >= 2) {                     // groups 2, 3 come from high nibbles left in place: 16 (q - 32)
+      fa[q] = h2_mul(fa[q], P1_16);
+      fb[q] = h2_mul(fb[q], P1_16);
+    }
+  }
+  const uint32_t lav[4] = {la.x, la.y, la.z, la.w}, lbv[4] = {lb.x, lb.y, lb.z, lb.w}, lhv[4] = {lh.x, lh.y, lh.z, lh.w};
+  const uint32_t kav[4] = {ka.x, ka.y, ka.z, ka.w}, kbv[4] = {kb.x, kb.y, kb.z, kb.w}, khv[4] = {kh.x, kh.y, kh.z, kh.w};
+  auto low = [mg](uint32_t l, uint32_t hs, uint32_t f) {
+    return h2_mul(h2_add(and_or<0x00300030u>(hs, and_or<0x000F000Fu>(l, mg)), M1056), f);
+  };
+  auto high = [mg](uint32_t l, uint32_t hs, uint32_t f) {
+    return h2_mul(h2_add(and_or<0x03000300u>(hs, and_or<0x00F000F0u>(l, mg)), M1536), f);
+  };
+#pragma unroll
+  for (int v = 0; v < 4; ++v) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      uint32_t e[4], o[4];            // the MMA's a0..a3 of groups 2c and 2c + 1
+      const uint32_t hA = lhv[v], hB = khv[v], hA8 = hA >> 8, hB8 = hB >> 8;
+      if (c == 0) {
+        e[0] = low(lav[v], hA << 4, fa[0]);
+        e[1] = low(kav[v], hB << 4, fb[0]);
+        e[2] = low(lav[v] >> 8, hA8 << 4, fa[0]);
+        e[3] = low(kav[v] >> 8, hB8 << 4, fb[0]);
+        o[0] = low(lbv[v], hA << 2, fa[1]);
+        o[1] = low(kbv[v], hB << 2, fb[1]);
+        o[2] = low(lbv[v] >> 8, hA8 << 2, fa[1]);
+        o[3] = low(kbv[v] >> 8, hB8 << 2, fb[1]);
+      } else {
+        e[0] = high(lav[v], hA << 4, fa[2]);
+        e[1] = high(kav[v], hB << 4, fb[2]);
+        e[2] = high(lav[v] >> 8, hA8 << 4, fa[2]);
+        e[3] = high(kav[v] >> 8, hB8 << 4, fb[2]);
+        o[0] = high(lbv[v], hA << 2, fa[3]);
+        o[1] = high(kbv[v], hB << 2, fb[3]);
+        o[2] = high(lbv[v] >> 8, hA8 << 2, fa[3]);
+        o[3] = high(kbv[v] >> 8, hB8 << 2, fb[3]);
+      }
+#pragma unroll
+      for (int n = 0; n < L; ++n) {
+        const uint4 x = lds128(xb + n * 8 * IMG_COL + (v * 2 + c) * 64);
+        mma_from(v + c == 0, D[n], e[0], e[1], e[2], e[3], x.x, x.y);
+        mma_from(L <= 2 && v + c == 0, L <= 2 ? E[L <= 2 ? n : 0] : D[n], o[0], o[1], o[2], o[3], x.z, x.w);
+      }
+    }
+  }
+  if (L <= 2) {
+#pragma unroll
+    for (int n = 0; n < L; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) D[n][i] += E[L <= 2 ? n : 0][i];
+  }
+  const uint32_t dwa = lds32(r0 + 208), dwb = lds32(r1 + 208);
+  block_scale<NT, L>(img, t, __low2float(*reinterpret_cast<const __half2*>(&dwa)),
+                  __low2float(*reinterpret_cast<const __half2*>(&dwb)), D, acc);
+}
+
+// Power of two of the largest of a Q8_0 row's eight scales, and the four scales of half h over it as fp16 pairs.
+__device__ __forceinline__ float q8_scales(const uint4& s, int h, uint32_t (&f)[4]) {
+  const uint32_t w[4] = {s.x, s.y, s.z, s.w};
+  __half2 m = __habs2(*reinterpret_cast<const __half2*>(&w[0]));
+#pragma unroll
+  for (int i = 1; i < 4; ++i) m = __hmax2(m, __habs2(*reinterpret_cast<const __half2*>(&w[i])));
+  const uint32_t e = __float_as_uint(fmaxf(__low2float(m), __high2float(m))) & 0x7F800000u;
+  const float inv = __uint_as_float(0x7F000000u - e);
+  const uint32_t w0 = h ? s.z : s.x, w1 = h ? s.w : s.y;
+  const float2 d0 = __half22float2(*reinterpret_cast<const __half2*>(&w0));
+  const float2 d1 = __half22float2(*reinterpret_cast<const __half2*>(&w1));
+  const float d[4] = {d0.x, d0.y, d1.x, d1.y};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __half2 p = __float2half2_rn(d[i] * inv);
+    f[i] = *reinterpret_cast<const uint32_t*>(&p);
+  }
+  return __uint_as_float(e);
+}
+
+// Q8_0: `p0` / `p1` are the region's planes [2][HT rows][128 bytes] (128-byte swizzle) and [HT rows][8 scales]; rows i0, i1.
+template <int NT, int L, int HT>
+__device__ __forceinline__ void block_q80(uint32_t p0, int i0, uint32_t p1, int i1, uint32_t img, int lane,
+                                          uint32_t mg, float (&acc)[NT][4]) {
+  const int g = lane >> 2, t = lane & 3, h = t >> 1, u = t & 1;
+  uint32_t fa[4], fb[4];
+  const float ea = q8_scales(lds128(p0 + 2 * HT * 128 + i0 * 16), h, fa);
+  const float eb = q8_scales(lds128(p1 + 2 * HT * 128 + i1 * 16), h, fb);
+  const uint32_t ra = p0 + h * HT * 128 + i0 * 128, rb = p1 + h * HT * 128 + i1 * 128;
+  float D[L][4], E[L <= 2 ? L : 1][4];      // few columns: two accumulators, half the dependent MMAs in a row
+  const uint32_t xb = img + g * IMG_COL + t * 16;
+  auto up = [mg](uint32_t w, uint32_t f) { return h2_mul(h2_add(and_or<0x00FF00FFu>(w, mg), M1152), f); };
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    uint4 a[2], b[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int chunk = 2 * (2 * c + q) + u;
+      a[q] = lds128(ra + ((chunk ^ (i0 & 7)) << 4));
+      b[q] = lds128(rb + ((chunk ^ (i1 & 7)) << 4));
+    }
+    const uint32_t av[2][4] = {{a[0].x, a[0].y, a[0].z, a[0].w}, {a[1].x, a[1].y, a[1].z, a[1].w}};
+    const uint32_t bv[2][4] = {{b[0].x, b[0].y, b[0].z, b[0].w}, {b[1].x, b[1].y, b[1].z, b[1].w}};
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      uint32_t e[2][4];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const uint32_t wa = av[q][v] ^ 0x80808080u, wb = bv[q][v] ^ 0x80808080u;
+        e[q][0] = up(wa, fa[2 * c + q]);
+        e[q][1] = up(wb, fb[2 * c + q]);
+        e[q][2] = up(wa >> 8, fa[2 * c + q]);
+        e[q][3] = up(wb >> 8, fb[2 * c + q]);
+      }
+#pragma unroll
+      for (int n = 0; n < L; ++n) {
+        const uint4 x = lds128(xb + n * 8 * IMG_COL + (v * 2 + c) * 64);
+        mma_from(v + c == 0, D[n], e[0][0], e[0][1], e[0][2], e[0][3], x.x, x.y);
+        mma_from(L <= 2 && v + c == 0, L <= 2 ? E[L <= 2 ? n : 0] : D[n], e[1][0], e[1][1], e[1][2], e[1][3], x.z, x.w);
+      }
+    }
+  }
+  if (L <= 2) {
+#pragma unroll
+    for (int n = 0; n < L; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) D[n][i] += E[L <= 2 ? n : 0][i];
+  }
+  block_scale<NT, L>(img, t, ea, eb, D, acc);
+}
+
+// Bounded wait whose polls the hardware suspends for up to ~10 us each: the polling loop of a waiting warp would take
+// issue slots from the warps that compute.
+__device__ __forceinline__ bool wait_long(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  for (uint32_t i = 0; i < (1u << 20); ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(sm100::smem_u32(bar)), "r"(parity), "r"(10000u)
+        : "memory");
+    if (ok) return true;
+    if (*abort_flag) return false;
+  }
+  *abort_flag = 1;
+  if (status != nullptr) atomicCAS(status, 0, code);
+  return false;
+}
+
+__device__ __forceinline__ void named_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void named_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(sm100::smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ float4 ldcg4(const float* p) {
+  float4 v;
+  asm volatile("ld.global.cg.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+
+// Eight consecutive columns (8 * lane) of a block of an activation row, as the fp16 fragments the kernel above loads: x over the power of two of the block's largest value; the sums of the rounded values per 32 columns in two parts.
+// (`also`: a second place to write to, or null)
+__device__ __forceinline__ void image_store(uint8_t* unit, uint8_t* also, int lane, const float (&v)[8]) {
+  float amax = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+  bool odd = false;                     // a NaN or an infinity stays one, under scale 1
+#pragma unroll
+  for (int i = 0; i < 8; ++i) odd |= !(fabsf(v[i]) <= 3.0e38f);
+  amax = warp_max(amax);
+  uint32_t e = min(__float_as_uint(amax) & 0x7F800000u, 0x7E800000u);
+  if (__any_sync(0xffffffffu, odd)) e = 0x3F800000u;
+  const float inv = __uint_as_float(0x7F000000u - e);
+  __half hv[8];
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    hv[i] = __float2half_rn(v[i] * inv);
+    s += __half2float(hv[i]);
+  }
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  const int h = lane >> 4, qt = (lane >> 2) & 3, u = (lane >> 1) & 1, v0 = (lane & 1) * 2, t = 2 * h + u;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    __half2 p[2] = {__halves2half2(hv[4 * q], hv[4 * q + 2]), __halves2half2(hv[4 * q + 1], hv[4 * q + 3])};
+    const int at = ((v0 + q) * 2 + (qt >> 1)) * 64 + t * 16 + (qt & 1) * 8;
+    *reinterpret_cast<uint2*>(unit + at) = *reinterpret_cast<const uint2*>(p);
+    if (also != nullptr) *reinterpret_cast<uint2*>(also + at) = *reinterpret_cast<const uint2*>(p);
+  }
+  if ((lane & 3) == 0) {
+    const int sub = lane >> 2;
+    const __half hi = __float2half_rn(s), lo = __float2half_rn(s - __half2float(hi));
+    const int at = SX_OFF + (sub >> 1) * 8 + (sub & 1) * 2;
+    *reinterpret_cast<__half*>(unit + at) = hi;
+    *reinterpret_cast<__half*>(unit + at + 4) = lo;
+    if (also != nullptr) {
+      *reinterpret_cast<__half*>(also + at) = hi;
+      *reinterpret_cast<__half*>(also + at + 4) = lo;
+    }
+  }
+  if (lane == 0) {
+    *reinterpret_cast<float*>(unit + XS_OFF) = __uint_as_float(e);
+    if (also != nullptr) *reinterpret_cast<float*>(also + XS_OFF) = __uint_as_float(e);
+  }
+}
+
+__device__ __forceinline__ void load_cols(const void* x, int dtype, size_t off, float (&v)[8]) {
+  if (dtype == 0) {
+    const float4* p = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(x) + off);
+    const float4 a = p[0], b = p[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  } else {
+    const uint4 u = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(x) + off);
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = __bfloat1622float2(h[i]);
+      v[2 * i] = f.x; v[2 * i + 1] = f.y;
+    }
+  }
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+inline EncodeTiledFn encode_fn() {
+  static const EncodeTiledFn fn = []() -> EncodeTiledFn {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      return reinterpret_cast<EncodeTiledFn>(p);
+    return nullptr;
+  }();
+  return fn;
+}
+
+// Weight rows as bytes: [rows][row_bytes], box {box_bytes, box_rows}
+inline int byte_map(CUtensorMap* m, const void* ptr, long long rows, long long row_bytes, int box_bytes, bool swizzle, int box_rows) {
+  const EncodeTiledFn enc = encode_fn();
+  if (enc == nullptr || (reinterpret_cast<uintptr_t>(ptr) & 15) != 0 || row_bytes % 16 != 0) return -HE_ERR_BAD_ARG;
+  const cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)row_bytes};
+  const cuuint32_t box[2] = {(cuuint32_t)box_bytes, (cuuint32_t)box_rows}, estr[2] = {1, 1};
+  const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), dims, strides, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : 1000 + (int)r;
+}
+
+inline int weight_maps(CUtensorMap* m, const void* w, int qtype, long long rows, int K, int box) {
+  if (w == nullptr) return -HE_ERR_BAD_ARG;
+  if (qtype == HE_Q4_K) return byte_map(m, w, rows, (long long)(K >> 8) * 144, 144, false, box);
+  if (qtype == HE_Q6_K) return byte_map(m, w, rows, (long long)(K >> 8) * 224, 224, false, box);
+  if (qtype != HE_Q8_0) return -HE_ERR_BAD_ARG;
+  const long long rb = (long long)K + (((K >> 4) + 15) / 16) * 16;
+  const int rc = byte_map(m, w, rows, rb, 128, true, box);
+  return rc != 0 ? rc : byte_map(m + 1, w, rows, rb, 16, false, box);
+}
+
+}  // namespace herows

@@ -15,6 +15,7 @@ launch; above that the projections run on the tcgen05 GEMM.
 """
 from __future__ import annotations
 
+import contextlib
 import os
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence, Tuple
@@ -23,12 +24,15 @@ import torch
 
 from ..loading.weights import ModelWeights, QTensor, ffn_norm_slot
 from ..ops import kernels as K
+from ..ops import rows as ROWS
 from ..ops.kernels import DeviceWeight, GemvSegment
 from ..quant.ggml import GGMLType
 from .config import ModelConfig
 
 PAGE = 16
 GEMV_MAX_ROWS = 8
+GEMV_ROWS = 5                 # packed batches of up to this many rows take the int8 GEMV where there are no few-row products
+FEW_MIN_WIDTH = 2048          # hidden width from which those take over above two rows
 
 
 @dataclass
@@ -137,6 +141,7 @@ class _Scratch:
 
 class HybridExecutor:
     keeps_hidden = True           # decode steps also store the post-norm hidden rows
+    few_rows = True               # a subclass with projections of its own (sharded, float, padded) turns the few-row products off
     packs_mixed = False           # can decode rows ride in a prompt's forward without costing more than a step of their own
 
     def __init__(self, weights: ModelWeights, device="cuda", max_slots: int = 4, max_context: int = 4608,
@@ -151,13 +156,6 @@ class HybridExecutor:
         self.n_pages = n_pages if n_pages is not None else max_slots * self.max_pages_per_slot + 1
         self.gemm_impl = gemm_impl or os.environ.get("HE_GEMM", "tcgen05")
         self.scratch = _Scratch(self.device)
-        # packed batches of up to small_rows rows take the quantised GEMV path, larger ones the tensor-core path
-        # (the int8 GEMV costs ~1.65 ms per extra row on the 27B geometry; the split-K tensor-core path streams the
-        # same quantised blocks once for any row count up to 128)
-        # measured on the 27B: a packed step costs 7.0 / 8.7 / 10.3 / 11.7 / 14.0 / 18.5 ms at 2 / 3 / 4 / 5 / 6 / 8
-        # rows on the GEMV path and 13.3 / 13.6 / 14.2 ms at 5 / 6 / 8 rows on the tensor-core path, so the switch is
-        # above five rows
-        self.small_rows = min(GEMV_MAX_ROWS, int(os.environ.get("HE_SMALL_ROWS", "5")))
         self.dw: Dict[str, DeviceWeight] = {}
         self.f32: Dict[str, torch.Tensor] = {}
         # per-stage device timing of the tensor-core (many rows) path, off unless HE_STAGE_TIMING=1 (the role of the
@@ -167,6 +165,60 @@ class HybridExecutor:
         self.timer = StageTimer(enabled=os.environ.get("HE_STAGE_TIMING", "0") == "1")
         self._load(weights)
         self._alloc_state()
+        # Packed batches of up to small_rows rows take the quantised GEMV, then up to 64 the few-row products
+        # (csrc/gemm_rows.cu), larger ones the tcgen05 GEMM.  With few-row products the GEMV keeps two rows: it takes about
+        # as long again for each further row (the four products of a 27B layer: 65 / 85 / 119 us at one / two / four rows),
+        # they take as long as for one (94 / 95 / 96 us).  On narrow models launches are all there is and the GEMV has one
+        # less for each norm, and without few-row products the choice is the tensor-core GEMM: five rows (a packed step
+        # of the 27B with 5 / 6 rows costs 11.7 / 14.0 ms on the GEMV, 13.3 / 13.6 ms on the tensor cores).
+        self.rows = self._make_rows()
+        self.small_rows = min(GEMV_MAX_ROWS, int(os.environ.get(
+            "HE_SMALL_ROWS", GEMV_ROWS if self.rows is None or self.cfg.hidden < FEW_MIN_WIDTH else 2)))
+
+    def _make_rows(self) -> Optional[ROWS.RowsSpace]:
+        """The few-row products, when every projection of the model is of a kind that they take."""
+        cfg = self.cfg
+        if not self.few_rows or self.gemm_impl != "tcgen05" or self.device.type != "cuda":
+            return None
+        used = [self.dw["output.weight"]]
+        for i in range(cfg.n_layers + cfg.nextn_layers):
+            full = i >= cfg.n_layers or cfg.is_full_attention_layer(i)
+            names = ["attn_q", "attn_k", "attn_v", "attn_output"] if full else ["attn_qkv", "attn_gate", "ssm_out"]
+            if i >= cfg.n_layers:
+                names.append("nextn.eh_proj")
+            pair = ("ffn_gate_shexp", "ffn_up_shexp") if cfg.is_moe else ("ffn_gate", "ffn_up")
+            if not cfg.is_moe or cfg.shared_ffn:
+                names += [*pair, "ffn_down_shexp" if cfg.is_moe else "ffn_down"]
+            ws = {n: self.dw.get(f"blk.{i}.{n}.weight") for n in names}
+            if any(w is None for w in ws.values()):
+                return None
+            if pair[0] in ws and ws[pair[0]].qtype != ws[pair[1]].qtype:
+                return None
+            used += ws.values()
+            if not full and f"blk.{i}.ssm_alpha.weight" not in self.f32:
+                return None
+        if not all(ROWS.weight_ok(w) for w in used):
+            return None
+        # the gates of the delta rule stay fp32: they ride with the rows' image (one matrix, alpha rows then beta rows)
+        self.ab_f32 = {i: torch.cat([self.F(i, "ssm_alpha.weight"), self.F(i, "ssm_beta.weight")], 0).contiguous()
+                       for i in range(cfg.n_layers) if not cfg.is_full_attention_layer(i)}
+        return ROWS.RowsSpace(self.scratch, self.device, max(w.n_rows for w in used))
+
+    def few(self, rows: int) -> bool:
+        """Do the projections of a batch of this many rows run as few-row products?"""
+        return self.rows is not None and self.small_rows < rows <= ROWS.MAX_ROWS
+
+    @contextlib.contextmanager
+    def gemv_numerics(self, rows: int):
+        """A verify chain of up to 8 rows must see the numerics of a plain single-row step (the int8 GEMV), or a near-tie
+        could make the verifier disagree with what autoregressive decoding would have produced."""
+        saved = self.small_rows
+        if rows <= GEMV_MAX_ROWS:
+            self.small_rows = GEMV_MAX_ROWS
+        try:
+            yield
+        finally:
+            self.small_rows = saved
 
     # ------------------------------------------------------------------ weights
     def _load(self, weights: ModelWeights) -> None:
@@ -299,7 +351,13 @@ class HybridExecutor:
     # calls _sync_resid first: a tensor-parallel executor defers the cross-rank sum of a row-parallel projection to
     # the next reader (folded into that GEMV's prologue, or a small stand-alone kernel).
     def _gemv_resid(self, h: torch.Tensor, segs, norm_w: torch.Tensor, eps: float) -> None:
-        K.gemv(h, segs, norm_w=norm_w, eps=eps)
+        self._few_gemm(h, segs, norm_w, eps)
+
+    def _few_gemm(self, x: torch.Tensor, segs, norm_w: Optional[torch.Tensor] = None, eps: float = 1e-6) -> None:
+        if self.few(x.shape[0]):
+            self.rows.gemm(x, segs, norm_w, eps)
+        else:
+            K.gemv(x, segs, norm_w=norm_w, eps=eps)
 
     def _sync_resid(self, h: torch.Tensor) -> None:
         return
@@ -323,7 +381,7 @@ class HybridExecutor:
     # Row-parallel ("output") projections: h += x @ W^T.  A tensor-parallel executor overrides these two to
     # reduce the partial products across ranks before the residual add.
     def _out_small(self, x: torch.Tensor, w: DeviceWeight, h: torch.Tensor) -> None:
-        K.gemv(x, [GemvSegment(w, h, K.EPI_ADD_F32)])
+        self._few_gemm(x, [GemvSegment(w, h, K.EPI_ADD_F32)])
 
     def _out_big(self, x: torch.Tensor, w: DeviceWeight, h: torch.Tensor, tag: str) -> None:
         T = x.shape[0]
@@ -405,10 +463,29 @@ class HybridExecutor:
         inner = cfg.ssm_inner
         a_p = sc.get("a_proj", (T, Hv), torch.float32)
         b_p = sc.get("b_proj", (T, Hv), torch.float32)
+        plain = (small and journal is None and b.n_seg == T and S == 128 and cfg.conv_kernel == 4
+                 and os.environ.get("HE_GDN_FUSED", "1") != "0")      # plain decode rows: two fused launches instead of five
+        gates = None
         if small:
             qkv = sc.get("qkv_f32", (T, C), torch.float32)
             z = sc.get("z_f32", (T, inner), torch.float32)
-            if i in self.ab_q8:
+            if self.few(T):
+                ab = sc.get("ab_proj", (T, 2 * Hv), torch.float32)
+                image, _ = self.rows.image(h, self.F(i, "attn_norm.weight"), cfg.rms_eps, self.ab_f32[i], ab)
+                self.rows.product(image, T, cfg.hidden, [GemvSegment(self.W(i, "attn_qkv.weight"), qkv),
+                                                         GemvSegment(self.W(i, "attn_gate.weight"), z)])
+                a_p, b_p = ab[:, :Hv], ab[:, Hv:]
+            elif self.rows is not None:
+                self._gemv_resid(h, [GemvSegment(self.W(i, "attn_qkv.weight"), qkv),
+                                     GemvSegment(self.W(i, "attn_gate.weight"), z)], self.F(i, "attn_norm.weight"),
+                                 cfg.rms_eps)
+                if plain and T == 1:
+                    gates = (self.ab_f32[i], h, self.F(i, "attn_norm.weight"), cfg.rms_eps)
+                else:                               # a verify chain: the same fp32 gates
+                    ab = sc.get("ab_proj", (T, 2 * Hv), torch.float32)
+                    self.rows.image(h, self.F(i, "attn_norm.weight"), cfg.rms_eps, self.ab_f32[i], ab)
+                    a_p, b_p = ab[:, :Hv], ab[:, Hv:]
+            elif i in self.ab_q8:
                 ab = sc.get("ab_proj", (T, 2 * Hv), torch.float32)
                 ab_split = os.environ.get("HE_AB_SPLIT", "1" if cfg.hidden >= 4096 else "0")
                 if ab_split != "0":
@@ -450,13 +527,11 @@ class HybridExecutor:
         decay = sc.get("decay", (T, Hv), torch.float32)
         beta = sc.get("beta", (T, Hv), torch.float32)
         og = sc.get("gdn_og", (T, inner), torch.bfloat16)
-        if (small and journal is None and b.n_seg == T and S == 128 and cfg.conv_kernel == 4
-                and os.environ.get("HE_GDN_FUSED", "1") != "0"):
-            # plain decode rows: two fused launches instead of five
+        if plain:
             K.gdn_decode(qkv, self.F(i, "ssm_conv1d.weight"), self.conv_state[i], a_p, b_p,
                          self.F(i, "ssm_a").reshape(-1), self.F(i, "ssm_dt.bias").reshape(-1), b.seg_slot, conv,
                          decay, beta, self.gdn_state[i], z, self.F(i, "ssm_norm.weight").reshape(-1), og, G, Hv,
-                         cfg.rms_eps)
+                         cfg.rms_eps, gates)
             self._out_small(og, self.W(i, "ssm_out.weight"), h)
             return
         cj = journal["conv"][i] if journal is not None else None
@@ -531,7 +606,7 @@ class HybridExecutor:
         ``head_greedy`` to fold in; otherwise the returned rows are complete."""
         cfg = self.cfg
         T = b.T
-        small = T <= self.small_rows
+        small = T <= self.small_rows or self.few(T)
         h = h_out if h_out is not None else self._resid_buffer(T)
         K.embed(self.dw["token_embd.weight"], b.tokens, h, cfg.embed_scale)
         for i in range(cfg.n_layers):
@@ -552,7 +627,7 @@ class HybridExecutor:
         head = self.dw["output.weight"]
         if out is None:
             out = self.scratch.get("logits", (R, cfg.vocab), torch.float32)
-        if R <= GEMV_MAX_ROWS:
+        if R <= GEMV_MAX_ROWS or self.few(R):
             self._gemv_resid(h_rows, [GemvSegment(head, out)], self.f32["output_norm.weight"], cfg.rms_eps)
         else:
             self._sync_resid(h_rows)
@@ -589,7 +664,7 @@ class HybridExecutor:
         cfg, sc = self.cfg, self.scratch
         i = cfg.n_layers
         T, H = b.T, cfg.hidden
-        small = T <= self.small_rows
+        small = T <= self.small_rows or self.few(T)
         table = self.dw.get(f"blk.{i}.nextn.embed_tokens.weight", self.dw["token_embd.weight"])
         e = sc.get("nx_e", (T, H), torch.float32)
         K.embed(table, b.tokens, e, cfg.embed_scale)
@@ -599,7 +674,7 @@ class HybridExecutor:
         h = sc.get("nx_h", (T, H), torch.float32)
         w = self.W(i, "nextn.eh_proj.weight")
         if small:
-            K.gemv(xcat, [GemvSegment(w, h, K.EPI_F32)])
+            self._few_gemm(xcat, [GemvSegment(w, h, K.EPI_F32)])
         else:
             xb = sc.get("nx_cat_bf", (T, 2 * H), torch.bfloat16)
             xb.copy_(xcat)

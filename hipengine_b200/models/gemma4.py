@@ -40,6 +40,8 @@ def _pad_q8_0_cols(t: QTensor, k_pad: int) -> QTensor:
 
 
 class Gemma4Executor(HybridExecutor):
+    few_rows = False              # projections of its own
+
     def __init__(self, weights: ModelWeights, **kw):
         cfg = weights.config
         self.expert_k = cfg.expert_ffn

@@ -52,6 +52,7 @@ class ExpertWeights:
 
 
 class ListedExecutor(HybridExecutor):
+    few_rows = False               # float weights, routes of their own
     keeps_hidden = False
     packs_mixed = True             # prompt portions and decode rows of one step run as one forward
 

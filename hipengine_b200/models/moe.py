@@ -26,8 +26,6 @@ from ..ops.kernels import GemvSegment
 from ..quant.ggml import GGMLType
 
 SEL_MAX_ROWS = 64
-
-
 class _MoeLayer:
     """Per-layer derived weights: router as a GEMV weight and as bf16 hi/lo halves for the tensor-core path."""
 
@@ -47,6 +45,7 @@ class _MoeLayer:
         pad = (-full.shape[0]) % 8
         if pad:
             full = torch.cat([full, torch.zeros(pad, full.shape[1], device=full.device)], 0)
+        self.full = full[:E + (1 if self.has_shared else 0)].contiguous()     # fp32 rows: experts, then the shared gate
         # fp32 router weights as two bf16 GEMM operands: hi + lo reproduces ~16 mantissa bits
         self.r_hi = full.to(torch.bfloat16).contiguous()
         self.r_lo = (full - self.r_hi.float()).to(torch.bfloat16).contiguous()
@@ -95,7 +94,14 @@ def _moe_selected(ex, i: int, h: torch.Tensor, target: torch.Tensor, T: int, nor
     act_sh = sc.get("moe_act_sh", (T, max(cfg.shared_ffn, 1)), torch.bfloat16) if L.has_shared else None
     epi = K.EPI_SILU_MUL if cfg.act == "silu" else K.EPI_GELU_MUL
     # everything that reads the residual stream runs before anything that adds to it
-    for r0 in range(0, T, 8):
+    few = ex.few(T)
+    if few:
+        # router and shared gate in fp32 beside the rows' images, the shared expert's gate/up from the image
+        image, _ = ex.rows.image(h, norm_w, cfg.rms_eps, L.full, logits)
+        if shared_here:
+            ex.rows.product(image, T, cfg.hidden, [GemvSegment(ex.W(i, "ffn_gate_shexp.weight"), act_sh, epi,
+                                                               ex.W(i, "ffn_up_shexp.weight"))])
+    for r0 in range(0, 0 if few else T, 8):
         r1 = min(T, r0 + 8)
         segs = [GemvSegment(L.router, logits[r0:r1, :E])]
         if L.has_shared:
@@ -110,6 +116,9 @@ def _moe_selected(ex, i: int, h: torch.Tensor, target: torch.Tensor, T: int, nor
     K.moe_down_sel(act_rows, ids, wts, ex.W(i, "ffn_down_exps.weight"), cfg.hidden, target, expert_range=er)
     if shared_here:
         K.moe_scale_rows(act_sh, logits[:, E:E + 1])
+        if few:
+            ex.rows.gemm(act_sh, [GemvSegment(ex.W(i, "ffn_down_shexp.weight"), target, K.EPI_ADD_F32)])
+            return
         for r0 in range(0, T, 8):
             r1 = min(T, r0 + 8)
             K.gemv(act_sh[r0:r1], [GemvSegment(ex.W(i, "ffn_down_shexp.weight"), target[r0:r1], K.EPI_ADD_F32)])
@@ -124,6 +133,18 @@ def _grouped(sc, a_sorted: torch.Tensor, w, out: torch.Tensor, n_groups: int, ti
     wb = sc.get("moe_deq", (w.n_rows, w.n_cols), torch.bfloat16)
     K.dequant_bf16(w, wb)
     GM.gemm_bf16_grouped(a_sorted, wb[:, :a_sorted.shape[1]], out, n_groups, tile_group)
+
+
+def _shared_rows(ex, i: int, xn: torch.Tensor, T: int) -> torch.Tensor:
+    """The shared expert's rows (before its gate), bf16."""
+    cfg, sc = ex.cfg, ex.scratch
+    Fs = cfg.shared_ffn
+    gus = sc.get("moe_gus", (T, 2 * Fs), torch.bfloat16)
+    ex._gemm(xn, ex.W(i, "ffn_gate_shexp.weight"), gus[:, :Fs], tag="g")
+    ex._gemm(xn, ex.W(i, "ffn_up_shexp.weight"), gus[:, Fs:], tag="g")
+    acts = sc.get("moe_acts", (T, Fs), torch.bfloat16)
+    K.act_mul(gus, acts, cfg.act)
+    return ex._gemm(acts, ex.W(i, "ffn_down_shexp.weight"), sc.get("y_bf", (T, cfg.hidden), torch.bfloat16), tag="d")
 
 
 def _moe_grouped(ex, i: int, h: torch.Tensor, target: torch.Tensor, T: int, norm_w: torch.Tensor, rng) -> None:
@@ -159,13 +180,5 @@ def _moe_grouped(ex, i: int, h: torch.Tensor, target: torch.Tensor, T: int, norm
     K.act_mul(gu, act, cfg.act)
     ys = sc.get("moe_ys", (bound, H), torch.bfloat16)
     _grouped(sc, act, wd, ys, El, tile_group)
-    ysh = None
-    if shared_here:
-        Fs = cfg.shared_ffn
-        gus = sc.get("moe_gus", (T, 2 * Fs), torch.bfloat16)
-        ex._gemm(xn, ex.W(i, "ffn_gate_shexp.weight"), gus[:, :Fs], tag="g")
-        ex._gemm(xn, ex.W(i, "ffn_up_shexp.weight"), gus[:, Fs:], tag="g")
-        acts = sc.get("moe_acts", (T, Fs), torch.bfloat16)
-        K.act_mul(gus, acts, cfg.act)
-        ysh = ex._gemm(acts, ex.W(i, "ffn_down_shexp.weight"), sc.get("y_bf", (T, H), torch.bfloat16), tag="d")
+    ysh = _shared_rows(ex, i, xn, T) if shared_here else None
     K.moe_combine(target, ys, pos, wts, k, ysh, logits[:, E:E + 1] if shared_here else None)

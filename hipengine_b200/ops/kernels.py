@@ -86,7 +86,8 @@ class _GdnDecodeArgs(C.Structure):
                 ("a_stride", c_ll), ("b_stride", c_ll), ("ssm_a", c_vp), ("dt_bias", c_vp), ("slot", c_vp),
                 ("qkv", c_vp), ("decay", c_vp), ("beta", c_vp), ("state", c_vp), ("z", c_vp), ("z_dtype", C.c_int),
                 ("z_stride", c_ll), ("norm_w", c_vp), ("out", c_vp), ("out_stride", c_ll), ("eps", C.c_float),
-                ("C", C.c_int), ("G", C.c_int), ("Hv", C.c_int), ("R", C.c_int)]
+                ("C", C.c_int), ("G", C.c_int), ("Hv", C.c_int), ("R", C.c_int), ("gate_w", c_vp), ("gate_x", c_vp),
+                ("gate_norm", c_vp), ("gate_eps", C.c_float), ("K", C.c_int)]
 
 
 class _GdnFrontArgs(C.Structure):
@@ -546,16 +547,24 @@ def gdn_gated_norm(o: torch.Tensor, z: torch.Tensor, w: torch.Tensor, out: torch
                                       C.c_int(Hv), C.c_int(Dv), C.c_float(eps), _stream()), "he_gdn_gated_norm")
 
 
-def gdn_decode(x: torch.Tensor, conv_w: torch.Tensor, conv_state: torch.Tensor, a: torch.Tensor, b: torch.Tensor,
+def gdn_decode(x: torch.Tensor, conv_w: torch.Tensor, conv_state: torch.Tensor, a: Optional[torch.Tensor],
+               b: Optional[torch.Tensor],
                ssm_a: torch.Tensor, dt_bias: torch.Tensor, slot: torch.Tensor, qkv: torch.Tensor,
                decay: torch.Tensor, beta: torch.Tensor, state: torch.Tensor, z: torch.Tensor, norm_w: torch.Tensor,
-               out: torch.Tensor, G: int, Hv: int, eps: float) -> None:
+               out: torch.Tensor, G: int, Hv: int, eps: float,
+               gates: Optional[Tuple[torch.Tensor, torch.Tensor, torch.Tensor, float]] = None) -> None:
     """Decode fast path of a gated delta-net layer (single-token segments): conv + gates, then one recurrent
-    step with the gated RMSNorm, in two launches."""
+    step with the gated RMSNorm, in two launches.  ``a``, ``b``: projections of the gates; or, for a single row, ``gates`` =
+    (fp32 weights [2 Hv, K], residual row [1, K], norm weight, norm eps) to compute them from."""
     _check_abi()
     p = _GdnDecodeArgs()
     p.x, p.x_stride, p.conv_w, p.conv_state = x.data_ptr(), x.stride(0), conv_w.data_ptr(), conv_state.data_ptr()
-    p.a, p.b, p.a_stride, p.b_stride = a.data_ptr(), b.data_ptr(), a.stride(0), b.stride(0)
+    if gates is not None:
+        gw, gx, gn, ge = gates
+        assert gw.is_contiguous() and gw.dtype == gx.dtype == torch.float32 and gw.shape == (2 * Hv, gx.shape[1])
+        p.gate_w, p.gate_x, p.gate_norm, p.gate_eps, p.K = gw.data_ptr(), gx.data_ptr(), gn.data_ptr(), ge, gx.shape[1]
+    else:
+        p.a, p.b, p.a_stride, p.b_stride = a.data_ptr(), b.data_ptr(), a.stride(0), b.stride(0)
     p.ssm_a, p.dt_bias, p.slot = ssm_a.data_ptr(), dt_bias.data_ptr(), slot.data_ptr()
     p.qkv, p.decay, p.beta, p.state = qkv.data_ptr(), decay.data_ptr(), beta.data_ptr(), state.data_ptr()
     p.z, p.z_dtype, p.z_stride, p.norm_w = z.data_ptr(), _dt(z), z.stride(0), norm_w.data_ptr()

@@ -33,6 +33,8 @@ from .sharding import TPPlan, shard_weights
 
 
 class TPHybridExecutor(HybridExecutor):
+    few_rows = False              # projections of its own
+
     def __init__(self, full_weights: ModelWeights, ctx: DistContext, comm: Optional[str] = None, **kw):
         self.ctx = ctx
         self.full_cfg = full_weights.config

@@ -13,11 +13,12 @@ Stages are recorded through ``SpecTransaction``.  Reference flow: ``hipengine/ru
 """
 from __future__ import annotations
 
+import os
 from typing import List, Optional, Sequence, Tuple
 
 import torch
 
-from ..models.executor import GEMV_MAX_ROWS, BatchDesc, make_batch
+from ..models.executor import GEMV_MAX_ROWS, GEMV_ROWS, BatchDesc, make_batch
 from ..ops import kernels as K
 from .contracts import SpecCycleResult, SpeculativeCapability
 from .transaction import SpecTransaction, Stage
@@ -30,6 +31,9 @@ class ChainVerifyCycle:
 
     def __init__(self, ex, max_depth: int = 3, max_requests: int = 8):
         self.ex = ex
+        # beside a verifier the plain steps of the smallest batches keep its numerics (the int8 GEMV): both then choose the
+        # same tokens
+        ex.small_rows = max(ex.small_rows, min(GEMV_ROWS, int(os.environ.get("HE_SMALL_ROWS", GEMV_ROWS))))
         self.max_depth = max_depth
         self.max_requests = max_requests
         dev = ex.device
@@ -71,20 +75,13 @@ class ChainVerifyCycle:
         vb.tokens = torch.cat([t0[:, None], drafts], 1).reshape(-1).contiguous()
         journal = {"conv": {i: t[:T] for i, t in self.journal["conv"].items()},
                    "gdn": {i: t[:T] for i, t in self.journal["gdn"].items()}}
-        # a verify chain must see the numerics of plain decode (the int8 GEMV path), or a near-tie could make the
-        # verifier disagree with what autoregressive decoding would have produced: keep chains of up to 8 rows there
-        saved_small = ex.small_rows
-        if T <= GEMV_MAX_ROWS:
-            ex.small_rows = GEMV_MAX_ROWS
-        try:
-            h = ex.forward(vb, journal=journal)
-        finally:
-            ex.small_rows = saved_small
         logits = ex.scratch.get("mtp_logits", (T, cfg.vocab), torch.float32)
         hid = ex.scratch.get("mtp_vhid", (T, cfg.hidden), torch.float32)
-        for r0 in range(0, T, GEMV_MAX_ROWS):
-            r1 = min(T, r0 + GEMV_MAX_ROWS)
-            ex.logits(h[r0:r1], out=logits[r0:r1], hidden_out=hid[r0:r1])
+        with ex.gemv_numerics(T):
+            h = ex.forward(vb, journal=journal)
+            for r0 in range(0, T, GEMV_MAX_ROWS):
+                r1 = min(T, r0 + GEMV_MAX_ROWS)
+                ex.logits(h[r0:r1], out=logits[r0:r1], hidden_out=hid[r0:r1])
         txn.advance(Stage.VERIFIED)
         # ---- accept
         out = torch.empty(R, Kd + 1, dtype=torch.int64, device=dev)
@@ -382,9 +379,7 @@ class GraphedMTPCycle(MTPCycle):
             txn.advance(st)
         head_rows = self.draft_head_rows if small_head else 0
         key = (R, Kd, ctx_bucket(max(positions) + Kd + 1), head_rows)
-        saved_small = ex.small_rows
-        ex.small_rows = GEMV_MAX_ROWS           # verify rows see the numerics of plain decode (see the parent)
-        try:
+        with ex.gemv_numerics(GEMV_MAX_ROWS):   # verify rows see the numerics of plain decode
             g = self.graphs.get(key)
             if g is None:
                 snap = self._snapshot(R)
@@ -399,8 +394,6 @@ class GraphedMTPCycle(MTPCycle):
                 self._restore(snap)
                 self.graphs[key] = g
                 self.graph_stats["captures"] += 1
-        finally:
-            ex.small_rows = saved_small
         exec_h = RT.graph_exec_handle(g)
         n_host = None
         if exec_h:

@@ -1,0 +1,116 @@
+"""Few-row products with quantised weights (csrc/gemm_rows.cu) against 64-bit products of the dequantised blocks."""
+import pytest
+import torch
+
+from hipengine_b200.quant import ggml as Q
+
+pytestmark = pytest.mark.gpu
+T = Q.GGMLType
+
+
+def _weight(t, n, k, seed):
+    from hipengine_b200.ops import kernels as K
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    raw = Q.quantize(torch.randn(n, k, generator=g, device="cuda") * 0.02, t)
+    return K.to_device_weight(raw, t, n, k), Q.dequantize_torch(raw, t, n, k).double()
+
+
+@pytest.fixture(scope="module")
+def space():
+    from hipengine_b200.models.executor import _Scratch
+    from hipengine_b200.ops.rows import RowsSpace
+    dev = torch.device("cuda", torch.cuda.current_device())
+    return RowsSpace(_Scratch(dev, canaries=True), dev, 5000)
+
+
+# fp32 rows round to 11 bits: at most 2^-11 of each value, so at most that of the result where the signs are random (2.1e-4 on
+# average for normal rows); Q6_K and Q8_0 operands round to 11 bits once more: sqrt(2) of it.  Q4_K operands and bf16 rows are exact
+BOUND = {T.Q4_K: 2 ** -11, T.Q6_K: 2 ** -10.5, T.Q8_0: 2 ** -10.5}
+
+
+@pytest.mark.parametrize("t", [T.Q4_K, T.Q6_K, T.Q8_0])
+@pytest.mark.parametrize("n,k", [(1, 256), (130, 512), (300, 768), (4999, 1280), (64, 17408)])
+def test_products_match_64_bit(space, t, n, k):
+    """Edges: fewer weight rows than a tile, remainders of it, one block, an odd number of blocks, tiles shared by many CTAs;
+    every group of eight activation rows."""
+    from hipengine_b200.ops import kernels as K
+    w, wd = _weight(t, n, k, n + k)
+    for R in (1, 2, 8, 9, 17, 32, 33, 41, 49, 64):
+        torch.manual_seed(R)
+        x = torch.randn(R, k, device="cuda") * torch.logspace(-3, 3, R, device="cuda")[:, None]
+        for xx in (x, x.bfloat16()):
+            out = torch.full((R, n), float("nan"), device="cuda")
+            space.gemm(xx, [K.GemvSegment(w, out)])
+            ref = xx.double() @ wd.t()
+            err = ((out.double() - ref).norm(dim=1) / ref.norm(dim=1)).max() if n > 1 else \
+                (out.double() - ref).abs().max() / (xx.double().norm(dim=1) * wd.norm()).max()
+            assert err < BOUND[t], (R, xx.dtype, float(err))
+        again = torch.zeros_like(out)
+        space.gemm(xx, [K.GemvSegment(w, again)])
+        assert torch.equal(out, again)
+    K.check_status()
+    assert int(space.counters.abs().sum()) == 0 and space.scratch.check_canaries() == []
+
+
+def test_a_row_does_not_depend_on_its_neighbours(space):
+    from hipengine_b200.ops import kernels as K
+    w, _ = _weight(T.Q4_K, 640, 2048, 3)
+    x = torch.randn(8, 2048, device="cuda")
+    out = torch.zeros(8, 640, device="cuda")
+    space.gemm(x, [K.GemvSegment(w, out)])
+    for r in range(8):
+        one = torch.zeros(1, 640, device="cuda")
+        space.gemm(x[r:r + 1], [K.GemvSegment(w, one)])
+        assert torch.equal(one[0], out[r])
+
+
+def test_segments_pairs_norm_side_rows(space):
+    """Segments of all block types in one launch; gate/up pair; adding into a strided residual; fp32 side rows."""
+    from hipengine_b200.ops import kernels as K
+    k = 1024
+    (g, gd), (u, ud) = _weight(T.Q4_K, 200, k, 1), _weight(T.Q4_K, 200, k, 2)
+    (a, ad), (b, bd) = _weight(T.Q6_K, 129, k, 3), _weight(T.Q8_0, 96, k, 4)
+    side = torch.randn(97, k, device="cuda") * 0.02
+    for R in (2, 7, 24, 40, 64):
+        x, nw = torch.randn(R, k, device="cuda"), torch.rand(k, device="cuda") + 0.5
+        act = torch.zeros(R, 208, device="cuda", dtype=torch.bfloat16)
+        add = torch.ones(R, 160, device="cuda")
+        pre = torch.zeros(R, 96, device="cuda")
+        so = torch.full((R, 104), float("nan"), device="cuda")
+        img, _ = space.image(x, nw, 1e-6, side, so)
+        space.product(img, R, k, [K.GemvSegment(g, act, K.EPI_SILU_MUL, u), K.GemvSegment(a, add[:, :129], K.EPI_ADD_F32),
+                                  K.GemvSegment(b, pre)])
+        xn = x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-6) * nw.double()
+        rel = lambda y, r: float((y.double() - r).norm() / r.norm())
+        assert rel(act[:, :200], torch.nn.functional.silu(xn @ gd.t()) * (xn @ ud.t())) < 4e-3       # bf16 result
+        assert rel(add[:, :129] - 1, xn @ ad.t()) < 2 ** -10.5 and bool((add[:, 129:] == 1).all())
+        assert rel(pre, xn @ bd.t()) < 2 ** -10.5
+        assert rel(so[:, :97], xn @ side.double().t()) < 3e-6 and bool(so[:, 97:].isnan().all())
+    K.check_status()
+
+
+def test_extreme_rows(space):
+    """Zero rows, the largest and smallest normal numbers, and a NaN that stays in its own row."""
+    from hipengine_b200.ops import kernels as K
+    w, wd = _weight(T.Q4_K, 128, 512, 9)
+    x = torch.randn(6, 512, device="cuda")
+    x[0] = 0
+    x[1] *= 1e30
+    x[2] *= 1e-30
+    x[3, 5] = float("nan")
+    x[4, 7] = float("inf")
+    out = torch.zeros(6, 128, device="cuda")
+    space.gemm(x, [K.GemvSegment(w, out)])
+    ref = x.double() @ wd.t()
+    assert bool((out[0] == 0).all()) and bool(out[3].isnan().all()) and not bool(out[4].isfinite().any())
+    for r in (1, 2, 5):
+        assert float((out[r].double() - ref[r]).norm() / ref[r].norm()) < 2 ** -11
+
+
+def test_refusals(space):
+    from hipengine_b200.ops import kernels as K
+    w, _ = _weight(T.Q4_K, 128, 512, 9)
+    with pytest.raises(RuntimeError):
+        space.gemm(torch.zeros(65, 512, device="cuda"), [K.GemvSegment(w, torch.zeros(65, 128, device="cuda"))])
+    with pytest.raises(RuntimeError):
+        space.image(torch.zeros(2, 516, device="cuda")[:, 2:514])         # rows that are not 16-byte aligned
