@@ -26,6 +26,14 @@ from ..ops.kernels import GemvSegment
 from ..quant.ggml import GGMLType
 
 SEL_MAX_ROWS = 64
+# Decode batches from this many rows on run their experts as jobs (csrc/moe_rows.cu): 256 experts, 8 used, a step of 4 / 8 / 32
+# rows takes 884 / 1033 / 1893 us with jobs, 873 / 1047 / 2471 us with one pass over an expert's rows per pair.
+JOBS_MIN_ROWS = 8
+# Pairs per expert up to which a prompt's do: 72 / 256 / 1024 / 2048 rows take 3.9 / 4.4 / 7.1 / 12.4 ms with jobs and
+# 6.1 / 7.3 / 8.6 / 10.6 ms in the grouped GEMM, whose 128-row tiles are mostly padding for few rows an expert.
+JOBS_MAX_LOAD = 32
+
+
 class _MoeLayer:
     """Per-layer derived weights: router as a GEMV weight and as bf16 hi/lo halves for the tensor-core path."""
 
@@ -95,9 +103,11 @@ def _moe_selected(ex, i: int, h: torch.Tensor, target: torch.Tensor, T: int, nor
     epi = K.EPI_SILU_MUL if cfg.act == "silu" else K.EPI_GELU_MUL
     # everything that reads the residual stream runs before anything that adds to it
     few = ex.few(T)
+    by_row = None
     if few:
         # router and shared gate in fp32 beside the rows' images, the shared expert's gate/up from the image
-        image, _ = ex.rows.image(h, norm_w, cfg.rms_eps, L.full, logits)
+        grouped = T >= JOBS_MIN_ROWS and _jobs_ok(ex, i, rng)
+        image, by_row = ex.rows.image(h, norm_w, cfg.rms_eps, L.full, logits, by_row=grouped)
         if shared_here:
             ex.rows.product(image, T, cfg.hidden, [GemvSegment(ex.W(i, "ffn_gate_shexp.weight"), act_sh, epi,
                                                                ex.W(i, "ffn_up_shexp.weight"))])
@@ -111,9 +121,13 @@ def _moe_selected(ex, i: int, h: torch.Tensor, target: torch.Tensor, T: int, nor
             K.gemv(h[r0:r1], [GemvSegment(ex.W(i, "ffn_gate_shexp.weight"), act_sh[r0:r1], epi,
                                           ex.W(i, "ffn_up_shexp.weight"))], norm_w=norm_w, eps=cfg.rms_eps)
     K.moe_route(logits, k, ids, wts, n_experts=E)
-    K.moe_gateup_sel(h, norm_w, cfg.rms_eps, ids, wts, ex.W(i, "ffn_gate_exps.weight"),
-                     ex.W(i, "ffn_up_exps.weight"), F, act_rows, cfg.act, expert_range=er)
-    K.moe_down_sel(act_rows, ids, wts, ex.W(i, "ffn_down_exps.weight"), cfg.hidden, target, expert_range=er)
+    if by_row is not None:
+        ys = _expert_jobs(ex, i, ids, by_row, k, act_rows, torch.float32)
+        ex.rows.sum_pairs(target, ys, wts)
+    else:
+        K.moe_gateup_sel(h, norm_w, cfg.rms_eps, ids, wts, ex.W(i, "ffn_gate_exps.weight"),
+                         ex.W(i, "ffn_up_exps.weight"), F, act_rows, cfg.act, expert_range=er)
+        K.moe_down_sel(act_rows, ids, wts, ex.W(i, "ffn_down_exps.weight"), cfg.hidden, target, expert_range=er)
     if shared_here:
         K.moe_scale_rows(act_sh, logits[:, E:E + 1])
         if few:
@@ -122,6 +136,36 @@ def _moe_selected(ex, i: int, h: torch.Tensor, target: torch.Tensor, T: int, nor
         for r0 in range(0, T, 8):
             r1 = min(T, r0 + 8)
             K.gemv(act_sh[r0:r1], [GemvSegment(ex.W(i, "ffn_down_shexp.weight"), target[r0:r1], K.EPI_ADD_F32)])
+
+
+def _jobs_ok(ex, i: int, rng) -> bool:
+    """Can the experts run as jobs (all of them local, block types and widths that the few-row products take)?"""
+    from ..ops import rows as ROWS
+    cfg = ex.cfg
+    w = [ex.W(i, f"ffn_{s}_exps.weight") for s in ("gate", "up", "down")]
+    return (ex.rows is not None and rng is None and cfg.n_experts <= 512 and cfg.hidden % 4 == 0 and
+            all(ROWS.weight_ok(x) for x in w) and w[0].qtype == w[1].qtype)
+
+
+def _job_cols(pairs: int, E: int) -> int:
+    """Rows per job: about twice what an expert gets on average (a job costs its columns' products whether they are
+    filled or not, a second job of an expert costs its weights again)."""
+    per = pairs / E
+    return 8 if per <= 4 else 16 if per <= 8 else 32
+
+
+def _expert_jobs(ex, i: int, ids: torch.Tensor, by_row: torch.Tensor, k: int, act: torch.Tensor, dtype) -> torch.Tensor:
+    """Rows of the pairs after their experts [T * k, hidden], from the token rows' image; ``act``: bf16 [T * k, expert width]."""
+    cfg, sc = ex.cfg, ex.scratch
+    P = ids.numel()
+    jobs = ex.rows.jobs(ids, cfg.n_experts, _job_cols(P, cfg.n_experts))
+    epi = K.EPI_SILU_MUL if cfg.act == "silu" else K.EPI_GELU_MUL
+    ex.rows.experts(jobs, by_row, k, ex.W(i, "ffn_gate_exps.weight"), act, epi, ex.W(i, "ffn_up_exps.weight"))
+    _, act_rows = ex.rows.image(act[:P], by_row=True, product=False)
+    ys = sc.get("moe_ys32" if dtype == torch.float32 else "moe_ys", (P, cfg.hidden), dtype)
+    ex.rows.experts(jobs, act_rows, 1, ex.W(i, "ffn_down_exps.weight"), ys,
+                    K.EPI_F32 if dtype == torch.float32 else K.EPI_BF16)
+    return ys
 
 
 def _grouped(sc, a_sorted: torch.Tensor, w, out: torch.Tensor, n_groups: int, tile_group: torch.Tensor) -> None:
@@ -164,6 +208,12 @@ def _moe_grouped(ex, i: int, h: torch.Tensor, target: torch.Tensor, T: int, norm
     wts = sc.get("moe_wts", (T, k), torch.float32)
     K.moe_route(logits, k, ids, wts, n_experts=E)
     P = T * k
+    if P <= JOBS_MAX_LOAD * E and _jobs_ok(ex, i, rng):
+        _, by_row = ex.rows.image(xn, by_row=True, product=False)
+        ys = _expert_jobs(ex, i, ids, by_row, k, sc.get("moe_act_g", (P, F), torch.bfloat16), torch.bfloat16)
+        ysh = _shared_rows(ex, i, xn, T) if shared_here else None
+        ex.rows.sum_pairs(target, ys, wts, ysh, logits[:, E:E + 1] if shared_here else None)
+        return
     bound = K.moe_sorted_rows_bound(P, El)
     pos = sc.get("moe_pos", (P,), torch.int32)
     tile_group = sc.get("moe_tiles", (bound // 128,), torch.int32)

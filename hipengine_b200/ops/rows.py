@@ -3,6 +3,7 @@ per product as an image of MMA fragments, times any number of weight rows stream
 from __future__ import annotations
 
 import ctypes as C
+from dataclasses import dataclass
 from typing import Optional, Sequence, Tuple
 
 import torch
@@ -29,6 +30,23 @@ class _Args(C.Structure):
                 ("w_bytes", C.c_int), ("tiles", C.c_int)]
 
 
+class _ExpertsArgs(C.Structure):
+    _fields_ = [("image", C.c_void_p), ("jobs", C.c_void_p), ("entries", C.c_void_p), ("meta", C.c_void_p),
+                ("out", C.c_void_p), ("out_stride", C.c_longlong), ("status", C.c_void_p), ("pairs_per_row", C.c_int),
+                ("N", C.c_int), ("K", C.c_int), ("E", C.c_int), ("expert_rows", C.c_int), ("qtype", C.c_int),
+                ("epi", C.c_int), ("stages", C.c_int), ("stage_bytes", C.c_int), ("w_bytes", C.c_int)]
+
+
+@dataclass
+class ExpertJobs:
+    entries: torch.Tensor      # [P] pair ids sorted by expert
+    list: torch.Tensor         # [bound, 4] (expert, first entry, entries, 0)
+    meta: torch.Tensor         # [0]: jobs
+    E: int
+    cols: int
+    P: int
+
+
 _CHECKED = False
 
 
@@ -38,6 +56,8 @@ def _lib():
     if not _CHECKED:
         if L.he_rows_args_size() != C.sizeof(_Args):
             raise RuntimeError(f"ABI mismatch for HeRowsArgs: C={L.he_rows_args_size()} Python={C.sizeof(_Args)}")
+        if L.he_rows_experts_args_size() != C.sizeof(_ExpertsArgs):
+            raise RuntimeError("ABI mismatch for RowsExpertsArgs")
         L.he_rows_image_bytes.restype = L.he_rows_ws_floats.restype = C.c_longlong
         _CHECKED = True
     return L
@@ -83,6 +103,51 @@ class RowsSpace:
                                 C.c_void_p(_p(side_out) if n_side else None),
                                 C.c_longlong(side_out.stride(0) if n_side else 0), _stream()), "he_rows_image")
         return img, rows
+
+    def jobs(self, ids: torch.Tensor, E: int, cols: int) -> "ExpertJobs":
+        """The (row, choice) pairs of ``ids`` [T, k] (int32) sorted by expert, cut into jobs of at most ``cols`` pairs."""
+        L = _lib()
+        L.he_moe_jobs_bound.restype = C.c_longlong
+        P = ids.numel()
+        n = int(L.he_moe_jobs_bound(C.c_longlong(P), C.c_int(E), C.c_int(cols)))
+        j = ExpertJobs(self.scratch.get("moe_entries", (P,), torch.int32),
+                       self.scratch.get("moe_job_list", (n, 4), torch.int32),
+                       self.scratch.get("moe_job_meta", (4,), torch.int32), E, cols, P)
+        assert ids.dtype == torch.int32 and ids.is_contiguous()
+        N.check(L.he_moe_jobs(C.c_void_p(ids.data_ptr()), C.c_int(P), C.c_int(E), C.c_int(cols),
+                              C.c_void_p(j.entries.data_ptr()), C.c_void_p(j.list.data_ptr()), C.c_int(n),
+                              C.c_void_p(j.meta.data_ptr()), _stream()), "he_moe_jobs")
+        return j
+
+    def experts(self, jobs: "ExpertJobs", by_row: torch.Tensor, pairs_per_row: int, w: DeviceWeight, out: torch.Tensor,
+                epi: int, w2: Optional[DeviceWeight] = None) -> None:
+        """out[pair] = (row of the pair) @ W[its expert]^T for the stacked expert weights ``w`` (gate, with ``w2`` up, for
+        the activation epilogues); ``by_row`` holds the image of pair // pairs_per_row."""
+        L = _lib()
+        assert w.n_rows % jobs.E == 0 and weight_ok(w) and out.shape[0] >= jobs.P and out.stride(1) == 1
+        a = _ExpertsArgs()
+        a.image, a.jobs, a.entries, a.meta = by_row.data_ptr(), jobs.list.data_ptr(), jobs.entries.data_ptr(), jobs.meta.data_ptr()
+        a.out, a.out_stride, a.status = out.data_ptr(), out.stride(0), status_tensor(out.device).data_ptr()
+        a.pairs_per_row, a.N, a.K, a.E = pairs_per_row, w.n_rows // jobs.E, w.n_cols, jobs.E
+        a.expert_rows, a.qtype, a.epi = w.n_rows // jobs.E, w.qtype, epi
+        if w2 is not None:
+            assert w2.qtype == w.qtype and w2.n_rows == w.n_rows and w2.n_cols == w.n_cols
+        N.check(L.he_rows_experts(C.byref(a), C.c_void_p(w.ptr), C.c_void_p(None if w2 is None else w2.ptr),
+                                  C.c_int(jobs.cols), C.c_int(N.num_sms()), _stream()), "he_rows_experts")
+
+    @staticmethod
+    def sum_pairs(h: torch.Tensor, y: torch.Tensor, wts: torch.Tensor, shared: Optional[torch.Tensor] = None,
+                  shared_gate: Optional[torch.Tensor] = None) -> None:
+        """h[t] += sum_j wts[t, j] * y[t * k + j] (+ sigmoid(shared_gate[t]) * shared[t])."""
+        T, k = wts.shape
+        assert h.dtype == torch.float32 and wts.is_contiguous() and wts.dtype == torch.float32
+        assert shared is None or shared.dtype == torch.bfloat16
+        N.check(_lib().he_moe_sum_pairs(
+            C.c_void_p(h.data_ptr()), C.c_longlong(h.stride(0)), C.c_void_p(y.data_ptr()), C.c_int(_dt(y)),
+            C.c_longlong(y.stride(0)), C.c_void_p(wts.data_ptr()), C.c_int(T), C.c_int(k), C.c_void_p(_p(shared)),
+            C.c_longlong(0 if shared is None else shared.stride(0)), C.c_void_p(_p(shared_gate)),
+            C.c_longlong(0 if shared_gate is None else shared_gate.stride(0)), C.c_int(h.shape[1]), _stream()),
+            "he_moe_sum_pairs")
 
     def product(self, image: torch.Tensor, R: int, K: int, segs: Sequence[GemvSegment]) -> None:
         """out (+)= rows @ W^T for every segment (see ``GemvSegment``), from the rows' image."""
