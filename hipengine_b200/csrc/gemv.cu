@@ -108,11 +108,26 @@ __device__ __forceinline__ void quant_store(const SmemView& s, int K, int r, int
 
 // (optional RMSNorm) + per-32 int8 quantisation.  With a norm and K <= 8192 the row is read once and kept in
 // registers between the statistics and the quantisation.
+constexpr int MAXG = 4;      // 8-column groups per thread of the one-pass prologue
+
+// The norm weights of the one-pass prologue, requested ahead of the predecessor's end (they are constants, and cold: their
+// way from HBM was on the chain between a launch's activations and its first product).  One row only: the registers.
+struct NormAhead {
+  float w[MAXG][8];
+};
+__device__ __forceinline__ void load_norm(const HeGemvArgs& a, NormAhead& n) {
+  if (a.norm_w == nullptr || a.K / 8 > MAXG * (int)blockDim.x) return;
+#pragma unroll
+  for (int u = 0; u < MAXG; ++u) {
+    const int g = u * (int)blockDim.x + (int)threadIdx.x;
+    if (g < a.K / 8) load8(a.norm_w, 0, (size_t)g * 8, n.w[u]);
+  }
+}
+
 template <int R, bool COMM>
-__device__ void prologue(const HeGemvArgs& a, const SmemView& s, float* red) {
+__device__ void prologue(const HeGemvArgs& a, const SmemView& s, float* red, const NormAhead& ahead) {
   const int K = a.K;
   const int n_groups = K / 8;
-  constexpr int MAXG = 4;
   const int nthr = (int)blockDim.x;
   const bool one_pass = a.norm_w != nullptr && n_groups <= MAXG * nthr;
   // reduce mode (the launcher admits it only with the one-pass prologue and fp32 rows): the rows are the residual
@@ -181,7 +196,10 @@ __device__ void prologue(const HeGemvArgs& a, const SmemView& s, float* red) {
         const int g = u * nthr + (int)threadIdx.x;
         if (u * nthr < n_groups) {  // uniform across the CTA
           const bool valid = g < n_groups;
-          if (valid) {
+          if (valid && R == 1) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[u][i] *= inv_rms * ahead.w[u][i];
+          } else if (valid) {
             const float4* wp = reinterpret_cast<const float4*>(a.norm_w + (size_t)g * 8);
             const float4 w0 = __ldg(wp), w1 = __ldg(wp + 1);
             v[u][0] *= inv_rms * w0.x; v[u][1] *= inv_rms * w0.y; v[u][2] *= inv_rms * w0.z; v[u][3] *= inv_rms * w0.w;
@@ -446,6 +464,8 @@ __global__ void __launch_bounds__(NW * 32, 1) gemv_kernel(const __grid_constant_
   // grid drains, start ours before the producer of the activations has finished, and only then wait for it.
   asm volatile("griddepcontrol.launch_dependents;");
   for (int i = 0; i < a.n_slots - 1; ++i) issue();
+  NormAhead ahead;
+  if (R == 1) load_norm(a, ahead);
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
   const bool push = COMM && (a.comm.mode & 1) != 0;
@@ -472,7 +492,7 @@ __global__ void __launch_bounds__(NW * 32, 1) gemv_kernel(const __grid_constant_
     }
     __syncthreads();
   } else {
-    prologue<R, COMM>(a, s, red);
+    prologue<R, COMM>(a, s, red, ahead);
   }
 
   if constexpr (P2) {

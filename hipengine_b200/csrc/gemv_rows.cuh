@@ -90,6 +90,10 @@ __device__ __forceinline__ void block_q4k(const uint8_t* blk, int b, const SmemV
   for (int r = 0; r < R; ++r) acc[r] += part[r];
 }
 
+// v - 32 in each byte, 0 <= v < 64: v + 96 has no carry, and flipping its top bit takes 128 off in two's complement (two
+// instructions; the byte-wise subtraction is a sequence of several).
+__device__ __forceinline__ uint32_t minus32x4(uint32_t v) { return (v + 0x60606060u) ^ 0x80808080u; }
+
 // ---------------------------------------------------------------- Q6_K: one 224-byte block
 template <int R>
 __device__ __forceinline__ void block_q6k(const uint8_t* blk, int b, const SmemView& s, float (&acc)[R]) {
@@ -107,10 +111,10 @@ __device__ __forceinline__ void block_q6k(const uint8_t* blk, int b, const SmemV
       uint32_t q[4][4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        q[0][u] = __vsub4((lav[u] & 0x0F0F0F0Fu) | ((hv[u] & 0x03030303u) << 4), 0x20202020u);
-        q[1][u] = __vsub4((lbv[u] & 0x0F0F0F0Fu) | (((hv[u] >> 2) & 0x03030303u) << 4), 0x20202020u);
-        q[2][u] = __vsub4(((lav[u] >> 4) & 0x0F0F0F0Fu) | (((hv[u] >> 4) & 0x03030303u) << 4), 0x20202020u);
-        q[3][u] = __vsub4(((lbv[u] >> 4) & 0x0F0F0F0Fu) | (((hv[u] >> 6) & 0x03030303u) << 4), 0x20202020u);
+        q[0][u] = minus32x4((lav[u] & 0x0F0F0F0Fu) | ((hv[u] & 0x03030303u) << 4));
+        q[1][u] = minus32x4((lbv[u] & 0x0F0F0F0Fu) | (((hv[u] >> 2) & 0x03030303u) << 4));
+        q[2][u] = minus32x4(((lav[u] >> 4) & 0x0F0F0F0Fu) | (((hv[u] >> 4) & 0x03030303u) << 4));
+        q[3][u] = minus32x4(((lbv[u] >> 4) & 0x0F0F0F0Fu) | (((hv[u] >> 6) & 0x03030303u) << 4));
       }
       float dsc[4];
 #pragma unroll
@@ -248,10 +252,10 @@ __device__ __forceinline__ void q6k_unpack16(const uint8_t* blk, int half, int l
   const uint32_t hv[4] = {hh.x, hh.y, hh.z, hh.w};
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
-    q[0][u] = __vsub4((lav[u] & 0x0F0F0F0Fu) | ((hv[u] & 0x03030303u) << 4), 0x20202020u);
-    q[1][u] = __vsub4((lbv[u] & 0x0F0F0F0Fu) | (((hv[u] >> 2) & 0x03030303u) << 4), 0x20202020u);
-    q[2][u] = __vsub4(((lav[u] >> 4) & 0x0F0F0F0Fu) | (((hv[u] >> 4) & 0x03030303u) << 4), 0x20202020u);
-    q[3][u] = __vsub4(((lbv[u] >> 4) & 0x0F0F0F0Fu) | (((hv[u] >> 6) & 0x03030303u) << 4), 0x20202020u);
+    q[0][u] = minus32x4((lav[u] & 0x0F0F0F0Fu) | ((hv[u] & 0x03030303u) << 4));
+    q[1][u] = minus32x4((lbv[u] & 0x0F0F0F0Fu) | (((hv[u] >> 2) & 0x03030303u) << 4));
+    q[2][u] = minus32x4(((lav[u] >> 4) & 0x0F0F0F0Fu) | (((hv[u] >> 4) & 0x03030303u) << 4));
+    q[3][u] = minus32x4(((lbv[u] >> 4) & 0x0F0F0F0Fu) | (((hv[u] >> 6) & 0x03030303u) << 4));
   }
 }
 
