@@ -20,6 +20,7 @@ import os
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence, Tuple
 
+import numpy as np
 import torch
 
 from ..loading.weights import ModelWeights, QTensor, ffn_norm_slot
@@ -52,28 +53,35 @@ class BatchDesc:
 
 
 def make_batch(segments: Sequence[Tuple[int, int, Sequence[int]]], device) -> BatchDesc:
-    """segments: (slot, start_pos, token_ids) per request.  Builds the packed descriptor (one H2D copy each)."""
-    toks: List[int] = []
-    slot: List[int] = []
-    pos: List[int] = []
-    seg_start = [0]
-    seg_slot: List[int] = []
-    tok_seg: List[int] = []
-    max_ctx = 1
+    """segments: (slot, start_pos, token_ids) per request.  Builds the packed descriptor: one pinned host buffer and one
+    copy, in stream order.  (A tensor per field made from a Python list was a pageable copy each, and every one of them
+    waited for the stream: the host's time for a prompt never overlapped the device's.)"""
+    device = torch.device(device)
+    counts = [len(ids) for _, _, ids in segments]
+    n, T = len(counts), sum(counts)
+    fields, words = [], (T + 1) // 2 * 2              # int64 tokens first; every field starts on 16 bytes
+    for length in (T, T, T, T, n + 1, n):
+        fields.append((2 * words, length))
+        words += (length + 3) // 4 * 2
+    host = torch.empty(words, dtype=torch.int64, pin_memory=device.type == "cuda")
+    tokens, ints = host.numpy(), host.numpy().view(np.int32)
+    slot, pos, ctx, tok_seg, seg_start, seg_slot = (ints[o:o + m] for o, m in fields)
+    seg_start[0], max_ctx, r1 = 0, 1, 0
     for si, (s, p0, ids) in enumerate(segments):
-        n = len(ids)
-        toks += list(ids)
-        slot += [s] * n
-        pos += list(range(p0, p0 + n))
-        tok_seg += [si] * n
-        seg_start.append(seg_start[-1] + n)
-        seg_slot.append(s)
-        max_ctx = max(max_ctx, p0 + n)
-    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=device)
-    pos_t = i32(pos)
-    return BatchDesc(torch.tensor(toks, dtype=torch.int64, device=device), i32(slot), pos_t, pos_t + 1,
-                     i32(seg_start), i32(seg_slot), i32(tok_seg), len(toks), len(segments), max_ctx,
-                     [(s, p0, len(ids)) for (s, p0, ids) in segments])
+        r0, r1 = r1, r1 + counts[si]
+        tokens[r0:r1] = ids.tolist() if isinstance(ids, torch.Tensor) else ids
+        slot[r0:r1] = s
+        pos[r0:r1] = np.arange(p0, p0 + counts[si], dtype=np.int32)
+        tok_seg[r0:r1] = si
+        seg_start[si + 1] = r1
+        seg_slot[si] = s
+        max_ctx = max(max_ctx, p0 + counts[si])
+    np.add(pos, 1, out=ctx)
+    dev = host.to(device, non_blocking=True) if device.type == "cuda" else host
+    d32 = dev.view(torch.int32)
+    v = [d32[o:o + m] for o, m in fields]
+    return BatchDesc(dev[:T], v[0], v[1], v[2], v[4], v[5], v[3], T, n, max_ctx,
+                     [(s, p0, c) for (s, p0, _), c in zip(segments, counts)])
 
 
 class _Scratch:
@@ -305,10 +313,9 @@ class HybridExecutor:
         self.am_i = torch.empty(GEMV_MAX_ROWS * 64 * 64, dtype=torch.int32, device=dev)
 
     def reset_slot(self, slot: int) -> None:
-        for t in self.conv_state.values():
-            t[slot].zero_()
-        for t in self.gdn_state.values():
-            t[slot].zero_()
+        held = [t[slot] for d in (self.conv_state, self.gdn_state) for t in d.values()]
+        if held:
+            torch._foreach_zero_(held)              # one launch for all layers
 
     def state_bytes(self) -> int:
         tot = 0
