@@ -7,15 +7,23 @@
 // registers and store them with tcgen05.st straight into a TMEM operand stage (row = TMEM lane).  The expanded
 // weight therefore never exists in shared or global memory: DRAM and L2 see 4.5 / 6.6 / 8.5 bits per weight, and
 // shared-memory bandwidth is left to the activation tiles.  Roles (24 warps):
-//   warp 0      : TMA producer of activation tiles X[mt][64] (128-byte swizzle, 5-stage ring)
-//   warp 1      : MMA issuer (tcgen05.mma 128 x mt x 16, A from TMEM, B from smem); owns the TMEM allocation
-//   warp 2      : TMA producer of raw weight blocks (one 256-column super-block of 128 rows per q-stage, 3 stages)
+//   warp 0      : TMA producer of activation tiles X[mt][64] (128-byte swizzle, 6-stage ring)
+//   warp 1, 3   : MMA issuers (tcgen05.mma 128 x mt x 16, A from TMEM, B from smem), one for each of the two activation
+//                 tiles of a unit; warp 1 alone where a unit has one tile and in the reduce-scatter form; warp 1 owns the
+//                 TMEM allocation
+//   warp 2      : TMA producer of raw weight blocks (one 256-column super-block of 128 rows per q-stage, 2 or more stages)
 //   warps 4..7  : epilogue (tcgen05.ld, transposed store: lane = weight row n, register = activation row m, so a
 //                 store instruction of a warp covers 32 consecutive n of one output row)
 //   warps 8..23 : unpack, four sets of four warps; set g expands k-block g of every super-block into TMEM
 //                 operand stage g (thread = weight row), so four k-blocks are in flight
 // TMEM (512 columns): two accumulators of 192 fp32 columns (epilogue of tile i overlaps the main loop of
 // tile i+1) + four operand stages of 32 columns.
+// What bounds it: the 1 kW power cap on large products (SM clock 1.3-1.5 GHz under load), below that the latency of the
+// single threads that issue.  A poll of a barrier that is ready costs such a thread 160 cycles, so one issuer of a k-block
+// (three barriers, eight MMAs of 64..96 cycles) took 1390 cycles where its MMAs take 768; two issuers and a producer without
+// divisions take 1020.  4096 x 17408 x 5120 Q4_K 708 -> 595 us, 4096 x 5120 x 17408 Q8_0 564 -> 488 us (1.5 PFLOP/s),
+// 777 x 17408 x 5120 167 -> 141 us.  A CTA pair (cta_group::2, half the activation traffic) gave another 4 % and is not
+// used: its issuers' last commits land in the other CTA's shared memory, where nothing waits for them.
 // Counterparts in the reference: hipengine/kernels/hip_gfx1100/quant/gguf_q4_k_prefill.hip:170-296 (raw 144-byte
 // blocks read inside the matrix-core loop), gguf_q8_0_prefill.hip, and the grouped expert form
 // quant/gguf_q4_k_selected_prefill.hip.
@@ -30,8 +38,7 @@ namespace {
 constexpr int WN = 128;                  // weight rows per tile (the MMA's M)
 constexpr int MT_MAX = 192;              // activation rows per tile (the MMA's N), multiple of 16
 constexpr int BK = 64, UK = 16;
-constexpr int XSTAGES = 5;                          // activation ring depth (stage = mt x 64 bf16, <= 24 KB); seven
-                                                    // stages (with three raw-block stages) measured slower in pair mode
+constexpr int XSTAGES = 6, XSTAGES_SMALL = 5;       // activation ring depth (stage = mt x 64 bf16, <= 24 KB)
 constexpr int QSTAGES_MAX = 12;                     // raw-block ring: as many stages as shared memory holds, up to 12
 constexpr int SMEM_BUDGET = 224 * 1024;             // dynamic shared memory the rings may use
 constexpr int N_SETS = 4;                           // unpack sets == TMEM operand stages == k-blocks per q-stage
@@ -380,20 +387,22 @@ __device__ __forceinline__ void gemm_wq_body(const CUtensorMap& tmX, const CUten
                                              const WqArgs& g, const WqFuse* f) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint8_t* qring = smem + XSTAGES * g.x_stage_bytes;
+  constexpr int XS = SMALL ? XSTAGES_SMALL : XSTAGES;
+  uint8_t* qring = smem + XS * g.x_stage_bytes;
   WqBarriers* bar = reinterpret_cast<WqBarriers*>(qring + g.q_stages * g.q_stage_bytes);
   const int QS = g.q_stages;
   volatile int* abort_flag = &bar->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int mt = g.mt;
+  const bool two = !RS && !SMALL && g.pair;            // an issuer for each of the two M-tiles of a unit
   const int tiles_m = (g.M + mt - 1) / mt, tiles_n = (g.N + WN - 1) / WN;
   const int units_m = g.pair ? (tiles_m + 1) >> 1 : tiles_m;
   const int n_tiles = (RS && !(f->phases & 1)) ? 0 : units_m * tiles_n * g.k_splits;   // work units
   const int sb_all = g.K >> 8;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < XSTAGES; ++s) {
+    for (int s = 0; s < XS; ++s) {
       mbar_init(&bar->x_full[s], 1);
       mbar_init(&bar->x_empty[s], 1);
     }
@@ -406,7 +415,7 @@ __device__ __forceinline__ void gemm_wq_body(const CUtensorMap& tmX, const CUten
     // the critical path when an MMA batch lasts tens of cycles -- waits and commits once per super-block
     for (int s = 0; s < A_STAGES_MAX; ++s) {
       mbar_init(&bar->a_full[s], SMALL ? N_UNPACK_WARPS : N_UNPACK_WARPS / N_SETS);
-      mbar_init(&bar->a_empty[s], 1);
+      mbar_init(&bar->a_empty[s], two ? 2 : 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&bar->d_full[a], 1);
@@ -435,7 +444,8 @@ __device__ __forceinline__ void gemm_wq_body(const CUtensorMap& tmX, const CUten
     // ------------------------------------------------------------ activation tiles
     if (elect_one()) {
       tma_prefetch_desc(&tmX);
-      uint32_t it = 0;
+      RingCursor xc;
+      const uint32_t x_bytes = (uint32_t)(XKB * mt * BK * 2);
       uint32_t ag_seen = 0;                     // owners whose rows are known to have arrived
       const uint32_t ag_want = g.ag_world > 0 ? *reinterpret_cast<const volatile uint32_t*>(g.ag_epoch) : 0u;
       for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
@@ -457,14 +467,19 @@ __device__ __forceinline__ void gemm_wq_body(const CUtensorMap& tmX, const CUten
           }
         }
         // a stage holds XKB k-blocks of one M-tile (XKB > 1 only with one tile per unit)
-        for (int kb = 4 * t.sb0; kb < 4 * t.sb1 && !*abort_flag; kb += XKB)
-          for (int j = 0; j < t.ntile; ++j, ++it) {
-            const int s = it % XSTAGES;
-            if (!mbar_wait(&bar->x_empty[s], ((it / XSTAGES) & 1) ^ 1, abort_flag, g.status, 301)) break;
-            mbar_expect_tx(&bar->x_full[s], (uint32_t)(XKB * mt * BK * 2));
+        for (int kb = 4 * t.sb0; kb < 4 * t.sb1; kb += XKB)
+          for (int j = 0; j < t.ntile; ++j) {
+            uint64_t* full = &bar->x_full[xc.s];
+            if (!mbar_try_wait(&bar->x_empty[xc.s], xc.ph ^ 1u) &&
+                !mbar_wait(&bar->x_empty[xc.s], xc.ph ^ 1u, abort_flag, g.status, 301)) {
+              kb = 4 * t.sb1;
+              break;
+            }
+            mbar_expect_tx(full, x_bytes);
+            uint8_t* dst = smem + xc.s * g.x_stage_bytes;
             for (int u = 0; u < XKB; ++u)
-              tma_load_2d(smem + s * g.x_stage_bytes + u * mt * BK * 2, &tmX, &bar->x_full[s], (kb + u) * BK,
-                          (t.tm + j) * mt);
+              tma_load_2d(dst + u * mt * BK * 2, &tmX, full, (kb + u) * BK, (t.tm + j) * mt);
+            xc.next(XS);
           }
         if (*abort_flag) break;
       }
@@ -501,39 +516,48 @@ __device__ __forceinline__ void gemm_wq_body(const CUtensorMap& tmX, const CUten
       }
       if (qprof) { g.dbg[16] = c_qe; g.dbg[17] = clock64() - c_qall; g.dbg[18] = qit; }
     }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    if (elect_one()) {
+  } else if (warp == 1 || (!RS && !SMALL && warp == 3)) {
+    // ------------------------------------------------------------ MMA issuers
+    const int me = warp == 1 ? 0 : 1;
+    if ((me == 0 || two) && elect_one()) {
       const uint32_t idesc = umma_idesc_bf16(WN, mt);
-      uint32_t it = 0, ait = 0, ucount = 0;
+      uint32_t ucount = 0;
       uint32_t par = 0;                         // bit b: parity of the completed uses of accumulator b
-      const bool mprof = HE_WQ_PROF_ON && g.dbg != nullptr && blockIdx.x == 0;
+      const bool mprof = HE_WQ_PROF_ON && g.dbg != nullptr && blockIdx.x == 0 && me == 0;
       long long c_af = 0, c_xf = 0, c_de = 0, c_all = mprof ? clock64() : 0;
+      // the single issuing thread is a chain of instruction latencies: a ready barrier costs it one poll, a descriptor
+      // one addition
+      auto wait = [&](uint64_t* b, uint32_t parity, int code) {
+        return mbar_try_wait(b, parity) || mbar_wait(b, parity, abort_flag, g.status, code);
+      };
+      uint32_t it = 0, ait = 0;                 // small tiles
+      uint32_t xs = 0, xph = 0, aph = 0;        // activation stage of the k-block's first M-tile; phase of the operand stages
+      const uint64_t desc0 = umma_desc_k_sw128(smem_u32(smem));
+      const uint32_t xq = (uint32_t)g.x_stage_bytes >> 4;
       for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
         const TileCoord t = tile_coord(g, tile, tiles_m, sb_all);
         if (t.skip) continue;
         // pair mode: tile j of the unit accumulates in buffer j; otherwise units alternate between the buffers so
         // that the epilogue of one overlaps the main loop of the next
         const int acc0 = g.pair ? 0 : (int)(ucount & 1);
+        const int j0 = two ? me : 0, j1 = two ? min(me + 1, t.ntile) : t.ntile;
         bool ok = true;
         long long d0 = mprof ? clock64() : 0;
-        for (int j = 0; j < t.ntile && ok; ++j)
-          ok = mbar_wait(&bar->d_empty[acc0 + j], ((par >> (acc0 + j)) & 1) ^ 1, abort_flag, g.status, 303);
+        for (int j = j0; j < j1 && ok; ++j) ok = wait(&bar->d_empty[acc0 + j], ((par >> (acc0 + j)) & 1) ^ 1, 303);
         if (!ok) break;
         if (mprof) c_de += clock64() - d0;
         tc_fence_after();
-        const int n_kb = 4 * (t.sb1 - t.sb0);
         if constexpr (SMALL) {
           // one super-block per iteration: slot sbi % AD of the operand ring, one activation stage (4 k-blocks)
           const uint32_t d_tmem = tmem_base + acc0 * d_cols;
           for (int sb = 0; sb < t.sb1 - t.sb0 && ok; ++sb, ait += N_SETS, ++it) {
             const uint32_t sbi = ait / N_SETS;
-            const int slot = (int)(sbi % AD), s = it % XSTAGES;
+            const int slot = (int)(sbi % AD), s = it % XS;
             long long m0 = 0;
             if (mprof) m0 = clock64();
-            if (!mbar_wait(&bar->a_full[slot], (sbi / AD) & 1, abort_flag, g.status, 305)) { ok = false; break; }
+            if (!wait(&bar->a_full[slot], (sbi / AD) & 1, 305)) { ok = false; break; }
             if (mprof) { c_af += clock64() - m0; m0 = clock64(); }
-            if (!mbar_wait(&bar->x_full[s], (it / XSTAGES) & 1, abort_flag, g.status, 304)) { ok = false; break; }
+            if (!wait(&bar->x_full[s], (it / XS) & 1, 304)) { ok = false; break; }
             if (mprof) c_xf += clock64() - m0;
             tc_fence_after();
             const uint32_t x_addr = smem_u32(smem + s * g.x_stage_bytes);
@@ -549,41 +573,42 @@ __device__ __forceinline__ void gemm_wq_body(const CUtensorMap& tmX, const CUten
             umma_commit(&bar->a_empty[slot]);
           }
         } else {
-        for (int kb = 0; kb < n_kb && ok; ++kb, ++ait) {
-            // operand stage of k-block c of the unit-spanning super-block count sbi: set c, slot sbi % AD
-            const uint32_t sbi = ait / N_SETS;
-            const int a = (int)(ait % N_SETS) + N_SETS * (int)(sbi % AD);
-            long long m0 = 0;
-            if (mprof) m0 = clock64();
-            if (!mbar_wait(&bar->a_full[a], (sbi / AD) & 1, abort_flag, g.status, 305)) { ok = false; break; }
-            if (mprof) c_af += clock64() - m0;
-            const uint32_t a_tmem = tmem_base + a_col0 + a * A_STAGE_COLS;
-            const int u = kb % XKB;           // k-block inside the activation stage
-            for (int j = 0; j < t.ntile; ++j) {
-              const int s = it % XSTAGES;
+          for (int sb = t.sb0; sb < t.sb1 && ok; ++sb, aph ^= 1u) {
+#pragma unroll
+            for (int c = 0; c < N_SETS; ++c) {
+              long long m0 = 0;
               if (mprof) m0 = clock64();
-              if (u == 0 && !mbar_wait(&bar->x_full[s], (it / XSTAGES) & 1, abort_flag, g.status, 304)) {
-                ok = false;
-                break;
+              if (!ok || !wait(&bar->a_full[c], aph, 305)) { ok = false; break; }
+              if (mprof) c_af += clock64() - m0;
+              const uint32_t a_tmem = tmem_base + a_col0 + c * A_STAGE_COLS;
+              for (int j = j0; j < j1; ++j) {
+                uint32_t sj = xs + j, pj = xph;
+                if (sj >= XS) { sj -= XS; pj ^= 1u; }
+                if (mprof) m0 = clock64();
+                if (!wait(&bar->x_full[sj], pj, 304)) { ok = false; break; }
+                if (mprof) c_xf += clock64() - m0;
+                tc_fence_after();
+                const uint64_t desc = desc0 + sj * xq;
+                const uint32_t d_tmem = tmem_base + (acc0 + j) * d_cols;
+#pragma unroll
+                for (int k = 0; k < BK / UK; ++k) {
+                  const uint32_t add = (c > 0 || k > 0) ? 1u : (sb > t.sb0 ? 1u : 0u);
+                  umma_f16_ts(d_tmem, a_tmem + k * (UK / 2), desc + k * (UK * 2 / 16), idesc, add);
+                }
+                umma_commit(&bar->x_empty[sj]);      // the smem stage is free once these MMAs have read it
               }
-              if (mprof) c_xf += clock64() - m0;
-              tc_fence_after();
-              const uint32_t x_addr = smem_u32(smem + s * g.x_stage_bytes + u * mt * BK * 2);
-              const uint32_t d_tmem = tmem_base + (acc0 + j) * d_cols;
-  #pragma unroll
-              for (int k = 0; k < BK / UK; ++k)
-                umma_f16_ts(d_tmem, a_tmem + k * (UK / 2), umma_desc_k_sw128(x_addr + k * UK * 2), idesc,
-                            (kb > 0 || k > 0) ? 1u : 0u);
-              if (u == XKB - 1) {
-                umma_commit(&bar->x_empty[s]);  // the smem stage is free once these MMAs have read it
-                ++it;
-              }
+              // ... and so is the TMEM operand stage, once both issuers are done with it (an issuer without a tile in this unit
+              // has no MMAs to wait for: nobody would see such a commit land before the block ends)
+              if (j0 < j1) umma_commit(&bar->a_empty[c]);
+              else mbar_arrive(&bar->a_empty[c]);
+              xs += t.ntile;
+              if (xs >= XS) { xs -= XS; xph ^= 1u; }
             }
-            umma_commit(&bar->a_empty[a]);    // ... and so is the TMEM operand stage
           }
+          if (mprof) ait += N_SETS * (t.sb1 - t.sb0);
         }
         if (!ok || *abort_flag) break;
-        for (int j = 0; j < t.ntile; ++j) {
+        for (int j = j0; j < j1; ++j) {
           umma_commit(&bar->d_full[acc0 + j]);
           par ^= 1u << (acc0 + j);
         }
@@ -928,7 +953,7 @@ int launch_wq(const void* A, long long lda, int a_cols, const void* B, int qtype
     const int tiles_m0 = (g.M + g.mt - 1) / g.mt;
     g.pair = (pair_mode_enabled() && g.tile_group == nullptr && g.k_splits == 1 && tiles_m0 >= 2) ? 1 : 0;
   }
-  g.q_stages = (SMEM_BUDGET - XSTAGES * g.x_stage_bytes) / g.q_stage_bytes;
+  g.q_stages = (SMEM_BUDGET - (small ? XSTAGES_SMALL : XSTAGES) * g.x_stage_bytes) / g.q_stage_bytes;
   if (g.q_stages > QSTAGES_MAX) g.q_stages = QSTAGES_MAX;
   if (g.q_stages < 2) return -HE_ERR_BAD_ARG;
   CUtensorMap tmX, q0, q1;
