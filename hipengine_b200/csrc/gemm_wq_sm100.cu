@@ -936,6 +936,40 @@ int pick_mt(int M, bool grouped) {
   return (M + 15) & ~15;
 }
 
+// Activation rows per tile of a plain product with several tiles.  A unit of two tiles costs its rows plus about as much again
+// as 390 of them (unit times of 4096 x 17408 x 5120: 55.1 / 52.9 / 51.4 / 48.3 us at 192 / 176 / 160 / 144 rows a tile), and the
+// busiest SM ends the kernel: take the tile for which that SM has the least to do.  Against 192 always: 2048 rows x 10240
+// 247 -> 219 us (160), x 17408 324 -> 308 us (176), 777 rows x 5120 72 -> 68 us (160); 4096 x 17408 stays at 192.
+int pick_mt_plain(int M, int N, int num_sms) {
+  if (M <= MT_MAX || !pair_mode_enabled()) return pick_mt(M, false);
+  constexpr int FIXED = 390;
+  const long long tiles_n = (N + WN - 1) / WN;
+  int best = MT_MAX;
+  long long best_cost = 0;
+  for (int mt = MT_MAX; mt >= 96; mt -= 16) {
+    const int tiles_m = (M + mt - 1) / mt, units_m = (tiles_m + 1) / 2;
+    const long long units = units_m * tiles_n, rounds = (units + num_sms - 1) / num_sms;
+    // units go to the SMs in turn, the last of every units_m has one tile when their number is odd: the fewest of those
+    // among the SMs that take part in the last round
+    long long singles = 0;
+    if (tiles_m & 1) {
+      const long long full = units - (rounds - 1) * num_sms;
+      singles = rounds;
+      for (int c = 0; c < units_m && c < full; ++c) {
+        long long n = 0;
+        for (long long r = 0; r < rounds; ++r) n += (c + r * num_sms) % units_m == units_m - 1;
+        if (n < singles) singles = n;
+      }
+    }
+    const long long cost = rounds * (2 * mt + FIXED) - singles * mt;
+    if (best_cost == 0 || cost < best_cost) {
+      best_cost = cost;
+      best = mt;
+    }
+  }
+  return best;
+}
+
 long long* g_debug_counters = nullptr;
 
 int launch_wq(const void* A, long long lda, int a_cols, const void* B, int qtype, long long b_rows, WqArgs g,
@@ -1015,7 +1049,7 @@ HE_API int he_gemm_q(const void* A, long long lda, int a_cols, const void* B, in
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   WqArgs g = {};
   g.C = C; g.ldc = ldc; g.M = M; g.N = N; g.K = K; g.epi = epi; g.qtype = qtype;
-  g.mt = pick_mt(M, tile_group != nullptr);
+  g.mt = tile_group != nullptr ? pick_mt(M, true) : pick_mt_plain(M, N, num_sms);
   g.k_splits = 1;
   g.sb_per = K >> 8;
   g.split_stride = 0;
