@@ -253,10 +253,12 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       for (int c = 0; c < 32; c += 2) {
         const float p0 = ex2(fmaf(__uint_as_float(r0[c]), sc, neg)), p1 = ex2(fmaf(__uint_as_float(r0[c + 1]), sc, neg));
         const float p2 = ex2(fmaf(__uint_as_float(r1[c]), sc, neg)), p3 = ex2(fmaf(__uint_as_float(r1[c + 1]), sc, neg));
-        s0 += p0 + p1;
-        s1 += p2 + p3;
         r0[c >> 1] = pack2(p0, p1);
         r1[c >> 1] = pack2(p2, p3);
+        // the sum takes the rounded weights: the largest one is not 1 under a reference that lags, and its rounding would
+        // stay in the quotient
+        s0 += __uint_as_float(r0[c >> 1] << 16) + __uint_as_float(r0[c >> 1] & 0xFFFF0000u);
+        s1 += __uint_as_float(r1[c >> 1] << 16) + __uint_as_float(r1[c >> 1] & 0xFFFF0000u);
       }
       l += s0 + s1;
 #pragma unroll
