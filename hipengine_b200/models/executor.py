@@ -9,9 +9,10 @@ through the same call, differing only in how many rows a segment has.
 Kernel sequence per layer follows the reference executors
 (``hipengine/runtime/qwen35_gguf_layer_attn.py:474-1147`` for linear / full
 attention, ``hipengine/runtime/qwen35_gguf_layer_ffn.py:301-1278`` for dense and
-MoE FFN) but the fusion boundaries are chosen for B200: for <= 8 rows each
-projection is a single fused [RMSNorm + int8 quantize + dp4a GEMV + epilogue]
-launch; above that the projections run on the tcgen05 GEMM.
+MoE FFN) but the fusion boundaries are chosen for B200: for one or two rows
+each projection is a single fused [RMSNorm + int8 quantize + dp4a GEMV +
+epilogue] launch (two launches for two rows); up to 64 rows the few-row products
+stream each weight once; above that the projections run on the tcgen05 GEMM.
 """
 from __future__ import annotations
 

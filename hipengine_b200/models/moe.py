@@ -1,11 +1,13 @@
 """Mixture-of-experts FFN block of the hybrid executor (Qwen3.5-MoE: 256 experts, top-8, shared expert).
 
-Two routes, chosen by the number of packed rows:
+Three routes, chosen by the number of packed rows:
 
 * ``T <= SEL_MAX_ROWS`` (decode, verify chains, short prefill chunks): *selected-expert GEMV*.  The router
   GEMV writes logits, ``he_moe_route`` picks the experts on the device, and two kernels walk the
-  (token, expert) pairs reading the experts' quantised rows in place.  No expert id is ever read by the host,
+  (token, expert) pairs reading the experts' quantised rows in place; from ``JOBS_MIN_ROWS`` rows the pairs are
+  sorted by expert and run as jobs (``csrc/moe_rows.cu``).  No expert id is ever read by the host,
   so the whole block is CUDA-graph capturable.
+* larger ``T`` with few pairs per expert (``JOBS_MAX_LOAD``): the same jobs, with the shared expert on the GEMM.
 * larger ``T``: *grouped tensor-core GEMM*.  Pairs are bucketed by expert (128-row padded segments), rows are
   gathered and the tcgen05 GEMM runs in grouped mode over the experts' quantised blocks (each 128-row tile
   carries its expert id; the blocks are expanded to bf16 inside the GEMM pipeline), followed by a combine kernel that applies the routing weights, the
