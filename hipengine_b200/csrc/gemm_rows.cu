@@ -115,7 +115,7 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
 
   if (warp >= S::MMA_WARPS) {
     if (warp == S::MMA_WARPS) {
-    // ------------------------------------------------------------ producer
+      // ------------------------------------------------------------ producer
       if (sm100::elect_one()) {
         const uint8_t* image = reinterpret_cast<const uint8_t*>(a.image);
         int si = 0, tile = u0 / nb, blk = u0 % nb;
