@@ -1,0 +1,54 @@
+"""Routed experts as jobs (csrc/moe_rows.cu): the job list, the products of the jobs and the weighted sum."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def space():
+    from hipengine_b200.models.executor import _Scratch
+    from hipengine_b200.ops.rows import RowsSpace
+    dev = torch.device("cuda", torch.cuda.current_device())
+    return RowsSpace(_Scratch(dev, canaries=True), dev, 5000)
+
+
+def _ids_of_counts(counts, k, seed):
+    """Expert ids [T, k] in which expert e appears counts[e] times, in random order."""
+    flat = torch.repeat_interleave(torch.arange(len(counts)), torch.tensor(counts))
+    flat = flat[torch.randperm(flat.numel(), generator=torch.Generator().manual_seed(seed))]
+    return flat.to(torch.int32).reshape(-1, k).cuda()
+
+
+def _weight(t, n, k, seed):
+    from hipengine_b200.ops import kernels as K
+    from hipengine_b200.quant import ggml as Q
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    raw = Q.quantize(torch.randn(n, k, generator=g, device="cuda") * 0.02, t)
+    return K.to_device_weight(raw, t, n, k), Q.dequantize_torch(raw, t, n, k).double()
+
+
+def _types():
+    from hipengine_b200.quant.ggml import GGMLType as T
+    return [T.Q4_K, T.Q6_K, T.Q8_0]
+
+
+@pytest.mark.parametrize("t", _types())
+def test_a_row_does_not_depend_on_its_job(space, t):
+    """Experts of more rows than a job: which of them fall into the short last one is a matter of chance."""
+    from hipengine_b200.ops import kernels as K
+    counts, n, k = [33, 48, 7, 40], 160, 768
+    w, _ = _weight(t, len(counts) * n, k, 3)
+    ids = _ids_of_counts(counts, 1, 0)
+    x = torch.randn(ids.shape[0], k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    first = None
+    for i in range(20):
+        perm = torch.randperm(ids.shape[0], generator=torch.Generator().manual_seed(i)).cuda()
+        out = torch.full((ids.shape[0], n), float("nan"), device="cuda")
+        jobs = space.jobs(ids[perm].contiguous(), len(counts), 32)
+        space.experts(jobs, space.image(x[perm].contiguous(), by_row=True, product=False)[1], 1, w, out, K.EPI_F32)
+        got = torch.empty_like(out)
+        got[perm] = out
+        first = got if first is None else first
+        assert torch.equal(got, first), i
+    K.check_status()
