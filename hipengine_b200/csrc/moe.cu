@@ -62,6 +62,9 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, long long ld,
       const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
       if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
     }
+    // nothing left above -infinity (logits that are NaN): expert 0, so that every id is one; its weight is that of the
+    // sentinel, NaN wherever a NaN logit is in the denominator
+    if (bi >= E) bi = 0;
     if ((bi & 31) == lane) {
 #pragma unroll
       for (int i = 0; i < MAXPL; ++i)

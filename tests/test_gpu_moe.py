@@ -24,6 +24,31 @@ def test_route_matches_reference(E, k, T):
     torch.testing.assert_close(wts.cpu(), rw, atol=1e-5, rtol=1e-4)
 
 
+@pytest.mark.parametrize("E,k", [(16, 4), (256, 8), (512, 10)])
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_route_names_experts_for_rows_without_enough_numbers(E, k, mode):
+    """Rows of NaN, of minus infinity, and with fewer numbers than choices: every id is an expert's, other rows as they were."""
+    from hipengine_b200.ops import kernels as K
+    g = torch.Generator(device="cuda").manual_seed(E)
+    clean = torch.randn(9, E, device="cuda", generator=g)
+    logits = clean.clone()
+    logits[1] = float("nan")
+    logits[3] = -float("inf")
+    logits[5, k - 1:] = float("nan")
+    logits[7, :E - 1] = -float("inf")
+    res = []
+    for x in (clean, logits):
+        ids = torch.full((9, k), -7, dtype=torch.int32, device="cuda")
+        wts = torch.zeros(9, k, device="cuda")
+        K.moe_route(x, k, ids, wts, n_experts=E, mode=mode)
+        res.append((ids.cpu(), wts.cpu()))
+    (ids0, w0), (ids1, w1) = res
+    assert int(ids1.min()) >= 0 and int(ids1.max()) < E
+    assert torch.equal(ids0[::2], ids1[::2]) and torch.equal(w0[::2], w1[::2])
+    assert sorted(ids1[5, :k - 1].tolist()) == list(range(k - 1)) and int(ids1[7, 0]) == E - 1
+    assert bool(w1[1].isnan().all())
+
+
 def test_group_and_gather_round_trip():
     from hipengine_b200.ops import kernels as K
     T, k, E, Hd = 300, 4, 16, 64
@@ -116,3 +141,22 @@ def test_moe_block_matches_reference_on_identical_input(T):
     assert torch.isfinite(got).all()
     err = (got - want).abs().amax(-1) / want.abs().amax(-1).clamp(min=1e-6)
     assert (err < 0.06).float().mean() >= 0.97, err
+
+
+@pytest.mark.parametrize("T", [3, 40, 100, 200], ids=["decode", "jobs", "prompt_jobs", "grouped"])
+def test_a_row_of_nan_stays_alone(T):
+    from hipengine_b200.loading.weights import ffn_norm_slot
+    from hipengine_b200.models import moe as M
+    from hipengine_b200.models.executor import HybridExecutor
+    from hipengine_b200.ops import kernels as K
+    cfg = TINY_HYBRID_MOE
+    ex = HybridExecutor(build_random_model(cfg, seed=2, std=0.05).to("cuda"), max_slots=1, max_context=64)
+    norm_w = ex.F(1, ffn_norm_slot(cfg))
+    clean = torch.randn(T, cfg.hidden, generator=torch.Generator().manual_seed(T)).cuda()
+    bad = clean.clone()
+    bad[1, 5] = float("nan")
+    for x in (clean, bad):
+        M.moe_ffn(ex, 1, x, T, norm_w, T <= 8)
+    K.check_status()
+    others = torch.arange(T, device="cuda") != 1
+    assert torch.equal(bad[others], clean[others]) and bool(bad[1].isnan().all())
