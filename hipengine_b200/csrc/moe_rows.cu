@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(1024) moe_jobs_kernel(const int* __restrict__ 
   __syncthreads();
   for (int p = tid; p < P; p += 1024) {
     const int e = ids[p];
-    if (HE_INDEX_OK(e, E, HE_SITE_MOE_EXPERT_ID)) atomicAdd(&cnt[e], 1);
+    if (HE_INDEX_OK(e, E, HE_SITE_MOE_EXPERT_ID) && e >= 0 && e < E) atomicAdd(&cnt[e], 1);
   }
   __syncthreads();
   // exclusive sums of the rows and of the jobs of the experts before

@@ -20,6 +20,29 @@ def _ids_of_counts(counts, k, seed):
     return flat.to(torch.int32).reshape(-1, k).cuda()
 
 
+@pytest.mark.parametrize("cols", [8, 16, 32])
+@pytest.mark.parametrize("E", [3, 32, 33, 512])
+def test_job_list(space, cols, E):
+    """Every pair in one job of its expert, jobs full except an expert's last; ids that are no expert's are in no job."""
+    g = torch.Generator().manual_seed(E + cols)
+    ids = torch.randint(0, E, (4 * cols + 3, 5), generator=g).int()
+    ids[:, 0] = E - 1                                   # one expert of several jobs
+    for k, bad in ((7, -1), (11, E), (12, 0x7FFFFFFF), (30, -0x80000000)):
+        ids.view(-1)[k] = bad
+    j = space.jobs(ids.cuda(), E, cols)
+    n, flat = int(j.meta[0]), ids.view(-1).tolist()
+    entries, jobs = j.entries.cpu().tolist(), j.list[:n].cpu().tolist()
+    seen, of = [], {}
+    for e, first, count, _ in jobs:
+        assert 1 <= count <= cols and 0 <= e < E
+        assert all(flat[p] == e for p in entries[first:first + count])
+        seen += entries[first:first + count]
+        of.setdefault(e, []).append(count)
+    assert sorted(seen) == [p for p, e in enumerate(flat) if 0 <= e < E]
+    assert all(c == cols for counts in of.values() for c in counts[:-1])
+    assert space.scratch.check_canaries() == []
+
+
 def _weight(t, n, k, seed):
     from hipengine_b200.ops import kernels as K
     from hipengine_b200.quant import ggml as Q
