@@ -50,6 +50,7 @@ struct GdnChunkArgs {
   int write_state;
   float* ws;              // he_gdn_chunk_ws_floats
   long long ws_floats;
+  int longest;            // tokens of the longest segment, or 0 where the caller does not know it
   int c_lo, c_hi;         // chunks [c_lo, c_hi) of every segment (set by the launcher)
 };
 
@@ -418,29 +419,42 @@ __global__ void __launch_bounds__(256) gdn_chain_kernel(const GdnChunkArgs p) {
   }
 }
 
-// Chunks per segment that one pass of both kernels covers: all of an ordinary prompt portion, at most ~160 in all, which
-// bounds the workspace (36 KB per chunk and head) whatever the number of tokens.
+// Chunks that one pass of both kernels covers, over all segments: 160 of them bound the workspace (37 KB per chunk and head)
+// whatever the number of tokens.  What fits is one pass, a longer scan goes in windows of as many chunks of every segment.
 constexpr int WINDOW_CHUNKS = 160;
-inline int window_chunks(int n_seg) { return n_seg >= WINDOW_CHUNKS ? 1 : WINDOW_CHUNKS / n_seg; }
+
+struct Windows {
+  long long units;        // workspace units of one pass
+  int per, count;         // chunks of a segment in one pass; passes
+};
+// (A scan that leaves the state alone has no place to carry it between windows: one window.)
+inline Windows windows(int T, int n_seg, int write_state, int longest) {
+  const long long all = T / CK + n_seg;                                // at least the sum of the rounded-up counts
+  const int chunks = ((longest > 0 && longest < T ? longest : T) + CK - 1) / CK;
+  if (!write_state || all <= WINDOW_CHUNKS) return {all, chunks, 1};
+  const int per = n_seg >= WINDOW_CHUNKS ? 1 : WINDOW_CHUNKS / n_seg;
+  const long long most = (long long)n_seg * per;
+  return {all < most ? all : most, per, (chunks + per - 1) / per};
+}
 
 }  // namespace
 
 // Floats of workspace that a scan of T tokens in n_seg segments needs.
-// (A scan that leaves the state alone has no place to carry it between windows: one window.)
 HE_API long long he_gdn_chunk_ws_floats(int T, int n_seg, int Hv, int write_state) {
   if (T <= 0 || n_seg <= 0) return 0;
-  long long chunks = T / CK + n_seg;                                   // at least the sum of the rounded-up counts
-  const long long most = (long long)n_seg * window_chunks(n_seg);
-  if (write_state && chunks > most) chunks = most;
-  return chunks * Hv * WS_UNIT;
+  return windows(T, n_seg, write_state, 0).units * Hv * WS_UNIT;
+}
+// Passes (of two launches each) that it makes; `longest` as in GdnChunkArgs.
+HE_API int he_gdn_chunk_windows(int T, int n_seg, int write_state, int longest) {
+  return T <= 0 || n_seg <= 0 ? 0 : windows(T, n_seg, write_state, longest).count;
 }
 
 // Chunked tensor-core scan.  Same arguments as he_gdn_scan minus the journal, plus the workspace; state size must be 128.
 HE_API int he_gdn_scan_chunked(const GdnChunkArgs* args, cudaStream_t stream) {
   GdnChunkArgs a = *args;
   if (a.T <= 0 || a.n_seg <= 0) return 0;
-  if (a.C != 2 * a.G * DK + a.Hv * DK || a.ws == nullptr || 
-      a.ws_floats < he_gdn_chunk_ws_floats(a.T, a.n_seg, a.Hv, a.write_state))
+  const Windows w = windows(a.T, a.n_seg, a.write_state, a.longest);
+  if (a.C != 2 * a.G * DK + a.Hv * DK || a.ws == nullptr || a.longest < 0 || a.ws_floats < w.units * a.Hv * WS_UNIT)
     return -HE_ERR_BAD_ARG;
   // set per call (cheap): the attribute belongs to the (function, device) pair, not to the process
   cudaError_t e = cudaFuncSetAttribute(gdn_prepare_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -454,14 +468,10 @@ HE_API int he_gdn_scan_chunked(const GdnChunkArgs* args, cudaStream_t stream) {
     e = narrow ? cudaFuncSetAttribute(gdn_chain_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chain_smem)
                : cudaFuncSetAttribute(gdn_chain_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chain_smem);
   if (e != cudaSuccess) return (int)e;
-  const int longest = (a.T + CK - 1) / CK;                             // chunks of one segment, at most
-  const int per = a.write_state ? window_chunks(a.n_seg) : longest;
-  for (int lo = 0; lo < longest; lo += per) {
-    a.c_lo = lo;
-    a.c_hi = lo + per;
-    long long grid = a.T / CK + a.n_seg;
-    if (grid > (long long)a.n_seg * per) grid = (long long)a.n_seg * per;
-    gdn_prepare_chunks_kernel<<<dim3((unsigned)grid, a.Hv), 128, sizeof(PrepSmem), stream>>>(a);
+  for (int i = 0; i < w.count; ++i) {
+    a.c_lo = i * w.per;
+    a.c_hi = a.c_lo + w.per;
+    gdn_prepare_chunks_kernel<<<dim3((unsigned)w.units, a.Hv), 128, sizeof(PrepSmem), stream>>>(a);
     HE_LAUNCH_CHECK();
     if (narrow) gdn_chain_kernel<32><<<dim3(a.n_seg, a.Hv, 4), 256, chain_smem, stream>>>(a);
     else gdn_chain_kernel<64><<<dim3(a.n_seg, a.Hv, 2), 256, chain_smem, stream>>>(a);

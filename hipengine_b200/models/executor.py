@@ -558,7 +558,8 @@ class HybridExecutor:
         if (journal is None and S == 128 and T >= 64 * b.n_seg and os.environ.get("HE_GDN_CHUNKED", "1") != "0"):
             # long prefill segments: 32-token chunks on the tensor cores instead of the token-serial recurrence
             ws = sc.get("gdn_ws", (K.gdn_chunk_ws_floats(T, b.n_seg, Hv),), torch.float32)
-            K.gdn_scan_chunked(conv, decay, beta, self.gdn_state[i], b.seg_start, b.seg_slot, o, G, Hv, ws=ws)
+            K.gdn_scan_chunked(conv, decay, beta, self.gdn_state[i], b.seg_start, b.seg_slot, o, G, Hv, ws=ws,
+                               longest=max(n for _, _, n in b.segs_host) if b.segs_host else 0)
         else:
             K.gdn_scan(conv, decay, beta, self.gdn_state[i], b.seg_start, b.seg_slot, o, G, Hv,
                        write_state=journal is None, journal=gj)

@@ -100,8 +100,8 @@ class _GdnFrontArgs(C.Structure):
 class _GdnChunkArgs(C.Structure):
     _fields_ = [("qkv", c_vp), ("decay", c_vp), ("beta", c_vp), ("state", c_vp), ("seg_start", c_vp),
                 ("seg_slot", c_vp), ("out", c_vp), ("C", C.c_int), ("G", C.c_int), ("Hv", C.c_int), ("T", C.c_int),
-                ("n_seg", C.c_int), ("write_state", C.c_int), ("ws", c_vp), ("ws_floats", c_ll), ("c_lo", C.c_int),
-                ("c_hi", C.c_int)]
+                ("n_seg", C.c_int), ("write_state", C.c_int), ("ws", c_vp), ("ws_floats", c_ll), ("longest", C.c_int),
+                ("c_lo", C.c_int), ("c_hi", C.c_int)]
 
 
 class _MoeSelArgs(C.Structure):
@@ -520,11 +520,17 @@ def gdn_chunk_ws_floats(T: int, n_seg: int, Hv: int, write_state: bool = True) -
     return int(L.he_gdn_chunk_ws_floats(C.c_int(T), C.c_int(n_seg), C.c_int(Hv), C.c_int(int(write_state))))
 
 
+def gdn_chunk_windows(T: int, n_seg: int, write_state: bool = True, longest: int = 0) -> int:
+    """Passes of a chunked scan, two launches each."""
+    return int(N.lib().he_gdn_chunk_windows(C.c_int(T), C.c_int(n_seg), C.c_int(int(write_state)), C.c_int(longest)))
+
+
 def gdn_scan_chunked(qkv: torch.Tensor, decay: torch.Tensor, beta: torch.Tensor, state: torch.Tensor,
                      seg_start: torch.Tensor, seg_slot: torch.Tensor, out: torch.Tensor, G: int, Hv: int,
-                     write_state: bool = True, ws: Optional[torch.Tensor] = None) -> None:
+                     write_state: bool = True, ws: Optional[torch.Tensor] = None, longest: int = 0) -> None:
     """Chunked (32-token, WY form) tensor-core scan for prefill segments; same contract as ``gdn_scan`` without the
-    journal.  Products run in TF32 with fp32 accumulation.  ``ws``: fp32 workspace of ``gdn_chunk_ws_floats``."""
+    journal.  Products run in TF32 with fp32 accumulation.  ``ws``: fp32 workspace of ``gdn_chunk_ws_floats``; ``longest``:
+    tokens of the longest segment where the host knows it (0: it could be all of them, which costs empty passes)."""
     _check_abi()
     p = _GdnChunkArgs()
     T, n_seg = qkv.shape[0], seg_slot.numel()
@@ -534,9 +540,10 @@ def gdn_scan_chunked(qkv: torch.Tensor, decay: torch.Tensor, beta: torch.Tensor,
     p.qkv, p.decay, p.beta, p.state = qkv.data_ptr(), decay.data_ptr(), beta.data_ptr(), state.data_ptr()
     p.seg_start, p.seg_slot, p.out = seg_start.data_ptr(), seg_slot.data_ptr(), out.data_ptr()
     p.C, p.G, p.Hv, p.T, p.n_seg, p.write_state = qkv.shape[1], G, Hv, T, n_seg, int(write_state)
-    p.ws, p.ws_floats = ws.data_ptr(), ws.numel()
+    p.ws, p.ws_floats, p.longest = ws.data_ptr(), ws.numel(), longest
     assert qkv.dtype == torch.float32 and qkv.is_contiguous() and ws.dtype == torch.float32
     N.check(N.lib().he_gdn_scan_chunked(C.byref(p), _stream()), "he_gdn_scan_chunked")
+    N.add_launches(2 * gdn_chunk_windows(T, n_seg, write_state, longest) - N.KERNELS_PER_CALL["he_gdn_scan_chunked"])
 
 
 def gdn_gated_norm(o: torch.Tensor, z: torch.Tensor, w: torch.Tensor, out: torch.Tensor, Hv: int, Dv: int,

@@ -67,6 +67,34 @@ def test_scan_windows_and_segments(lens, Hv):
     assert torch.equal(st, state0) and float((out - outs[1]).norm() / outs[1].norm()) < 1e-6
 
 
+@pytest.mark.parametrize("lens", [[700] * 8, [64] * 40, [5200, 64, 300], [65] * 165, [2000, 100, 33]])
+def test_scan_of_packed_prompts_makes_no_empty_passes(lens):
+    """With the longest segment given: as many passes as it has windows, the results of the scan that was not told."""
+    from hipengine_b200.ops import kernels as K
+    G, Hv, S, T, n = 1, 1, 128, sum(lens), len(lens)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    q, k = R.l2norm(rand(T, G, S)) * S ** -0.5, R.l2norm(rand(T, G, S))
+    qkv = torch.cat([q.reshape(T, -1), k.reshape(T, -1), rand(T, Hv * S) * 0.5], 1).contiguous()
+    decay, beta = torch.exp(-0.2 * rand(T, Hv).abs()), torch.sigmoid(rand(T, Hv))
+    start = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+    slot = torch.arange(n, dtype=torch.int32, device="cuda")
+    state0 = rand(n, Hv, S, S) * 0.1
+    per = max(1, 160 // n) if T // 32 + n > 160 else -(-max(lens) // 32)
+    res = []
+    for longest in (0, max(lens)):
+        st, out = state0.clone(), torch.zeros(T, Hv, S, device="cuda")
+        before = K.launch_count()
+        K.gdn_scan_chunked(qkv, decay, beta, st, start, slot, out, G, Hv, longest=longest)
+        res.append((st, out, K.launch_count() - before))
+    assert res[1][2] == 2 * -(-(-(-max(lens) // 32)) // per) <= res[0][2]
+    assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
+    st, out = state0.clone(), torch.zeros(T, Hv, S, device="cuda")
+    K.gdn_scan(qkv, decay, beta, st, start, slot, out, G, Hv)
+    for a, b in ((res[1][1], out), (res[1][0], st)):
+        assert float((a - b).norm() / b.norm()) < 2e-3          # TF32 products against fp32
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("lens", [[1], [2, 3, 40], [17, 1, 16, 100]])
 def test_front_is_convolution_then_preparation(dtype, lens):
