@@ -26,23 +26,34 @@ struct MoeJob {
   int expert, first, count, pad;      // rows entries[first .. first + count)
 };
 
-// One CTA.  entries: pair ids sorted by expert (in any order within one); meta[0] = number of jobs.
-__global__ void __launch_bounds__(1024) moe_jobs_kernel(const int* __restrict__ ids, int P, int E, int cols,
-                                                        int* __restrict__ entries, MoeJob* __restrict__ jobs,
-                                                        int max_jobs, int* __restrict__ meta) {
-  __shared__ int cnt[512], off[512], wsum[2][32];
+constexpr int JOB_WARPS = 16, MAX_EXPERTS = JOB_WARPS * 32;
+
+// One CTA, a contiguous part of the pairs per warp.  entries: pair ids sorted by expert, in ascending order within one, so that
+// the jobs (and the sums of their rows) are the same in every run; meta[0] = number of jobs.
+__global__ void __launch_bounds__(MAX_EXPERTS) moe_jobs_kernel(const int* __restrict__ ids, int P, int E, int cols,
+                                                               int* __restrict__ entries, MoeJob* __restrict__ jobs,
+                                                               int max_jobs, int* __restrict__ meta) {
+  __shared__ int at[JOB_WARPS][MAX_EXPERTS];      // pairs of a warp's part per expert, then where its next one goes
+  __shared__ int wsum[2][JOB_WARPS];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int part = (P + MAX_EXPERTS - 1) / MAX_EXPERTS * 32, p0 = warp * part, p1 = min(P, p0 + part);
   pdl_wait();
   pdl_launch();
-  if (tid < 512) cnt[tid] = 0;
+  for (int w = 0; w < JOB_WARPS; ++w) at[w][tid] = 0;
   __syncthreads();
-  for (int p = tid; p < P; p += 1024) {
+  for (int p = p0 + lane; p < p1; p += 32) {
     const int e = ids[p];
-    if (HE_INDEX_OK(e, E, HE_SITE_MOE_EXPERT_ID) && e >= 0 && e < E) atomicAdd(&cnt[e], 1);
+    if (HE_INDEX_OK(e, E, HE_SITE_MOE_EXPERT_ID) && e >= 0 && e < E) atomicAdd(&at[warp][e], 1);
   }
   __syncthreads();
-  // exclusive sums of the rows and of the jobs of the experts before
-  const int n = tid < E ? cnt[tid] : 0, nj = (n + cols - 1) / cols;
+  // exclusive sums: of an expert's pairs over the parts before, of the pairs and the jobs of the experts before
+  int n = 0;
+  for (int w = 0; w < JOB_WARPS; ++w) {
+    const int c = at[w][tid];
+    at[w][tid] = n;
+    n += c;
+  }
+  const int nj = (n + cols - 1) / cols;
   int a = n, b = nj;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -52,17 +63,20 @@ __global__ void __launch_bounds__(1024) moe_jobs_kernel(const int* __restrict__ 
   if (lane == 31) { wsum[0][warp] = a; wsum[1][warp] = b; }
   __syncthreads();
   for (int w = 0; w < warp; ++w) { a += wsum[0][w]; b += wsum[1][w]; }
-  if (tid < E) {
-    off[tid] = a - n;
-    cnt[tid] = 0;
-    for (int i = 0; i < nj; ++i)
-      if (b - nj + i < max_jobs) jobs[b - nj + i] = MoeJob{tid, a - n + i * cols, min(cols, n - i * cols), 0};
-  }
-  if (tid == E - 1) meta[0] = min(b, max_jobs);
+  for (int w = 0; w < JOB_WARPS; ++w) at[w][tid] += a - n;
+  for (int i = 0; i < nj; ++i)
+    if (b - nj + i < max_jobs) jobs[b - nj + i] = MoeJob{tid, a - n + i * cols, min(cols, n - i * cols), 0};
+  if (tid == MAX_EXPERTS - 1) meta[0] = min(b, max_jobs);
   __syncthreads();
-  for (int p = tid; p < P; p += 1024) {
-    const int e = ids[p];
-    if (e >= 0 && e < E) entries[off[e] + atomicAdd(&cnt[e], 1)] = p;
+  for (int q = p0; q < p1; q += 32) {
+    const int p = q + lane, e = p < p1 ? ids[p] : -1;
+    const bool ok = e >= 0 && e < E;
+    const unsigned same = __match_any_sync(0xffffffffu, e);
+    const int rank = __popc(same & ((1u << lane) - 1u)), first = ok ? at[warp][e] : 0;
+    if (ok) entries[first + rank] = p;
+    __syncwarp();
+    if (ok && rank == 0) at[warp][e] = first + __popc(same);
+    __syncwarp();
   }
 }
 
@@ -310,12 +324,12 @@ HE_API long long he_moe_jobs_bound(long long P, int E, int cols) {
   return full < P ? full : P;
 }
 
-// ids[P] (0 <= id < E <= 512) -> entries[P], jobs (4 ints each), meta[0].  cols: 8, 16 or 32.
+// ids[P] (0 <= id < E <= 512; pairs with others are in no job) -> entries[P], jobs (4 ints each), meta[0].  cols: 8, 16 or 32.
 HE_API int he_moe_jobs(const int* ids, int P, int E, int cols, int* entries, void* jobs, int max_jobs, int* meta,
                        cudaStream_t stream) {
   if (P <= 0) return 0;
-  if (E < 1 || E > 512 || cols < 1 || max_jobs < he_moe_jobs_bound(P, E, cols)) return -HE_ERR_BAD_ARG;
-  return (int)launch_pdl(moe_jobs_kernel, dim3(1), dim3(1024), 0, stream, ids, P, E, cols, entries, (MoeJob*)jobs, max_jobs, meta);
+  if (E < 1 || E > MAX_EXPERTS || cols < 1 || max_jobs < he_moe_jobs_bound(P, E, cols)) return -HE_ERR_BAD_ARG;
+  return (int)launch_pdl(moe_jobs_kernel, dim3(1), dim3(MAX_EXPERTS), 0, stream, ids, P, E, cols, entries, (MoeJob*)jobs, max_jobs, meta);
 }
 
 // Products of the jobs' rows with their experts' weights `w` (and `w2`: the up weights of epi 3, 4), [E * expert_rows][K]

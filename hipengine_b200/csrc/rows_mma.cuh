@@ -100,10 +100,6 @@ __device__ __forceinline__ uint32_t opaque(uint32_t c) {
 // byte i of w as the fp16 pair (1024 + byte, 1024 + byte)
 __device__ __forceinline__ uint32_t dup_byte(uint32_t w, uint32_t i) { return prmt(w, 0x64646464u, 0x4040u | i | (i << 8)); }
 
-// Few columns: two accumulators of a block, half the dependent MMAs in a row.  Chosen by NT and not by L, so that a row's sum
-// is the same whatever the number of rows beside it in its job.
-constexpr bool split_sums(int nt) { return nt <= 2; }
-
 // One block (256 columns) of the 16 weight rows of a warp: `r0`, `r1` are the shared addresses of rows g and g + 8 in
 // the stage, `img` that of the block's image.  acc[nt] += the block's product in the MMA's C layout (rows g / g + 8,
 // activation rows 8 nt + 2t, + 1); only the first L groups of eight rows are computed.
@@ -120,8 +116,7 @@ __device__ __forceinline__ void block_q4k(uint32_t r0, uint32_t r1, uint32_t img
   const uint32_t scb = ((h ? mb.w : mb.y) & low_bits) | ((mb.y >> 2) & high_bits);
   const uint32_t mna = ((h ? ma.w >> 4 : ma.z) & low_bits) | ((ma.z >> 2) & high_bits);
   const uint32_t mnb = ((h ? mb.w >> 4 : mb.z) & low_bits) | ((mb.z >> 2) & high_bits);
-  constexpr bool SPLIT = split_sums(NT);
-  float D[L][4], E[SPLIT ? L : 1][4];
+  float D[L][4], E[L <= 2 ? L : 1][4];      // few columns: two accumulators, half the dependent MMAs in a row
   const uint32_t xb = img + g * IMG_COL + t * 16;
 #pragma unroll
   for (int c = 0; c < 2; ++c) {      // chunk 2h + c: low nibbles are group 2c of the half, high nibbles group 2c + 1
@@ -142,15 +137,15 @@ __device__ __forceinline__ void block_q4k(uint32_t r0, uint32_t r1, uint32_t img
       for (int n = 0; n < L; ++n) {
         const uint4 x = lds128(xb + n * 8 * IMG_COL + (v * 2 + c) * 64);
         mma_from(v + c == 0, D[n], l0, l1, l2, l3, x.x, x.y);
-        mma_from(SPLIT && v + c == 0, SPLIT ? E[SPLIT ? n : 0] : D[n], u0, u1, u2, u3, x.z, x.w);
+        mma_from(L <= 2 && v + c == 0, L <= 2 ? E[L <= 2 ? n : 0] : D[n], u0, u1, u2, u3, x.z, x.w);
       }
     }
   }
-  if (SPLIT) {
+  if (L <= 2) {
 #pragma unroll
     for (int n = 0; n < L; ++n)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) D[n][i] += E[SPLIT ? n : 0][i];
+      for (int i = 0; i < 4; ++i) D[n][i] += E[L <= 2 ? n : 0][i];
   }
   // minima: slots (2t, 2t + 1) meet the high parts of the sums of sub-blocks 2t, 2t + 1, slots + 8 the low parts
   const uint32_t msel = 0x4040u | (2 * u) | ((2 * u + 1) << 8);
@@ -196,8 +191,7 @@ __device__ __forceinline__ void block_q6k(uint32_t r0, uint32_t r1, uint32_t img
   // signed scales of the four groups (byte 2 qt + u), one per byte, as byte + 128
   const uint32_t ssel = u ? 0x7531u : 0x6420u;
   const uint32_t sca = prmt(sa.x, sa.y, ssel) ^ 0x80808080u, scb = prmt(sb.x, sb.y, ssel) ^ 0x80808080u;
-  constexpr bool SPLIT = split_sums(NT);
-  float D[L][4], E[SPLIT ? L : 1][4];
+  float D[L][4], E[L <= 2 ? L : 1][4];      // few columns: two accumulators, half the dependent MMAs in a row
   const uint32_t xb = img + g * IMG_COL + t * 16;
   uint32_t fa[4], fb[4];
 #pragma unroll
@@ -246,15 +240,15 @@ __device__ __forceinline__ void block_q6k(uint32_t r0, uint32_t r1, uint32_t img
       for (int n = 0; n < L; ++n) {
         const uint4 x = lds128(xb + n * 8 * IMG_COL + (v * 2 + c) * 64);
         mma_from(v + c == 0, D[n], e[0], e[1], e[2], e[3], x.x, x.y);
-        mma_from(SPLIT && v + c == 0, SPLIT ? E[SPLIT ? n : 0] : D[n], o[0], o[1], o[2], o[3], x.z, x.w);
+        mma_from(L <= 2 && v + c == 0, L <= 2 ? E[L <= 2 ? n : 0] : D[n], o[0], o[1], o[2], o[3], x.z, x.w);
       }
     }
   }
-  if (SPLIT) {
+  if (L <= 2) {
 #pragma unroll
     for (int n = 0; n < L; ++n)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) D[n][i] += E[SPLIT ? n : 0][i];
+      for (int i = 0; i < 4; ++i) D[n][i] += E[L <= 2 ? n : 0][i];
   }
   const uint32_t dwa = lds32(r0 + 208), dwb = lds32(r1 + 208);
   block_scale<NT, L>(img, t, __low2float(*reinterpret_cast<const __half2*>(&dwa)),
@@ -290,8 +284,7 @@ __device__ __forceinline__ void block_q80(uint32_t p0, int i0, uint32_t p1, int 
   const float ea = q8_scales(lds128(p0 + 2 * HT * 128 + i0 * 16), h, fa);
   const float eb = q8_scales(lds128(p1 + 2 * HT * 128 + i1 * 16), h, fb);
   const uint32_t ra = p0 + h * HT * 128 + i0 * 128, rb = p1 + h * HT * 128 + i1 * 128;
-  constexpr bool SPLIT = split_sums(NT);
-  float D[L][4], E[SPLIT ? L : 1][4];
+  float D[L][4], E[L <= 2 ? L : 1][4];      // few columns: two accumulators, half the dependent MMAs in a row
   const uint32_t xb = img + g * IMG_COL + t * 16;
   auto up = [mg](uint32_t w, uint32_t f) { return h2_mul(h2_add(and_or<0x00FF00FFu>(w, mg), M1152), f); };
 #pragma unroll
@@ -320,15 +313,15 @@ __device__ __forceinline__ void block_q80(uint32_t p0, int i0, uint32_t p1, int 
       for (int n = 0; n < L; ++n) {
         const uint4 x = lds128(xb + n * 8 * IMG_COL + (v * 2 + c) * 64);
         mma_from(v + c == 0, D[n], e[0][0], e[0][1], e[0][2], e[0][3], x.x, x.y);
-        mma_from(SPLIT && v + c == 0, SPLIT ? E[SPLIT ? n : 0] : D[n], e[1][0], e[1][1], e[1][2], e[1][3], x.z, x.w);
+        mma_from(L <= 2 && v + c == 0, L <= 2 ? E[L <= 2 ? n : 0] : D[n], e[1][0], e[1][1], e[1][2], e[1][3], x.z, x.w);
       }
     }
   }
-  if (SPLIT) {
+  if (L <= 2) {
 #pragma unroll
     for (int n = 0; n < L; ++n)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) D[n][i] += E[SPLIT ? n : 0][i];
+      for (int i = 0; i < 4; ++i) D[n][i] += E[L <= 2 ? n : 0][i];
   }
   block_scale<NT, L>(img, t, ea, eb, D, acc);
 }

@@ -21,11 +21,12 @@ def _ids_of_counts(counts, k, seed):
 
 
 @pytest.mark.parametrize("cols", [8, 16, 32])
-@pytest.mark.parametrize("E", [3, 32, 33, 512])
-def test_job_list(space, cols, E):
-    """Every pair in one job of its expert, jobs full except an expert's last; ids that are no expert's are in no job."""
+@pytest.mark.parametrize("E,rows", [(3, 4), (32, 4), (33, 1), (512, 4), (512, 70)])
+def test_job_list(space, cols, E, rows):
+    """Every pair in one job of its expert, in ascending order, jobs full except an expert's last; ids that are no expert's
+    are in no job."""
     g = torch.Generator().manual_seed(E + cols)
-    ids = torch.randint(0, E, (4 * cols + 3, 5), generator=g).int()
+    ids = torch.randint(0, E, (rows * cols + 3, 5), generator=g).int()
     ids[:, 0] = E - 1                                   # one expert of several jobs
     for k, bad in ((7, -1), (11, E), (12, 0x7FFFFFFF), (30, -0x80000000)):
         ids.view(-1)[k] = bad
@@ -38,7 +39,7 @@ def test_job_list(space, cols, E):
         assert all(flat[p] == e for p in entries[first:first + count])
         seen += entries[first:first + count]
         of.setdefault(e, []).append(count)
-    assert sorted(seen) == [p for p, e in enumerate(flat) if 0 <= e < E]
+    assert seen == sorted((p for p, e in enumerate(flat) if 0 <= e < E), key=lambda p: (flat[p], p))
     assert all(c == cols for counts in of.values() for c in counts[:-1])
     assert space.scratch.check_canaries() == []
 
@@ -57,21 +58,18 @@ def _types():
 
 
 @pytest.mark.parametrize("t", _types())
-def test_a_row_does_not_depend_on_its_job(space, t):
-    """Experts of more rows than a job: which of them fall into the short last one is a matter of chance."""
+def test_crowded_experts_repeat(space, t):
+    """Experts of more rows than a job: the same rows fall into the short last one, whose sums take another order, every time."""
     from hipengine_b200.ops import kernels as K
     counts, n, k = [33, 48, 7, 40], 160, 768
     w, _ = _weight(t, len(counts) * n, k, 3)
     ids = _ids_of_counts(counts, 1, 0)
     x = torch.randn(ids.shape[0], k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    rows = space.image(x, by_row=True, product=False)[1]
     first = None
     for i in range(20):
-        perm = torch.randperm(ids.shape[0], generator=torch.Generator().manual_seed(i)).cuda()
         out = torch.full((ids.shape[0], n), float("nan"), device="cuda")
-        jobs = space.jobs(ids[perm].contiguous(), len(counts), 32)
-        space.experts(jobs, space.image(x[perm].contiguous(), by_row=True, product=False)[1], 1, w, out, K.EPI_F32)
-        got = torch.empty_like(out)
-        got[perm] = out
-        first = got if first is None else first
-        assert torch.equal(got, first), i
+        space.experts(space.jobs(ids, len(counts), 32), rows, 1, w, out, K.EPI_F32)
+        first = out if first is None else first
+        assert torch.equal(out, first), i
     K.check_status()
