@@ -7,19 +7,24 @@
 //              sc * q an integer below 2^10 and m one below 2^6: both are exact in fp16, so ONE packed fp16 FMA makes two
 //              operands (1024 + q is the nibble under an exponent byte; (1024 + q) * sc - 1024 * sc), the 256-column block
 //              accumulates in fp32, and d / dmin come in once per block.  The minima are one more MMA against the sums of
-//              the activations per 32 columns (as an fp16 high and low part).  Q6_K: sc * (q - 32) (13 bits, rounded to 11);
-//              Q8_0: q times the sub-block scale over the block's power of two (11 bits).  The weights are thus exact or
-//              carry 11 bits (bf16 operands carried 8), at ~2 instructions per weight and lane.
-//   activations: fp16 under a power of two per row and block of 256 columns, 11 bits each (bf16 rows exactly), written once
-//              per launch by he_rows_image in the very order of the MMA's B fragments (one 16-byte load per lane feeds two
-//              MMAs), so no CTA repeats the normalisation.
-//   k order  : lane (g, t) of an MMA holds columns of ITS OWN sub-blocks -- t = (h, u) owns, in half h of the block, the 16
+//              the activations per 32 columns (as an fp16 high and low part).  Q8_0, and Q6_K up to 8 rows: the integers
+//              themselves are the operands, an MMA (two for Q8_0) covers one sub-block, and the sub-block's scale meets
+//              its fp32 sums: exact as well, and for Q8_0 cheaper than a product per operand (17408 x 5120, 4 / 16 / 32 rows
+//              24.7 / 29.0 / 47.9 -> 21.8 / 24.2 / 42.6 us; 64 rows 50.3 -> 50.9).  Q6_K above 8 rows: sc * (q - 32), 13
+//              bits, rounded to 11: the exact form costs two packed FMAs per MMA (17408 x 5120, 16 / 32 / 64 rows 27.5 / 40.7
+//              / 55.2 us against 25.3 / 35.1 / 45.1; at 8 rows 22.3 against 22.8).
+//   activations: fp16 under a power of two per row and block of 256 columns, 11 bits each down to 2^-14 of the block's largest
+//              value and 2^-25 of it below (bf16 values down to 2^-17 of it exactly), written once per launch by he_rows_image
+//              in the order of the MMA's B fragments (one 16-byte load per lane feeds two MMAs), so no CTA repeats the
+//              normalisation.
+//   k order  : lane (g, t) of an MMA with scaled operands holds columns of ITS OWN sub-blocks -- t = (h, u) owns, in half h of the block, the 16
 //              positions of half u of each of the four 32-column groups -- because that is what a 16-byte load of Q6_K
 //              low nibbles, high nibbles and Q4_K nibbles delivers; the scale is then a per-lane constant.
 //   split    : the (tile of 128 weight rows) x (block) units of all segments are dealt out as one contiguous range
 //              per SM (equal to one unit), so there is no last wave.  A tile that several CTAs share leaves fp32 partial
 //              tiles in `ws`; whoever arrives last (a counter per tile, reset by it) adds them in CTA order:
-//              bit-reproducible, and the same for any number of rows.
+//              bit-reproducible for a given number of rows.  (A row's last bits depend on that number: up to 16 rows sum a
+//              block in two chains, up to 32 two warp groups take every other block, above that neither.)
 //   roles    : one producer warp (TMA boxes of weight rows x 1 block, bulk copies of the image), one warp that signals shared
 //              tiles, 8 or 16 MMA warps.  The ring holds ~200 KB: with programmatic dependent launch the
 //              next product's weights arrive while the previous kernels drain.
@@ -86,6 +91,7 @@ template <int NT>
 __global__ void __launch_bounds__(Shape<NT>::THREADS, 1)
 rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ HeRowsArgs a) {
   using S = Shape<NT>;
+  constexpr bool SPLIT = NT <= 2;                                  // registers for more sums than that are not left
   constexpr int IMG = IMG_COL * 8 * NT, SLOT = TILE * 8 * NT;      // image bytes of a block, floats of a partial tile
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -278,10 +284,13 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
     };
     if (qtype == HE_Q4_K) {
       const uint32_t o0 = p0 + i0 * 144, o1 = p1 + i1 * 144;
-      blocks([&](uint32_t st0, uint32_t img) { block_q4k<NT, NT>(st0 + o0, st0 + o1, img, lane, mg, acc); });
+      blocks([&](uint32_t st0, uint32_t img) { block_q4k<NT, NT, SPLIT>(st0 + o0, st0 + o1, img, lane, mg, acc); });
     } else if (qtype == HE_Q6_K) {
       const uint32_t o0 = p0 + i0 * 224, o1 = p1 + i1 * 224;
-      blocks([&](uint32_t st0, uint32_t img) { block_q6k<NT, NT>(st0 + o0, st0 + o1, img, lane, mg, acc); });
+      blocks([&](uint32_t st0, uint32_t img) {
+        if constexpr (NT == 1) block_q6k_exact<NT, NT>(st0 + o0, st0 + o1, img, lane, mg, acc);
+        else block_q6k<NT, NT, SPLIT>(st0 + o0, st0 + o1, img, lane, mg, acc);
+      });
     } else {
       blocks([&](uint32_t st0, uint32_t img) { block_q80<NT, NT, HALF>(st0 + p0, i0, st0 + p1, i1, img, lane, mg, acc); });
     }

@@ -212,8 +212,11 @@ rows_experts_kernel(const __grid_constant__ ExpertMaps maps, const __grid_consta
       for (int blk = 0; blk < nb; ++blk) {
         if (wait_long(&sh->full[s], ph, abort_flag, a.status, 412)) {
           const uint32_t st = ring + (uint32_t)s * a.stage_bytes, img = st + w_bytes;
-          if (a.qtype == HE_Q4_K) block_q4k<NT, L>(st + p0 + i0 * 144, st + p1 + i1 * 144, img, lane, mg, acc);
-          else if (a.qtype == HE_Q6_K) block_q6k<NT, L>(st + p0 + i0 * 224, st + p1 + i1 * 224, img, lane, mg, acc);
+          if (a.qtype == HE_Q4_K) block_q4k<NT, L, L <= 2>(st + p0 + i0 * 144, st + p1 + i1 * 144, img, lane, mg, acc);
+          else if (a.qtype == HE_Q6_K) {      // prompts: 11 bits; the exact form takes 15-20 % longer at 32 rows a job
+            if constexpr (NT <= 2) block_q6k_exact<NT, L>(st + p0 + i0 * 224, st + p1 + i1 * 224, img, lane, mg, acc);
+            else block_q6k<NT, L, L <= 2>(st + p0 + i0 * 224, st + p1 + i1 * 224, img, lane, mg, acc);
+          }
           else block_q80<NT, L, XH>(st + p0, i0, st + p1, i1, img, lane, mg, acc);
           __syncwarp();
           if (lane == 0) sm100::mbar_arrive(&sh->empty[s]);

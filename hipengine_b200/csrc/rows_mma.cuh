@@ -8,8 +8,10 @@ namespace herows {
 
 using namespace he;
 
-// Image of one block of one activation row: 16 units [v][c] of 64 bytes (lane t's 16 bytes of two MMAs), the eight sums per
-// 32 columns in two parts, the scale, and padding that puts neighbouring rows half a bank cycle apart.
+// Image of one block of one activation row: 8 units [v][c] of 64 bytes, the eight sums per 32 columns in two parts, the
+// scale, and padding that puts neighbouring rows half a bank cycle apart.  A unit holds the quads v (columns 4 v .. + 3) of the
+// 16-column groups (h, 2 c, u) and (h, 2 c + 1, u), h and u at position (2 h + u) ^ v: lanes that read one position of four units
+// meet no bank twice either.
 constexpr int IMG_COL = 576, SX_OFF = 512, XS_OFF = 544;
 constexpr int MAX_STAGES = 8;
 constexpr int SMEM_TOTAL = 220 * 1024;
@@ -102,8 +104,9 @@ __device__ __forceinline__ uint32_t dup_byte(uint32_t w, uint32_t i) { return pr
 
 // One block (256 columns) of the 16 weight rows of a warp: `r0`, `r1` are the shared addresses of rows g and g + 8 in
 // the stage, `img` that of the block's image.  acc[nt] += the block's product in the MMA's C layout (rows g / g + 8,
-// activation rows 8 nt + 2t, + 1); only the first L groups of eight rows are computed.
-template <int NT, int L>
+// activation rows 8 nt + 2t, + 1); only the first L groups of eight rows are computed.  SPLIT: two accumulators of a block, half
+// the dependent MMAs in a row.  A row's sum is the same for every L.
+template <int NT, int L, bool SPLIT>
 __device__ __forceinline__ void block_q4k(uint32_t r0, uint32_t r1, uint32_t img, int lane, uint32_t mg,
                                           float (&acc)[NT][4]) {
   const int g = lane >> 2, t = lane & 3, h = t >> 1, u = t & 1;
@@ -116,7 +119,7 @@ __device__ __forceinline__ void block_q4k(uint32_t r0, uint32_t r1, uint32_t img
   const uint32_t scb = ((h ? mb.w : mb.y) & low_bits) | ((mb.y >> 2) & high_bits);
   const uint32_t mna = ((h ? ma.w >> 4 : ma.z) & low_bits) | ((ma.z >> 2) & high_bits);
   const uint32_t mnb = ((h ? mb.w >> 4 : mb.z) & low_bits) | ((mb.z >> 2) & high_bits);
-  float D[L][4], E[L <= 2 ? L : 1][4];      // few columns: two accumulators, half the dependent MMAs in a row
+  float D[L][4], E[SPLIT ? L : 1][4];
   const uint32_t xb = img + g * IMG_COL + t * 16;
 #pragma unroll
   for (int c = 0; c < 2; ++c) {      // chunk 2h + c: low nibbles are group 2c of the half, high nibbles group 2c + 1
@@ -133,19 +136,20 @@ __device__ __forceinline__ void block_q4k(uint32_t r0, uint32_t r1, uint32_t img
       const uint32_t l2 = h2_fma(and_or<0x000F000Fu>(a8, mg), sla, cla), l3 = h2_fma(and_or<0x000F000Fu>(b8, mg), slb, clb);
       const uint32_t u0 = h2_fma(and_or<0x00F000F0u>(a, mg), sha, cha), u1 = h2_fma(and_or<0x00F000F0u>(b, mg), shb, chb);
       const uint32_t u2 = h2_fma(and_or<0x00F000F0u>(a8, mg), sha, cha), u3 = h2_fma(and_or<0x00F000F0u>(b8, mg), shb, chb);
+      const uint32_t xv = xb ^ (v * 16);
 #pragma unroll
       for (int n = 0; n < L; ++n) {
-        const uint4 x = lds128(xb + n * 8 * IMG_COL + (v * 2 + c) * 64);
+        const uint4 x = lds128(xv + n * 8 * IMG_COL + (v * 2 + c) * 64);
         mma_from(v + c == 0, D[n], l0, l1, l2, l3, x.x, x.y);
-        mma_from(L <= 2 && v + c == 0, L <= 2 ? E[L <= 2 ? n : 0] : D[n], u0, u1, u2, u3, x.z, x.w);
+        mma_from(SPLIT && v + c == 0, SPLIT ? E[SPLIT ? n : 0] : D[n], u0, u1, u2, u3, x.z, x.w);
       }
     }
   }
-  if (L <= 2) {
+  if (SPLIT) {
 #pragma unroll
     for (int n = 0; n < L; ++n)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) D[n][i] += E[L <= 2 ? n : 0][i];
+      for (int i = 0; i < 4; ++i) D[n][i] += E[SPLIT ? n : 0][i];
   }
   // minima: slots (2t, 2t + 1) meet the high parts of the sums of sub-blocks 2t, 2t + 1, slots + 8 the low parts
   const uint32_t msel = 0x4040u | (2 * u) | ((2 * u + 1) << 8);
@@ -180,7 +184,7 @@ __device__ __forceinline__ void block_scale(uint32_t img, int t, float da, float
   }
 }
 
-template <int NT, int L>
+template <int NT, int L, bool SPLIT>
 __device__ __forceinline__ void block_q6k(uint32_t r0, uint32_t r1, uint32_t img, int lane, uint32_t mg,
                                           float (&acc)[NT][4]) {
   const int g = lane >> 2, t = lane & 3, h = t >> 1, u = t & 1;
@@ -191,7 +195,7 @@ __device__ __forceinline__ void block_q6k(uint32_t r0, uint32_t r1, uint32_t img
   // signed scales of the four groups (byte 2 qt + u), one per byte, as byte + 128
   const uint32_t ssel = u ? 0x7531u : 0x6420u;
   const uint32_t sca = prmt(sa.x, sa.y, ssel) ^ 0x80808080u, scb = prmt(sb.x, sb.y, ssel) ^ 0x80808080u;
-  float D[L][4], E[L <= 2 ? L : 1][4];      // few columns: two accumulators, half the dependent MMAs in a row
+  float D[L][4], E[SPLIT ? L : 1][4];
   const uint32_t xb = img + g * IMG_COL + t * 16;
   uint32_t fa[4], fb[4];
 #pragma unroll
@@ -236,94 +240,160 @@ __device__ __forceinline__ void block_q6k(uint32_t r0, uint32_t r1, uint32_t img
         o[2] = high(lbv[v] >> 8, hA8 << 2, fa[3]);
         o[3] = high(kbv[v] >> 8, hB8 << 2, fb[3]);
       }
+      const uint32_t xv = xb ^ (v * 16);
 #pragma unroll
       for (int n = 0; n < L; ++n) {
-        const uint4 x = lds128(xb + n * 8 * IMG_COL + (v * 2 + c) * 64);
+        const uint4 x = lds128(xv + n * 8 * IMG_COL + (v * 2 + c) * 64);
         mma_from(v + c == 0, D[n], e[0], e[1], e[2], e[3], x.x, x.y);
-        mma_from(L <= 2 && v + c == 0, L <= 2 ? E[L <= 2 ? n : 0] : D[n], o[0], o[1], o[2], o[3], x.z, x.w);
+        mma_from(SPLIT && v + c == 0, SPLIT ? E[SPLIT ? n : 0] : D[n], o[0], o[1], o[2], o[3], x.z, x.w);
       }
     }
   }
-  if (L <= 2) {
+  if (SPLIT) {
 #pragma unroll
     for (int n = 0; n < L; ++n)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) D[n][i] += E[L <= 2 ? n : 0][i];
+      for (int i = 0; i < 4; ++i) D[n][i] += E[SPLIT ? n : 0][i];
   }
   const uint32_t dwa = lds32(r0 + 208), dwb = lds32(r1 + 208);
   block_scale<NT, L>(img, t, __low2float(*reinterpret_cast<const __half2*>(&dwa)),
                   __low2float(*reinterpret_cast<const __half2*>(&dwb)), D, acc);
 }
 
-// Power of two of the largest of a Q8_0 row's eight scales, and the four scales of half h over it as fp16 pairs.
-__device__ __forceinline__ float q8_scales(const uint4& s, int h, uint32_t (&f)[4]) {
-  const uint32_t w[4] = {s.x, s.y, s.z, s.w};
-  __half2 m = __habs2(*reinterpret_cast<const __half2*>(&w[0]));
+// Byte i of w, an integer - 128 with its sign bit flipped, as a float times 1 / div (exact: 2^23 + byte).
+template <int DIV>
+__device__ __forceinline__ float byte_scale(uint32_t w, uint32_t i) {
+  const float f = __uint_as_float(prmt(w, 0x4B000000u, 0x7440u | i));
+  return DIV == 1 ? f - 8388736.f : fmaf(f, 1.f / DIV, -8388736.f / DIV);
+}
+// acc += (row g's scale, row g + 8's scale) * D, two sums an instruction
+__device__ __forceinline__ void add_scaled(float (&acc)[4], float sa, float sb, const float (&D)[4]) {
+  asm("{\n\t.reg .b64 x, y, s;\n\t"
+      "mov.b64 s, {%4, %4};\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%6, %7};\n\t"
+      "fma.rn.f32x2 x, s, y, x;\n\tmov.b64 {%0, %1}, x;\n\t"
+      "mov.b64 s, {%5, %5};\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%8, %9};\n\t"
+      "fma.rn.f32x2 x, s, y, x;\n\tmov.b64 {%2, %3}, x;\n\t}"
+      : "+f"(acc[0]), "+f"(acc[1]), "+f"(acc[2]), "+f"(acc[3])
+      : "f"(sa), "f"(sb), "f"(D[0]), "f"(D[1]), "f"(D[2]), "f"(D[3]));
+}
+
+// The same with exact weights: an MMA takes the 16 columns of one sub-block (lane t its quad t), its integers q - 32 as they are,
+// and the sub-block's scale meets the fp32 sums.
+template <int NT, int L>
+__device__ __forceinline__ void block_q6k_exact(uint32_t r0, uint32_t r1, uint32_t img, int lane, uint32_t mg,
+                                                float (&acc)[NT][4]) {
+  const int g = lane >> 2, t = lane & 3;
+  const uint4 sa = lds128(r0 + 192), sb = lds128(r1 + 192);
+  const uint32_t wa[4] = {sa.x ^ 0x80808080u, sa.y ^ 0x80808080u, sa.z ^ 0x80808080u, sa.w ^ 0x80808080u};
+  const uint32_t wb[4] = {sb.x ^ 0x80808080u, sb.y ^ 0x80808080u, sb.z ^ 0x80808080u, sb.w ^ 0x80808080u};
+  const uint32_t xb = img + g * IMG_COL + t * 128 + t * 16, q0 = r0 + 4 * t, q1 = r1 + 4 * t;
+  auto low = [mg](uint32_t l, uint32_t hs) { return h2_add(and_or<0x00300030u>(hs, and_or<0x000F000Fu>(l, mg)), M1056); };
+  auto high = [mg](uint32_t l, uint32_t hs) {       // 16 (q - 32)
+    return h2_add(and_or<0x03000300u>(hs, and_or<0x00F000F0u>(l, mg)), M1536);
+  };
+  float D[L][4];
 #pragma unroll
-  for (int i = 1; i < 4; ++i) m = __hmax2(m, __habs2(*reinterpret_cast<const __half2*>(&w[i])));
-  const uint32_t e = __float_as_uint(fmaxf(__low2float(m), __high2float(m))) & 0x7F800000u;
-  const float inv = __uint_as_float(0x7F000000u - e);
-  const uint32_t w0 = h ? s.z : s.x, w1 = h ? s.w : s.y;
-  const float2 d0 = __half22float2(*reinterpret_cast<const __half2*>(&w0));
-  const float2 d1 = __half22float2(*reinterpret_cast<const __half2*>(&w1));
-  const float d[4] = {d0.x, d0.y, d1.x, d1.y};
+  for (int n = 0; n < L; ++n) D[n][0] = D[n][1] = D[n][2] = D[n][3] = 0.f;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const __half2 p = __float2half2_rn(d[i] * inv);
-    f[i] = *reinterpret_cast<const uint32_t*>(&p);
+  for (int s = 0; s < 4; ++s) {
+    const int h = s >> 1, u = s & 1, lo = 64 * h + 16 * u, ho = 128 + 32 * h + 16 * u;
+    const uint32_t la = lds32(q0 + lo), lb = lds32(q0 + lo + 32), lh = lds32(q0 + ho);
+    const uint32_t ka = lds32(q1 + lo), kb = lds32(q1 + lo + 32), kh = lds32(q1 + ho);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      uint32_t e[4], o[4];            // groups 2c and 2c + 1
+      if (c == 0) {
+        e[0] = low(la, lh << 4);
+        e[1] = low(ka, kh << 4);
+        e[2] = low(la >> 8, lh >> 4);
+        e[3] = low(ka >> 8, kh >> 4);
+        o[0] = low(lb, lh << 2);
+        o[1] = low(kb, kh << 2);
+        o[2] = low(lb >> 8, lh >> 6);
+        o[3] = low(kb >> 8, kh >> 6);
+      } else {
+        e[0] = high(la, lh << 4);
+        e[1] = high(ka, kh << 4);
+        e[2] = high(la >> 8, lh >> 4);
+        e[3] = high(ka >> 8, kh >> 4);
+        o[0] = high(lb, lh << 2);
+        o[1] = high(kb, kh << 2);
+        o[2] = high(lb >> 8, lh >> 6);
+        o[3] = high(kb >> 8, kh >> 6);
+      }
+      constexpr int W = 16;
+      const float ea = c == 0 ? byte_scale<1>(wa[2 * h], u) : byte_scale<W>(wa[2 * h + 1], u);
+      const float eb = c == 0 ? byte_scale<1>(wb[2 * h], u) : byte_scale<W>(wb[2 * h + 1], u);
+      const float oa = c == 0 ? byte_scale<1>(wa[2 * h], 2 + u) : byte_scale<W>(wa[2 * h + 1], 2 + u);
+      const float ob = c == 0 ? byte_scale<1>(wb[2 * h], 2 + u) : byte_scale<W>(wb[2 * h + 1], 2 + u);
+#pragma unroll
+      for (int n = 0; n < L; ++n) {
+        const uint4 x = lds128((xb ^ (s * 16)) + n * 8 * IMG_COL + c * 64);
+        float P[4], R[4];
+        mma_from(true, P, e[0], e[1], e[2], e[3], x.x, x.y);
+        mma_from(true, R, o[0], o[1], o[2], o[3], x.z, x.w);
+        add_scaled(D[n], ea, eb, P);
+        add_scaled(D[n], oa, ob, R);
+      }
+    }
   }
-  return __uint_as_float(e);
+  const uint32_t dwa = lds32(r0 + 208), dwb = lds32(r1 + 208);
+  block_scale<NT, L>(img, t, __low2float(*reinterpret_cast<const __half2*>(&dwa)),
+                  __low2float(*reinterpret_cast<const __half2*>(&dwb)), D, acc);
 }
 
 // Q8_0: `p0` / `p1` are the region's planes [2][HT rows][128 bytes] (128-byte swizzle) and [HT rows][8 scales]; rows i0, i1.
+// Two MMAs take the 32 columns of one sub-block, its bytes as they are (lane t the quads 2 (t / 2), + 1 of the 16 columns
+// t % 2), and the sub-block's scale meets the fp32 sums: exact weights.
 template <int NT, int L, int HT>
 __device__ __forceinline__ void block_q80(uint32_t p0, int i0, uint32_t p1, int i1, uint32_t img, int lane,
                                           uint32_t mg, float (&acc)[NT][4]) {
-  const int g = lane >> 2, t = lane & 3, h = t >> 1, u = t & 1;
-  uint32_t fa[4], fb[4];
-  const float ea = q8_scales(lds128(p0 + 2 * HT * 128 + i0 * 16), h, fa);
-  const float eb = q8_scales(lds128(p1 + 2 * HT * 128 + i1 * 16), h, fb);
-  const uint32_t ra = p0 + h * HT * 128 + i0 * 128, rb = p1 + h * HT * 128 + i1 * 128;
-  float D[L][4], E[L <= 2 ? L : 1][4];      // few columns: two accumulators, half the dependent MMAs in a row
-  const uint32_t xb = img + g * IMG_COL + t * 16;
-  auto up = [mg](uint32_t w, uint32_t f) { return h2_mul(h2_add(and_or<0x00FF00FFu>(w, mg), M1152), f); };
+  const int g = lane >> 2, t = lane & 3, u = t & 1;
+  const uint4 sa = lds128(p0 + 2 * HT * 128 + i0 * 16), sb = lds128(p1 + 2 * HT * 128 + i1 * 16);
+  const uint32_t wa[4] = {sa.x, sa.y, sa.z, sa.w}, wb[4] = {sb.x, sb.y, sb.z, sb.w};
+  const uint32_t ra = p0 + i0 * 128 + (t >> 1) * 8, rb = p1 + i1 * 128 + (t >> 1) * 8;
+  const uint32_t xb = img + g * IMG_COL + (t >> 1) * 256 + t * 16;
+  auto up = [mg](uint32_t w) { return h2_add(and_or<0x00FF00FFu>(w, mg), M1152); };
+  float D[L][4];
 #pragma unroll
-  for (int c = 0; c < 2; ++c) {
-    uint4 a[2], b[2];
+  for (int n = 0; n < L; ++n) D[n][0] = D[n][1] = D[n][2] = D[n][3] = 0.f;
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int chunk = 2 * (2 * c + q) + u;
-      a[q] = lds128(ra + ((chunk ^ (i0 & 7)) << 4));
-      b[q] = lds128(rb + ((chunk ^ (i1 & 7)) << 4));
-    }
-    const uint32_t av[2][4] = {{a[0].x, a[0].y, a[0].z, a[0].w}, {a[1].x, a[1].y, a[1].z, a[1].w}};
-    const uint32_t bv[2][4] = {{b[0].x, b[0].y, b[0].z, b[0].w}, {b[1].x, b[1].y, b[1].z, b[1].w}};
+  for (int h = 0; h < 2; ++h)
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      uint32_t e[2][4];
+    for (int c = 0; c < 2; ++c) {
+      uint2 va[2], vb[2];             // sub-blocks 2c, 2c + 1 of the half
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
-        const uint32_t wa = av[q][v] ^ 0x80808080u, wb = bv[q][v] ^ 0x80808080u;
-        e[q][0] = up(wa, fa[2 * c + q]);
-        e[q][1] = up(wb, fb[2 * c + q]);
-        e[q][2] = up(wa >> 8, fa[2 * c + q]);
-        e[q][3] = up(wb >> 8, fb[2 * c + q]);
+        const int chunk = 2 * (2 * c + q) + u;
+        va[q] = lds64(ra + h * HT * 128 + ((chunk ^ (i0 & 7)) << 4));
+        vb[q] = lds64(rb + h * HT * 128 + ((chunk ^ (i1 & 7)) << 4));
       }
+      const float2 da = __half22float2(*reinterpret_cast<const __half2*>(&wa[2 * h + c]));
+      const float2 db = __half22float2(*reinterpret_cast<const __half2*>(&wb[2 * h + c]));
 #pragma unroll
-      for (int n = 0; n < L; ++n) {
-        const uint4 x = lds128(xb + n * 8 * IMG_COL + (v * 2 + c) * 64);
-        mma_from(v + c == 0, D[n], e[0][0], e[0][1], e[0][2], e[0][3], x.x, x.y);
-        mma_from(L <= 2 && v + c == 0, L <= 2 ? E[L <= 2 ? n : 0] : D[n], e[1][0], e[1][1], e[1][2], e[1][3], x.z, x.w);
+      for (int i = 0; i < 2; ++i) {
+        uint32_t a[2][4];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const uint32_t ka = (i ? va[q].y : va[q].x) ^ 0x80808080u, kb = (i ? vb[q].y : vb[q].x) ^ 0x80808080u;
+          a[q][0] = up(ka);
+          a[q][1] = up(kb);
+          a[q][2] = up(ka >> 8);
+          a[q][3] = up(kb >> 8);
+        }
+        const uint32_t xv = xb ^ ((2 * h ^ i) * 16);
+#pragma unroll
+        for (int n = 0; n < L; ++n) {
+          const uint4 x = lds128(xv + n * 8 * IMG_COL + i * 128 + c * 64);
+          float P[4], R[4];
+          mma_from(true, P, a[0][0], a[0][1], a[0][2], a[0][3], x.x, x.y);
+          mma_from(true, R, a[1][0], a[1][1], a[1][2], a[1][3], x.z, x.w);
+          add_scaled(D[n], da.x, db.x, P);
+          add_scaled(D[n], da.y, db.y, R);
+        }
       }
     }
-  }
-  if (L <= 2) {
-#pragma unroll
-    for (int n = 0; n < L; ++n)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) D[n][i] += E[L <= 2 ? n : 0][i];
-  }
-  block_scale<NT, L>(img, t, ea, eb, D, acc);
+  block_scale<NT, L>(img, t, 1.f, 1.f, D, acc);
 }
 
 // Bounded wait whose polls the hardware suspends for up to ~10 us each: the polling loop of a waiting warp would take
@@ -384,7 +454,7 @@ __device__ __forceinline__ void image_store(uint8_t* unit, uint8_t* also, int la
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
     __half2 p[2] = {__halves2half2(hv[4 * q], hv[4 * q + 2]), __halves2half2(hv[4 * q + 1], hv[4 * q + 3])};
-    const int at = ((v0 + q) * 2 + (qt >> 1)) * 64 + t * 16 + (qt & 1) * 8;
+    const int at = ((v0 + q) * 2 + (qt >> 1)) * 64 + (t ^ (v0 + q)) * 16 + (qt & 1) * 8;
     *reinterpret_cast<uint2*>(unit + at) = *reinterpret_cast<const uint2*>(p);
     if (also != nullptr) *reinterpret_cast<uint2*>(also + at) = *reinterpret_cast<const uint2*>(p);
   }

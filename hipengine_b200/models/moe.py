@@ -149,18 +149,19 @@ def _jobs_ok(ex, i: int, rng) -> bool:
             all(ROWS.weight_ok(x) for x in w) and w[0].qtype == w[1].qtype)
 
 
-def _job_cols(pairs: int, E: int) -> int:
+def _job_cols(pairs: int, E: int, decode: bool) -> int:
     """Rows per job: about twice what an expert gets on average (a job costs its columns' products whether they are
-    filled or not, a second job of an expert costs its weights again)."""
+    filled or not, a second job of an expert costs its weights again).  Decode batches keep to jobs of 16 rows, whose Q6_K
+    weights enter exactly, as in the selected-expert GEMV that smaller batches take."""
     per = pairs / E
-    return 8 if per <= 4 else 16 if per <= 8 else 32
+    return 8 if per <= 4 else 16 if per <= 8 or decode else 32
 
 
 def _expert_jobs(ex, i: int, ids: torch.Tensor, by_row: torch.Tensor, k: int, act: torch.Tensor, dtype) -> torch.Tensor:
     """Rows of the pairs after their experts [T * k, hidden], from the token rows' image; ``act``: bf16 [T * k, expert width]."""
     cfg, sc = ex.cfg, ex.scratch
     P = ids.numel()
-    jobs = ex.rows.jobs(ids, cfg.n_experts, _job_cols(P, cfg.n_experts))
+    jobs = ex.rows.jobs(ids, cfg.n_experts, _job_cols(P, cfg.n_experts, decode=dtype == torch.float32))
     epi = K.EPI_SILU_MUL if cfg.act == "silu" else K.EPI_GELU_MUL
     ex.rows.experts(jobs, by_row, k, ex.W(i, "ffn_gate_exps.weight"), act, epi, ex.W(i, "ffn_up_exps.weight"))
     _, act_rows = ex.rows.image(act[:P], by_row=True, product=False)

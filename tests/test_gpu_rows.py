@@ -24,8 +24,8 @@ def space():
 
 
 # fp32 rows round to 11 bits: at most 2^-11 of each value, so at most that of the result where the signs are random (2.1e-4 on
-# average for normal rows); Q6_K and Q8_0 operands round to 11 bits once more: sqrt(2) of it.  Q4_K operands and bf16 rows are exact
-BOUND = {T.Q4_K: 2 ** -11, T.Q6_K: 2 ** -10.5, T.Q8_0: 2 ** -10.5}
+# average for normal rows).  The weights are exact, but for Q6_K above eight rows: rounded to 11 bits as well, sqrt(2) of it
+BOUND = {T.Q4_K: 2 ** -11, T.Q6_K: 2 ** -10.5, T.Q8_0: 2 ** -11}
 
 
 @pytest.mark.parametrize("t", [T.Q4_K, T.Q6_K, T.Q8_0])
@@ -50,6 +50,26 @@ def test_products_match_64_bit(space, t, n, k):
         assert torch.equal(out, again)
     K.check_status()
     assert int(space.counters.abs().sum()) == 0 and space.scratch.check_canaries() == []
+
+
+@pytest.mark.parametrize("t", [T.Q4_K, T.Q6_K, T.Q8_0])
+@pytest.mark.parametrize("R", [1, 8, 9, 24, 40, 64])
+def test_weights_enter_exactly(space, t, R):
+    """Rows that their image holds exactly: what is left is the rounding of fp32 sums.  Scales from the type's largest to its
+    smallest within a block."""
+    from hipengine_b200.ops import kernels as K
+    n, k = 200, 1280
+    g = torch.Generator(device="cuda").manual_seed(R)
+    wf = torch.randn(n, k // 16, 16, generator=g, device="cuda") * 10 ** (-4 * torch.rand(n, k // 16, 1, generator=g, device="cuda"))
+    raw = Q.quantize(wf.reshape(n, k), t)
+    w, wd = K.to_device_weight(raw, t, n, k), Q.dequantize_torch(raw, t, n, k).double()
+    x = torch.randint(-31, 32, (R, k), generator=g, device="cuda").float()
+    out = torch.zeros(R, n, device="cuda")
+    space.gemm(x, [K.GemvSegment(w, out)])
+    ref = x.double() @ wd.t()
+    # 1280 terms in fp32: sqrt(1280) 2^-24 of the terms' norm; above eight rows Q6_K operands round to 11 bits
+    assert float((out.double() - ref).norm() / ref.norm()) < (2 ** -11 if t == T.Q6_K and R > 8 else 36 * 2 ** -24)
+    K.check_status()
 
 
 def test_a_row_does_not_depend_on_its_neighbours(space):
