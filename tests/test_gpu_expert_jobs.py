@@ -73,3 +73,57 @@ def test_crowded_experts_repeat(space, t):
         first = out if first is None else first
         assert torch.equal(out, first), i
     K.check_status()
+
+
+@pytest.mark.parametrize("t", _types())
+@pytest.mark.parametrize("cols,n", [(8, 96), (16, 130), (32, 300), (8, 512)])
+def test_products_of_jobs_match_64_bit(space, t, cols, n):
+    """Experts of no row, one, a job's worth, one more and several jobs; tiles that end inside an expert's rows (the box reaches
+    into the next expert); token rows that two pairs share and rows of their own; rows that the image holds exactly."""
+    from hipengine_b200.ops import kernels as K
+    counts, k = [0, 1, cols, cols + 1, 3 * cols + 4], 768
+    E = len(counts)
+    (a, ad), (b, bd) = _weight(t, E * n, k, n), _weight(t, E * n, k, n + 1)
+    ids = _ids_of_counts(counts, 2, cols)
+    P = ids.numel()
+    jobs = space.jobs(ids, E, cols)
+    e = ids.view(-1).long()
+    ad, bd = ad.reshape(E, n, k)[e], bd.reshape(E, n, k)[e]
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    rel = lambda y, r: float((y.double() - r).norm(dim=1).div(r.norm(dim=1)).max())
+    x = torch.randint(-31, 32, (P // 2, k), generator=g, device="cuda").float() / 16
+    img = space.image(x, by_row=True, product=False)[1]
+    up = lambda m: torch.einsum("pk,pnk->pn", x.double()[torch.arange(P, device="cuda") // 2], m)
+    for epi, f in ((K.EPI_SILU_MUL, torch.nn.functional.silu), (K.EPI_GELU_MUL, lambda v: torch.nn.functional.gelu(v, approximate="tanh"))):
+        act = torch.full((P + 1, n + 8), 7.0, device="cuda", dtype=torch.bfloat16)
+        space.experts(jobs, img, 2, a, act[:P, :n], epi, b)
+        assert rel(act[:P, :n], f(up(ad)) * up(bd)) < 4e-3                       # bf16 result
+        assert bool((act[P] == 7).all()) and bool((act[:, n:] == 7).all())
+    rows = torch.randint(-31, 32, (P, k), generator=g, device="cuda").bfloat16()
+    img = space.image(rows, by_row=True, product=False)[1]
+    want = torch.einsum("pk,pnk->pn", rows.double(), ad)
+    out = torch.full((P + 1, n + 4), 7.0, device="cuda")
+    space.experts(jobs, img, 1, a, out[:P, :n], K.EPI_F32)
+    # fp32 sums of 768 terms; Q6_K operands of 32-row jobs round to 11 bits
+    assert rel(out[:P, :n], want) < (2 ** -11 if t == _types()[1] and cols == 32 else 28 * 2 ** -24)
+    assert bool((out[P] == 7).all()) and bool((out[:, n:] == 7).all())
+    half = torch.zeros(P, n, device="cuda", dtype=torch.bfloat16)
+    space.experts(jobs, img, 1, a, half, K.EPI_BF16)
+    assert torch.equal(half, out[:P, :n].bfloat16())
+    K.check_status()
+    assert space.scratch.check_canaries() == []
+
+
+@pytest.mark.parametrize("T,k,n", [(1, 1, 4), (3, 8, 1028), (70, 2, 256)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_sum_of_pairs(space, T, k, n, dtype):
+    g = torch.Generator(device="cuda").manual_seed(n)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    h, y, w = rand(T, n + 4)[:, :n], rand(T * k, n).to(dtype), torch.rand(T, k, generator=g, device="cuda")
+    sh, gate = rand(T, n).bfloat16(), rand(T, 3)
+    want = h.double() + (w.double()[..., None] * y.double().reshape(T, k, n)).sum(1)
+    for shared in (False, True):
+        got = h.clone()
+        space.sum_pairs(got, y, w, sh if shared else None, gate[:, 1:2] if shared else None)
+        ref = want + torch.sigmoid(gate[:, 1:2].double()) * sh.double() if shared else want
+        assert float((got.double() - ref).abs().max()) < 1e-5                    # fp32 sums of at most ten terms below 30
