@@ -107,6 +107,8 @@ class GpuRunner(BaseRunner):
                                                    draft_model=config.speculative.draft_model),
                 max_requests=min(self.max_slots, 8))
         self.supports_mtp = self.mtp is not None
+        if self.mtp is not None:
+            self.graphs.beside_verifier()
         self.spec_uses_history = self.mtp is not None and hasattr(self.mtp, "drafter")
         # hot-vocabulary draft head: per-request rule over the request's own committed tokens decides, cycle by
         # cycle, whether the NextN draft may score only the leading slice of the head

@@ -19,7 +19,7 @@ import torch
 
 from ..core import native as N
 from ..ops import kernels as K
-from .executor import GEMV_MAX_ROWS, BatchDesc, HybridExecutor
+from .executor import GEMV_MAX_ROWS, GEMV_ROWS, BatchDesc, HybridExecutor
 
 CTX_BUCKETS = (1024, 4096, 8192, 16384, 32768, 65536, 131072, 262144)
 
@@ -54,7 +54,14 @@ class DecodeGraphRunner:
         # replay through the native launcher (validated control block + cudaGraphLaunch) when torch exposes the
         # instantiated graph; otherwise through torch's own replay
         self.native_launch = os.environ.get("HE_NATIVE_GRAPH_LAUNCH", "1") != "0"
+        # rows up to which these steps keep the numerics of verify chains (the int8 GEMV).  Whoever runs plain steps beside a
+        # verifier sets it before the first step (``beside_verifier``): both then choose the same tokens
+        self.gemv_rows = 0
         self._execs: Dict[Tuple[int, int, bool], int] = {}
+
+    def beside_verifier(self) -> None:
+        assert not self.graphs, "captured steps keep the numerics that they were captured with"
+        self.gemv_rows = min(GEMV_ROWS, int(os.environ.get("HE_SMALL_ROWS", GEMV_ROWS)))
 
     def batch(self, rows: int, max_ctx: int) -> BatchDesc:
         return BatchDesc(self.tokens[:rows], self.slot[:rows], self.pos[:rows], self.ctx_len[:rows],
@@ -73,13 +80,14 @@ class DecodeGraphRunner:
     def _step_body(self, rows: int, max_ctx: int, greedy: bool) -> None:
         ex = self.ex
         b = self.batch(rows, max_ctx)
-        h = ex.forward(b, defer_resid=True)
-        hid = self.hidden[:rows] if ex.keeps_hidden else None
-        if greedy:
-            ex.head_greedy(h, self.next_ids[:rows], logits_out=self.logits[:rows], hidden_out=hid)
-            self.publish(rows)
-        else:
-            ex.logits(h, out=self.logits[:rows], hidden_out=hid)
+        with ex.gemv_numerics(rows, self.gemv_rows):
+            h = ex.forward(b, defer_resid=True)
+            hid = self.hidden[:rows] if ex.keeps_hidden else None
+            if greedy:
+                ex.head_greedy(h, self.next_ids[:rows], logits_out=self.logits[:rows], hidden_out=hid)
+                self.publish(rows)
+            else:
+                ex.logits(h, out=self.logits[:rows], hidden_out=hid)
 
     def publish(self, rows: int) -> None:
         """next_ids -> tokens, advance positions (device side)."""

@@ -218,12 +218,13 @@ class HybridExecutor:
         return self.rows is not None and self.small_rows < rows <= ROWS.MAX_ROWS
 
     @contextlib.contextmanager
-    def gemv_numerics(self, rows: int):
+    def gemv_numerics(self, rows: int, limit: int = GEMV_MAX_ROWS):
         """A verify chain of up to 8 rows must see the numerics of a plain single-row step (the int8 GEMV), or a near-tie
-        could make the verifier disagree with what autoregressive decoding would have produced."""
+        could make the verifier disagree with what autoregressive decoding would have produced.  ``limit``: rows up to which
+        the batch is held to it."""
         saved = self.small_rows
-        if rows <= GEMV_MAX_ROWS:
-            self.small_rows = GEMV_MAX_ROWS
+        if rows <= limit:
+            self.small_rows = max(saved, limit)
         try:
             yield
         finally:

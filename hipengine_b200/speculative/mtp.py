@@ -13,12 +13,11 @@ Stages are recorded through ``SpecTransaction``.  Reference flow: ``hipengine/ru
 """
 from __future__ import annotations
 
-import os
 from typing import List, Optional, Sequence, Tuple
 
 import torch
 
-from ..models.executor import GEMV_MAX_ROWS, GEMV_ROWS, BatchDesc, make_batch
+from ..models.executor import GEMV_MAX_ROWS, BatchDesc, make_batch
 from ..ops import kernels as K
 from .contracts import SpecCycleResult, SpeculativeCapability
 from .transaction import SpecTransaction, Stage
@@ -31,9 +30,6 @@ class ChainVerifyCycle:
 
     def __init__(self, ex, max_depth: int = 3, max_requests: int = 8):
         self.ex = ex
-        # beside a verifier the plain steps of the smallest batches keep its numerics (the int8 GEMV): both then choose the
-        # same tokens
-        ex.small_rows = max(ex.small_rows, min(GEMV_ROWS, int(os.environ.get("HE_SMALL_ROWS", GEMV_ROWS))))
         self.max_depth = max_depth
         self.max_requests = max_requests
         dev = ex.device

@@ -214,6 +214,32 @@ def test_hot_vocab_draft_head_scores_a_row_prefix_and_keeps_greedy_output(graphe
         assert mtp.graph_stats["captures"] == 2 and mtp.graph_stats["eager"] == 0
 
 
+def test_a_verifier_leaves_other_steps_of_its_executor_alone():
+    """Making one changes nothing for the executor; steps that are declared to run beside one keep the GEMV's numerics."""
+    from hipengine_b200.models.decode_graph import DecodeGraphRunner
+    from hipengine_b200.models.executor import HybridExecutor
+    from hipengine_b200.speculative.mtp import ChainVerifyCycle
+    w = build_random_model(TINY_HYBRID, seed=0, std=0.05).to("cuda")
+    ex = HybridExecutor(w, max_slots=4, max_context=256)
+    ex.small_rows = 2                          # as for a wide model
+    assert ex.few(4)
+    ChainVerifyCycle(ex, max_depth=3, max_requests=1)
+    assert ex.small_rows == 2 and ex.few(4)
+    logits = {}
+    for name, small, beside in (("few", 2, False), ("gemv", 5, False), ("beside", 2, True)):
+        ex.small_rows = small
+        for s in range(4):
+            ex.reset_slot(s)
+        run = DecodeGraphRunner(ex, max_rows=4)
+        if beside:
+            run.beside_verifier()
+        run.set_rows(range(4), [3, 5, 7, 9], [0] * 4)
+        run.step(4, 16, greedy=False)
+        logits[name] = run.logits.clone()
+        assert ex.small_rows == small
+    assert torch.equal(logits["beside"], logits["gemv"]) and not torch.equal(logits["beside"], logits["few"])
+
+
 def test_lookup_cycle_with_known_chains_needs_no_nextn_block():
     """Chain verify with host-supplied drafts on a checkpoint WITHOUT a NextN block: the true greedy continuation is
     accepted in full (plus the bonus token), a corrupted chain is cut at the first wrong token, and the committed
