@@ -518,14 +518,9 @@ int launch_rows(HeRowsArgs a, int num_sms, cudaStream_t stream) {
   if (S::GROUPS == 2) a.stages &= ~1;
   if (a.stages < 2) return -HE_ERR_BAD_ARG;
   const size_t smem = (size_t)a.stages * a.stage_bytes + S::XBUF + sizeof(RowsShared) + 1024;
-  static size_t configured[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
-  if (smem > configured[dev]) {
-    const cudaError_t e = cudaFuncSetAttribute(rows_gemm_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    configured[dev] = smem;
-  }
+  static std::atomic<unsigned long long> allowed{0};
+  const cudaError_t e = allow_smem(rows_gemm_kernel<NT>, SMEM_TOTAL, allowed);
+  if (e != cudaSuccess) return (int)e;
   const long long units = (long long)a.tiles * (a.K >> 8);
   const int grid = (int)(units < num_sms ? units : num_sms);
   if (2ll * grid * TILE * 8 * NT > a.ws_floats || a.tiles > a.n_counters) return -HE_ERR_BAD_ARG;
@@ -561,15 +556,11 @@ HE_API int he_rows_image(const void* x, int x_dtype, long long x_stride, const f
     if (norm_w == nullptr || side_w == nullptr || side_out == nullptr || (reinterpret_cast<uintptr_t>(side_w) & 15) != 0)
       return -HE_ERR_BAD_ARG;
     smem = (size_t)2 * K * sizeof(float);
-    if (smem > 200 * 1024) return -HE_ERR_BAD_ARG;
-    static size_t configured[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
-    if (smem > 40 * 1024 && smem > configured[dev]) {
-      const cudaError_t e = cudaFuncSetAttribute(rows_image_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return (int)e;
-      configured[dev] = smem;
-    }
+    constexpr int most = 200 * 1024;
+    if (smem > most) return -HE_ERR_BAD_ARG;
+    static std::atomic<unsigned long long> allowed{0};
+    const cudaError_t e = allow_smem(rows_image_kernel, most, allowed);
+    if (e != cudaSuccess) return (int)e;
   }
   const int parts = norm_w != nullptr ? 1 : (nb + 3) / 4;
   const unsigned grid = (unsigned)(R * parts + (side_n > 0 ? (side_n + 1) / 2 : 0));

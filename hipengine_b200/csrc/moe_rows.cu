@@ -307,15 +307,11 @@ int launch_experts(const ExpertMaps& maps, RowsExpertsArgs a, int num_sms, cudaS
   if (a.stages > MAX_STAGES) a.stages = MAX_STAGES;
   if (a.stages < 2) return -HE_ERR_BAD_ARG;
   const size_t smem = (size_t)a.stages * a.stage_bytes + sizeof(ExpertShared) + 1024;
-  static size_t configured[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
-  if (smem > configured[dev]) {
-    if (!registers_ok(rows_experts_kernel<NT>)) return -HE_ERR_BAD_ARG;
-    const cudaError_t e = cudaFuncSetAttribute(rows_experts_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    configured[dev] = smem;
-  }
+  static const bool ok = registers_ok(rows_experts_kernel<NT>);
+  if (!ok) return -HE_ERR_BAD_ARG;
+  static std::atomic<unsigned long long> allowed{0};
+  const cudaError_t e = allow_smem(rows_experts_kernel<NT>, SMEM_TOTAL, allowed);
+  if (e != cudaSuccess) return (int)e;
   return (int)launch_pdl(rows_experts_kernel<NT>, dim3(num_sms), dim3(XTHREADS), smem, stream, maps, a);
 }
 

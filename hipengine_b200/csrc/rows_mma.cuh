@@ -1,6 +1,8 @@
 // Operands and host helpers of the few-row products (gemm_rows.cu, moe_rows.cu): quantised weight blocks as fp16 MMA
 // operands, the activation image, waits, tensor maps of weight rows.  See gemm_rows.cu for the method.
 #pragma once
+#include <atomic>
+
 #include "common.cuh"
 #include "sm100.cuh"
 
@@ -505,6 +507,20 @@ inline EncodeTiledFn encode_fn() {
     return nullptr;
   }();
   return fn;
+}
+
+// Dynamic shared memory that a kernel may ask for, set once per device.  `bytes` is the kernel's largest need, the same in every
+// call: threads that set it at the same time agree, and none takes back what another one's launch relies on.
+template <typename F>
+inline cudaError_t allow_smem(F kernel, int bytes, std::atomic<unsigned long long>& devices) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
+  if (e == cudaSuccess && (devices.load(std::memory_order_acquire) & bit) == 0) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) devices.fetch_or(bit, std::memory_order_release);
+  }
+  return e;
 }
 
 // Weight rows as bytes: [rows][row_bytes], box {box_bytes, box_rows}

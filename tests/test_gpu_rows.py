@@ -134,3 +134,53 @@ def test_refusals(space):
         space.gemm(torch.zeros(65, 512, device="cuda"), [K.GemvSegment(w, torch.zeros(65, 128, device="cuda"))])
     with pytest.raises(RuntimeError):
         space.image(torch.zeros(2, 516, device="cuda")[:, 2:514])         # rows that are not 16-byte aligned
+
+
+FIRST_LAUNCHES = """
+import sys, threading
+sys.path.insert(0, %r)
+import torch
+from hipengine_b200.models.executor import _Scratch
+from hipengine_b200.ops import kernels as K
+from hipengine_b200.ops.rows import RowsSpace
+from hipengine_b200.quant import ggml as Q
+dev = torch.device("cuda", 0)
+T, k, bad = Q.GGMLType, 1024, []
+raw = {t: Q.quantize(torch.randn(200, k, device=dev), t) for t in (T.Q4_K, T.Q6_K, T.Q8_0)}
+w = {t: (K.to_device_weight(r, t, 200, k), Q.dequantize_torch(r, t, 200, k).double()) for t, r in raw.items()}
+x = torch.randint(-9, 9, (24, k), device=dev).float()
+side = torch.randn(8, k, device=dev)
+torch.cuda.synchronize()
+gate = threading.Barrier(9)
+def run(i):
+    t = list(w)[i %% 3]
+    space = RowsSpace(_Scratch(dev), dev, 256)
+    out, so = torch.zeros(24, 200, device=dev), torch.zeros(24, 8, device=dev)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        torch.cuda.synchronize()
+        gate.wait()
+        for _ in range(5):
+            img, _ = space.image(x, torch.ones(k, device=dev), 1e-6, side, so)
+            space.product(img, 24, k, [K.GemvSegment(w[t][0], out)])
+    torch.cuda.synchronize()
+    xn = x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-6)
+    ref = xn @ w[t][1].t()
+    if not float((out.double() - ref).norm() / ref.norm()) < 2 ** -10:
+        bad.append((i, float((out.double() - ref).norm() / ref.norm())))
+threads = [threading.Thread(target=run, args=(i,)) for i in range(9)]
+[t.start() for t in threads]
+[t.join(120) for t in threads]
+K.check_status()
+print("bad", bad, "alive", sum(t.is_alive() for t in threads))
+"""
+
+
+def test_first_launches_from_several_threads():
+    """The shared memory that the kernels ask for depends on the block type; the first launches of a process, from nine threads
+    with streams of their own, do not take it from one another."""
+    import subprocess
+    import sys
+    from pathlib import Path
+    r = subprocess.run([sys.executable, "-c", FIRST_LAUNCHES % str(Path(__file__).resolve().parent.parent)], capture_output=True,
+                       text=True, timeout=300)
+    assert r.returncode == 0 and "bad [] alive 0" in r.stdout and "Error" not in r.stderr, (r.stdout, r.stderr[-2000:])
