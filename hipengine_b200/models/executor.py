@@ -204,9 +204,9 @@ class HybridExecutor:
             if pair[0] in ws and ws[pair[0]].qtype != ws[pair[1]].qtype:
                 return None
             used += ws.values()
-            if not full and f"blk.{i}.ssm_alpha.weight" not in self.f32:
+            if not full and not all(f"blk.{i}.ssm_{n}.weight" in self.f32 for n in ("alpha", "beta")):
                 return None
-        if not all(ROWS.weight_ok(w) for w in used):
+        if not all(ROWS.weight_ok(w) for w in used) or cfg.hidden > ROWS.SIDE_MAX_COLS:
             return None
         # the gates of the delta rule stay fp32: they ride with the rows' image (one matrix, alpha rows then beta rows)
         self.ab_f32 = {i: torch.cat([self.F(i, "ssm_alpha.weight"), self.F(i, "ssm_beta.weight")], 0).contiguous()

@@ -16,6 +16,7 @@ MAX_SEGMENTS = 4
 QTYPES = (8, 12, 14)         # Q8_0, Q4_K, Q6_K
 HALF_TILE = 64               # smallest tile: weight rows of each weight of a gate/up pair
 IMAGE_UNIT = 576             # image bytes of 256 columns of a row
+SIDE_MAX_COLS = 25600        # widest rows that products with fp32 side weights take: two of those in shared memory
 
 
 class _Seg(C.Structure):

@@ -134,6 +134,15 @@ def test_refusals(space):
         space.gemm(torch.zeros(65, 512, device="cuda"), [K.GemvSegment(w, torch.zeros(65, 128, device="cuda"))])
     with pytest.raises(RuntimeError):
         space.image(torch.zeros(2, 516, device="cuda")[:, 2:514])         # rows that are not 16-byte aligned
+    from hipengine_b200.ops.rows import SIDE_MAX_COLS
+    for k in (SIDE_MAX_COLS, SIDE_MAX_COLS + 256):
+        z = torch.zeros(2, k, device="cuda")
+        side = lambda: space.image(z[:1], torch.ones(k, device="cuda"), 1e-6, z, torch.zeros(1, 2, device="cuda"))
+        if k == SIDE_MAX_COLS:
+            side()
+        else:
+            with pytest.raises(RuntimeError):
+                side()
 
 
 FIRST_LAUNCHES = """
@@ -184,3 +193,26 @@ def test_first_launches_from_several_threads():
     r = subprocess.run([sys.executable, "-c", FIRST_LAUNCHES % str(Path(__file__).resolve().parent.parent)], capture_output=True,
                        text=True, timeout=300)
     assert r.returncode == 0 and "bad [] alive 0" in r.stdout and "Error" not in r.stderr, (r.stdout, r.stderr[-2000:])
+
+
+def test_models_that_the_products_cannot_take_keep_the_other_routes(monkeypatch):
+    """Rows too wide for the fp32 side products, gates of which one is quantised: the executor does without."""
+    from hipengine_b200.loading.synth import build_random_model
+    from hipengine_b200.loading.weights import QTensor
+    from hipengine_b200.models.config import TINY_HYBRID
+    from hipengine_b200.models.executor import HybridExecutor
+    from hipengine_b200.ops import rows as ROWS
+    w = build_random_model(TINY_HYBRID, seed=0, std=0.05).to("cuda")
+    toks = list(range(1, 13))
+    build = lambda: HybridExecutor(w, device="cuda", max_slots=1, max_context=64)
+    assert build().rows is not None
+    with monkeypatch.context() as m:
+        m.setattr(ROWS, "SIDE_MAX_COLS", TINY_HYBRID.hidden - 1)
+        ex = build()
+    assert ex.rows is None and bool(ex.prefill(0, toks).isfinite().all())
+    name = next(n for n in w.tensors if n.endswith("ssm_beta.weight"))
+    t = w.tensors[name]
+    n, k = t.shape
+    w.tensors[name] = QTensor(name, T.Q8_0, t.shape, Q.quantize(t.float(), T.Q8_0).reshape(n, -1))
+    ex = build()
+    assert ex.rows is None
