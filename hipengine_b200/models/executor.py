@@ -167,6 +167,8 @@ class HybridExecutor:
         self.scratch = _Scratch(self.device)
         self.dw: Dict[str, DeviceWeight] = {}
         self.f32: Dict[str, torch.Tensor] = {}
+        self.ab_bf16: Dict[int, torch.Tensor] = {}     # gates of the delta rule, [alpha rows | beta rows], for prompts ...
+        self.ab_q8: Dict[int, DeviceWeight] = {}       # ... and for decode without the few-row products
         # per-stage device timing of the tensor-core (many rows) path, off unless HE_STAGE_TIMING=1 (the role of the
         # reference's stage timers, hipengine/runtime/qwen35_gguf_timing.py:1-80): CUDA events around each stage,
         # read back once by stage_summary()
@@ -181,6 +183,8 @@ class HybridExecutor:
         # less for each norm, and without few-row products the choice is the tensor-core GEMM: five rows (a packed step
         # of the 27B with 5 / 6 rows costs 11.7 / 14.0 ms on the GEMV, 13.3 / 13.6 ms on the tensor cores).
         self.rows = self._make_rows()
+        if self.rows is None:
+            self._quantise_gates()
         self.small_rows = min(GEMV_MAX_ROWS, int(os.environ.get(
             "HE_SMALL_ROWS", GEMV_ROWS if self.rows is None or self.cfg.hidden < FEW_MIN_WIDTH else 2)))
 
@@ -248,11 +252,6 @@ class HybridExecutor:
         if "output.weight" not in self.dw:
             self.dw["output.weight"] = self.dw["token_embd.weight"]
         # prefill path: the two small F32 gate projections of a linear layer run as one bf16 tensor-core GEMM
-        # ... and for decode they ride the int8 block path of the fused GEMV as one Q8_0 segment: as fp32 rows each
-        # was a 20 KB dot product walked by a single warp, a latency-bound tail twice as long as the rest of the launch
-        self.ab_bf16: Dict[int, torch.Tensor] = {}
-        self.ab_q8: Dict[int, DeviceWeight] = {}
-        from ..quant.ggml import quantize
         for i in range(self.cfg.n_layers):
             a_name, b_name = f"blk.{i}.ssm_alpha.weight", f"blk.{i}.ssm_beta.weight"
             if a_name in self.f32 and b_name in self.f32:
@@ -263,9 +262,17 @@ class HybridExecutor:
                 pad = (-ab.shape[0]) % 8
                 abp = torch.cat([ab, ab.new_zeros(pad, ab.shape[1])], 0) if pad else ab
                 self.ab_bf16[i] = abp.to(torch.bfloat16).contiguous()
-                if ab.shape[1] % 256 == 0 and os.environ.get("HE_AB_Q8", "1") != "0":
-                    raw = quantize(ab, GGMLType.Q8_0).reshape(ab.shape[0], -1).contiguous()
-                    self.ab_q8[i] = K.to_device_weight(raw, GGMLType.Q8_0, ab.shape[0], ab.shape[1])
+
+    def _quantise_gates(self) -> None:
+        """Decode without the few-row products: the two gate projections ride the int8 block path of the fused GEMV as one
+        Q8_0 segment (as fp32 rows each was a 20 KB dot product walked by a single warp, a latency-bound tail twice as long
+        as the rest of the launch)."""
+        from ..quant.ggml import quantize
+        for i in self.ab_bf16:
+            ab = torch.cat([self.F(i, "ssm_alpha.weight"), self.F(i, "ssm_beta.weight")], 0)
+            if ab.shape[1] % 256 == 0 and os.environ.get("HE_AB_Q8", "1") != "0":
+                raw = quantize(ab, GGMLType.Q8_0).reshape(ab.shape[0], -1).contiguous()
+                self.ab_q8[i] = K.to_device_weight(raw, GGMLType.Q8_0, ab.shape[0], ab.shape[1])
 
     def _stage(self, name: str):
         """Context manager timing one stage (a no-op when timing is off or the stream is being captured)."""

@@ -55,7 +55,8 @@ class _MoeLayer:
         pad = (-full.shape[0]) % 8
         if pad:
             full = torch.cat([full, torch.zeros(pad, full.shape[1], device=full.device)], 0)
-        self.full = full[:E + (1 if self.has_shared else 0)].contiguous()     # fp32 rows: experts, then the shared gate
+        # fp32 rows for the few-row products: experts, then the shared gate
+        self.full = None if ex.rows is None else full[:E + (1 if self.has_shared else 0)].contiguous()
         # fp32 router weights as two bf16 GEMM operands: hi + lo reproduces ~16 mantissa bits
         self.r_hi = full.to(torch.bfloat16).contiguous()
         self.r_lo = (full - self.r_hi.float()).to(torch.bfloat16).contiguous()

@@ -205,11 +205,12 @@ def test_models_that_the_products_cannot_take_keep_the_other_routes(monkeypatch)
     w = build_random_model(TINY_HYBRID, seed=0, std=0.05).to("cuda")
     toks = list(range(1, 13))
     build = lambda: HybridExecutor(w, device="cuda", max_slots=1, max_context=64)
-    assert build().rows is not None
+    ex = build()
+    assert ex.rows is not None and not ex.ab_q8          # one form of the gates, the one that is used
     with monkeypatch.context() as m:
         m.setattr(ROWS, "SIDE_MAX_COLS", TINY_HYBRID.hidden - 1)
         ex = build()
-    assert ex.rows is None and bool(ex.prefill(0, toks).isfinite().all())
+    assert ex.rows is None and ex.ab_q8 and bool(ex.prefill(0, toks).isfinite().all())
     name = next(n for n in w.tensors if n.endswith("ssm_beta.weight"))
     t = w.tensors[name]
     n, k = t.shape
