@@ -161,3 +161,30 @@ def test_projection_rows_match_the_per_head_kernel(dtype, gated, rope, qk_norm):
         res.append((qo, go, kv))
     for a, b in zip(*res):
         assert torch.allclose(a.float(), b.float(), rtol=8e-3, atol=1e-5)      # one bf16 rounding apart at most
+
+
+@pytest.mark.parametrize("K", [256, 5120, 6144, 6148, 9000])
+def test_single_row_gates_in_the_decode_step(K):
+    """Gates from the residual row inside the step against gates given to it: fewer columns than threads, all that a thread keeps
+    in registers (6144), and what it loads in place beyond."""
+    from hipengine_b200.ops import kernels as Kn
+    G, Hv, S = 2, 6, 128
+    C = 2 * G * S + Hv * S
+    g = torch.Generator(device="cuda").manual_seed(K)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    h, norm, gw = 3 * rand(1, K), rand(K).abs() + 0.5, rand(2 * Hv, K) * K ** -0.5
+    xn = h.double() * torch.rsqrt(h.double().square().mean(-1, keepdim=True) + 1e-6) * norm.double()
+    ab = (xn @ gw.double().t()).float()
+    x, w, z = rand(1, C), rand(C, 4) * 0.5, rand(1, Hv * S)
+    ssm_a, dt, nw, slot = -rand(Hv).abs(), rand(Hv), rand(S).abs(), torch.tensor([1], dtype=torch.int32, device="cuda")
+    conv0, state0 = rand(2, C, 3), rand(2, Hv, S, S) * 0.1
+    res = []
+    for gates in (None, (gw, h, norm, 1e-6)):
+        conv, state = conv0.clone(), state0.clone()
+        qkv, decay, beta = torch.zeros(1, C, device="cuda"), torch.zeros(1, Hv, device="cuda"), torch.zeros(1, Hv, device="cuda")
+        out = torch.zeros(1, Hv * S, device="cuda", dtype=torch.bfloat16)
+        a, b = (ab[:, :Hv], ab[:, Hv:]) if gates is None else (None, None)
+        Kn.gdn_decode(x, w, conv, a, b, ssm_a, dt, slot, qkv, decay, beta, state, z, nw, out, G, Hv, 1e-6, gates)
+        res.append((decay, beta, state, conv, out.float()))
+    for got, want, tol in zip(res[1], res[0], (1e-5, 1e-5, 1e-5, 0, 8e-3)):       # fp32 sums; the output is bf16
+        assert torch.allclose(got, want, rtol=tol, atol=tol)
