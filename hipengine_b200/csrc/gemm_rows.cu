@@ -537,14 +537,15 @@ HE_API long long he_rows_ws_floats(int R, int num_sms) {
 }
 
 // Images of (RMSNorm with norm_w of) the R rows x[r][0..K), fp32 or bf16.  K % 256 == 0, 16-byte rows.  `image` (may be
-// null): block by block, for a product of 1..64 rows; `by_row` (may be null): row by row, for he_rows_experts, any R.
+// null): block by block, for a product of 1..64 rows; `by_row` (may be null): row by row, for he_rows_experts, any R; both null:
+// the side rows alone.
 // With `side_n` > 0 (at most 64 rows) also side_out[r][j] = (normalised row r) . side_w[j], j < side_n: fp32 weights
 // [side_n][K], in fp32.
 HE_API int he_rows_image(const void* x, int x_dtype, long long x_stride, const float* norm_w, float eps, int K, int R,
                          void* image, void* by_row, const float* side_w, int side_n, float* side_out, long long side_ld,
                          cudaStream_t stream) {
   if (K <= 0 || K % 256 != 0 || R < 1 || ((image != nullptr || side_n > 0) && R > 64) || x == nullptr ||
-      (image == nullptr && by_row == nullptr) || (reinterpret_cast<uintptr_t>(by_row) & 15) != 0)
+      (image == nullptr && by_row == nullptr && side_n <= 0) || (reinterpret_cast<uintptr_t>(by_row) & 15) != 0)
     return -HE_ERR_BAD_ARG;
   const int es = x_dtype == 0 ? 4 : 2;
   if ((reinterpret_cast<uintptr_t>(x) & 15) != 0 || (x_stride * es) % 16 != 0 ||
@@ -562,7 +563,7 @@ HE_API int he_rows_image(const void* x, int x_dtype, long long x_stride, const f
     const cudaError_t e = allow_smem(rows_image_kernel, most, allowed);
     if (e != cudaSuccess) return (int)e;
   }
-  const int parts = norm_w != nullptr ? 1 : (nb + 3) / 4;
+  const int parts = image == nullptr && by_row == nullptr ? 0 : norm_w != nullptr ? 1 : (nb + 3) / 4;
   const unsigned grid = (unsigned)(R * parts + (side_n > 0 ? (side_n + 1) / 2 : 0));
   return (int)launch_pdl(rows_image_kernel, dim3(grid), dim3(norm_w != nullptr ? 512 : 128), smem, stream, x, x_dtype,
                          x_stride, norm_w, eps, K, R, col_groups(R) * 8, parts, (uint8_t*)image, (uint8_t*)by_row, side_w, side_n,

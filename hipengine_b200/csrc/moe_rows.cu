@@ -149,11 +149,8 @@ rows_experts_kernel(const __grid_constant__ ExpertMaps maps, const __grid_consta
       for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
         const MoeJob job = a.jobs[it / tiles];
         const int n0 = (it % tiles) * per;
-        const uint8_t* src[2] = {image, image};
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-          if (i * 32 + lane < job.count)
-            src[i] = image + (size_t)(a.entries[job.first + i * 32 + lane] / a.rows_per_image_row) * nb * IMG_COL;
+        const uint8_t* src = image;                  // a job has at most 32 rows: one a lane
+        if (lane < job.count) src += (size_t)(a.entries[job.first + lane] / a.rows_per_image_row) * nb * IMG_COL;
         for (int blk = 0; blk < nb; ++blk, ++n) {
           ok = __all_sync(0xffffffffu, wait_long(&sh->empty[s], ph ^ 1u, abort_flag, a.status, 411));
           if (!ok) break;
@@ -175,11 +172,8 @@ rows_experts_kernel(const __grid_constant__ ExpertMaps maps, const __grid_consta
             }
           }
           __syncwarp();
-#pragma unroll
-          for (int i = 0; i < 2; ++i)
-            if (i * 32 + lane < job.count)
-              bulk_load(sm100::smem_u32(dst + a.w_bytes + (i * 32 + lane) * IMG_COL), src[i] + (size_t)blk * IMG_COL, IMG_COL,
-                        &sh->full[s]);
+          if (lane < job.count)
+            bulk_load(sm100::smem_u32(dst + a.w_bytes + lane * IMG_COL), src + (size_t)blk * IMG_COL, IMG_COL, &sh->full[s]);
           if (++s == a.stages) { s = 0; ph ^= 1u; }
         }
       }

@@ -5,6 +5,7 @@
 
 #include "common.cuh"
 #include "sm100.cuh"
+#include "tmap.cuh"
 
 namespace herows {
 
@@ -493,22 +494,6 @@ __device__ __forceinline__ void load_cols(const void* x, int dtype, size_t off, 
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-inline EncodeTiledFn encode_fn() {
-  static const EncodeTiledFn fn = []() -> EncodeTiledFn {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      return reinterpret_cast<EncodeTiledFn>(p);
-    return nullptr;
-  }();
-  return fn;
-}
-
 // Dynamic shared memory that a kernel may ask for, set once per device.  `bytes` is the kernel's largest need, the same in every
 // call: threads that set it at the same time agree, and none takes back what another one's launch relies on.
 template <typename F>
@@ -525,7 +510,7 @@ inline cudaError_t allow_smem(F kernel, int bytes, std::atomic<unsigned long lon
 
 // Weight rows as bytes: [rows][row_bytes], box {box_bytes, box_rows}
 inline int byte_map(CUtensorMap* m, const void* ptr, long long rows, long long row_bytes, int box_bytes, bool swizzle, int box_rows) {
-  const EncodeTiledFn enc = encode_fn();
+  const EncodeTiledFn enc = get_encode();
   if (enc == nullptr || (reinterpret_cast<uintptr_t>(ptr) & 15) != 0 || row_bytes % 16 != 0) return -HE_ERR_BAD_ARG;
   const cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)row_bytes};
   const cuuint32_t box[2] = {(cuuint32_t)box_bytes, (cuuint32_t)box_rows}, estr[2] = {1, 1};

@@ -497,9 +497,9 @@ class HybridExecutor:
                                  cfg.rms_eps)
                 if plain and T == 1:
                     gates = (self.ab_f32[i], h, self.F(i, "attn_norm.weight"), cfg.rms_eps)
-                else:                               # a verify chain: the same fp32 gates
+                else:                               # two rows, a verify chain: the same fp32 gates
                     ab = sc.get("ab_proj", (T, 2 * Hv), torch.float32)
-                    self.rows.image(h, self.F(i, "attn_norm.weight"), cfg.rms_eps, self.ab_f32[i], ab)
+                    self.rows.image(h, self.F(i, "attn_norm.weight"), cfg.rms_eps, self.ab_f32[i], ab, product=False)
                     a_p, b_p = ab[:, :Hv], ab[:, Hv:]
             elif i in self.ab_q8:
                 ab = sc.get("ab_proj", (T, 2 * Hv), torch.float32)

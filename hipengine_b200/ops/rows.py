@@ -83,7 +83,7 @@ class RowsSpace:
               by_row: bool = False, product: bool = True) -> Tuple[Optional[torch.Tensor], Optional[torch.Tensor]]:
         """The fragments of (RMSNorm of) the rows ``x`` [R, K] (fp32 or bf16): (for ``product``, for ``experts``), each on
         demand.  With ``side_w`` (fp32 [n, K]) the same launch also writes ``side_out`` [R, >= n] = normalised rows @
-        side_w^T, all in fp32."""
+        side_w^T, all in fp32, or nothing else."""
         _check_device(x)
         R, K = x.shape
         assert x.stride(1) == 1

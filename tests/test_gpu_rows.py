@@ -106,6 +106,9 @@ def test_segments_pairs_norm_side_rows(space):
         assert rel(add[:, :129] - 1, xn @ ad.t()) < 2 ** -10.5 and bool((add[:, 129:] == 1).all())
         assert rel(pre, xn @ bd.t()) < 2 ** -10.5
         assert rel(so[:, :97], xn @ side.double().t()) < 3e-6 and bool(so[:, 97:].isnan().all())
+        alone = torch.full((R, 104), float("nan"), device="cuda")
+        assert space.image(x, nw, 1e-6, side, alone, product=False) == (None, None)
+        assert torch.equal(alone[:, :97], so[:, :97])
     K.check_status()
 
 
