@@ -72,16 +72,43 @@ def test_weights_enter_exactly(space, t, R):
     K.check_status()
 
 
-def test_a_row_does_not_depend_on_its_neighbours(space):
+@pytest.mark.parametrize("t", [T.Q4_K, T.Q6_K, T.Q8_0])
+def test_a_row_beside_others(space, t):
+    """A row's bits are the same for every number of rows that takes the same kernel; between kernels the sums take another
+    order and Q6_K operands another rounding (11 bits above eight rows)."""
     from hipengine_b200.ops import kernels as K
-    w, _ = _weight(T.Q4_K, 640, 2048, 3)
-    x = torch.randn(8, 2048, device="cuda")
-    out = torch.zeros(8, 640, device="cuda")
-    space.gemm(x, [K.GemvSegment(w, out)])
-    for r in range(8):
-        one = torch.zeros(1, 640, device="cuda")
-        space.gemm(x[r:r + 1], [K.GemvSegment(w, one)])
-        assert torch.equal(one[0], out[r])
+    w, _ = _weight(t, 640, 2048, 3)
+    x = torch.randn(64, 2048, device="cuda", generator=torch.Generator(device="cuda").manual_seed(7))
+    first = {}
+    for R in (1, 3, 8, 9, 16, 17, 24, 25, 32, 33, 40, 41, 48, 49, 64):
+        out = torch.zeros(R, 640, device="cuda")
+        space.gemm(x[:R], [K.GemvSegment(w, out)])
+        kernel = min((R + 7) // 8, 7)
+        seen = first.setdefault(kernel, out)
+        n = min(R, seen.shape[0])
+        assert torch.equal(out[:n], seen[:n]), R
+        if R > seen.shape[0]:
+            first[kernel] = out
+        rel = float((out[0] - first[1][0]).norm() / first[1][0].norm())
+        assert rel < (2 ** -11 if t == T.Q6_K and R > 8 else 2e-6), R
+
+
+@pytest.mark.parametrize("t", [T.Q4_K, T.Q6_K, T.Q8_0])
+def test_outliers_cost_the_other_columns_of_their_block_an_absolute_error(space, t):
+    """One value a block a million times the others: those are fp16 subnormals under the block's power of two, off by at most
+    2^-25 of it each (bf16 rows too, whose small values the image no longer holds exactly)."""
+    from hipengine_b200.ops import kernels as K
+    n, k = 96, 1024
+    w, wd = _weight(t, n, k, 11)
+    x = torch.randn(4, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2)) * 1e-6
+    x[:, 37::256] = torch.tensor([1.0, 1.5, -1.25, 1.75], device="cuda")[:, None]
+    for xx in (x, x.bfloat16()):
+        out = torch.zeros(4, n, device="cuda")
+        space.gemm(xx, [K.GemvSegment(w, out)])
+        err = (out.double() - xx.double() @ wd.t()).abs()
+        # the rounding of the small values, and of fp32 sums of at most 1.75 times the outliers' weights
+        bound = 2 ** -25 * wd.abs().sum(1) + 2 ** -20 * 1.75 * wd[:, 37::256].abs().sum(1)
+        assert bool((err <= bound[None]).all()), float((err / bound[None]).max())
 
 
 def test_segments_pairs_norm_side_rows(space):
