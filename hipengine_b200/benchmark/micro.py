@@ -360,7 +360,7 @@ def gemm_role_counters(M, N, K, qtype="q4_k"):
 def bench_decode_step(rows_list, model="qwen35-27b", ctx=1024, small_rows=None):
     """Whole-model packed decode step (captured graph) at R concurrent rows, each at context `ctx`: the cost a
     continuous-batching round or a verify chain pays.  `small_rows` overrides the row count up to which the int8 GEMV
-    path is taken (above it the split-K tensor-core path streams the quantised blocks once for all rows)."""
+    path is taken (above it the few-row products stream the quantised blocks once for all rows)."""
     from hipengine_b200.loading.synth import build_random_model
     from hipengine_b200.models import make_executor
     from hipengine_b200.models.config import NAMED_CONFIGS

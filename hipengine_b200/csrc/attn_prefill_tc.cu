@@ -11,11 +11,12 @@
 // cores.  The accumulator is rescaled only when a row's maximum has grown by more than 2^8 (exact: sums and weights use the
 // same reference).
 //
-// Bound by shared memory and L2: a tile of 64 keys costs 1024 tensor-core cycles, 1500 cycles of shared-memory traffic (the
-// 64 KB of queries are read again for every tile, 64-wide score products cannot do better) and 64 KB of L2 reads.  The
+// What bounds it: a tile of 64 keys costs 1024 tensor-core cycles, about 1500 cycles of operand reads from shared memory by count
+// (the 64 KB of queries are read again for every tile, 64-wide score products cannot do better) and 64 KB from L2.  Counters at
+// 4096 rows after 4096 tokens: tensor pipe 51 %, L2 7.3 TB/s, issue 28 %, DRAM 2 %.  The
 // register form (mma.sync, 64 query rows) is bound by the rate of mma.sync and re-reads keys and values twice as often:
-// 24 heads on 4, 4096 rows 1159 us there, 403 us here (512 TFLOP/s); after 12288 tokens 6694 / 1508 us (957 TFLOP/s); 777 rows
-// 107 / 78 us; 16 heads on 2, 2048 rows 287 / 119 us.
+// 24 heads on 4, 4096 rows 1159 us there, 406 us here (508 TFLOP/s); after 12288 tokens 6694 / 1516 us (952 TFLOP/s); 777 rows
+// 107 / 80 us; 16 heads on 2, 2048 rows 287 / 127 us.
 #include "common.cuh"
 #include "sm100.cuh"
 #include "tmap.cuh"

@@ -14,9 +14,10 @@
 //   gdn_prepare_chunks : one CTA per (chunk, V head), all chunks at once: W, U, P and the log-sums to a workspace
 //   gdn_chain          : one CTA per (segment, V head, 32 or 64 columns of the state), the chunks in order: three products per
 //                        step, the state in registers, the next chunk's operands in flight (cp.async)
-// The chain is bound by its operands' way from L2 (56 KB per step and CTA) and by the latency of its two barriers per
-// step; 32 tokens per chunk halve the steps of 16 and keep the inverse cheap (64 measured no better on paper: the same
-// bytes, a four times larger inverse).  Measured on B200, 4096 tokens: 48 heads 585 us (147 + 438) against
+// The chain is bound by latency: dependent products and conversions, operands from shared memory, two barriers per step, on the
+// 96 SMs that 48 heads fill (issue 42 %, shared memory 41 %, tensor pipe 26 %, L2 2.8 TB/s); a step needs 56 KB from L2 per CTA of
+// 32 columns, 60 KB of 64.  32 tokens per chunk halve the steps of 16 and keep the inverse cheap.  (64 were not built: the same
+// bytes per token and an inverse of eight times the work.)  Measured on B200, 4096 tokens: 48 heads 585 us (147 + 438) against
 // 938 us, 2048 tokens x 32 heads 207 us (54 + 153) against 395 us.
 // All products run as mma.sync m16n8k8 TF32 with rounded operands (fp32 accumulate).  Used for prefill segments without a
 // state journal; decode rows, verify chains and short segments keep the serial kernel in gdn.cu.  V head h reads K head

@@ -2,7 +2,9 @@
 // out[r][n] = sum_k x[r][k] W[n][k], the weights streamed once whatever the row count.  Decode steps, verify chains and
 // short prompts are these products and little else.
 //
-// What bounds it: the weight stream (HBM), as long as turning a block into operands stays cheaper than reading it.
+// What has to move is the weight stream (HBM).  What bounds it in fact (17408 x 5120 Q4_K, 4 / 16 / 64 rows): up to 16 rows ramp,
+// image wait and the sum of shared tiles around a steady part that the expansion of blocks sets (DRAM 25 / 22 %, issue 44 / 43 %,
+// tensor pipe 14 / 23 %); at 64 rows the reads of the image and mma.sync (shared memory 59 %, tensor pipe 45 %, DRAM 11 %).
 //   operands : fp16 m16n8k16 MMAs with the WEIGHT as the A operand.  A k-quant weight is d * (sc * q) - dmin * m with
 //              sc * q an integer below 2^10 and m one below 2^6: both are exact in fp16, so ONE packed fp16 FMA makes two
 //              operands (1024 + q is the nibble under an exponent byte; (1024 + q) * sc - 1024 * sc), the 256-column block

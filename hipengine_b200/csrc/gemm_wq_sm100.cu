@@ -937,7 +937,8 @@ int pick_mt(int M, bool grouped) {
 }
 
 // Activation rows per tile of a plain product with several tiles.  A unit of two tiles costs its rows plus about as much again
-// as 390 of them (unit times of 4096 x 17408 x 5120: 55.1 / 52.9 / 51.4 / 48.3 us at 192 / 176 / 160 / 144 rows a tile), and the
+// as 390 of them (unit times of 4096 x 17408 x 5120, Q4_K: 55.1 / 52.9 / 51.4 / 48.3 us at 192 / 176 / 160 / 144 rows a tile; the
+// other types, whose blocks cost about the same to expand, use the figure too), and the
 // busiest SM ends the kernel: take the tile for which that SM has the least to do.  Against 192 always: 2048 rows x 10240
 // 247 -> 219 us (160), x 17408 324 -> 308 us (176), 777 rows x 5120 72 -> 68 us (160); 4096 x 17408 stays at 192.
 int pick_mt_plain(int M, int N, int num_sms) {

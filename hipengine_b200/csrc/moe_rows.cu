@@ -1,7 +1,7 @@
 // Routed experts over the rows that chose them: every expert's quantised weights are streamed once per 8, 16 or 32 of its rows,
 // with the operands of the few-row products (rows_mma.cuh).
 //
-//   he_moe_jobs      : the (row, expert) pairs sorted by expert and cut into jobs of at most `cols` rows
+//   he_moe_jobs      : the (row, expert) pairs sorted by expert, ascending within one, and cut into jobs of at most `cols` rows
 //   he_rows_experts  : a CTA takes (job, tile of 256 weight rows) items; the activation image is gathered row by row with
 //                      bulk copies while the tile's blocks arrive by TMA.  Gate/up: act(g) * u per pair as bf16; down: one
 //                      row per pair
@@ -11,7 +11,8 @@
 // Why: a decode batch (256 pairs over ~160 of 256 experts at 32 rows, top 8) had one CTA group per PAIR that normalised and
 // quantised its row again and read the expert's blocks with 16-byte loads; a prompt (64 rows per expert at 2048) had its
 // rows padded to 128 for a tile of the tcgen05 GEMM, whose expansion of 128 x 256 weights costs the same whatever the rows.
-// Bound by the weight stream for few rows per expert, by mma.sync for many.  A layer's experts (256, 8 used, hidden 2048,
+// At 32 rows DRAM is at 43-47 % and the issue slots at 60 % (expansion of the blocks); with more rows per expert mma.sync and the
+// image reads grow.  A layer's experts (256, 8 used, hidden 2048,
 // width 512): 32 rows 100 us for both products (172 us before), a step of 8 layers 2471 -> 1893 us; prompts of 72 / 256 / 1024
 // rows 6.1 / 7.3 / 8.6 ms -> 3.9 / 4.4 / 7.1 ms, of 2048 rows 10.6 -> 12.4 ms (those stay on the grouped GEMM).
 // Reference: hipengine/kernels/hip_gfx1100/quant/gguf_q4_k_selected_prefill.hip, moe/group_scatter.hip.

@@ -29,7 +29,9 @@ from ..quant.ggml import GGMLType
 
 SEL_MAX_ROWS = 64
 # Decode batches from this many rows on run their experts as jobs (csrc/moe_rows.cu): 256 experts, 8 used, a step of 4 / 8 / 32
-# rows takes 884 / 1033 / 1893 us with jobs, 873 / 1047 / 2471 us with one pass over an expert's rows per pair.
+# rows takes 884 / 1033 / 1893 us with jobs, 873 / 1047 / 2471 us with one pass over an expert's rows per pair.  (What jobs save
+# is the weights that pairs share: with fewer experts per pair used they would pay from fewer rows; that was the only geometry
+# measured.)
 JOBS_MIN_ROWS = 8
 # Pairs per expert up to which a prompt's do: 72 / 256 / 1024 / 2048 rows take 3.9 / 4.4 / 7.1 / 12.4 ms with jobs and
 # 6.1 / 7.3 / 8.6 / 10.6 ms in the grouped GEMM, whose 128-row tiles are mostly padding for few rows an expert.
