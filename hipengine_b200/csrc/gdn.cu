@@ -534,7 +534,8 @@ HE_API int he_gdn_front(const GdnFrontArgs* args, cudaStream_t stream) {
   if (a.T <= 0 || a.n_seg <= 0) return 0;
   const int es = a.in_dtype == 0 ? 4 : 2;
   if (a.C != 2 * a.G * 128 + a.Hv * 128 || (reinterpret_cast<uintptr_t>(a.x) & 15) != 0 || (a.x_stride * es) % 8 != 0 ||
-      (a.in_dtype == 0 && a.x_stride % 4 != 0) || (reinterpret_cast<uintptr_t>(a.conv_state) & 15) != 0)
+      (a.in_dtype == 0 && a.x_stride % 4 != 0) ||
+      ((reinterpret_cast<uintptr_t>(a.conv_state) | reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.out)) & 15) != 0)
     return -HE_ERR_BAD_ARG;
   gdn_front_kernel<<<dim3(a.T / FRONT_TOK + a.n_seg, (a.C / 128 + 7) / 8), 256, 0, stream>>>(a);
   HE_LAUNCH_CHECK();

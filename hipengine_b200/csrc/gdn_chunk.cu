@@ -455,7 +455,8 @@ HE_API int he_gdn_scan_chunked(const GdnChunkArgs* args, cudaStream_t stream) {
   GdnChunkArgs a = *args;
   if (a.T <= 0 || a.n_seg <= 0) return 0;
   const Windows w = windows(a.T, a.n_seg, a.write_state, a.longest);
-  if (a.C != 2 * a.G * DK + a.Hv * DK || a.ws == nullptr || a.longest < 0 || a.ws_floats < w.units * a.Hv * WS_UNIT)
+  if (a.C != 2 * a.G * DK + a.Hv * DK || a.ws == nullptr || a.longest < 0 || a.ws_floats < w.units * a.Hv * WS_UNIT ||
+      ((reinterpret_cast<uintptr_t>(a.ws) | reinterpret_cast<uintptr_t>(a.qkv)) & 15) != 0)
     return -HE_ERR_BAD_ARG;
   // set per call (cheap): the attribute belongs to the (function, device) pair, not to the process
   cudaError_t e = cudaFuncSetAttribute(gdn_prepare_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -352,7 +352,9 @@ HE_API int he_rows_experts_args_size() { return (int)sizeof(RowsExpertsArgs); }
 HE_API int he_moe_sum_pairs(float* h, long long ldh, const void* y, int y_dtype, long long ldy, const float* wts, int T, int k,
                             const void* ysh, long long ldsh, const float* sg, long long ldsg, int N, cudaStream_t stream) {
   if (T <= 0) return 0;
-  if (N % 4 != 0 || ldh % 4 != 0 || ldy % 4 != 0 || ldsh % 4 != 0) return -HE_ERR_BAD_ARG;
+  if (N % 4 != 0 || ldh % 4 != 0 || ldy % 4 != 0 || ldsh % 4 != 0 || (reinterpret_cast<uintptr_t>(h) & 15) != 0 ||
+      (reinterpret_cast<uintptr_t>(y) & (y_dtype == 0 ? 15 : 7)) != 0 || (reinterpret_cast<uintptr_t>(ysh) & 7) != 0)
+    return -HE_ERR_BAD_ARG;
   const dim3 grid((N / 4 + 255) / 256, T);
   if (y_dtype == 0)
     return (int)launch_pdl(moe_sum_pairs_kernel<float>, grid, dim3(256), 0, stream, h, ldh, (const float*)y, ldy, wts, k,

@@ -127,3 +127,13 @@ def test_sum_of_pairs(space, T, k, n, dtype):
         space.sum_pairs(got, y, w, sh if shared else None, gate[:, 1:2] if shared else None)
         ref = want + torch.sigmoid(gate[:, 1:2].double()) * sh.double() if shared else want
         assert float((got.double() - ref).abs().max()) < 1e-5                    # fp32 sums of at most ten terms below 30
+
+
+def test_sum_of_pairs_refuses_rows_that_are_not_aligned(space):
+    """Rows are read four columns at once."""
+    h, y, w = torch.zeros(2, 12, device="cuda"), torch.zeros(4, 12, device="cuda"), torch.zeros(2, 2, device="cuda")
+    sh = torch.zeros(2, 12, device="cuda", dtype=torch.bfloat16)
+    for a, b, c in ((h[:, 1:9], y[:, :8], None), (h[:, :8], y[:, 2:10], None), (h[:, :8], y.bfloat16()[:, 2:10], None),
+                    (h[:, :8], y[:, :8], sh[:, 1:9])):
+        with pytest.raises(RuntimeError):
+            space.sum_pairs(a, b, w, c)

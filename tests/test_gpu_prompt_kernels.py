@@ -124,6 +124,22 @@ def test_front_is_convolution_then_preparation(dtype, lens):
         assert torch.allclose(p, q, rtol=1e-5, atol=1e-6)
 
 
+def test_front_and_scan_refuse_operands_that_are_not_aligned():
+    from hipengine_b200.ops import kernels as K
+    G, Hv, T = 1, 1, 64
+    C = 3 * 128
+    z = lambda *s: torch.zeros(*s, device="cuda")
+    start, slot = torch.tensor([0, T], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    odd = lambda *s: z(torch.Size(s).numel() + 1)[1:].view(*s)
+    ab, one = z(T, Hv), z(Hv)
+    for w, out in ((odd(C, 4), z(T, C)), (z(C, 4), odd(T, C))):
+        with pytest.raises(RuntimeError):
+            K.gdn_front(z(T, C), w, z(1, C, 3), start, slot, out, ab, ab, one, one, z(T, Hv), z(T, Hv), G, Hv)
+    for qkv, ws in ((odd(T, C), None), (z(T, C), odd(K.gdn_chunk_ws_floats(T, 1, Hv)))):
+        with pytest.raises(RuntimeError):
+            K.gdn_scan_chunked(qkv, z(T, Hv), z(T, Hv), z(1, Hv, 128, 128), start, slot, z(T, Hv, 128), G, Hv, ws=ws)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("T", [1, 33])
 def test_gated_norm_of_128_columns(dtype, T):
