@@ -4,19 +4,23 @@
 //   warps 0-3 : softmax; a thread owns one of the tile's 128 query rows (= a TMEM lane)
 //   warp 4, 5 : TMA producers of keys / values: a tile is 64 keys = 4 pages x 4 boxes of 16 keys x 64 columns, one box a lane
 //   warp 6    : MMA issuer; owns the tensor memory
-// Tensor memory: two score buffers of 64 columns and the 256-column accumulator; the bf16 weights overwrite the scores they
-// came from and are the A operand of the value product.  Queries and keys are K-major operands as they lie in memory; values
+// Tensor memory: two score buffers of 64 columns and the 256-column accumulator; the weights overwrite the scores they came from
+// and are the A operand of the value product.  Queries and keys are K-major operands as they lie in memory; values
 // are too -- [key][column] rows are the MN-major form of the B operand, so the cache is read in place by both products.
 // While the softmax of a tile runs, the scores of the next tile and the value product of the last one occupy the tensor
-// cores.  The accumulator is rescaled only when a row's maximum has grown by more than 2^8 (exact: sums and weights use the
-// same reference).
+// cores.  The accumulator is rescaled only when a row's maximum has grown by more than 2^8: sums and weights use the same
+// reference, but the largest weight is then not 1 and a bf16 weight would be off by its rounding, which it is not in the register
+// form.  So a weight is two bf16 numbers, its upper 16 bits and the rest (64 columns of 64 keys: the buffer that the scores had), and
+// the value product takes both.  Error against 64 bits at 600 rows after 2000, queries of twice unit size: 1.66e-3, the rounding of
+// the output; 2.19e-3 with one number, 1.89e-3 in the register form.  It costs 14-24 % (4096 rows 406 -> 462 us, after 12288 tokens
+// 1516 -> 1878 us); rescaling at every growth instead, with one number, 493 / 1924 us.
 //
-// What bounds it: a tile of 64 keys costs 1024 tensor-core cycles, about 1500 cycles of operand reads from shared memory by count
-// (the 64 KB of queries are read again for every tile, 64-wide score products cannot do better) and 64 KB from L2.  Counters at
-// 4096 rows after 4096 tokens: tensor pipe 51 %, L2 7.3 TB/s, issue 28 %, DRAM 2 %.  The
-// register form (mma.sync, 64 query rows) is bound by the rate of mma.sync and re-reads keys and values twice as often:
-// 24 heads on 4, 4096 rows 1159 us there, 406 us here (508 TFLOP/s); after 12288 tokens 6694 / 1516 us (952 TFLOP/s); 777 rows
-// 107 / 80 us; 16 heads on 2, 2048 rows 287 / 127 us.
+// What bounds it: a tile of 64 keys costs 1536 tensor-core cycles, about 1750 cycles of operand reads from shared memory by count
+// (the 64 KB of queries are read again for every tile, 64-wide score products cannot do better) and 64 KB from L2; with one
+// bf16 number a weight 1024 and 1500.  The register form (mma.sync, 64 query rows) is bound by the rate of mma.sync and re-reads keys
+// and values twice as often: 24 heads on 4, 4096 rows 1159 us there, 462 us here (447 TFLOP/s); after 12288 tokens 6694 / 1878 us (769
+// TFLOP/s); 777 rows 107 / 91 us; 16 heads on 2, 2048 rows 287 / 147 us.  Counters at 4096 rows after 4096 tokens: tensor pipe 62 %,
+// L2 5.5 TB/s, issue 27 %, DRAM 2 %.
 #include "common.cuh"
 #include "sm100.cuh"
 #include "tmap.cuh"
@@ -59,6 +63,8 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
   __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
 }
+// The upper half of a float: a bf16 number; what it leaves fits another one to 2^-9 of itself.
+__device__ __forceinline__ float upper(float x) { return __uint_as_float(__float_as_uint(x) & 0xFFFF0000u); }
 // Bounded wait that goes on after an abort.
 __device__ __forceinline__ void drain_wait(uint64_t* bar, uint32_t parity) {
   for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
@@ -189,8 +195,11 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         tc_fence_after();
         const uint32_t va = smem_u32(sV + s * KV_STAGE);
 #pragma unroll
-        for (int u = 0; u < KN / 16; ++u)
-          umma_f16_ts(o_col, s_col(b) + u * 8, desc_mn_sw128(va + u * 2048), id_o, (j > 0 || u > 0) ? 1u : 0u);
+        for (int u = 0; u < KN / 16; ++u) {
+          const uint64_t vd = desc_mn_sw128(va + u * 2048);
+          umma_f16_ts(o_col, s_col(b) + u * 8, vd, id_o, (j > 0 || u > 0) ? 1u : 0u);
+          umma_f16_ts(o_col, s_col(b) + KN / 2 + u * 8, vd, id_o, 1u);        // the weights' low parts
+        }
         umma_commit(&bar->o_done);
         umma_commit(&bar->v_empty[s]);
       }
@@ -250,21 +259,21 @@ flash_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       }
       const float neg = m_ref == -INFINITY ? 0.f : -m_ref;     // nothing seen yet: every weight is 2^-inf = 0
       float s0 = 0.f, s1 = 0.f;
+      uint32_t hi[32], lo[32];                                 // 32 columns each: weights of 64 keys, two to a column
 #pragma unroll
       for (int c = 0; c < 32; c += 2) {
         const float p0 = ex2(fmaf(__uint_as_float(r0[c]), sc, neg)), p1 = ex2(fmaf(__uint_as_float(r0[c + 1]), sc, neg));
         const float p2 = ex2(fmaf(__uint_as_float(r1[c]), sc, neg)), p3 = ex2(fmaf(__uint_as_float(r1[c + 1]), sc, neg));
-        r0[c >> 1] = pack2(p0, p1);
-        r1[c >> 1] = pack2(p2, p3);
-        // the sum takes the rounded weights: the largest one is not 1 under a reference that lags, and its rounding would
-        // stay in the quotient
-        s0 += __uint_as_float(r0[c >> 1] << 16) + __uint_as_float(r0[c >> 1] & 0xFFFF0000u);
-        s1 += __uint_as_float(r1[c >> 1] << 16) + __uint_as_float(r1[c >> 1] & 0xFFFF0000u);
+        s0 += p0 + p1;
+        s1 += p2 + p3;
+        hi[c >> 1] = __byte_perm(__float_as_uint(p0), __float_as_uint(p1), 0x7632);
+        hi[16 + (c >> 1)] = __byte_perm(__float_as_uint(p2), __float_as_uint(p3), 0x7632);
+        lo[c >> 1] = pack2(p0 - upper(p0), p1 - upper(p1));
+        lo[16 + (c >> 1)] = pack2(p2 - upper(p2), p3 - upper(p3));
       }
       l += s0 + s1;
-#pragma unroll
-      for (int c = 0; c < 16; ++c) r0[16 + c] = r1[c];
-      tmem_st_32x32(s_col(b) + lane_off, r0);
+      tmem_st_32x32(s_col(b) + lane_off, hi);
+      tmem_st_32x32(s_col(b) + lane_off + KN / 2, lo);
       tmem_st_wait();
       if (k0 + KN > kv_end) {
         // keys past the last visible one: their weights are zero, their values may be anything (also NaN): zero them

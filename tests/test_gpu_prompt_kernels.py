@@ -40,6 +40,26 @@ def test_tensor_memory_attention_matches_64_bit(T, H, Hkv, pos0):
     K.check_status()
 
 
+@pytest.mark.parametrize("T,pos0,size", [(777, 0, 1.0), (600, 2000, 2.0), (512, 3000, 3.0), (300, 100, 8.0)])
+def test_tensor_memory_attention_loses_nothing_but_the_output_rounding(T, pos0, size):
+    """Flat to peaked weights, maxima that grow a little at a time: what is left is the output's bf16."""
+    from hipengine_b200.ops import attention as A
+    H, G, D, last = 8, 2, 256, pos0 + T
+    n = -(-last // 16)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    kv = torch.randn(n, 2, G, 16, D, device="cuda", generator=g).bfloat16()
+    q = (size * torch.randn(T, H, D, device="cuda", generator=g)).bfloat16()
+    out = torch.zeros(T, H * D, device="cuda", dtype=torch.bfloat16)
+    A.flash_prefill(q, None, kv, torch.arange(n, device="cuda", dtype=torch.int32)[None].contiguous(), 0, pos0, out, H, G, D, 16, 1 / 16)
+    k, v = (kv[:, i].permute(1, 0, 2, 3).reshape(G, -1, D)[:, :last].double() for i in (0, 1))
+    s = torch.einsum("thgd,hkd->thgk", q.double().reshape(T, G, H // G, D), k) / 16
+    dark = torch.arange(last, device="cuda")[None] > pos0 + torch.arange(T, device="cuda")[:, None]
+    want = torch.einsum("thgk,hkd->thgd", torch.softmax(s.masked_fill(dark[:, None, None], -math.inf), -1), v).reshape(T, -1)
+    least = float((want.bfloat16().double() - want).norm())
+    # scores are fp32 sums of 256 products: 2^-20 of scores up to 60 beside the output's 2^-9
+    assert float((out.double() - want).norm()) < 1.01 * least
+
+
 @pytest.mark.parametrize("lens,Hv", [([5500], 1), ([64, 1, 95], 2), ([100, 2600, 33], 2)])
 def test_scan_windows_and_segments(lens, Hv):
     """More chunks than one window holds, segments of uneven length: the same recurrence as the serial kernel."""
