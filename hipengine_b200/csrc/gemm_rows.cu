@@ -12,9 +12,9 @@
 //              the activations per 32 columns (as an fp16 high and low part).  Q8_0, and Q6_K up to 8 rows: the integers
 //              themselves are the operands, an MMA (two for Q8_0) covers one sub-block, and the sub-block's scale meets
 //              its fp32 sums: exact as well, and for Q8_0 cheaper than a product per operand (17408 x 5120, 4 / 16 / 32 rows
-//              24.7 / 29.0 / 47.9 -> 21.8 / 24.2 / 42.6 us; 64 rows 50.3 -> 50.9).  Q6_K above 8 rows: sc * (q - 32), 13
+//              24.7 / 29.2 / 48.1 -> 21.4 / 24.0 / 42.5 us; 64 rows 51.0 -> 52.4).  Q6_K above 8 rows: sc * (q - 32), 13
 //              bits, rounded to 11: the exact form costs two packed FMAs per MMA (17408 x 5120, 16 / 32 / 64 rows 27.5 / 40.7
-//              / 55.2 us against 25.3 / 35.1 / 45.1; at 8 rows 22.3 against 22.8).
+//              / 55.2 us against 25.0 / 35.2 / 44.5; at 8 rows 22.1 against 22.8).
 //   activations: fp16 under a power of two per row and block of 256 columns, 11 bits each down to 2^-14 of the block's largest
 //              value and 2^-25 of it below (bf16 values down to 2^-17 of it exactly), written once per launch by he_rows_image
 //              in the order of the MMA's B fragments (one 16-byte load per lane feeds two MMAs), so no CTA repeats the

@@ -11,11 +11,11 @@ namespace herows {
 
 using namespace he;
 
-// Image of one block of one activation row: 8 units [v][c] of 64 bytes, the eight sums per 32 columns in two parts, the
-// scale, and padding that puts neighbouring rows half a bank cycle apart.  A unit holds the quads v (columns 4 v .. + 3) of the
-// 16-column groups (h, 2 c, u) and (h, 2 c + 1, u), h and u at position (2 h + u) ^ v: lanes that read one position of four units
-// meet no bank twice either.
-constexpr int IMG_COL = 576, SX_OFF = 512, XS_OFF = 544;
+// Image of one block of one activation row: four parts v of 144 bytes.  Part v holds the quads v (columns 4 v .. + 3) of all
+// 16-column groups (h, qt, u): unit c = qt / 2 of 64 bytes, in it 16 bytes per (h, u), quads of qt = 2 c and 2 c + 1.  The last 16
+// bytes of parts 0 and 1 hold the eight sums per 32 columns in two parts, those of part 2 the scale.  With them lanes that read one
+// part and lanes that read one place of four parts both meet no bank twice; 576 bytes put neighbouring rows half a bank cycle apart.
+constexpr int IMG_COL = 576, PART = 144, SX_OFF = 128, XS_OFF = 2 * PART + 128;
 constexpr int MAX_STAGES = 8;
 constexpr int SMEM_TOTAL = 220 * 1024;
 
@@ -139,10 +139,9 @@ __device__ __forceinline__ void block_q4k(uint32_t r0, uint32_t r1, uint32_t img
       const uint32_t l2 = h2_fma(and_or<0x000F000Fu>(a8, mg), sla, cla), l3 = h2_fma(and_or<0x000F000Fu>(b8, mg), slb, clb);
       const uint32_t u0 = h2_fma(and_or<0x00F000F0u>(a, mg), sha, cha), u1 = h2_fma(and_or<0x00F000F0u>(b, mg), shb, chb);
       const uint32_t u2 = h2_fma(and_or<0x00F000F0u>(a8, mg), sha, cha), u3 = h2_fma(and_or<0x00F000F0u>(b8, mg), shb, chb);
-      const uint32_t xv = xb ^ (v * 16);
 #pragma unroll
       for (int n = 0; n < L; ++n) {
-        const uint4 x = lds128(xv + n * 8 * IMG_COL + (v * 2 + c) * 64);
+        const uint4 x = lds128(xb + n * 8 * IMG_COL + v * PART + c * 64);
         mma_from(v + c == 0, D[n], l0, l1, l2, l3, x.x, x.y);
         mma_from(SPLIT && v + c == 0, SPLIT ? E[SPLIT ? n : 0] : D[n], u0, u1, u2, u3, x.z, x.w);
       }
@@ -159,7 +158,7 @@ __device__ __forceinline__ void block_q4k(uint32_t r0, uint32_t r1, uint32_t img
   const uint32_t na = h2_add(prmt(mna, 0x64646464u, msel), M1024), nb = h2_add(prmt(mnb, 0x64646464u, msel), M1024);
   const float2 da = __half22float2(*reinterpret_cast<const __half2*>(&ma.x));
   const float2 db = __half22float2(*reinterpret_cast<const __half2*>(&mb.x));
-  const uint32_t sx = img + g * IMG_COL + SX_OFF + t * 8, xs = img + 2 * t * IMG_COL + XS_OFF;
+  const uint32_t sx = img + g * IMG_COL + SX_OFF + (t >> 1) * PART + (t & 1) * 8, xs = img + 2 * t * IMG_COL + XS_OFF;
 #pragma unroll
   for (int n = 0; n < L; ++n) {
     float M[4];
@@ -243,10 +242,9 @@ __device__ __forceinline__ void block_q6k(uint32_t r0, uint32_t r1, uint32_t img
         o[2] = high(lbv[v] >> 8, hA8 << 2, fa[3]);
         o[3] = high(kbv[v] >> 8, hB8 << 2, fb[3]);
       }
-      const uint32_t xv = xb ^ (v * 16);
 #pragma unroll
       for (int n = 0; n < L; ++n) {
-        const uint4 x = lds128(xv + n * 8 * IMG_COL + (v * 2 + c) * 64);
+        const uint4 x = lds128(xb + n * 8 * IMG_COL + v * PART + c * 64);
         mma_from(v + c == 0, D[n], e[0], e[1], e[2], e[3], x.x, x.y);
         mma_from(SPLIT && v + c == 0, SPLIT ? E[SPLIT ? n : 0] : D[n], o[0], o[1], o[2], o[3], x.z, x.w);
       }
@@ -289,7 +287,7 @@ __device__ __forceinline__ void block_q6k_exact(uint32_t r0, uint32_t r1, uint32
   const uint4 sa = lds128(r0 + 192), sb = lds128(r1 + 192);
   const uint32_t wa[4] = {sa.x ^ 0x80808080u, sa.y ^ 0x80808080u, sa.z ^ 0x80808080u, sa.w ^ 0x80808080u};
   const uint32_t wb[4] = {sb.x ^ 0x80808080u, sb.y ^ 0x80808080u, sb.z ^ 0x80808080u, sb.w ^ 0x80808080u};
-  const uint32_t xb = img + g * IMG_COL + t * 128 + t * 16, q0 = r0 + 4 * t, q1 = r1 + 4 * t;
+  const uint32_t xb = img + g * IMG_COL + t * PART, q0 = r0 + 4 * t, q1 = r1 + 4 * t;
   auto low = [mg](uint32_t l, uint32_t hs) { return h2_add(and_or<0x00300030u>(hs, and_or<0x000F000Fu>(l, mg)), M1056); };
   auto high = [mg](uint32_t l, uint32_t hs) {       // 16 (q - 32)
     return h2_add(and_or<0x03000300u>(hs, and_or<0x00F000F0u>(l, mg)), M1536);
@@ -331,7 +329,7 @@ __device__ __forceinline__ void block_q6k_exact(uint32_t r0, uint32_t r1, uint32
       const float ob = c == 0 ? byte_scale<1>(wb[2 * h], 2 + u) : byte_scale<W>(wb[2 * h + 1], 2 + u);
 #pragma unroll
       for (int n = 0; n < L; ++n) {
-        const uint4 x = lds128((xb ^ (s * 16)) + n * 8 * IMG_COL + c * 64);
+        const uint4 x = lds128(xb + n * 8 * IMG_COL + s * 16 + c * 64);
         float P[4], R[4];
         mma_from(true, P, e[0], e[1], e[2], e[3], x.x, x.y);
         mma_from(true, R, o[0], o[1], o[2], o[3], x.z, x.w);
@@ -355,7 +353,7 @@ __device__ __forceinline__ void block_q80(uint32_t p0, int i0, uint32_t p1, int 
   const uint4 sa = lds128(p0 + 2 * HT * 128 + i0 * 16), sb = lds128(p1 + 2 * HT * 128 + i1 * 16);
   const uint32_t wa[4] = {sa.x, sa.y, sa.z, sa.w}, wb[4] = {sb.x, sb.y, sb.z, sb.w};
   const uint32_t ra = p0 + i0 * 128 + (t >> 1) * 8, rb = p1 + i1 * 128 + (t >> 1) * 8;
-  const uint32_t xb = img + g * IMG_COL + (t >> 1) * 256 + t * 16;
+  const uint32_t xb = img + g * IMG_COL + (t >> 1) * 2 * PART + u * 16;
   auto up = [mg](uint32_t w) { return h2_add(and_or<0x00FF00FFu>(w, mg), M1152); };
   float D[L][4];
 #pragma unroll
@@ -384,10 +382,9 @@ __device__ __forceinline__ void block_q80(uint32_t p0, int i0, uint32_t p1, int 
           a[q][2] = up(ka >> 8);
           a[q][3] = up(kb >> 8);
         }
-        const uint32_t xv = xb ^ ((2 * h ^ i) * 16);
 #pragma unroll
         for (int n = 0; n < L; ++n) {
-          const uint4 x = lds128(xv + n * 8 * IMG_COL + i * 128 + c * 64);
+          const uint4 x = lds128(xb + n * 8 * IMG_COL + i * PART + c * 64 + h * 32);
           float P[4], R[4];
           mma_from(true, P, a[0][0], a[0][1], a[0][2], a[0][3], x.x, x.y);
           mma_from(true, R, a[1][0], a[1][1], a[1][2], a[1][3], x.z, x.w);
@@ -457,14 +454,14 @@ __device__ __forceinline__ void image_store(uint8_t* unit, uint8_t* also, int la
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
     __half2 p[2] = {__halves2half2(hv[4 * q], hv[4 * q + 2]), __halves2half2(hv[4 * q + 1], hv[4 * q + 3])};
-    const int at = ((v0 + q) * 2 + (qt >> 1)) * 64 + (t ^ (v0 + q)) * 16 + (qt & 1) * 8;
+    const int at = (v0 + q) * PART + (qt >> 1) * 64 + t * 16 + (qt & 1) * 8;
     *reinterpret_cast<uint2*>(unit + at) = *reinterpret_cast<const uint2*>(p);
     if (also != nullptr) *reinterpret_cast<uint2*>(also + at) = *reinterpret_cast<const uint2*>(p);
   }
   if ((lane & 3) == 0) {
     const int sub = lane >> 2;
     const __half hi = __float2half_rn(s), lo = __float2half_rn(s - __half2float(hi));
-    const int at = SX_OFF + (sub >> 1) * 8 + (sub & 1) * 2;
+    const int at = SX_OFF + (sub >> 2) * PART + ((sub >> 1) & 1) * 8 + (sub & 1) * 2;
     *reinterpret_cast<__half*>(unit + at) = hi;
     *reinterpret_cast<__half*>(unit + at + 4) = lo;
     if (also != nullptr) {

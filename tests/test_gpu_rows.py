@@ -72,6 +72,18 @@ def test_weights_enter_exactly(space, t, R):
     K.check_status()
 
 
+def test_a_row_does_not_depend_on_its_neighbours(space):
+    from hipengine_b200.ops import kernels as K
+    w, _ = _weight(T.Q4_K, 640, 2048, 3)
+    x = torch.randn(8, 2048, device="cuda")
+    out = torch.zeros(8, 640, device="cuda")
+    space.gemm(x, [K.GemvSegment(w, out)])
+    for r in range(8):
+        one = torch.zeros(1, 640, device="cuda")
+        space.gemm(x[r:r + 1], [K.GemvSegment(w, one)])
+        assert torch.equal(one[0], out[r])
+
+
 @pytest.mark.parametrize("t", [T.Q4_K, T.Q6_K, T.Q8_0])
 def test_a_row_beside_others(space, t):
     """A row's bits are the same for every number of rows that takes the same kernel; between kernels the sums take another
