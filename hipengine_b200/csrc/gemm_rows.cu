@@ -19,9 +19,9 @@
 //              value and 2^-25 of it below (bf16 values down to 2^-17 of it exactly), written once per launch by he_rows_image
 //              in the order of the MMA's B fragments (one 16-byte load per lane feeds two MMAs), so no CTA repeats the
 //              normalisation.
-//   k order  : lane (g, t) of an MMA with scaled operands holds columns of ITS OWN sub-blocks -- t = (h, u) owns, in half h of the block, the 16
-//              positions of half u of each of the four 32-column groups -- because that is what a 16-byte load of Q6_K
-//              low nibbles, high nibbles and Q4_K nibbles delivers; the scale is then a per-lane constant.
+//   k order  : lane (g, t) of an MMA with scaled operands holds columns of ITS OWN sub-blocks -- t = (h, u) owns, in half h of
+//              the block, the 16 positions of half u of each of the four 32-column groups -- because that is what a 16-byte load
+//              of Q6_K low nibbles, high nibbles and Q4_K nibbles delivers; the scale is then a per-lane constant.
 //   split    : the (tile of 128 weight rows) x (block) units of all segments are dealt out as one contiguous range
 //              per SM (equal to one unit), so there is no last wave.  A tile that several CTAs share leaves fp32 partial
 //              tiles in `ws`; whoever arrives last (a counter per tile, reset by it) adds them in CTA order:

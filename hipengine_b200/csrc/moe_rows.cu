@@ -323,7 +323,8 @@ HE_API int he_moe_jobs(const int* ids, int P, int E, int cols, int* entries, voi
                        cudaStream_t stream) {
   if (P <= 0) return 0;
   if (E < 1 || E > MAX_EXPERTS || cols < 1 || max_jobs < he_moe_jobs_bound(P, E, cols)) return -HE_ERR_BAD_ARG;
-  return (int)launch_pdl(moe_jobs_kernel, dim3(1), dim3(MAX_EXPERTS), 0, stream, ids, P, E, cols, entries, (MoeJob*)jobs, max_jobs, meta);
+  return (int)launch_pdl(moe_jobs_kernel, dim3(1), dim3(MAX_EXPERTS), 0, stream, ids, P, E, cols, entries, (MoeJob*)jobs, max_jobs,
+                         meta);
 }
 
 // Products of the jobs' rows with their experts' weights `w` (and `w2`: the up weights of epi 3, 4), [E * expert_rows][K]

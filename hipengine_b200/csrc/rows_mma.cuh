@@ -2,6 +2,7 @@
 // operands, the activation image, waits, tensor maps of weight rows.  See gemm_rows.cu for the method.
 #pragma once
 #include <atomic>
+#include <cfloat>
 
 #include "common.cuh"
 #include "sm100.cuh"
@@ -108,7 +109,7 @@ __device__ __forceinline__ uint32_t dup_byte(uint32_t w, uint32_t i) { return pr
 // One block (256 columns) of the 16 weight rows of a warp: `r0`, `r1` are the shared addresses of rows g and g + 8 in
 // the stage, `img` that of the block's image.  acc[nt] += the block's product in the MMA's C layout (rows g / g + 8,
 // activation rows 8 nt + 2t, + 1); only the first L groups of eight rows are computed.  SPLIT: two accumulators of a block, half
-// the dependent MMAs in a row.  A row's sum is the same for every L.
+// the dependent MMAs in a row.  A row's sum is the same for every L of one SPLIT.
 template <int NT, int L, bool SPLIT>
 __device__ __forceinline__ void block_q4k(uint32_t r0, uint32_t r1, uint32_t img, int lane, uint32_t mg,
                                           float (&acc)[NT][4]) {
@@ -428,15 +429,16 @@ __device__ __forceinline__ float4 ldcg4(const float* p) {
   return v;
 }
 
-// Eight consecutive columns (8 * lane) of a block of an activation row, as the fp16 fragments the kernel above loads: x over the power of two of the block's largest value; the sums of the rounded values per 32 columns in two parts.
-// (`also`: a second place to write to, or null)
+// Eight consecutive columns (8 * lane) of a block of an activation row, as the fp16 fragments that the products load: x over the
+// power of two of the block's largest value (at most 2^126, whose reciprocal is the smallest normal number: up to 4 then); the
+// sums of the rounded values per 32 columns in two parts.  (`also`: a second place to write to, or null)
 __device__ __forceinline__ void image_store(uint8_t* unit, uint8_t* also, int lane, const float (&v)[8]) {
   float amax = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
   bool odd = false;                     // a NaN or an infinity stays one, under scale 1
 #pragma unroll
-  for (int i = 0; i < 8; ++i) odd |= !(fabsf(v[i]) <= 3.0e38f);
+  for (int i = 0; i < 8; ++i) odd |= !(fabsf(v[i]) <= FLT_MAX);
   amax = warp_max(amax);
   uint32_t e = min(__float_as_uint(amax) & 0x7F800000u, 0x7E800000u);
   if (__any_sync(0xffffffffu, odd)) e = 0x3F800000u;

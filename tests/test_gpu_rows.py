@@ -152,20 +152,22 @@ def test_segments_pairs_norm_side_rows(space):
 
 
 def test_extreme_rows(space):
-    """Zero rows, the largest and smallest normal numbers, and a NaN that stays in its own row."""
+    """Zero rows, large and small numbers up to the largest of all, and a NaN that stays in its own row."""
     from hipengine_b200.ops import kernels as K
     w, wd = _weight(T.Q4_K, 128, 512, 9)
-    x = torch.randn(6, 512, device="cuda")
+    x = torch.randn(7, 512, device="cuda")
     x[0] = 0
     x[1] *= 1e30
     x[2] *= 1e-30
     x[3, 5] = float("nan")
     x[4, 7] = float("inf")
-    out = torch.zeros(6, 128, device="cuda")
+    x[6] *= 1e38 / x[6].abs().max()
+    x[6, 300] = torch.finfo(torch.float32).max
+    out = torch.zeros(7, 128, device="cuda")
     space.gemm(x, [K.GemvSegment(w, out)])
     ref = x.double() @ wd.t()
     assert bool((out[0] == 0).all()) and bool(out[3].isnan().all()) and not bool(out[4].isfinite().any())
-    for r in (1, 2, 5):
+    for r in (1, 2, 5, 6):
         assert float((out[r].double() - ref[r]).norm() / ref[r].norm()) < 2 ** -11
 
 
