@@ -1,10 +1,11 @@
 // Products of a few activation rows (1..64) with QUANTISED weights (Q4_K / Q6_K / Q8_0 in their device layouts):
 // out[r][n] = sum_k x[r][k] W[n][k], the weights streamed once whatever the row count.  Decode steps, verify chains and
-// short prompts are these products and little else.
+// short prompts are these products and little else.  This file: the rows' image for all of them, and the products of up to 24
+// rows on mma.sync; more rows run on tcgen05 (gemm_rows_tc.cu; ops/rows.py has the line).
 //
-// What has to move is the weight stream (HBM).  What bounds it in fact (17408 x 5120 Q4_K, 4 / 16 / 64 rows): up to 16 rows ramp,
+// What has to move is the weight stream (HBM).  What bounds it in fact (17408 x 5120 Q4_K, 4 / 16 rows: 18.4 / 22.2 us): ramp,
 // image wait and the sum of shared tiles around a steady part that the expansion of blocks sets (DRAM 25 / 22 %, issue 44 / 43 %,
-// tensor pipe 14 / 23 %); at 64 rows the reads of the image and mma.sync (shared memory 59 %, tensor pipe 45 %, DRAM 11 %).
+// tensor pipe 14 / 23 %).
 //   operands : fp16 m16n8k16 MMAs with the WEIGHT as the A operand.  A k-quant weight is d * (sc * q) - dmin * m with
 //              sc * q an integer below 2^10 and m one below 2^6: both are exact in fp16, so ONE packed fp16 FMA makes two
 //              operands (1024 + q is the nibble under an exponent byte; (1024 + q) * sc - 1024 * sc), the 256-column block
@@ -12,9 +13,8 @@
 //              the activations per 32 columns (as an fp16 high and low part).  Q8_0, and Q6_K up to 8 rows: the integers
 //              themselves are the operands, an MMA (two for Q8_0) covers one sub-block, and the sub-block's scale meets
 //              its fp32 sums: exact as well, and for Q8_0 cheaper than a product per operand (17408 x 5120, 4 / 16 / 32 rows
-//              24.7 / 29.2 / 48.1 -> 21.4 / 24.0 / 42.5 us; 64 rows 51.0 -> 52.4).  Q6_K above 8 rows: sc * (q - 32), 13
-//              bits, rounded to 11: the exact form costs two packed FMAs per MMA (17408 x 5120, 16 / 32 / 64 rows 27.5 / 40.7
-//              / 55.2 us against 25.0 / 35.2 / 44.5; at 8 rows 22.1 against 22.8).
+//              24.7 / 29.2 / 48.1 -> 21.4 / 24.0 / 42.5 us).  Q6_K above 8 rows: sc * (q - 32), 13 bits, rounded to 11: the exact
+//              form costs two packed FMAs per MMA (17408 x 5120, 16 rows 27.5 us against 25.0; at 8 rows 22.1 against 22.8).
 //   activations: fp16 under a power of two per row and block of 256 columns, 11 bits each down to 2^-14 of the block's largest
 //              value and 2^-25 of it below (bf16 values down to 2^-17 of it exactly), written once per launch by he_rows_image
 //              in the order of the MMA's B fragments (one 16-byte load per lane feeds two MMAs), so no CTA repeats the
@@ -26,9 +26,10 @@
 //              per SM (equal to one unit), so there is no last wave.  A tile that several CTAs share leaves fp32 partial
 //              tiles in `ws`; whoever arrives last (a counter per tile, reset by it) adds them in CTA order:
 //              bit-reproducible for a given number of rows.  (A row's last bits depend on that number: up to 16 rows sum a
-//              block in two chains, up to 32 two warp groups take every other block, above that neither.)
+//              block in two chains, more in one, on tcgen05 in the order of its sums.)  The host divides: with the CTAs' ranges
+//              from eight 64-bit divisions a thread and old residual values loaded one by one 4 / 16 rows took 20.0 / 23.1 us.
 //   roles    : one producer warp (TMA boxes of weight rows x 1 block, bulk copies of the image), one warp that signals shared
-//              tiles, 8 or 16 MMA warps.  The ring holds ~200 KB: with programmatic dependent launch the
+//              tiles, 16 MMA warps.  The ring holds ~200 KB: with programmatic dependent launch the
 //              next product's weights arrive while the previous kernels drain.
 //
 // Counterparts in the reference: hipengine/kernels/hip_gfx1100/quant/gguf_q4_k_gemv.hip and the packed-row forms in
@@ -38,37 +39,7 @@
 using namespace he;
 using namespace herows;
 
-constexpr int ROWS_MAX_SEG = 4;
-
-struct HeRowsSeg {
-  const void* w;
-  const void* w2;          // second weight of a gate/up pair (epi 3, 4), same block type
-  void* out;
-  long long out_stride;    // elements between the outputs of two activation rows
-  int n_rows;
-  int qtype;
-  int epi;                 // 0: f32 store, 1: bf16 store, 2: f32 +=, 3: silu(g) * u -> bf16, 4: gelu_tanh(g) * u -> bf16
-  int tile0;               // first tile of the segment (set by the launcher)
-};
-
-struct HeRowsArgs {
-  HeRowsSeg seg[ROWS_MAX_SEG];
-  int n_seg;
-  int K, R;
-  const void* image;       // he_rows_image of the R rows
-  float* ws;               // partial tiles: 2 * SMs * 128 * (R rounded up to 8) floats
-  long long ws_floats;
-  int* counters;           // zero before the first launch; every launch leaves them zero
-  int n_counters;
-  int* status;
-  int stages, stage_bytes, w_bytes, tiles;   // set by the launcher
-};
-
 namespace {
-
-struct RowsMaps {
-  CUtensorMap m[ROWS_MAX_SEG][4];   // [2 * (second weight of a pair) + (scale plane of Q8_0)]
-};
 
 struct RowsShared {
   uint64_t full[MAX_STAGES];
@@ -79,35 +50,30 @@ struct RowsShared {
 
 constexpr int TILE = 128, HALF = 64;                  // weight rows of a tile; of a TMA box, of each weight of a pair
 
-// MMA warps: eight side by side, 16 weight rows each; up to 32 activation rows a second group of eight takes every other
-// block (their sums meet in shared memory at the end of a tile), for more the accumulators leave no registers for it.
-// Measured against this: 8 warps of 32 rows and 16 warps side by side over 256 rows, both slower for one of the widths.
+// MMA warps: two groups of eight side by side, 16 weight rows each, that take every other block (their sums meet in shared memory
+// at the end of a tile).
+constexpr int MMA_WARPS = 16, THREADS = MMA_WARPS * 32 + 64;       // + producer warp + signal warp
 template <int NT>
 struct Shape {
-  static constexpr int GROUPS = NT <= 4 ? 2 : 1;
-  static constexpr int MMA_WARPS = 8 * GROUPS, THREADS = MMA_WARPS * 32 + 64;   // + producer warp + signal warp
-  static constexpr int XBUF = GROUPS == 2 ? TILE * 8 * NT * 4 : 0;              // exchange of the second group's sums
+  static constexpr int XBUF = TILE * 8 * NT * 4;                   // exchange of the second group's sums
 };
 
 template <int NT>
-__global__ void __launch_bounds__(Shape<NT>::THREADS, 1)
-rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ HeRowsArgs a) {
+__global__ void __launch_bounds__(THREADS, 1)
+rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ HeRowsArgs a, const RowsPlan plan) {
   using S = Shape<NT>;
-  constexpr bool SPLIT = NT <= 2;                                  // registers for more sums than that are not left
   constexpr int IMG = IMG_COL * 8 * NT, SLOT = TILE * 8 * NT;      // image bytes of a block, floats of a partial tile
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   float* xbuf = reinterpret_cast<float*>(smem + (size_t)a.stages * a.stage_bytes);
   RowsShared* sh = reinterpret_cast<RowsShared*>(smem + (size_t)a.stages * a.stage_bytes + S::XBUF);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nb = a.K >> 8, U = a.tiles * nb, G = gridDim.x, b = blockIdx.x;
-  const int u0 = (int)((long long)U * b / G), u1 = (int)((long long)U * (b + 1) / G);
+  const int nb = a.K >> 8, b = blockIdx.x, u0 = plan.begin(b), u1 = plan.begin(b + 1);
   // CTAs that share a tile: those that hold its first and last unit and all between
-  const auto first_cta = [&](int tile) { return (int)((((long long)tile * nb + 1) * G - 1) / U); };
-  const auto last_cta = [&](int tile) { return (int)((((long long)tile + 1) * nb * G - 1) / U); };
+  const auto first_cta = [&](int tile) { return plan.cta_of(tile * nb); };
+  const auto last_cta = [&](int tile) { return plan.cta_of((tile + 1) * nb - 1); };
   const int tile_a = u0 / nb, tile_z = (u1 - 1) / nb;           // only the first and the last tile can be shared
-  const bool share_a = first_cta(tile_a) != last_cta(tile_a);
-  const bool share_z = tile_z != tile_a && first_cta(tile_z) != last_cta(tile_z);
+  const bool share_a = u0 > tile_a * nb || u1 < (tile_a + 1) * nb, share_z = tile_z != tile_a && u1 < (tile_z + 1) * nb;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < a.stages; ++s) {
@@ -121,8 +87,8 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
   pdl_launch();
   volatile int* abort_flag = &sh->abort_flag;
 
-  if (warp >= S::MMA_WARPS) {
-    if (warp == S::MMA_WARPS) {
+  if (warp >= MMA_WARPS) {
+    if (warp == MMA_WARPS) {
       // ------------------------------------------------------------ producer
       if (sm100::elect_one()) {
         const uint8_t* image = reinterpret_cast<const uint8_t*>(a.image);
@@ -202,10 +168,10 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
 
   // -------------------------------------------------------------- MMA warps
   const uint32_t mg = opaque(MAGIC);
-  const int grp = S::GROUPS == 2 ? warp >> 3 : 0, w = warp & 7, g = lane >> 2, t = lane & 3;
+  const int grp = warp >> 3, w = warp & 7, g = lane >> 2, t = lane & 3;
   pdl_wait();
-  // this group's stages: every one, or (two groups) the slots of its parity
-  const uint32_t ring = sm100::smem_u32(smem), step = (uint32_t)(S::GROUPS * a.stage_bytes);
+  // this group's stages: the slots of its parity
+  const uint32_t ring = sm100::smem_u32(smem), step = (uint32_t)(2 * a.stage_bytes);
   const uint32_t first = ring + (uint32_t)(grp * a.stage_bytes), end = ring + (uint32_t)(a.stages * a.stage_bytes);
   const uint32_t w_bytes = (uint32_t)a.w_bytes;
   uint32_t st = first, ph = 0;
@@ -227,6 +193,17 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
         }
       return;
     }
+    // a residual's old values first, all of them: they could lie where the stores go, for the compiler
+    float old[NT][4];
+    if (sg.epi == 2) {
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int row = tl * TILE + 16 * w + g + 8 * (i >> 1), r = 8 * n + 2 * t + (i & 1);
+          old[n][i] = row < sg.n_rows && r < a.R ? reinterpret_cast<const float*>(sg.out)[(size_t)r * sg.out_stride + row] : 0.f;
+        }
+    }
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       const int row = tl * TILE + 16 * w + g + 8 * k;
@@ -239,9 +216,8 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
           if (r >= a.R) continue;
           const size_t off = (size_t)r * sg.out_stride + row;
           const float v = acc[n][2 * k + j];
-          if (sg.epi == 0) reinterpret_cast<float*>(sg.out)[off] = v;
-          else if (sg.epi == 1) reinterpret_cast<__nv_bfloat16*>(sg.out)[off] = f32_to_bf16(v);
-          else reinterpret_cast<float*>(sg.out)[off] += v;
+          if (sg.epi == 1) reinterpret_cast<__nv_bfloat16*>(sg.out)[off] = f32_to_bf16(v);
+          else reinterpret_cast<float*>(sg.out)[off] = sg.epi == 2 ? old[n][2 * k + j] + v : v;
         }
     }
   };
@@ -265,17 +241,17 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
     float acc[NT][4];
 #pragma unroll
     for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
-    const int skip = S::GROUPS == 2 ? (u - u0 + grp) & 1 : 0;    // the tile's first unit is the other group's
+    const int skip = (u - u0 + grp) & 1;    // the tile's first unit is the other group's
     auto blocks = [&](auto&& one) {
-      for (int i = skip; i < n_blk; i += S::GROUPS) {
+      for (int i = skip; i < n_blk; i += 2) {
         if (wait_long(full, ph, abort_flag, a.status, 402)) {
           one(st, st + w_bytes);
           __syncwarp();
           if (lane == 0) sm100::mbar_arrive(empty);
         }
         st += step;
-        full += S::GROUPS;
-        empty += S::GROUPS;
+        full += 2;
+        empty += 2;
         if (st >= end) {
           st = first;
           full = sh->full + grp;
@@ -286,35 +262,33 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
     };
     if (qtype == HE_Q4_K) {
       const uint32_t o0 = p0 + i0 * 144, o1 = p1 + i1 * 144;
-      blocks([&](uint32_t st0, uint32_t img) { block_q4k<NT, NT, SPLIT>(st0 + o0, st0 + o1, img, lane, mg, acc); });
+      blocks([&](uint32_t st0, uint32_t img) { block_q4k<NT, NT, NT <= 2>(st0 + o0, st0 + o1, img, lane, mg, acc); });
     } else if (qtype == HE_Q6_K) {
       const uint32_t o0 = p0 + i0 * 224, o1 = p1 + i1 * 224;
       blocks([&](uint32_t st0, uint32_t img) {
         if constexpr (NT == 1) block_q6k_exact<NT, NT>(st0 + o0, st0 + o1, img, lane, mg, acc);
-        else block_q6k<NT, NT, SPLIT>(st0 + o0, st0 + o1, img, lane, mg, acc);
+        else block_q6k<NT, NT, NT <= 2>(st0 + o0, st0 + o1, img, lane, mg, acc);
       });
     } else {
       blocks([&](uint32_t st0, uint32_t img) { block_q80<NT, NT, HALF>(st0 + p0, i0, st0 + p1, i1, img, lane, mg, acc); });
     }
     u += n_blk;
-    if (S::GROUPS == 2) {
-      float4* xb = reinterpret_cast<float4*>(xbuf) + w * NT * 32 + lane;
-      if (grp == 1) {
-        if (wrote) named_sync(5, 512);          // group 0 has read the previous tile's sums
-        wrote = true;
+    float4* xb = reinterpret_cast<float4*>(xbuf) + w * NT * 32 + lane;
+    if (grp == 1) {
+      if (wrote) named_sync(5, 512);          // group 0 has read the previous tile's sums
+      wrote = true;
 #pragma unroll
-        for (int n = 0; n < NT; ++n) xb[n * 32] = make_float4(acc[n][0], acc[n][1], acc[n][2], acc[n][3]);
-        named_arrive(4, 512);
-        continue;
-      }
-      named_sync(4, 512);
-#pragma unroll
-      for (int n = 0; n < NT; ++n) {
-        const float4 v = xb[n * 32];
-        acc[n][0] += v.x; acc[n][1] += v.y; acc[n][2] += v.z; acc[n][3] += v.w;
-      }
-      named_arrive(5, 512);
+      for (int n = 0; n < NT; ++n) xb[n * 32] = make_float4(acc[n][0], acc[n][1], acc[n][2], acc[n][3]);
+      named_arrive(4, 512);
+      continue;
     }
+    named_sync(4, 512);
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      const float4 v = xb[n * 32];
+      acc[n][0] += v.x; acc[n][1] += v.y; acc[n][2] += v.z; acc[n][3] += v.w;
+    }
+    named_arrive(5, 512);
     if ((tile == tile_a && share_a) || (tile == tile_z && share_z)) {
       // a partial tile: the CTA's own slot 1 if it holds the tile's first unit, else slot 0
       float* mine = a.ws + (size_t)(2 * b + (blk0 == 0 ? 1 : 0)) * SLOT + (w * NT * 32 + lane) * 4;
@@ -327,7 +301,7 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
     }
     epilogue(sg, tile, acc);
   }
-  if (S::GROUPS == 2 && grp == 1) {
+  if (grp == 1) {
     if (wrote) named_sync(5, 512);
     return;
   }
@@ -340,14 +314,22 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
     float acc[NT][4];
 #pragma unroll
     for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
-    for (int c = c0; c <= c1; ++c) {
-      // the first of them holds the tile's first unit (slot 1 of its CTA), the others' ranges start inside it (slot 0)
-      const float* p = a.ws + (size_t)(2 * c + (c == c0 ? 1 : 0)) * SLOT + (w * NT * 32 + lane) * 4;
+    constexpr int FLY = NT == 1 ? 8 : 4;         // partial tiles in flight (one after the other each took a trip to L2)
+    for (int c = c0; c <= c1; c += FLY) {
+      float4 v[FLY][NT];
 #pragma unroll
-      for (int n = 0; n < NT; ++n) {
-        const float4 v = ldcg4(p + n * 128);
-        acc[n][0] += v.x; acc[n][1] += v.y; acc[n][2] += v.z; acc[n][3] += v.w;
+      for (int e = 0; e < FLY; ++e) {
+        // the first of them holds the tile's first unit (slot 1 of its CTA), the others' ranges start inside it (slot 0)
+        const float* p = a.ws + (size_t)(2 * (c + e) + (c + e == c0 ? 1 : 0)) * SLOT + (w * NT * 32 + lane) * 4;
+#pragma unroll
+        for (int n = 0; n < NT; ++n) v[e][n] = c + e <= c1 ? ldcg4(p + n * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
+#pragma unroll
+      for (int e = 0; e < FLY; ++e)
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+          acc[n][0] += v[e][n].x; acc[n][1] += v[e][n].y; acc[n][2] += v[e][n].z; acc[n][3] += v[e][n].w;
+        }
     }
     epilogue(a.seg[segment(tile)], tile, acc);
   }
@@ -421,9 +403,10 @@ __device__ void side_rows(const float* w, int n, int n0, float* out, long long l
 
 // With a norm: one CTA per row, the row kept in registers between the statistics and the fragments (up to 4 blocks a
 // warp), a warp per block; CTAs from `R` on take two side rows each.  Without: the blocks of a row are spread over CTAs.
+template <bool TC>                    // the image for tcgen05
 __global__ void __launch_bounds__(512) rows_image_kernel(const void* __restrict__ x, int x_dtype, long long x_stride,
                                                          const float* __restrict__ norm_w, float eps, int K, int R,
-                                                         int blk_units, int parts, uint8_t* __restrict__ image,
+                                                         int pad_rows, int parts, uint8_t* __restrict__ image,
                                                          uint8_t* __restrict__ by_row,
                                                          const float* __restrict__ side_w, int side_n,
                                                          float* __restrict__ side_out, long long side_ld) {
@@ -439,8 +422,9 @@ __global__ void __launch_bounds__(512) rows_image_kernel(const void* __restrict_
   const int nw = (int)(blockDim.x >> 5) * parts, w0 = (int)(blockIdx.x % parts) * (int)(blockDim.x >> 5) + warp;
   const auto store = [&](int blk, const float (&v)[8]) {
     uint8_t* row = by_row == nullptr ? nullptr : by_row + ((size_t)r * nb + blk) * IMG_COL;
-    if (image == nullptr) image_store(row, nullptr, lane, v);
-    else image_store(image + ((size_t)blk * blk_units + r) * IMG_COL, row, lane, v);
+    if (TC) image_store<true>(image + (size_t)blk * tc_image(pad_rows), row, pad_rows, r, lane, v);
+    else if (image == nullptr) image_store<false>(row, nullptr, 0, 0, lane, v);
+    else image_store<false>(image + ((size_t)blk * pad_rows + r) * IMG_COL, row, 0, 0, lane, v);
   };
   constexpr int KEEP = 4;
   float nwv[KEEP][8];
@@ -515,9 +499,9 @@ int launch_rows(HeRowsArgs a, int num_sms, cudaStream_t stream) {
   a.stage_bytes = (a.w_bytes + IMG + 1023) & ~1023;
   a.stages = (SMEM_TOTAL - S::XBUF - (int)sizeof(RowsShared) - 1024) / a.stage_bytes;
   if (a.stages > MAX_STAGES) a.stages = MAX_STAGES;
-  // two groups: an even ring, so that a slot always belongs to one group.  A phase bit tells only neighbours apart: a
+  // an even ring, so that a slot always belongs to one group.  A phase bit tells only neighbours apart: a
   // group that skipped the other group's use of a slot could take the phase before that use for its own
-  if (S::GROUPS == 2) a.stages &= ~1;
+  a.stages &= ~1;
   if (a.stages < 2) return -HE_ERR_BAD_ARG;
   const size_t smem = (size_t)a.stages * a.stage_bytes + S::XBUF + sizeof(RowsShared) + 1024;
   static std::atomic<unsigned long long> allowed{0};
@@ -525,17 +509,20 @@ int launch_rows(HeRowsArgs a, int num_sms, cudaStream_t stream) {
   if (e != cudaSuccess) return (int)e;
   const long long units = (long long)a.tiles * (a.K >> 8);
   const int grid = (int)(units < num_sms ? units : num_sms);
-  if (2ll * grid * TILE * 8 * NT > a.ws_floats || a.tiles > a.n_counters) return -HE_ERR_BAD_ARG;
-  return (int)launch_pdl(rows_gemm_kernel<NT>, dim3(grid), dim3(S::THREADS), smem, stream, maps, a);
+  if (units > 0x7FFFFFFF || 2ll * grid * TILE * 8 * NT > a.ws_floats || a.tiles > a.n_counters) return -HE_ERR_BAD_ARG;
+  return (int)launch_pdl(rows_gemm_kernel<NT>, dim3(grid), dim3(THREADS), smem, stream, maps, a,
+                         RowsPlan{(int)(units / grid), (int)(units % grid)});
 }
 
 }  // namespace
 
 // Bytes of the activation image of R rows of K columns.
-HE_API long long he_rows_image_bytes(int R, int K) { return (long long)(K >> 8) * col_groups(R) * 8 * IMG_COL; }
+HE_API long long he_rows_image_bytes(int R, int K, int tc) {
+  return (long long)(K >> 8) * (tc ? tc_image(tc_rows(R)) : col_groups(R) * 8 * IMG_COL);
+}
 // Floats of the partial-tile workspace for R rows.
-HE_API long long he_rows_ws_floats(int R, int num_sms) {
-  return 2ll * num_sms * TILE * col_groups(R) * 8;
+HE_API long long he_rows_ws_floats(int R, int num_sms, int tc) {
+  return 2ll * num_sms * TILE * (tc ? tc_rows(R) : col_groups(R) * 8);
 }
 
 // Images of (RMSNorm with norm_w of) the R rows x[r][0..K), fp32 or bf16.  K % 256 == 0, 16-byte rows.  `image` (may be
@@ -544,9 +531,9 @@ HE_API long long he_rows_ws_floats(int R, int num_sms) {
 // With `side_n` > 0 (at most 64 rows) also side_out[r][j] = (normalised row r) . side_w[j], j < side_n: fp32 weights
 // [side_n][K], in fp32.
 HE_API int he_rows_image(const void* x, int x_dtype, long long x_stride, const float* norm_w, float eps, int K, int R,
-                         void* image, void* by_row, const float* side_w, int side_n, float* side_out, long long side_ld,
+                         void* image, int tc, void* by_row, const float* side_w, int side_n, float* side_out, long long side_ld,
                          cudaStream_t stream) {
-  if (K <= 0 || K % 256 != 0 || R < 1 || ((image != nullptr || side_n > 0) && R > 64) || x == nullptr ||
+  if (K <= 0 || K % 256 != 0 || R < 1 || ((image != nullptr || side_n > 0) && R > (image != nullptr && !tc ? MMA_MAX_ROWS : 64)) || x == nullptr ||
       (image == nullptr && by_row == nullptr && side_n <= 0) || (reinterpret_cast<uintptr_t>(by_row) & 15) != 0)
     return -HE_ERR_BAD_ARG;
   const int es = x_dtype == 0 ? 4 : 2;
@@ -554,6 +541,7 @@ HE_API int he_rows_image(const void* x, int x_dtype, long long x_stride, const f
       (reinterpret_cast<uintptr_t>(norm_w) & 15) != 0 || (reinterpret_cast<uintptr_t>(image) & 15) != 0)
     return -HE_ERR_BAD_ARG;
   const int nb = K >> 8;
+  if (image == nullptr) tc = 0;
   size_t smem = 0;
   if (side_n > 0) {
     if (norm_w == nullptr || side_w == nullptr || side_out == nullptr || (reinterpret_cast<uintptr_t>(side_w) & 15) != 0)
@@ -561,14 +549,14 @@ HE_API int he_rows_image(const void* x, int x_dtype, long long x_stride, const f
     smem = (size_t)2 * K * sizeof(float);
     constexpr int most = 200 * 1024;
     if (smem > most) return -HE_ERR_BAD_ARG;
-    static std::atomic<unsigned long long> allowed{0};
-    const cudaError_t e = allow_smem(rows_image_kernel, most, allowed);
+    static std::atomic<unsigned long long> allowed[2];
+    const cudaError_t e = tc ? allow_smem(rows_image_kernel<true>, most, allowed[1]) : allow_smem(rows_image_kernel<false>, most, allowed[0]);
     if (e != cudaSuccess) return (int)e;
   }
   const int parts = image == nullptr && by_row == nullptr ? 0 : norm_w != nullptr ? 1 : (nb + 3) / 4;
   const unsigned grid = (unsigned)(R * parts + (side_n > 0 ? (side_n + 1) / 2 : 0));
-  return (int)launch_pdl(rows_image_kernel, dim3(grid), dim3(norm_w != nullptr ? 512 : 128), smem, stream, x, x_dtype,
-                         x_stride, norm_w, eps, K, R, col_groups(R) * 8, parts, (uint8_t*)image, (uint8_t*)by_row, side_w, side_n,
+  return (int)launch_pdl(tc ? rows_image_kernel<true> : rows_image_kernel<false>, dim3(grid), dim3(norm_w != nullptr ? 512 : 128), smem, stream, x, x_dtype,
+                         x_stride, norm_w, eps, K, R, tc ? tc_rows(R) : col_groups(R) * 8, parts, (uint8_t*)image, (uint8_t*)by_row, side_w, side_n,
                          side_out, side_ld);
 }
 
@@ -578,14 +566,12 @@ HE_API int he_rows_gemm(const HeRowsArgs* args, int num_sms, cudaStream_t stream
       a.image == nullptr || a.ws == nullptr || a.counters == nullptr || (reinterpret_cast<uintptr_t>(a.image) & 15) != 0 ||
       (reinterpret_cast<uintptr_t>(a.ws) & 15) != 0)
     return -HE_ERR_BAD_ARG;
+  if (a.tc) return launch_rows_tc(a, num_sms, stream);
   switch (col_groups(a.R)) {
     case 1: return launch_rows<1>(a, num_sms, stream);
     case 2: return launch_rows<2>(a, num_sms, stream);
     case 3: return launch_rows<3>(a, num_sms, stream);
-    case 4: return launch_rows<4>(a, num_sms, stream);
-    case 5: return launch_rows<5>(a, num_sms, stream);
-    case 6: return launch_rows<6>(a, num_sms, stream);
-    default: return launch_rows<8>(a, num_sms, stream);
+    default: return -HE_ERR_BAD_ARG;
   }
 }
 HE_API int he_rows_args_size() { return (int)sizeof(HeRowsArgs); }

@@ -8,6 +8,33 @@
 #include "sm100.cuh"
 #include "tmap.cuh"
 
+constexpr int ROWS_MAX_SEG = 4;
+
+struct HeRowsSeg {
+  const void* w;
+  const void* w2;          // second weight of a gate/up pair (epi 3, 4), same block type
+  void* out;
+  long long out_stride;    // elements between the outputs of two activation rows
+  int n_rows;
+  int qtype;
+  int epi;                 // 0: f32 store, 1: bf16 store, 2: f32 +=, 3: silu(g) * u -> bf16, 4: gelu_tanh(g) * u -> bf16
+  int tile0;               // first tile of the segment (set by the launcher)
+};
+
+struct HeRowsArgs {
+  HeRowsSeg seg[ROWS_MAX_SEG];
+  int n_seg;
+  int K, R;
+  int tc;                  // products and image on tcgen05 (up to 64 rows), else on mma.sync (up to MMA_MAX_ROWS)
+  const void* image;       // he_rows_image of the R rows, with the same `tc`
+  float* ws;               // partial tiles (he_rows_ws_floats)
+  long long ws_floats;
+  int* counters;           // zero before the first launch; every launch leaves them zero
+  int n_counters;
+  int* status;
+  int stages, stage_bytes, w_bytes, tiles;   // set by the launcher
+};
+
 namespace herows {
 
 using namespace he;
@@ -17,14 +44,22 @@ using namespace he;
 // bytes of parts 0 and 1 hold the eight sums per 32 columns in two parts, those of part 2 the scale.  With them lanes that read one
 // part and lanes that read one place of four parts both meet no bank twice; 576 bytes put neighbouring rows half a bank cycle apart.
 constexpr int IMG_COL = 576, PART = 144, SX_OFF = 128, XS_OFF = 2 * PART + 128;
+// Products of more rows than a few run on tcgen05 (gemm_rows_tc.cu), from an image of their own: of one block of n rows (32, 48 or 64)
+//   [4 groups of 64 columns][n rows][128 bytes], 128-byte swizzle : the B operand, columns of a quad in the order 0 2 1 3
+//   [n / 8][2: high, low parts][8 rows][8 sums per 32 columns], fp16: the B operand of the minima (no swizzle)
+//   [n] fp32                                                      : the rows' powers of two
+constexpr int MMA_MAX_ROWS = 24;
+__host__ __device__ constexpr int tc_rows(int R) { return R <= 32 ? 32 : (R + 15) & ~15; }
+__host__ __device__ constexpr int tc_sums(int n) { return n * 512; }
+__host__ __device__ constexpr int tc_scales(int n) { return n * 544; }
+__host__ __device__ constexpr int tc_image(int n) { return n * 548; }
+__host__ __device__ constexpr int tc_image_pad(int n) { return (tc_image(n) + 1023) & ~1023; }
+
 constexpr int MAX_STAGES = 8;
 constexpr int SMEM_TOTAL = 220 * 1024;
 
 __host__ __device__ inline int rows_block_bytes(int qt) { return qt == HE_Q4_K ? 144 : qt == HE_Q6_K ? 224 : 272; }
-__host__ __device__ inline int col_groups(int R) {             // n8 tiles of R rows
-  const int n = (R + 7) / 8;
-  return n == 7 ? 8 : n;
-}
+__host__ __device__ inline int col_groups(int R) { return (R + 7) / 8; }       // n8 tiles of R rows
 
 __device__ __forceinline__ uint4 lds128(uint32_t a) {
   uint4 v;
@@ -431,8 +466,10 @@ __device__ __forceinline__ float4 ldcg4(const float* p) {
 
 // Eight consecutive columns (8 * lane) of a block of an activation row, as the fp16 fragments that the products load: x over the
 // power of two of the block's largest value (at most 2^126, whose reciprocal is the smallest normal number: up to 4 then); the
-// sums of the rounded values per 32 columns in two parts.  (`also`: a second place to write to, or null)
-__device__ __forceinline__ void image_store(uint8_t* unit, uint8_t* also, int lane, const float (&v)[8]) {
+// sums of the rounded values per 32 columns in two parts.  Into the row's unit `unit` or, TC, as row r of the block's image `unit` of n
+// rows; and into the row's unit `also` (or null).
+template <bool TC>
+__device__ __forceinline__ void image_store(uint8_t* unit, uint8_t* also, int n, int r, int lane, const float (&v)[8]) {
   float amax = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
@@ -452,28 +489,43 @@ __device__ __forceinline__ void image_store(uint8_t* unit, uint8_t* also, int la
   }
   s += __shfl_xor_sync(0xffffffffu, s, 1);
   s += __shfl_xor_sync(0xffffffffu, s, 2);
+  const int sub = lane >> 2;
+  if (TC) {
+    const __half2 p[4] = {__halves2half2(hv[0], hv[2]), __halves2half2(hv[1], hv[3]), __halves2half2(hv[4], hv[6]),
+                          __halves2half2(hv[5], hv[7])};
+    *reinterpret_cast<uint4*>(unit + (lane >> 3) * n * 128 + r * 128 + (((lane & 7) ^ (r & 7)) << 4)) =
+        *reinterpret_cast<const uint4*>(p);
+    if ((lane & 3) == 0) {
+      const __half hi = __float2half_rn(s), lo = __float2half_rn(s - __half2float(hi));
+      uint8_t* at = unit + tc_sums(n) + (r >> 3) * 256 + (r & 7) * 16 + sub * 2;
+      *reinterpret_cast<__half*>(at) = hi;
+      *reinterpret_cast<__half*>(at + 128) = lo;
+    }
+    if (lane == 0) *reinterpret_cast<float*>(unit + tc_scales(n) + r * 4) = __uint_as_float(e);
+    if (also == nullptr) return;
+    unit = also;
+  }
   const int h = lane >> 4, qt = (lane >> 2) & 3, u = (lane >> 1) & 1, v0 = (lane & 1) * 2, t = 2 * h + u;
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
     __half2 p[2] = {__halves2half2(hv[4 * q], hv[4 * q + 2]), __halves2half2(hv[4 * q + 1], hv[4 * q + 3])};
     const int at = (v0 + q) * PART + (qt >> 1) * 64 + t * 16 + (qt & 1) * 8;
     *reinterpret_cast<uint2*>(unit + at) = *reinterpret_cast<const uint2*>(p);
-    if (also != nullptr) *reinterpret_cast<uint2*>(also + at) = *reinterpret_cast<const uint2*>(p);
+    if (!TC && also != nullptr) *reinterpret_cast<uint2*>(also + at) = *reinterpret_cast<const uint2*>(p);
   }
   if ((lane & 3) == 0) {
-    const int sub = lane >> 2;
     const __half hi = __float2half_rn(s), lo = __float2half_rn(s - __half2float(hi));
     const int at = SX_OFF + (sub >> 2) * PART + ((sub >> 1) & 1) * 8 + (sub & 1) * 2;
     *reinterpret_cast<__half*>(unit + at) = hi;
     *reinterpret_cast<__half*>(unit + at + 4) = lo;
-    if (also != nullptr) {
+    if (!TC && also != nullptr) {
       *reinterpret_cast<__half*>(also + at) = hi;
       *reinterpret_cast<__half*>(also + at + 4) = lo;
     }
   }
   if (lane == 0) {
     *reinterpret_cast<float*>(unit + XS_OFF) = __uint_as_float(e);
-    if (also != nullptr) *reinterpret_cast<float*>(also + XS_OFF) = __uint_as_float(e);
+    if (!TC && also != nullptr) *reinterpret_cast<float*>(also + XS_OFF) = __uint_as_float(e);
   }
 }
 
@@ -528,5 +580,23 @@ inline int weight_maps(CUtensorMap* m, const void* w, int qtype, long long rows,
   const int rc = byte_map(m, w, rows, rb, 128, true, box);
   return rc != 0 ? rc : byte_map(m + 1, w, rows, rb, 16, false, box);
 }
+
+struct RowsMaps {
+  CUtensorMap m[ROWS_MAX_SEG][4];   // [2 * (second weight of a pair) + (scale plane of Q8_0)]
+};
+
+// Units per CTA: the first `rem` take base + 1, the others base.  (Divided once, by the host: eight 64-bit divisions a thread were
+// 3 us at the start of every launch.)
+struct RowsPlan {
+  int base, rem;
+  __host__ __device__ int begin(int cta) const { return base * cta + (cta < rem ? cta : rem); }
+  __host__ __device__ int cta_of(int unit) const {
+    const unsigned big = (unsigned)rem * (unsigned)(base + 1), x = (unsigned)unit;
+    return x < big ? (int)(x / (unsigned)(base + 1)) : rem + (int)((x - big) / (unsigned)base);
+  }
+};
+
+// Products of up to 64 rows on tcgen05 (gemm_rows_tc.cu)
+int launch_rows_tc(const HeRowsArgs& a, int num_sms, cudaStream_t stream);
 
 }  // namespace herows

@@ -215,7 +215,8 @@ class HybridExecutor:
         # the gates of the delta rule stay fp32: they ride with the rows' image (one matrix, alpha rows then beta rows)
         self.ab_f32 = {i: torch.cat([self.F(i, "ssm_alpha.weight"), self.F(i, "ssm_beta.weight")], 0).contiguous()
                        for i in range(cfg.n_layers) if not cfg.is_full_attention_layer(i)}
-        return ROWS.RowsSpace(self.scratch, self.device, max(w.n_rows for w in used))
+        return ROWS.RowsSpace(self.scratch, self.device, max(w.n_rows for w in used),
+                              ROWS.MMA_ROWS_Q8 if any(w.qtype == GGMLType.Q8_0 for w in used) else ROWS.MMA_ROWS)
 
     def few(self, rows: int) -> bool:
         """Do the projections of a batch of this many rows run as few-row products?"""

@@ -12,6 +12,10 @@ from ..core import native as N
 from .kernels import EPI_GELU_MUL, EPI_SILU_MUL, DeviceWeight, GemvSegment, _check_device, _dt, _p, _stream, status_tensor
 
 MAX_ROWS = 64
+# Rows up to which products run on mma.sync, above them on tcgen05 (csrc/gemm_rows_tc.cu): 17408 x 5120 weights at 16 rows 22.2 us
+# (Q4_K), 24.7 (Q8_0), Q6_K 5120 x 17408 24.8; at 24 rows tcgen05 takes 20.7 / 36.5 / 27.0 us, mma.sync 24.4 / 29.5 / 27.4.
+MMA_ROWS = 16
+MMA_ROWS_Q8 = 24             # ... of models with Q8_0 projections
 MAX_SEGMENTS = 4
 QTYPES = (8, 12, 14)         # Q8_0, Q4_K, Q6_K
 HALF_TILE = 64               # smallest tile: weight rows of each weight of a gate/up pair
@@ -25,7 +29,7 @@ class _Seg(C.Structure):
 
 
 class _Args(C.Structure):
-    _fields_ = [("seg", _Seg * MAX_SEGMENTS), ("n_seg", C.c_int), ("K", C.c_int), ("R", C.c_int),
+    _fields_ = [("seg", _Seg * MAX_SEGMENTS), ("n_seg", C.c_int), ("K", C.c_int), ("R", C.c_int), ("tc", C.c_int),
                 ("image", C.c_void_p), ("ws", C.c_void_p), ("ws_floats", C.c_longlong), ("counters", C.c_void_p),
                 ("n_counters", C.c_int), ("status", C.c_void_p), ("stages", C.c_int), ("stage_bytes", C.c_int),
                 ("w_bytes", C.c_int), ("tiles", C.c_int)]
@@ -72,8 +76,9 @@ class RowsSpace:
     """What the products of one stream share: the activation image and the partial tiles (named scratch of the owner)
     and the arrival counters of the tiles (zero between launches)."""
 
-    def __init__(self, scratch, device: torch.device, max_weight_rows: int):
+    def __init__(self, scratch, device: torch.device, max_weight_rows: int, mma_rows: int = MMA_ROWS):
         self.scratch = scratch
+        self.mma_rows = mma_rows
         # tiles of a launch: at most MAX_SEGMENTS segments of the largest weight, in half tiles when they are pairs
         n = MAX_SEGMENTS * (-(-max_weight_rows // HALF_TILE))
         self.counters = torch.zeros(n, dtype=torch.int32, device=device)
@@ -89,8 +94,9 @@ class RowsSpace:
         assert x.stride(1) == 1
         L = _lib()
         img = rows = None
+        tc = C.c_int(int(R > self.mma_rows))
         if product:
-            img = self.scratch.get("rows_image", (int(L.he_rows_image_bytes(C.c_int(R), C.c_int(K))),), torch.uint8)
+            img = self.scratch.get("rows_image", (int(L.he_rows_image_bytes(C.c_int(R), C.c_int(K), tc)),), torch.uint8)
         if by_row:
             rows = self.scratch.get("rows_by_row", (R * (K // 256) * IMAGE_UNIT,), torch.uint8)
         n_side = 0
@@ -99,7 +105,7 @@ class RowsSpace:
             assert side_w.dtype == side_out.dtype == torch.float32 and side_w.is_contiguous() and side_w.shape[1] == K
             assert side_out.shape[0] >= R and side_out.shape[1] >= n_side and side_out.stride(1) == 1
         N.check(L.he_rows_image(C.c_void_p(x.data_ptr()), C.c_int(_dt(x)), C.c_longlong(x.stride(0)),
-                                C.c_void_p(_p(norm_w)), C.c_float(eps), C.c_int(K), C.c_int(R), C.c_void_p(_p(img)),
+                                C.c_void_p(_p(norm_w)), C.c_float(eps), C.c_int(K), C.c_int(R), C.c_void_p(_p(img)), tc,
                                 C.c_void_p(_p(rows)), C.c_void_p(_p(side_w)), C.c_int(n_side),
                                 C.c_void_p(_p(side_out) if n_side else None),
                                 C.c_longlong(side_out.stride(0) if n_side else 0), _stream()), "he_rows_image")
@@ -162,8 +168,8 @@ class RowsSpace:
                 g.w2 = s.w2.ptr
             g.w, g.out, g.n_rows, g.qtype, g.epi = s.w.ptr, s.out.data_ptr(), s.w.n_rows, s.w.qtype, s.epi
             g.out_stride = s.out.stride(0) if s.out.dim() > 1 else s.out.numel()
-        n_ws = int(L.he_rows_ws_floats(C.c_int(R), C.c_int(N.num_sms())))
-        a.n_seg, a.K, a.R = len(segs), K, R
+        a.n_seg, a.K, a.R, a.tc = len(segs), K, R, int(R > self.mma_rows)
+        n_ws = int(L.he_rows_ws_floats(C.c_int(R), C.c_int(N.num_sms()), C.c_int(a.tc)))
         a.image = image.data_ptr()
         a.ws, a.ws_floats = self.scratch.get("rows_ws", (n_ws,), torch.float32).data_ptr(), n_ws
         a.counters, a.n_counters = self.counters.data_ptr(), self.counters.numel()
