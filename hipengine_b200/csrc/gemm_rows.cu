@@ -338,9 +338,10 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
 // Two fp32 weight rows against all activation rows, in fp32 (the few projections that checkpoints keep as floats: expert
 // routers, the gates of the delta rule).  They ride in the image's launch because they need the same rows at the same
 // time and leave nearly all of the chip free.  The weight rows times the norm wait in shared memory; a warp takes a row,
-// or with fewer rows than warps a slice of one; the row's sum of squares falls out of the same pass.
+// or with fewer rows than warps a slice of one; the row's sum of squares falls out of the same pass.  `steady`: all warps a slice of
+// one row after the other, so that a row's sums do not depend on how many rows there are.
 __device__ void side_rows(const float* w, int n, int n0, float* out, long long ld, const void* x, int x_dtype,
-                          long long x_stride, const float* norm_w, float eps, int K, int R, float* wsm) {
+                          long long x_stride, const float* norm_w, float eps, int K, int R, bool steady, float* wsm) {
   __shared__ float part[16][3];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool two = n0 + 1 < n;
@@ -354,7 +355,8 @@ __device__ void side_rows(const float* w, int n, int n0, float* out, long long l
   pdl_wait();
   __syncthreads();
   int slices = 1;
-  while (slices * R <= 8) slices <<= 1;                       // R * slices <= 16 warps
+  if (steady) slices = 16;
+  else while (slices * R <= 8) slices <<= 1;                  // R * slices <= 16 warps
   const int sl = warp % slices, r_step = 16 / slices;
   for (int r0 = 0; r0 < R; r0 += r_step) {
     const int r = r0 + warp / slices;
@@ -409,13 +411,13 @@ __global__ void __launch_bounds__(512) rows_image_kernel(const void* __restrict_
                                                          int pad_rows, int parts, uint8_t* __restrict__ image,
                                                          uint8_t* __restrict__ by_row,
                                                          const float* __restrict__ side_w, int side_n,
-                                                         float* __restrict__ side_out, long long side_ld) {
+                                                         float* __restrict__ side_out, long long side_ld, bool steady) {
   extern __shared__ __align__(16) float side_sm[];
   __shared__ float red[33];
   pdl_launch();
   if ((int)blockIdx.x >= R * parts) {
     side_rows(side_w, side_n, ((int)blockIdx.x - R * parts) * 2, side_out, side_ld, x, x_dtype, x_stride, norm_w, eps, K, R,
-              side_sm);
+              steady, side_sm);
     return;
   }
   const int r = blockIdx.x / parts, nb = K >> 8, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -529,10 +531,10 @@ HE_API long long he_rows_ws_floats(int R, int num_sms, int tc) {
 // null): block by block, for a product of 1..64 rows; `by_row` (may be null): row by row, for he_rows_experts, any R; both null:
 // the side rows alone.
 // With `side_n` > 0 (at most 64 rows) also side_out[r][j] = (normalised row r) . side_w[j], j < side_n: fp32 weights
-// [side_n][K], in fp32.
+// [side_n][K], in fp32.  `side_steady`: a row's are the same bits beside any number of others.
 HE_API int he_rows_image(const void* x, int x_dtype, long long x_stride, const float* norm_w, float eps, int K, int R,
                          void* image, int tc, void* by_row, const float* side_w, int side_n, float* side_out, long long side_ld,
-                         cudaStream_t stream) {
+                         int side_steady, cudaStream_t stream) {
   if (K <= 0 || K % 256 != 0 || R < 1 || ((image != nullptr || side_n > 0) && R > (image != nullptr && !tc ? MMA_MAX_ROWS : 64)) || x == nullptr ||
       (image == nullptr && by_row == nullptr && side_n <= 0) || (reinterpret_cast<uintptr_t>(by_row) & 15) != 0)
     return -HE_ERR_BAD_ARG;
@@ -557,7 +559,7 @@ HE_API int he_rows_image(const void* x, int x_dtype, long long x_stride, const f
   const unsigned grid = (unsigned)(R * parts + (side_n > 0 ? (side_n + 1) / 2 : 0));
   return (int)launch_pdl(tc ? rows_image_kernel<true> : rows_image_kernel<false>, dim3(grid), dim3(norm_w != nullptr ? 512 : 128), smem, stream, x, x_dtype,
                          x_stride, norm_w, eps, K, R, tc ? tc_rows(R) : col_groups(R) * 8, parts, (uint8_t*)image, (uint8_t*)by_row, side_w, side_n,
-                         side_out, side_ld);
+                         side_out, side_ld, side_steady != 0);
 }
 
 HE_API int he_rows_gemm(const HeRowsArgs* args, int num_sms, cudaStream_t stream) {

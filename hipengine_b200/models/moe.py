@@ -118,10 +118,14 @@ def _moe_selected(ex, i: int, h: torch.Tensor, target: torch.Tensor, T: int, nor
                                                                ex.W(i, "ffn_up_shexp.weight"))])
     for r0 in range(0, 0 if few else T, 8):
         r1 = min(T, r0 + 8)
-        segs = [GemvSegment(L.router, logits[r0:r1, :E])]
-        if L.has_shared:
-            segs.append(GemvSegment(L.shexp_gate, logits[r0:r1, E:E + 1]))
-        K.gemv(h[r0:r1], segs, norm_w=norm_w, eps=cfg.rms_eps)
+        if L.full is not None:
+            # two rows of the fp32 router a block (one row, hidden 2048, 257 rows: 4 us; as GEMV rows, each the chain of one warp, 20)
+            ex.rows.image(h[r0:r1], norm_w, cfg.rms_eps, L.full, logits[r0:r1], product=False, steady=True)
+        else:
+            segs = [GemvSegment(L.router, logits[r0:r1, :E])]
+            if L.has_shared:
+                segs.append(GemvSegment(L.shexp_gate, logits[r0:r1, E:E + 1]))
+            K.gemv(h[r0:r1], segs, norm_w=norm_w, eps=cfg.rms_eps)
         if shared_here:
             K.gemv(h[r0:r1], [GemvSegment(ex.W(i, "ffn_gate_shexp.weight"), act_sh[r0:r1], epi,
                                           ex.W(i, "ffn_up_shexp.weight"))], norm_w=norm_w, eps=cfg.rms_eps)

@@ -85,10 +85,10 @@ class RowsSpace:
 
     def image(self, x: torch.Tensor, norm_w: Optional[torch.Tensor] = None, eps: float = 1e-6,
               side_w: Optional[torch.Tensor] = None, side_out: Optional[torch.Tensor] = None,
-              by_row: bool = False, product: bool = True) -> Tuple[Optional[torch.Tensor], Optional[torch.Tensor]]:
+              by_row: bool = False, product: bool = True, steady: bool = False) -> Tuple[Optional[torch.Tensor], Optional[torch.Tensor]]:
         """The fragments of (RMSNorm of) the rows ``x`` [R, K] (fp32 or bf16): (for ``product``, for ``experts``), each on
         demand.  With ``side_w`` (fp32 [n, K]) the same launch also writes ``side_out`` [R, >= n] = normalised rows @
-        side_w^T, all in fp32, or nothing else."""
+        side_w^T, all in fp32, or nothing else; ``steady``: a row's are the same bits beside any number of others."""
         _check_device(x)
         R, K = x.shape
         assert x.stride(1) == 1
@@ -108,7 +108,7 @@ class RowsSpace:
                                 C.c_void_p(_p(norm_w)), C.c_float(eps), C.c_int(K), C.c_int(R), C.c_void_p(_p(img)), tc,
                                 C.c_void_p(_p(rows)), C.c_void_p(_p(side_w)), C.c_int(n_side),
                                 C.c_void_p(_p(side_out) if n_side else None),
-                                C.c_longlong(side_out.stride(0) if n_side else 0), _stream()), "he_rows_image")
+                                C.c_longlong(side_out.stride(0) if n_side else 0), C.c_int(int(steady)), _stream()), "he_rows_image")
         return img, rows
 
     def jobs(self, ids: torch.Tensor, E: int, cols: int) -> "ExpertJobs":

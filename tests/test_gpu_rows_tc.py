@@ -38,3 +38,22 @@ def test_forms_agree_and_add(t, n, k):
     K.check_status()
     for space in spaces:
         assert int(space.counters.abs().sum()) == 0 and space.scratch.check_canaries() == []
+
+
+def test_steady_side_rows():
+    """fp32 side rows whose sums do not depend on the rows beside: a verify chain routes like a plain step."""
+    from hipengine_b200.models.executor import _Scratch
+    from hipengine_b200.ops.rows import RowsSpace
+    dev = torch.device("cuda", torch.cuda.current_device())
+    space = RowsSpace(_Scratch(dev), dev, 256)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x, nw = torch.randn(8, 2304, generator=g, device="cuda"), torch.rand(2304, generator=g, device="cuda") + 0.5
+    side = torch.randn(257, 2304, generator=g, device="cuda") * 0.02
+    out, one = (torch.zeros(8, 264, device="cuda") for _ in range(2))
+    space.image(x, nw, 1e-6, side, out, product=False, steady=True)
+    for r in range(8):
+        space.image(x[r:r + 1], nw, 1e-6, side, one[r:r + 1], product=False, steady=True)
+    assert torch.equal(out, one)
+    xn = x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-6) * nw.double()
+    ref = xn @ side.double().t()
+    assert float((out[:, :257].double() - ref).norm() / ref.norm()) < 3e-6 and bool((out[:, 257:] == 0).all())
