@@ -18,6 +18,10 @@
 // Against mma.sync, whose warps each read the whole image for 16 weight rows (17408 x 5120, 32 / 48 / 64 rows, us in a graph):
 // Q4_K 30.7 / 37.9 / 46.8 -> 20.7 / 22.4 / 25.4, Q8_0 44.5 / 42.5 / 54.4 -> 36.3 / 38.0 / 40.3, Q6_K (5120 x 17408) 35.2 / 37.7 / 45.8
 // -> 27.0 / 29.4 / 32.6; a step of 64 rows, 8 layers of the 27B, 3295 -> 2315 us.
+// Experts of prompts: the same pipeline over (job of up to 64 rows of an expert, tile) items.  A job's rows are first gathered into an
+// image of their own (43 us for 16384 rows of 2048 columns), which its tiles read from L2.  2048 rows, 256 experts, 8 used, hidden 2048,
+// width 512: gate/up 180-215 us and down 163 us a layer; the grouped GEMM took 130 + 124 + 52 (activation) and 190, with 128-row tiles
+// half padding, and rounds its weights to bf16, which these do not.
 #include "rows_tc.cuh"
 
 using namespace he;
@@ -25,12 +29,22 @@ using namespace herows;
 
 namespace {
 
+struct TcExperts {
+  const int4* jobs;        // (expert, first entry, entries, 0)
+  const int* entries;      // pairs
+  const int* meta;         // [0]: number of jobs
+  int expert_rows;
+};
+
 constexpr int TILE = 128, HALF = TC_HALF;              // weight rows of a tile, of each weight of a pair
 
-// N: activation rows, padded to the next multiple of 16; TYPE: block type of all segments, or 0 where they differ
-template <int N, int TYPE>
+// N: activation rows, padded to the next multiple of 16; TYPE: block type of all segments, or 0 where they differ.
+// EXPERTS: instead of units dealt out, whole (job, tile) items in turn; segment 0 describes an expert's weights, a job's rows have an
+// image of their own (he_tc_gather) and results go to the rows of their pairs.
+template <int N, int TYPE, bool EXPERTS>
 __global__ void __launch_bounds__(TC_THREADS, 1)
-rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ HeRowsArgs a, const RowsPlan plan) {
+rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ HeRowsArgs a, const RowsPlan plan,
+                 const TcExperts x) {
   constexpr int SUMS = TC_SUM_WARPS, NC = 4 * N / SUMS, SLOT = TILE * N;   // columns of a summing thread, floats of a partial tile
   constexpr int IMG = tc_image(N), IMG_PAD = tc_image_pad(N);
   constexpr int PRODUCER = TC_UNPACK_WARPS + SUMS, SIGNAL = PRODUCER + 1, ISSUER = PRODUCER + 2;     // two issuers
@@ -42,13 +56,18 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
   const uint32_t ring = sm100::smem_u32(smem), minima = ring + (uint32_t)stages * stage_bytes;
   TcBars* bar = reinterpret_cast<TcBars*>(smem + (size_t)stages * stage_bytes + 2 * TC_MIN_BYTES);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nb = a.K >> 8, b = blockIdx.x, u0 = plan.begin(b), u1 = plan.begin(b + 1);
+  if (EXPERTS) pdl_wait();               // the jobs come from the kernels before
+  const int nb = a.K >> 8, b = blockIdx.x, u0 = EXPERTS ? b : plan.begin(b);
+  const int u1 = EXPERTS ? *reinterpret_cast<const volatile int*>(x.meta) * a.tiles : plan.begin(b + 1);
+  const int step = EXPERTS ? (int)gridDim.x : 0;        // to a CTA's next item
   // CTAs that share a tile: those that hold its first and last unit and all between
   const auto first_cta = [&](int tile) { return plan.cta_of(tile * nb); };
   const auto last_cta = [&](int tile) { return plan.cta_of((tile + 1) * nb - 1); };
   const int tile_a = u0 / nb, tile_z = (u1 - 1) / nb;           // only the first and the last tile can be shared
-  const bool share_a = u0 > tile_a * nb || u1 < (tile_a + 1) * nb, share_z = tile_z != tile_a && u1 < (tile_z + 1) * nb;
+  const bool share_a = !EXPERTS && (u0 > tile_a * nb || u1 < (tile_a + 1) * nb);
+  const bool share_z = !EXPERTS && tile_z != tile_a && u1 < (tile_z + 1) * nb;
   const auto segment = [&](int tile) {
+    if (EXPERTS) return 0;
     int si = 0;
     while (si + 1 < a.n_seg && tile >= a.seg[si + 1].tile0) ++si;
     return si;
@@ -90,7 +109,10 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
   // The results of weight row 32 q + lane of a tile for columns col .. col + C (C even)
   const auto epilogue = [&](const HeRowsSeg& sg, int tile, int q, int col, const auto& acc) {
     constexpr int C = sizeof(acc) / sizeof(float);
-    const int tl = tile - sg.tile0;
+    const int tl = EXPERTS ? tile % a.tiles : tile - sg.tile0;
+    int4 job = make_int4(0, 0, a.R, 0);
+    if (EXPERTS) job = x.jobs[tile / a.tiles];
+    const auto to = [&](int r) { return (size_t)(EXPERTS ? x.entries[job.y + r] : r) * sg.out_stride; };
     if (sg.epi >= 3) {
       // lanes l and l + 16 hold the gate row and its up row: the lower one finishes the first half of the columns
       const bool up = lane >= 16;
@@ -102,27 +124,27 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
         const float gv = up ? other : acc[j], uv = up ? acc[j + C / 2] : other;
         const int r = col + j + (up ? C / 2 : 0);
         const float ga = sg.epi == 3 ? silu_f(gv) : gelu_tanh_f(gv);
-        if (r < a.R && row < sg.n_rows) o[(size_t)r * sg.out_stride] = f32_to_bf16(ga * uv);
+        if (r < job.z && row < sg.n_rows) o[to(r)] = f32_to_bf16(ga * uv);
       }
       return;
     }
     const int row = tl * TILE + 32 * q + lane;
     if (row >= sg.n_rows) return;
-    const int n = min(C, a.R - col);
+    const int n = min(C, job.z - col);
     if (sg.epi == 1) {
-      __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(sg.out) + (size_t)col * sg.out_stride + row;
+      __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(sg.out) + row;
 #pragma unroll
       for (int j = 0; j < C; ++j)
-        if (j < n) o[(size_t)j * sg.out_stride] = f32_to_bf16(acc[j]);
+        if (j < n) o[to(col + j)] = f32_to_bf16(acc[j]);
       return;
     }
-    float* o = reinterpret_cast<float*>(sg.out) + (size_t)col * sg.out_stride + row;
+    float* o = reinterpret_cast<float*>(sg.out) + row;
     float old[C];                       // all loads before the first store: they could be of the same address, for the compiler
 #pragma unroll
-    for (int j = 0; j < C; ++j) old[j] = sg.epi == 2 && j < n ? o[(size_t)j * sg.out_stride] : 0.f;
+    for (int j = 0; j < C; ++j) old[j] = sg.epi == 2 && j < n ? o[to(col + j)] : 0.f;
 #pragma unroll
     for (int j = 0; j < C; ++j)
-      if (j < n) o[(size_t)j * sg.out_stride] = sg.epi == 2 ? old[j] + acc[j] : acc[j];
+      if (j < n) o[to(col + j)] = sg.epi == 2 ? old[j] + acc[j] : acc[j];
   };
   // Shared tiles that this CTA was the last to arrive at: sums of the partial tiles in CTA order, by all unpacking and summing
   // warps with four partial tiles in flight (by the summing warps alone, one after the other: 4 us of a launch)
@@ -182,12 +204,12 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
       __syncwarp();
     };
     for (int u = u0; u < u1 && ok;) {
-      const int tile = u / nb, n_blk = min(nb - (u - tile * nb), u1 - u);
+      const int tile = EXPERTS ? u : u / nb, n_blk = EXPERTS ? nb : min(nb - (u - tile * nb), u1 - u);
       const HeRowsSeg& sg = a.seg[segment(tile)];
       const bool pair = sg.epi >= 3;
       const int qtype = type_of(sg), bb = rows_block_bytes(qtype);
       const TcRow at_row(pair, q, lane, bb, qtype);
-      u += n_blk;
+      u += EXPERTS ? step : n_blk;
       for (int k = 0; k < n_blk; ++k, ++j) {
         const bool mine = (j & 1) == grp;
         if (mine || !own) {
@@ -251,7 +273,7 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
     uint32_t j = 0;
     int s = 0;
     for (int u = u0; u < u1;) {
-      const int tile = u / nb, blk0 = u - tile * nb, n_blk = min(nb - blk0, u1 - u);
+      const int tile = EXPERTS ? u : u / nb, blk0 = EXPERTS ? 0 : u - tile * nb, n_blk = min(nb - blk0, EXPERTS ? nb : u1 - u);
       const HeRowsSeg& sg = a.seg[segment(tile)];
       const bool pair = sg.epi >= 3;
       const int qtype = type_of(sg), bb = rows_block_bytes(qtype);
@@ -259,7 +281,7 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
       uint64_t sum[NC / 2];
 #pragma unroll
       for (int k = 0; k < NC / 2; ++k) sum[k] = 0;
-      u += n_blk;
+      u += EXPERTS ? step : n_blk;
       for (int k = 0; k < n_blk; ++k, ++j) {
         const uint32_t slot = j & 1;
         const uint32_t st = ring + (uint32_t)s * stage_bytes, t = dt + slot * (2 * N);
@@ -307,9 +329,9 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
     // -------------------------------------------------------------- producer
     const uint8_t* image = reinterpret_cast<const uint8_t*>(a.image);
     const bool leader = sm100::elect_one();
-    int si = segment(u0 / nb), tile = u0 / nb, blk = u0 % nb;
+    int si = EXPERTS ? 0 : segment(u0 / nb), tile = EXPERTS ? u0 : u0 / nb, blk = EXPERTS ? 0 : u0 % nb;
     const auto weights = [&](int s) {
-      while (si + 1 < a.n_seg && tile >= a.seg[si + 1].tile0) ++si;
+      while (!EXPERTS && si + 1 < a.n_seg && tile >= a.seg[si + 1].tile0) ++si;
       const HeRowsSeg& sg = a.seg[si];
       const int qtype = type_of(sg), bb = rows_block_bytes(qtype);
       const bool pair = sg.epi >= 3;
@@ -317,7 +339,8 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
         uint8_t* dst = smem + (size_t)s * stage_bytes + IMG_PAD;
         uint64_t* full = &bar->full[s];
         sm100::mbar_expect_tx(full, (uint32_t)(TILE * bb + IMG));
-        const int n0 = (tile - sg.tile0) * (pair ? HALF : TILE);
+        const int n0 = EXPERTS ? x.jobs[tile / a.tiles].x * x.expert_rows + tile % a.tiles * (pair ? HALF : TILE)
+                               : (tile - sg.tile0) * (pair ? HALF : TILE);
         if (qtype == HE_Q8_0) {
           const int h = pair ? HALF : TILE;
 #pragma unroll 1
@@ -333,13 +356,13 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
         }
       }
       __syncwarp();
-      if (++blk == nb) { blk = 0; ++tile; }
+      if (++blk == nb) { blk = 0; tile += EXPERTS ? step : 1; }
     };
     const auto rows = [&](int s, int blk) {
       if (leader) bulk_load(ring + (uint32_t)s * stage_bytes, image + (size_t)blk * IMG, IMG, &bar->full[s]);
       __syncwarp();
     };
-    const int n = u1 - u0, pre = min(n, stages);
+    const int n = EXPERTS ? (u1 > u0 ? (u1 - u0 + step - 1) / step * nb : 0) : u1 - u0, pre = EXPERTS ? 0 : min(n, stages);
     for (int i = 0; i < pre; ++i) weights(i);
     pdl_wait();                         // the rows (and so their image) come from the kernels before
     for (int i = 0; i < pre; ++i) rows(i, (u0 + i) % nb);
@@ -347,8 +370,8 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
     uint32_t ph = 0;
     int issued = pre;
     for (int i = pre; i < n; ++i) {
-      if (!wait(&bar->empty[s], ph, 401)) break;
-      const int bi = blk;
+      if (EXPERTS ? i >= stages && !wait(&bar->empty[s], ph ^ 1u, 401) : !wait(&bar->empty[s], ph, 401)) break;
+      const int bi = EXPERTS ? tile / a.tiles * nb + blk : blk;
       weights(s);
       rows(s, bi);
       ++issued;
@@ -372,9 +395,9 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
     int s = 0;
     bool ok = true;
     for (int u = u0; u < u1 && ok;) {
-      const int tile = u / nb, n_blk = min(nb - (u - tile * nb), u1 - u);
+      const int tile = EXPERTS ? u : u / nb, n_blk = EXPERTS ? nb : min(nb - (u - tile * nb), u1 - u);
       const int qtype = type_of(a.seg[segment(tile)]);
-      u += n_blk;
+      u += EXPERTS ? step : n_blk;
       for (int k = 0; k < n_blk && ok; ++k, ++j) {
         if ((j & 1) == me) {
           const uint32_t img = ring + (uint32_t)s * stage_bytes;
@@ -457,12 +480,24 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
   }
 }
 
-template <int N, int TYPE>
-int launch_typed(const RowsMaps& maps, const HeRowsArgs& a, size_t smem, int grid, const RowsPlan& plan, cudaStream_t stream) {
+template <int N, int TYPE, bool EXPERTS>
+int launch_typed(const RowsMaps& maps, const HeRowsArgs& a, size_t smem, int grid, const RowsPlan& plan, const TcExperts& x,
+                 cudaStream_t stream) {
   static std::atomic<unsigned long long> allowed{0};
-  const cudaError_t e = allow_smem(rows_gemm_kernel<N, TYPE>, TC_SMEM, allowed);
+  const cudaError_t e = allow_smem(rows_gemm_kernel<N, TYPE, EXPERTS>, TC_SMEM, allowed);
   if (e != cudaSuccess) return (int)e;
-  return (int)launch_pdl(rows_gemm_kernel<N, TYPE>, dim3(grid), dim3(TC_THREADS), smem, stream, maps, a, plan);
+  return (int)launch_pdl(rows_gemm_kernel<N, TYPE, EXPERTS>, dim3(grid), dim3(TC_THREADS), smem, stream, maps, a, plan, x);
+}
+
+// Stages of the ring, set in `a`; dynamic shared memory of a block, or 0 where it does not hold two stages
+template <int N>
+size_t ring(HeRowsArgs& a) {
+  a.stage_bytes = tc_image_pad(N) + ((a.w_bytes + 1023) & ~1023);
+  constexpr int fixed = 1024 + 2 * TC_MIN_BYTES + (int)sizeof(TcBars);
+  a.stages = (TC_SMEM - fixed) / a.stage_bytes;
+  if (a.stages > TC_MAX_STAGES) a.stages = TC_MAX_STAGES;
+  if (a.stages > 4) a.stages &= ~1;
+  return a.stages < 2 ? 0 : (size_t)a.stages * a.stage_bytes + fixed;
 }
 
 template <int N>
@@ -484,22 +519,64 @@ int launch_rows(HeRowsArgs a, int num_sms, cudaStream_t stream) {
     if (wb > a.w_bytes) a.w_bytes = wb;
     if (sg.qtype != type) type = 0;
   }
-  a.stage_bytes = tc_image_pad(N) + ((a.w_bytes + 1023) & ~1023);
-  constexpr int fixed = 1024 + 2 * TC_MIN_BYTES + (int)sizeof(TcBars);
-    a.stages = (TC_SMEM - fixed) / a.stage_bytes;
-  if (a.stages > TC_MAX_STAGES) a.stages = TC_MAX_STAGES;
-  if (a.stages < 2) return -HE_ERR_BAD_ARG;
-  if (a.stages > 4) a.stages &= ~1;
-  const size_t smem = (size_t)a.stages * a.stage_bytes + fixed;
+  const size_t smem = ring<N>(a);
+  if (smem == 0) return -HE_ERR_BAD_ARG;
   const long long units = (long long)a.tiles * (a.K >> 8);
   const int grid = (int)(units < num_sms ? units : num_sms);
   if (units > 0x7FFFFFFF || 2ll * grid * TILE * N > a.ws_floats || a.tiles > a.n_counters) return -HE_ERR_BAD_ARG;
   const RowsPlan plan{(int)(units / grid), (int)(units % grid)};
   switch (type) {
-    case HE_Q4_K: return launch_typed<N, HE_Q4_K>(maps, a, smem, grid, plan, stream);
-    case HE_Q6_K: return launch_typed<N, HE_Q6_K>(maps, a, smem, grid, plan, stream);
-    case HE_Q8_0: return launch_typed<N, HE_Q8_0>(maps, a, smem, grid, plan, stream);
-    default: return launch_typed<N, 0>(maps, a, smem, grid, plan, stream);
+    case HE_Q4_K: return launch_typed<N, HE_Q4_K, false>(maps, a, smem, grid, plan, TcExperts{}, stream);
+    case HE_Q6_K: return launch_typed<N, HE_Q6_K, false>(maps, a, smem, grid, plan, TcExperts{}, stream);
+    case HE_Q8_0: return launch_typed<N, HE_Q8_0, false>(maps, a, smem, grid, plan, TcExperts{}, stream);
+    default: return launch_typed<N, 0, false>(maps, a, smem, grid, plan, TcExperts{}, stream);
+  }
+}
+
+template <int N>
+int launch_experts(HeRowsArgs a, const TcExperts& x, long long rows, int num_sms, cudaStream_t stream) {
+  const HeRowsSeg& sg = a.seg[0];
+  const int per = sg.epi >= 3 ? HALF : TILE;
+  RowsMaps maps;
+  int rc = weight_maps(&maps.m[0][0], sg.w, sg.qtype, rows, a.K, per);
+  if (rc == 0 && sg.epi >= 3) rc = weight_maps(&maps.m[0][2], sg.w2, sg.qtype, rows, a.K, per);
+  if (rc != 0) return rc;
+  a.n_seg = 1;
+  a.tiles = (sg.n_rows + per - 1) / per;
+  a.w_bytes = TILE * rows_block_bytes(sg.qtype);
+  const size_t smem = ring<N>(a);
+  if (smem == 0) return -HE_ERR_BAD_ARG;
+  const RowsPlan plan{1, 0};
+  switch (sg.qtype) {
+    case HE_Q4_K: return launch_typed<N, HE_Q4_K, true>(maps, a, smem, num_sms, plan, x, stream);
+    case HE_Q6_K: return launch_typed<N, HE_Q6_K, true>(maps, a, smem, num_sms, plan, x, stream);
+    case HE_Q8_0: return launch_typed<N, HE_Q8_0, true>(maps, a, smem, num_sms, plan, x, stream);
+    default: return -HE_ERR_BAD_ARG;
+  }
+}
+
+// Images of the jobs' rows: row entries[first + c] / per_row of x becomes row c of its job's image.  A CTA a (job, block), a warp a row,
+// four rows of a warp in flight.  (A CTA a job: 52 us for 16384 rows of 2048 columns, a chain of loads a warp.)
+__global__ void __launch_bounds__(512) gather_kernel(const void* __restrict__ rows, int dtype, long long stride, int K,
+                                                     const int4* __restrict__ jobs, const int* __restrict__ entries,
+                                                     const int* __restrict__ meta, int per_row, int n, uint8_t* __restrict__ image) {
+  pdl_wait();
+  pdl_launch();
+  if ((int)blockIdx.x >= *meta) return;
+  const int4 job = jobs[blockIdx.x];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, blk = blockIdx.y;
+  uint8_t* img = image + ((size_t)blockIdx.x * (K >> 8) + blk) * tc_image(n);
+  float v[4][8];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int c = warp + 16 * e;
+    if (c < job.z)
+      load_cols(rows, dtype, (size_t)(entries[job.y + c] / per_row) * stride + blk * 256 + lane * 8, v[e]);
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int c = warp + 16 * e;
+    if (c < job.z) image_store<true>(img, nullptr, n, c, lane, v[e]);
   }
 }
 
@@ -511,4 +588,34 @@ int herows::launch_rows_tc(const HeRowsArgs& a, int num_sms, cudaStream_t stream
     case 48: return launch_rows<48>(a, num_sms, stream);
     default: return launch_rows<64>(a, num_sms, stream);
   }
+}
+
+// Bytes of the images of `jobs` jobs of up to `cols` (32 or 64) rows of K columns.
+HE_API long long he_tc_gather_bytes(long long jobs, int cols, int K) { return jobs * (K >> 8) * (long long)tc_image(cols); }
+
+// Images of the rows of `max_jobs` jobs at most (he_moe_jobs with the same `cols`): fp32 or bf16 rows, 16-byte aligned.
+HE_API int he_tc_gather(const void* rows, int dtype, long long stride, int K, const void* jobs, const int* entries, const int* meta,
+                        int per_row, int cols, int max_jobs, void* image, cudaStream_t stream) {
+  if (K <= 0 || K % 256 != 0 || per_row < 1 || max_jobs < 1 || !(cols == 32 || cols == 64) || rows == nullptr || image == nullptr ||
+      (reinterpret_cast<uintptr_t>(rows) & 15) != 0 || (stride * (dtype == 0 ? 4 : 2)) % 16 != 0 ||
+      (reinterpret_cast<uintptr_t>(image) & 15) != 0 || (reinterpret_cast<uintptr_t>(jobs) & 15) != 0)
+    return -HE_ERR_BAD_ARG;
+  return (int)launch_pdl(gather_kernel, dim3(max_jobs, K >> 8), dim3(512), 0, stream, rows, dtype, stride, K, (const int4*)jobs, entries,
+                         meta, per_row, cols, (uint8_t*)image);
+}
+
+// Products of the jobs' rows with their experts' weights, from the images of he_tc_gather; see he_rows_experts.  `a`: segment 0 (n_rows
+// of an expert, out by pair), K, image, status.
+HE_API int he_tc_experts(const HeRowsArgs* args, int experts, const void* jobs, const int* entries, const int* meta, int cols,
+                         int num_sms, cudaStream_t stream) {
+  HeRowsArgs a = *args;
+  const HeRowsSeg& sg = a.seg[0];
+  if (a.K <= 0 || a.K % 256 != 0 || sg.n_rows < 1 || experts < 1 || num_sms < 1 || a.image == nullptr || sg.out == nullptr ||
+      (reinterpret_cast<uintptr_t>(a.image) & 15) != 0 || jobs == nullptr || entries == nullptr || meta == nullptr ||
+      !(sg.epi == 0 || sg.epi == 1 || sg.epi == 3 || sg.epi == 4))
+    return -HE_ERR_BAD_ARG;
+  const TcExperts x{(const int4*)jobs, entries, meta, sg.n_rows};
+  const long long rows = (long long)experts * sg.n_rows;
+  return cols == 32 ? launch_experts<32>(a, x, rows, num_sms, stream)
+       : cols == 64 ? launch_experts<64>(a, x, rows, num_sms, stream) : -HE_ERR_BAD_ARG;
 }

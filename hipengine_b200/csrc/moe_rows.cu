@@ -14,7 +14,7 @@
 // At 32 rows DRAM is at 43-47 % and the issue slots at 60 % (expansion of the blocks); with more rows per expert mma.sync and the
 // image reads grow.  A layer's experts (256, 8 used, hidden 2048,
 // width 512): 32 rows 100 us for both products (172 us before), a step of 8 layers 2471 -> 1893 us; prompts of 72 / 256 / 1024
-// rows 6.1 / 7.3 / 8.6 ms -> 3.9 / 4.4 / 7.1 ms, of 2048 rows 10.6 -> 12.4 ms (those stay on the grouped GEMM).
+// rows 6.1 / 7.3 / 8.6 ms -> 3.9 / 4.4 / 7.1 ms, of 2048 rows 10.6 -> 12.4 ms (those take the jobs of gemm_rows_tc.cu).
 // Reference: hipengine/kernels/hip_gfx1100/quant/gguf_q4_k_selected_prefill.hip, moe/group_scatter.hip.
 #include "rows_mma.cuh"
 

@@ -7,7 +7,8 @@ Three routes, chosen by the number of packed rows:
   (token, expert) pairs reading the experts' quantised rows in place; from ``JOBS_MIN_ROWS`` rows the pairs are
   sorted by expert and run as jobs (``csrc/moe_rows.cu``).  No expert id is ever read by the host,
   so the whole block is CUDA-graph capturable.
-* larger ``T`` with few pairs per expert (``JOBS_MAX_LOAD``): the same jobs, with the shared expert on the GEMM.
+* larger ``T`` with few pairs per expert (``JOBS_MAX_LOAD``): the same jobs, with the shared expert on the GEMM; up to
+  ``JOBS_TC_LOAD`` jobs of 64 rows on tcgen05.
 * larger ``T``: *grouped tensor-core GEMM*.  Pairs are bucketed by expert (128-row padded segments), rows are
   gathered and the tcgen05 GEMM runs in grouped mode over the experts' quantised blocks (each 128-row tile
   carries its expert id; the blocks are expanded to bf16 inside the GEMM pipeline), followed by a combine kernel that applies the routing weights, the
@@ -33,9 +34,10 @@ SEL_MAX_ROWS = 64
 # is the weights that pairs share: with fewer experts per pair used they would pay from fewer rows; that was the only geometry
 # measured.)
 JOBS_MIN_ROWS = 8
-# Pairs per expert up to which a prompt's do: 72 / 256 / 1024 / 2048 rows take 3.9 / 4.4 / 7.1 / 12.4 ms with jobs and
-# 6.1 / 7.3 / 8.6 / 10.6 ms in the grouped GEMM, whose 128-row tiles are mostly padding for few rows an expert.
-JOBS_MAX_LOAD = 32
+# Pairs per expert up to which a prompt's do, and above that up to which its jobs are of 64 rows on tcgen05 (csrc/gemm_rows_tc.cu): 600
+# / 800 / 1000 / 2048 / 4096 rows (19 / 25 / 31 / 64 / 128 pairs an expert) take 4.8 / 5.4 / 6.1 / 12.4 / - ms with the former, 5.2 /
+# 5.5 / 5.9 / 8.3 / 13.7 with the latter, - / - / - / 9.3 / 13.7 in the grouped GEMM, whose 128-row tiles are half padding at 64.
+JOBS_MAX_LOAD, JOBS_TC_LOAD = 28, 112
 
 
 class _MoeLayer:
@@ -218,6 +220,17 @@ def _moe_grouped(ex, i: int, h: torch.Tensor, target: torch.Tensor, T: int, norm
     wts = sc.get("moe_wts", (T, k), torch.float32)
     K.moe_route(logits, k, ids, wts, n_experts=E)
     P = T * k
+    if JOBS_MAX_LOAD * E < P <= JOBS_TC_LOAD * E and _jobs_ok(ex, i, rng):
+        jobs = ex.rows.jobs(ids, E, 64)
+        act = sc.get("moe_act_g", (P, F), torch.bfloat16)
+        epi = K.EPI_SILU_MUL if cfg.act == "silu" else K.EPI_GELU_MUL
+        ex.rows.experts_tc(jobs, ex.rows.gather(jobs, xn, k), ex.W(i, "ffn_gate_exps.weight"), act, epi,
+                           ex.W(i, "ffn_up_exps.weight"))
+        ys = sc.get("moe_ys", (P, H), torch.bfloat16)
+        ex.rows.experts_tc(jobs, ex.rows.gather(jobs, act, 1), ex.W(i, "ffn_down_exps.weight"), ys, K.EPI_BF16)
+        ysh = _shared_rows(ex, i, xn, T) if shared_here else None
+        ex.rows.sum_pairs(target, ys, wts, ysh, logits[:, E:E + 1] if shared_here else None)
+        return
     if P <= JOBS_MAX_LOAD * E and _jobs_ok(ex, i, rng):
         _, by_row = ex.rows.image(xn, by_row=True, product=False)
         ys = _expert_jobs(ex, i, ids, by_row, k, sc.get("moe_act_g", (P, F), torch.bfloat16), torch.bfloat16)

@@ -57,3 +57,45 @@ def test_steady_side_rows():
     xn = x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-6) * nw.double()
     ref = xn @ side.double().t()
     assert float((out[:, :257].double() - ref).norm() / ref.norm()) < 3e-6 and bool((out[:, 257:] == 0).all())
+
+
+@pytest.mark.parametrize("t", [T.Q4_K, T.Q6_K, T.Q8_0])
+@pytest.mark.parametrize("cols", [32, 64])
+def test_expert_jobs(t, cols):
+    """Experts without rows, with one, with a job more or less than full; tiles with a remainder of weight rows; ids of no expert."""
+    from hipengine_b200.models.executor import _Scratch
+    from hipengine_b200.ops import kernels as K
+    from hipengine_b200.ops.rows import RowsSpace
+    dev = torch.device("cuda", torch.cuda.current_device())
+    space = RowsSpace(_Scratch(dev, canaries=True), dev, 256)
+    counts, k, H, F = [0, 1, cols - 1, cols, cols + 1, 2 * cols + 3, 0, 5], 2, 512, 200
+    E, P = len(counts), sum(counts) + 2
+    P += P % 2
+    g = torch.Generator().manual_seed(cols)
+    ids = torch.tensor([e for e, c in enumerate(counts) for _ in range(c)] + [-1] * (P - sum(counts)), dtype=torch.int32)
+    ids = ids[torch.randperm(P, generator=g)].reshape(-1, k).cuda()
+    gd = torch.Generator(device="cuda").manual_seed(cols)
+    def weight(n, kk):
+        raw = Q.quantize(torch.randn(E * n, kk, generator=gd, device="cuda") * 0.05, t)
+        return K.to_device_weight(raw, t, E * n, kk), Q.dequantize_torch(raw, t, E * n, kk).double().reshape(E, n, kk)
+    (wg, g64), (wu, u64), (wd, d64) = weight(F, H), weight(F, H), weight(300, 256)
+    x = torch.randn(P // k, H, generator=gd, device="cuda").bfloat16()
+    jobs = space.jobs(ids, E, cols)
+    act = torch.full((P, F), float("nan"), device="cuda", dtype=torch.bfloat16)
+    space.experts_tc(jobs, space.gather(jobs, x, k), wg, act, K.EPI_SILU_MUL, wu)
+    y = torch.randn(P, 256, generator=gd, device="cuda")
+    down = torch.full((P, 300), float("nan"), device="cuda")
+    space.experts_tc(jobs, space.gather(jobs, y, 1), wd, down, K.EPI_F32)
+    flat = ids.reshape(-1).tolist()
+    for p, e in enumerate(flat):
+        if e < 0:
+            assert bool(act[p].isnan().all()) and bool(down[p].isnan().all())
+            continue
+        xp, yp = x[p // k].double(), y[p].double()
+        ref = torch.nn.functional.silu(g64[e] @ xp) * (u64[e] @ xp)
+        assert float((act[p].double() - ref).norm() / ref.norm()) < 6e-3, (p, e)          # bf16 result
+        ref = d64[e] @ yp
+        # rows round to 11 bits; Q6_K operands as well
+        assert float((down[p].double() - ref).norm() / ref.norm()) < (2 ** -10.5 if t == T.Q6_K else 2 ** -11), (p, e)
+    K.check_status()
+    assert space.scratch.check_canaries() == []
