@@ -79,6 +79,7 @@ class RowsSpace:
     def __init__(self, scratch, device: torch.device, max_weight_rows: int, mma_rows: int = MMA_ROWS):
         self.scratch = scratch
         self.mma_rows = mma_rows
+        self._image_bytes, self._ws_floats = {}, {}      # by (rows, columns), by rows
         # tiles of a launch: at most MAX_SEGMENTS segments of the largest weight, in half tiles when they are pairs
         n = MAX_SEGMENTS * (-(-max_weight_rows // HALF_TILE))
         self.counters = torch.zeros(n, dtype=torch.int32, device=device)
@@ -96,7 +97,10 @@ class RowsSpace:
         img = rows = None
         tc = C.c_int(int(R > self.mma_rows))
         if product:
-            img = self.scratch.get("rows_image", (int(L.he_rows_image_bytes(C.c_int(R), C.c_int(K), tc)),), torch.uint8)
+            size = self._image_bytes.get((R, K))
+            if size is None:
+                size = self._image_bytes[R, K] = int(L.he_rows_image_bytes(C.c_int(R), C.c_int(K), tc))
+            img = self.scratch.get("rows_image", (size,), torch.uint8)
         if by_row:
             rows = self.scratch.get("rows_by_row", (R * (K // 256) * IMAGE_UNIT,), torch.uint8)
         n_side = 0
@@ -197,7 +201,9 @@ class RowsSpace:
             g.w, g.out, g.n_rows, g.qtype, g.epi = s.w.ptr, s.out.data_ptr(), s.w.n_rows, s.w.qtype, s.epi
             g.out_stride = s.out.stride(0) if s.out.dim() > 1 else s.out.numel()
         a.n_seg, a.K, a.R, a.tc = len(segs), K, R, int(R > self.mma_rows)
-        n_ws = int(L.he_rows_ws_floats(C.c_int(R), C.c_int(N.num_sms()), C.c_int(a.tc)))
+        n_ws = self._ws_floats.get(R)
+        if n_ws is None:
+            n_ws = self._ws_floats[R] = int(L.he_rows_ws_floats(C.c_int(R), C.c_int(N.num_sms()), C.c_int(a.tc)))
         a.image = image.data_ptr()
         a.ws, a.ws_floats = self.scratch.get("rows_ws", (n_ws,), torch.float32).data_ptr(), n_ws
         a.counters, a.n_counters = self.counters.data_ptr(), self.counters.numel()
