@@ -77,7 +77,7 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
       sm100::mbar_init(&bar->full[s], 1);
-      sm100::mbar_init(&bar->empty[s], SUMS);
+      sm100::mbar_init(&bar->empty[s], tc_empty_arrivals(stages));
     }
     for (int s = 0; s < 4; ++s) {
       sm100::mbar_init(&bar->ready[s], TC_UNPACK_WARPS / 2);
@@ -188,9 +188,7 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
     const int q = warp & 3;
     const uint32_t at = tmem + ((uint32_t)(q * 32) << 16) + TC_A_COL + grp * TC_A_SLOT;
     const uint32_t mins = minima + grp * TC_MIN_BYTES + (uint32_t)((4 * q + (lane >> 3)) * 256 + (lane & 7) * 16);
-    // Blocks go to the groups in turn.  With an even ring a group has stages of its own, else it waits for the other one's too: a
-    // phase bit tells only neighbours apart
-    const bool own = (stages & 1) == 0;
+    const bool own = tc_own_stages(stages);
     uint32_t j = 0, ph = 0, done_ph = 1;
     int s = 0;
     bool ok = true;
@@ -215,6 +213,10 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
         if (mine || !own) {
           ok = wait(&bar->full[s], ph, 402);
           if (!ok) break;
+        }
+        if (!mine && !own) {
+          __syncwarp();
+          if (lane == 0) sm100::mbar_arrive(&bar->empty[s]);
         }
         const uint32_t row = ring + (uint32_t)s * stage_bytes + IMG_PAD + at_row.off;
         if (mine && qtype == HE_Q8_0) {
@@ -489,15 +491,21 @@ int launch_typed(const RowsMaps& maps, const HeRowsArgs& a, size_t smem, int gri
   return (int)launch_pdl(rows_gemm_kernel<N, TYPE, EXPERTS>, dim3(grid), dim3(TC_THREADS), smem, stream, maps, a, plan, x);
 }
 
+constexpr int TC_FIXED = 1024 + 2 * TC_MIN_BYTES + (int)sizeof(TcBars);
+
+// Stages of a ring for n activation rows and a block of `w_bytes` of weights
+int ring_stages(int n, int w_bytes) {
+  int s = (TC_SMEM - TC_FIXED) / (tc_image_pad(n) + ((w_bytes + 1023) & ~1023));
+  if (s > TC_MAX_STAGES) s = TC_MAX_STAGES;
+  return s > 4 ? s & ~1 : s;
+}
+
 // Stages of the ring, set in `a`; dynamic shared memory of a block, or 0 where it does not hold two stages
 template <int N>
 size_t ring(HeRowsArgs& a) {
   a.stage_bytes = tc_image_pad(N) + ((a.w_bytes + 1023) & ~1023);
-  constexpr int fixed = 1024 + 2 * TC_MIN_BYTES + (int)sizeof(TcBars);
-  a.stages = (TC_SMEM - fixed) / a.stage_bytes;
-  if (a.stages > TC_MAX_STAGES) a.stages = TC_MAX_STAGES;
-  if (a.stages > 4) a.stages &= ~1;
-  return a.stages < 2 ? 0 : (size_t)a.stages * a.stage_bytes + fixed;
+  a.stages = ring_stages(N, a.w_bytes);
+  return a.stages < 2 ? 0 : (size_t)a.stages * a.stage_bytes + TC_FIXED;
 }
 
 template <int N>
@@ -588,6 +596,14 @@ int herows::launch_rows_tc(const HeRowsArgs& a, int num_sms, cudaStream_t stream
     case 48: return launch_rows<48>(a, num_sms, stream);
     default: return launch_rows<64>(a, num_sms, stream);
   }
+}
+
+// Stages of the ring of a product of R rows with blocks of the largest type `qtype`, and how many
+// unpacking warps have to arrive, beside the summing ones, before one is loaded again.
+HE_API int he_rows_tc_ring(int R, int qtype, int* arrivals) {
+  const int s = ring_stages(tc_rows(R), TILE * rows_block_bytes(qtype));
+  *arrivals = tc_empty_arrivals(s) - TC_SUM_WARPS;
+  return s;
 }
 
 // Bytes of the images of `jobs` jobs of up to `cols` (32 or 64) rows of K columns.
