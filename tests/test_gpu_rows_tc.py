@@ -99,3 +99,35 @@ def test_expert_jobs(t, cols):
         assert float((down[p].double() - ref).norm() / ref.norm()) < (2 ** -10.5 if t == T.Q6_K else 2 ** -11), (p, e)
     K.check_status()
     assert space.scratch.check_canaries() == []
+
+
+@pytest.mark.parametrize("top,small", [(10, -12), (15, -7), (15, -14), (-14, -14)])
+def test_q8_scales_far_apart_within_a_block(top, small):
+    """Q8_0 scales of a block up to 2^22 apart enter exactly; beyond that a small one is a multiple of 2^-32 of the power of two of the
+    largest, off by at most half of it.  Rows that are zero where the scales are large show what is left of the small ones; the largest
+    scale (511.75 under its power) meets -128, the largest integer."""
+    from hipengine_b200.models.executor import _Scratch
+    from hipengine_b200.ops import kernels as K
+    from hipengine_b200.ops.rows import RowsSpace
+    dev = torch.device("cuda", torch.cuda.current_device())
+    space, n, k = RowsSpace(_Scratch(dev, canaries=True), dev, 256), 200, 1024
+    g = torch.Generator(device="cuda").manual_seed(top - small)
+    scale = (1 + torch.rand(n, k // 32, generator=g, device="cuda")) * 2.0 ** small
+    scale[:, ::8] = (2 - 2 ** -10) * 2.0 ** top
+    q = torch.randint(-128, 128, (n, k // 32, 32), generator=g, device="cuda").to(torch.int8)
+    raw = torch.cat([scale.half().view(torch.uint8).view(n, k // 32, 2), q.view(torch.uint8)], 2).reshape(n, -1).contiguous()
+    w, wd = K.to_device_weight(raw, T.Q8_0, n, k), Q.dequantize_torch(raw, T.Q8_0, n, k).double()
+    off = (q.double().abs() * 2.0 ** (top - 33)).reshape(n, k) if top - small > 22 else torch.zeros(n, k, dtype=torch.double, device="cuda")
+    for R in (8, 32, 48, 64):
+        x = torch.randint(-31, 32, (R, k), generator=g, device="cuda").float()
+        x.view(R, k // 32, 32)[::2, ::8] = 0
+        out = torch.zeros(R, n, device="cuda")
+        space.gemm(x, [K.GemvSegment(w, out)])
+        ref = x.double() @ wd.t()
+        # fp32 sums: of at most k terms, each a rounding of the terms' sum
+        bound = x.double().abs() @ (off + k * 2 ** -24 * wd.abs()).t()
+        assert bool(((out.double() - ref).abs() <= bound).all()), (R, float(((out.double() - ref).abs() / bound).max()))
+        small_rows = (out.double() - ref)[::2].norm() / ref[::2].norm()
+        assert top - small > 22 or float(small_rows) < k ** 0.5 * 2 ** -24, (R, float(small_rows))
+    K.check_status()
+    assert space.scratch.check_canaries() == []
