@@ -35,9 +35,14 @@ SEL_MAX_ROWS = 64
 # measured.)
 JOBS_MIN_ROWS = 8
 # Pairs per expert up to which a prompt's do, and above that up to which its jobs are of 64 rows on tcgen05 (csrc/gemm_rows_tc.cu): 600
-# / 800 / 1000 / 2048 / 4096 rows (19 / 25 / 31 / 64 / 128 pairs an expert) take 4.8 / 5.4 / 6.1 / 12.4 / - ms with the former, 5.2 /
-# 5.5 / 5.9 / 8.3 / 13.7 with the latter, - / - / - / 9.3 / 13.7 in the grouped GEMM, whose 128-row tiles are half padding at 64.
+# / 800 / 1000 rows (19 / 25 / 31 pairs an expert) take 4.8 / 5.4 / 6.1 ms with the former, 5.2 / 5.5 / 5.9 with the latter; 2048 /
+# 2560 / 3072 / 3584 / 4096 rows (64 / 80 / 96 / 112 / 128 pairs) 8.3 / 9.8 / 10.8 / 12.4 / 13.7 with the latter, 9.3 / 10.1 / 11.0 /
+# 12.4 / 14.1 in the grouped GEMM, whose 128-row tiles are half padding at 64.
 JOBS_MAX_LOAD, JOBS_TC_LOAD = 28, 112
+# ... and with Q8_0 experts, two operands a weight on tcgen05: 912 / 976 / 1020 rows (29 / 31 / 32 pairs) 6.2 / 6.4 / 6.5 ms with the
+# former, 6.7 / 6.7 / 6.7 with the latter; 1152 / 1792 / 2048 / 2304 / 2560 rows (36 / 56 / 64 / 72 / 80 pairs) 6.9 / 8.3 / 9.4 / 10.5 /
+# 11.4 with the latter, 7.9 / 9.3 / 9.6 / 9.9 / 10.3 in the grouped GEMM.
+JOBS_MAX_LOAD_Q8, JOBS_TC_LOAD_Q8 = 32, 64
 
 
 class _MoeLayer:
@@ -158,6 +163,15 @@ def _jobs_ok(ex, i: int, rng) -> bool:
             all(ROWS.weight_ok(x) for x in w) and w[0].qtype == w[1].qtype)
 
 
+def _prompt_route(ex, i: int, pairs: int, rng) -> str:
+    """How a prompt's (token, expert) pairs run: as "jobs", as jobs of 64 rows on tcgen05 ("jobs_tc") or in the "grouped" GEMM."""
+    if pairs > JOBS_TC_LOAD * ex.cfg.n_experts or not _jobs_ok(ex, i, rng):
+        return "grouped"
+    q8 = any(ex.W(i, f"ffn_{s}_exps.weight").qtype == GGMLType.Q8_0 for s in ("gate", "down"))
+    few, tc = (JOBS_MAX_LOAD_Q8, JOBS_TC_LOAD_Q8) if q8 else (JOBS_MAX_LOAD, JOBS_TC_LOAD)
+    return "jobs" if pairs <= few * ex.cfg.n_experts else "jobs_tc" if pairs <= tc * ex.cfg.n_experts else "grouped"
+
+
 def _job_cols(pairs: int, E: int, decode: bool) -> int:
     """Rows per job: about twice what an expert gets on average (a job costs its columns' products whether they are
     filled or not, a second job of an expert costs its weights again).  Decode batches keep to jobs of 16 rows, whose Q6_K
@@ -220,7 +234,8 @@ def _moe_grouped(ex, i: int, h: torch.Tensor, target: torch.Tensor, T: int, norm
     wts = sc.get("moe_wts", (T, k), torch.float32)
     K.moe_route(logits, k, ids, wts, n_experts=E)
     P = T * k
-    if JOBS_MAX_LOAD * E < P <= JOBS_TC_LOAD * E and _jobs_ok(ex, i, rng):
+    route = _prompt_route(ex, i, P, rng)
+    if route == "jobs_tc":
         jobs = ex.rows.jobs(ids, E, 64)
         act = sc.get("moe_act_g", (P, F), torch.bfloat16)
         epi = K.EPI_SILU_MUL if cfg.act == "silu" else K.EPI_GELU_MUL
@@ -231,7 +246,7 @@ def _moe_grouped(ex, i: int, h: torch.Tensor, target: torch.Tensor, T: int, norm
         ysh = _shared_rows(ex, i, xn, T) if shared_here else None
         ex.rows.sum_pairs(target, ys, wts, ysh, logits[:, E:E + 1] if shared_here else None)
         return
-    if P <= JOBS_MAX_LOAD * E and _jobs_ok(ex, i, rng):
+    if route == "jobs":
         _, by_row = ex.rows.image(xn, by_row=True, product=False)
         ys = _expert_jobs(ex, i, ids, by_row, k, sc.get("moe_act_g", (P, F), torch.bfloat16), torch.bfloat16)
         ysh = _shared_rows(ex, i, xn, T) if shared_here else None

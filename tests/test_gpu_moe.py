@@ -96,16 +96,31 @@ def _kl(p_logits, q_logits):
     return (p.exp() * (p - q)).sum(-1)
 
 
-@pytest.mark.parametrize("n_prompt,n_decode", [(4, 5), (40, 2), (150, 2)], ids=["decode", "selected", "grouped"])
-def test_moe_executor_matches_reference(n_prompt, n_decode):
+# (rows, route of the prompt's pairs) with 16 experts, 4 used: a quarter of the rows an expert
+ROUTES = [(100, "jobs"), (113, "jobs_tc"), (200, "jobs_tc"), (448, "jobs_tc"), (449, "grouped")]
+
+
+@pytest.fixture
+def routes(monkeypatch):
+    """The routes that prompts took, in order."""
+    from hipengine_b200.models import moe as M
+    seen, choose = [], M._prompt_route
+    monkeypatch.setattr(M, "_prompt_route", lambda *a: seen.append(choose(*a)) or seen[-1])
+    return seen
+
+
+@pytest.mark.parametrize("n_prompt,n_decode,route", [(4, 5, None), (40, 2, None), (150, 2, "jobs_tc"), (460, 2, "grouped")],
+                         ids=["decode", "selected", "prompt_jobs_tc", "grouped"])
+def test_moe_executor_matches_reference(n_prompt, n_decode, route, routes):
     from hipengine_b200.models.executor import HybridExecutor
     cfg = TINY_HYBRID_MOE
     w = build_random_model(cfg, seed=0, std=0.05)
     ref = RefModel(w)
-    ex = HybridExecutor(w.to("cuda"), max_slots=2, max_context=256)
+    ex = HybridExecutor(w.to("cuda"), max_slots=2, max_context=512)
     toks = torch.randint(0, cfg.vocab, (n_prompt + n_decode,), generator=torch.Generator().manual_seed(1))
     ref_logits, _ = ref.forward(toks)
     got = [ex.forward_logits(1, toks[:n_prompt].tolist(), 0).cpu()]
+    assert set(routes) == ({route} if route else set())
     for t in range(n_prompt, n_prompt + n_decode):
         got.append(ex.forward_logits(1, [int(toks[t])], t).cpu())
     got = torch.cat(got, 0)
@@ -120,8 +135,8 @@ def test_moe_executor_matches_reference(n_prompt, n_decode):
     assert kl.mean() < 0.01 and kl.max() < 0.15 and top1 >= 0.8 and rel < 1.5, (kl.mean().item(), kl.max().item(), top1, rel)
 
 
-@pytest.mark.parametrize("T", [3, 8, 40, 100, 200], ids=["decode", "jobs8", "jobs16", "prompt_jobs", "grouped"])
-def test_moe_block_matches_reference_on_identical_input(T):
+@pytest.mark.parametrize("T,route", [(3, None), (8, None), (40, None), *ROUTES])
+def test_moe_block_matches_reference_on_identical_input(T, route, routes):
     """The FFN block alone, fed the same residual rows as the reference: only an exact router near-tie can
     differ, so nearly every row must agree closely."""
     from hipengine_b200.loading.weights import ffn_norm_slot
@@ -137,14 +152,15 @@ def test_moe_block_matches_reference_on_identical_input(T):
     want = ref.ffn(i, R.rmsnorm(h0, ref.W(i, ffn_norm_slot(cfg)), cfg.rms_eps))
     h = h0.cuda().clone()
     M.moe_ffn(ex, i, h, T, norm_w, T <= 8)
+    assert routes == ([route] if route else [])
     got = (h.cpu() - h0)
     assert torch.isfinite(got).all()
     err = (got - want).abs().amax(-1) / want.abs().amax(-1).clamp(min=1e-6)
     assert (err < 0.06).float().mean() >= 0.97, err
 
 
-@pytest.mark.parametrize("T", [3, 40, 100, 200], ids=["decode", "jobs", "prompt_jobs", "grouped"])
-def test_a_row_of_nan_stays_alone(T):
+@pytest.mark.parametrize("T,route", [(3, None), (40, None), *ROUTES])
+def test_a_row_of_nan_stays_alone(T, route, routes):
     from hipengine_b200.loading.weights import ffn_norm_slot
     from hipengine_b200.models import moe as M
     from hipengine_b200.models.executor import HybridExecutor
@@ -157,6 +173,7 @@ def test_a_row_of_nan_stays_alone(T):
     bad[1, 5] = float("nan")
     for x in (clean, bad):
         M.moe_ffn(ex, 1, x, T, norm_w, T <= 8)
+    assert routes == ([route] * 2 if route else [])
     K.check_status()
     others = torch.arange(T, device="cuda") != 1
     assert torch.equal(bad[others], clean[others]) and bool(bad[1].isnan().all())
