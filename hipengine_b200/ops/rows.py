@@ -79,7 +79,7 @@ class RowsSpace:
     def __init__(self, scratch, device: torch.device, max_weight_rows: int, mma_rows: int = MMA_ROWS):
         self.scratch = scratch
         self.mma_rows = mma_rows
-        self._image_bytes, self._ws_floats = {}, {}      # by (rows, columns), by rows
+        self._image_bytes, self._ws_floats = {}, {}      # by (rows, columns, form), by (rows, form)
         # tiles of a launch: at most MAX_SEGMENTS segments of the largest weight, in half tiles when they are pairs
         n = MAX_SEGMENTS * (-(-max_weight_rows // HALF_TILE))
         self.counters = torch.zeros(n, dtype=torch.int32, device=device)
@@ -95,11 +95,11 @@ class RowsSpace:
         assert x.stride(1) == 1
         L = _lib()
         img = rows = None
-        tc = C.c_int(int(R > self.mma_rows))
+        tc = int(R > self.mma_rows)
         if product:
-            size = self._image_bytes.get((R, K))
+            size = self._image_bytes.get((R, K, tc))
             if size is None:
-                size = self._image_bytes[R, K] = int(L.he_rows_image_bytes(C.c_int(R), C.c_int(K), tc))
+                size = self._image_bytes[R, K, tc] = int(L.he_rows_image_bytes(C.c_int(R), C.c_int(K), C.c_int(tc)))
             img = self.scratch.get("rows_image", (size,), torch.uint8)
         if by_row:
             rows = self.scratch.get("rows_by_row", (R * (K // 256) * IMAGE_UNIT,), torch.uint8)
@@ -109,7 +109,7 @@ class RowsSpace:
             assert side_w.dtype == side_out.dtype == torch.float32 and side_w.is_contiguous() and side_w.shape[1] == K
             assert side_out.shape[0] >= R and side_out.shape[1] >= n_side and side_out.stride(1) == 1
         N.check(L.he_rows_image(C.c_void_p(x.data_ptr()), C.c_int(_dt(x)), C.c_longlong(x.stride(0)),
-                                C.c_void_p(_p(norm_w)), C.c_float(eps), C.c_int(K), C.c_int(R), C.c_void_p(_p(img)), tc,
+                                C.c_void_p(_p(norm_w)), C.c_float(eps), C.c_int(K), C.c_int(R), C.c_void_p(_p(img)), C.c_int(tc),
                                 C.c_void_p(_p(rows)), C.c_void_p(_p(side_w)), C.c_int(n_side),
                                 C.c_void_p(_p(side_out) if n_side else None),
                                 C.c_longlong(side_out.stride(0) if n_side else 0), C.c_int(int(steady)), _stream()), "he_rows_image")
@@ -201,9 +201,9 @@ class RowsSpace:
             g.w, g.out, g.n_rows, g.qtype, g.epi = s.w.ptr, s.out.data_ptr(), s.w.n_rows, s.w.qtype, s.epi
             g.out_stride = s.out.stride(0) if s.out.dim() > 1 else s.out.numel()
         a.n_seg, a.K, a.R, a.tc = len(segs), K, R, int(R > self.mma_rows)
-        n_ws = self._ws_floats.get(R)
+        n_ws = self._ws_floats.get((R, a.tc))
         if n_ws is None:
-            n_ws = self._ws_floats[R] = int(L.he_rows_ws_floats(C.c_int(R), C.c_int(N.num_sms()), C.c_int(a.tc)))
+            n_ws = self._ws_floats[R, a.tc] = int(L.he_rows_ws_floats(C.c_int(R), C.c_int(N.num_sms()), C.c_int(a.tc)))
         a.image = image.data_ptr()
         a.ws, a.ws_floats = self.scratch.get("rows_ws", (n_ws,), torch.float32).data_ptr(), n_ws
         a.counters, a.n_counters = self.counters.data_ptr(), self.counters.numel()
