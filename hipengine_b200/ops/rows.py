@@ -150,8 +150,9 @@ class RowsSpace:
         """Images of the jobs' rows (of 32 or 64) for ``experts_tc``: row pair // pairs_per_row of ``x`` (fp32 or bf16)."""
         L = _lib()
         n, K = jobs.list.shape[0], x.shape[1]
-        img = self.scratch.get("moe_job_image", (int(L.he_tc_gather_bytes(C.c_longlong(n), C.c_int(jobs.cols), C.c_int(K))),),
-                               torch.uint8)
+        # (in the buffer that the grouped GEMM gathers its rows into, of the same size: an expert block takes one route or the other)
+        size = int(L.he_tc_gather_bytes(C.c_longlong(n), C.c_int(jobs.cols), C.c_int(K)))
+        img = self.scratch.get("moe_xs", (size // 2,), torch.bfloat16).view(torch.uint8)
         assert x.stride(1) == 1 and x.shape[0] * pairs_per_row >= jobs.P
         N.check(L.he_tc_gather(C.c_void_p(x.data_ptr()), C.c_int(_dt(x)), C.c_longlong(x.stride(0)), C.c_int(K),
                                C.c_void_p(jobs.list.data_ptr()), C.c_void_p(jobs.entries.data_ptr()),
