@@ -37,6 +37,7 @@ struct TcExperts {
 };
 
 constexpr int TILE = 128, HALF = TC_HALF;              // weight rows of a tile, of each weight of a pair
+constexpr int TC_JOB_ROWS = 64;                        // rows of an expert job
 
 // N: activation rows, padded to the next multiple of 16; TYPE: block type of all segments, or 0 where they differ.
 // EXPERTS: instead of units dealt out, whole (job, tile) items in turn; segment 0 describes an expert's weights, a job's rows have an
@@ -541,8 +542,8 @@ int launch_rows(HeRowsArgs a, int num_sms, cudaStream_t stream) {
   }
 }
 
-template <int N>
 int launch_experts(HeRowsArgs a, const TcExperts& x, long long rows, int num_sms, cudaStream_t stream) {
+  constexpr int N = TC_JOB_ROWS;
   const HeRowsSeg& sg = a.seg[0];
   const int per = sg.epi >= 3 ? HALF : TILE;
   RowsMaps maps;
@@ -567,7 +568,8 @@ int launch_experts(HeRowsArgs a, const TcExperts& x, long long rows, int num_sms
 // four rows of a warp in flight.  (A CTA a job: 52 us for 16384 rows of 2048 columns, a chain of loads a warp.)
 __global__ void __launch_bounds__(512) gather_kernel(const void* __restrict__ rows, int dtype, long long stride, int K,
                                                      const int4* __restrict__ jobs, const int* __restrict__ entries,
-                                                     const int* __restrict__ meta, int per_row, int n, uint8_t* __restrict__ image) {
+                                                     const int* __restrict__ meta, int per_row, uint8_t* __restrict__ image) {
+  constexpr int n = TC_JOB_ROWS;
   pdl_wait();
   pdl_launch();
   if ((int)blockIdx.x >= *meta) return;
@@ -606,23 +608,23 @@ HE_API int he_rows_tc_ring(int R, int qtype, int* arrivals) {
   return s;
 }
 
-// Bytes of the images of `jobs` jobs of up to `cols` (32 or 64) rows of K columns.
-HE_API long long he_tc_gather_bytes(long long jobs, int cols, int K) { return jobs * (K >> 8) * (long long)tc_image(cols); }
+// Bytes of the images of `jobs` jobs of up to 64 rows of K columns.
+HE_API long long he_tc_gather_bytes(long long jobs, int K) { return jobs * (K >> 8) * (long long)tc_image(TC_JOB_ROWS); }
 
-// Images of the rows of `max_jobs` jobs at most (he_moe_jobs with the same `cols`): fp32 or bf16 rows, 16-byte aligned.
+// Images of the rows of `max_jobs` jobs at most (he_moe_jobs with 64 columns): fp32 or bf16 rows, 16-byte aligned.
 HE_API int he_tc_gather(const void* rows, int dtype, long long stride, int K, const void* jobs, const int* entries, const int* meta,
-                        int per_row, int cols, int max_jobs, void* image, cudaStream_t stream) {
-  if (K <= 0 || K % 256 != 0 || per_row < 1 || max_jobs < 1 || !(cols == 32 || cols == 64) || rows == nullptr || image == nullptr ||
+                        int per_row, int max_jobs, void* image, cudaStream_t stream) {
+  if (K <= 0 || K % 256 != 0 || per_row < 1 || max_jobs < 1 || rows == nullptr || image == nullptr ||
       (reinterpret_cast<uintptr_t>(rows) & 15) != 0 || (stride * (dtype == 0 ? 4 : 2)) % 16 != 0 ||
       (reinterpret_cast<uintptr_t>(image) & 15) != 0 || (reinterpret_cast<uintptr_t>(jobs) & 15) != 0)
     return -HE_ERR_BAD_ARG;
   return (int)launch_pdl(gather_kernel, dim3(max_jobs, K >> 8), dim3(512), 0, stream, rows, dtype, stride, K, (const int4*)jobs, entries,
-                         meta, per_row, cols, (uint8_t*)image);
+                         meta, per_row, (uint8_t*)image);
 }
 
 // Products of the jobs' rows with their experts' weights, from the images of he_tc_gather; see he_rows_experts.  `a`: segment 0 (n_rows
 // of an expert, out by pair), K, image, status.
-HE_API int he_tc_experts(const HeRowsArgs* args, int experts, const void* jobs, const int* entries, const int* meta, int cols,
+HE_API int he_tc_experts(const HeRowsArgs* args, int experts, const void* jobs, const int* entries, const int* meta,
                          int num_sms, cudaStream_t stream) {
   HeRowsArgs a = *args;
   const HeRowsSeg& sg = a.seg[0];
@@ -631,7 +633,5 @@ HE_API int he_tc_experts(const HeRowsArgs* args, int experts, const void* jobs, 
       !(sg.epi == 0 || sg.epi == 1 || sg.epi == 3 || sg.epi == 4))
     return -HE_ERR_BAD_ARG;
   const TcExperts x{(const int4*)jobs, entries, meta, sg.n_rows};
-  const long long rows = (long long)experts * sg.n_rows;
-  return cols == 32 ? launch_experts<32>(a, x, rows, num_sms, stream)
-       : cols == 64 ? launch_experts<64>(a, x, rows, num_sms, stream) : -HE_ERR_BAD_ARG;
+  return launch_experts(a, x, (long long)experts * sg.n_rows, num_sms, stream);
 }

@@ -147,23 +147,23 @@ class RowsSpace:
                                   C.c_int(jobs.cols), C.c_int(N.num_sms()), _stream()), "he_rows_experts")
 
     def gather(self, jobs: "ExpertJobs", x: torch.Tensor, pairs_per_row: int) -> torch.Tensor:
-        """Images of the jobs' rows (of 32 or 64) for ``experts_tc``: row pair // pairs_per_row of ``x`` (fp32 or bf16)."""
+        """Images of the jobs' rows (of 64) for ``experts_tc``: row pair // pairs_per_row of ``x`` (fp32 or bf16)."""
         L = _lib()
         n, K = jobs.list.shape[0], x.shape[1]
         # (in the buffer that the grouped GEMM gathers its rows into, of the same size: an expert block takes one route or the other)
-        size = int(L.he_tc_gather_bytes(C.c_longlong(n), C.c_int(jobs.cols), C.c_int(K)))
+        size = int(L.he_tc_gather_bytes(C.c_longlong(n), C.c_int(K)))
         img = self.scratch.get("moe_xs", (size // 2,), torch.bfloat16).view(torch.uint8)
-        assert x.stride(1) == 1 and x.shape[0] * pairs_per_row >= jobs.P
+        assert jobs.cols == 64 and x.stride(1) == 1 and x.shape[0] * pairs_per_row >= jobs.P
         N.check(L.he_tc_gather(C.c_void_p(x.data_ptr()), C.c_int(_dt(x)), C.c_longlong(x.stride(0)), C.c_int(K),
                                C.c_void_p(jobs.list.data_ptr()), C.c_void_p(jobs.entries.data_ptr()),
-                               C.c_void_p(jobs.meta.data_ptr()), C.c_int(pairs_per_row), C.c_int(jobs.cols), C.c_int(n),
+                               C.c_void_p(jobs.meta.data_ptr()), C.c_int(pairs_per_row), C.c_int(n),
                                C.c_void_p(img.data_ptr()), _stream()), "he_tc_gather")
         return img
 
     def experts_tc(self, jobs: "ExpertJobs", image: torch.Tensor, w: DeviceWeight, out: torch.Tensor, epi: int,
                    w2: Optional[DeviceWeight] = None) -> None:
-        """``experts`` for jobs of 32 or 64 rows on tcgen05, from the images of ``gather``."""
-        assert w.n_rows % jobs.E == 0 and weight_ok(w) and out.shape[0] >= jobs.P and out.stride(1) == 1
+        """``experts`` for jobs of 64 rows on tcgen05, from the images of ``gather``."""
+        assert jobs.cols == 64 and w.n_rows % jobs.E == 0 and weight_ok(w) and out.shape[0] >= jobs.P and out.stride(1) == 1
         a = _Args()
         g = a.seg[0]
         g.w, g.out, g.out_stride, g.n_rows, g.qtype, g.epi = w.ptr, out.data_ptr(), out.stride(0), w.n_rows // jobs.E, w.qtype, epi
@@ -172,7 +172,7 @@ class RowsSpace:
             g.w2 = w2.ptr
         a.K, a.R, a.tc, a.image, a.status = w.n_cols, jobs.cols, 1, image.data_ptr(), status_tensor(out.device).data_ptr()
         N.check(_lib().he_tc_experts(C.byref(a), C.c_int(jobs.E), C.c_void_p(jobs.list.data_ptr()),
-                                     C.c_void_p(jobs.entries.data_ptr()), C.c_void_p(jobs.meta.data_ptr()), C.c_int(jobs.cols),
+                                     C.c_void_p(jobs.entries.data_ptr()), C.c_void_p(jobs.meta.data_ptr()),
                                      C.c_int(N.num_sms()), _stream()), "he_tc_experts")
 
     @staticmethod

@@ -69,6 +69,6 @@ def test_job_images_take_the_buffer_of_the_grouped_gemm(monkeypatch, pairs, E, K
     n = int(lib.he_moe_jobs_bound(C.c_longlong(pairs), C.c_int(E), C.c_int(64)))
     jobs = ROWS.ExpertJobs(torch.zeros(1), torch.zeros(n, 4), torch.zeros(4), E, 64, pairs)
     img = space.gather(jobs, torch.zeros(pairs // 4, K, dtype=torch.bfloat16), 4)
-    assert img.dtype == torch.uint8 and img.numel() == lib.he_tc_gather_bytes(C.c_longlong(n), C.c_int(64), C.c_int(K))
+    assert img.dtype == torch.uint8 and img.numel() == lib.he_tc_gather_bytes(C.c_longlong(n), C.c_int(K))
     assert set(asked) == {"moe_xs"} and asked["moe_xs"][1] == torch.bfloat16
     assert asked["moe_xs"][0] <= KN.moe_sorted_rows_bound(pairs, E) * K
