@@ -77,8 +77,9 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
-      sm100::mbar_init(&bar->full[s], 1);
-      sm100::mbar_init(&bar->empty[s], tc_empty_arrivals(stages));
+      sm100::mbar_init(&bar->full[0][s], 1);
+      sm100::mbar_init(&bar->full[1][s], 1);
+      sm100::mbar_init(&bar->empty[s], SUMS);
     }
     for (int s = 0; s < 4; ++s) {
       sm100::mbar_init(&bar->ready[s], TC_UNPACK_WARPS / 2);
@@ -189,9 +190,9 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
     const int q = warp & 3;
     const uint32_t at = tmem + ((uint32_t)(q * 32) << 16) + TC_A_COL + grp * TC_A_SLOT;
     const uint32_t mins = minima + grp * TC_MIN_BYTES + (uint32_t)((4 * q + (lane >> 3)) * 256 + (lane & 7) * 16);
-    const bool own = tc_own_stages(stages);
-    uint32_t j = 0, ph = 0, done_ph = 1;
-    int s = 0;
+    uint64_t* full = bar->full[grp];
+    uint32_t j = 0, done_ph = 1;
+    TcWalk at_stage;
     bool ok = true;
     const auto slot_free = [&](int half) {
       ok = ok && wait(&bar->done[2 * grp + half], done_ph, 403);
@@ -211,15 +212,11 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
       u += EXPERTS ? step : n_blk;
       for (int k = 0; k < n_blk; ++k, ++j) {
         const bool mine = (j & 1) == grp;
-        if (mine || !own) {
-          ok = wait(&bar->full[s], ph, 402);
+        if (mine) {
+          ok = wait(&full[at_stage.s], at_stage.ph, 402);
           if (!ok) break;
         }
-        if (!mine && !own) {
-          __syncwarp();
-          if (lane == 0) sm100::mbar_arrive(&bar->empty[s]);
-        }
-        const uint32_t row = ring + (uint32_t)s * stage_bytes + IMG_PAD + at_row.off;
+        const uint32_t row = ring + (uint32_t)at_stage.s * stage_bytes + IMG_PAD + at_row.off;
         if (mine && qtype == HE_Q8_0) {
           // 64 columns at a time: first and second operands in a half of the slot
           const float inv = __uint_as_float(0x7F000000u - __float_as_uint(tc_q80_pow(row, at_row)));
@@ -262,7 +259,7 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
           done_ph ^= 1u;
         }
         if (!ok) break;
-        if (++s == stages) { s = 0; ph ^= 1u; }
+        at_stage.next(stages);
       }
     }
     pdl_wait();
@@ -333,14 +330,14 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
     const uint8_t* image = reinterpret_cast<const uint8_t*>(a.image);
     const bool leader = sm100::elect_one();
     int si = EXPERTS ? 0 : segment(u0 / nb), tile = EXPERTS ? u0 : u0 / nb, blk = EXPERTS ? 0 : u0 % nb;
-    const auto weights = [&](int s) {
+    const auto weights = [&](int i, int s) {
       while (!EXPERTS && si + 1 < a.n_seg && tile >= a.seg[si + 1].tile0) ++si;
       const HeRowsSeg& sg = a.seg[si];
       const int qtype = type_of(sg), bb = rows_block_bytes(qtype);
       const bool pair = sg.epi >= 3;
       if (leader) {
         uint8_t* dst = smem + (size_t)s * stage_bytes + IMG_PAD;
-        uint64_t* full = &bar->full[s];
+        uint64_t* full = &bar->full[i & 1][s];
         sm100::mbar_expect_tx(full, (uint32_t)(TILE * bb + IMG));
         const int n0 = EXPERTS ? x.jobs[tile / a.tiles].x * x.expert_rows + tile % a.tiles * (pair ? HALF : TILE)
                                : (tile - sg.tile0) * (pair ? HALF : TILE);
@@ -361,28 +358,29 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
       __syncwarp();
       if (++blk == nb) { blk = 0; tile += EXPERTS ? step : 1; }
     };
-    const auto rows = [&](int s, int blk) {
-      if (leader) bulk_load(ring + (uint32_t)s * stage_bytes, image + (size_t)blk * IMG, IMG, &bar->full[s]);
+    const auto rows = [&](int i, int s, int blk) {
+      if (leader) bulk_load(ring + (uint32_t)s * stage_bytes, image + (size_t)blk * IMG, IMG, &bar->full[i & 1][s]);
       __syncwarp();
     };
     const int n = EXPERTS ? (u1 > u0 ? (u1 - u0 + step - 1) / step * nb : 0) : u1 - u0, pre = EXPERTS ? 0 : min(n, stages);
-    for (int i = 0; i < pre; ++i) weights(i);
+    for (int i = 0; i < pre; ++i) weights(i, i);
     pdl_wait();                         // the rows (and so their image) come from the kernels before
-    for (int i = 0; i < pre; ++i) rows(i, (u0 + i) % nb);
+    for (int i = 0; i < pre; ++i) rows(i, i, (u0 + i) % nb);
     int s = 0;
     uint32_t ph = 0;
     int issued = pre;
     for (int i = pre; i < n; ++i) {
       if (EXPERTS ? i >= stages && !wait(&bar->empty[s], ph ^ 1u, 401) : !wait(&bar->empty[s], ph, 401)) break;
       const int bi = EXPERTS ? tile / a.tiles * nb + blk : blk;
-      weights(s);
-      rows(s, bi);
+      weights(i, s);
+      rows(i, s, bi);
       ++issued;
       if (++s == stages) { s = 0; ph ^= 1u; }
     }
     if (issued < n) {                   // gave up: let the copies in flight land before the CTA leaves
-      for (int i = max(0, issued - stages); i < issued; ++i)
-        for (int p = 0; p < (1 << 16) && !sm100::mbar_test_wait(&bar->full[i % stages], (i / stages) & 1); ++p)
+      TcWalk at_stage;
+      for (int i = 0; i < issued; ++i, at_stage.next(stages))
+        for (int p = 0; i >= issued - stages && p < (1 << 16) && !sm100::mbar_test_wait(&bar->full[i & 1][at_stage.s], at_stage.ph); ++p)
           __nanosleep(64);
     }
   } else if (warp >= ISSUER) {
@@ -600,12 +598,16 @@ int herows::launch_rows_tc(const HeRowsArgs& a, int num_sms, cudaStream_t stream
   }
 }
 
-// Stages of the ring of a product of R rows with blocks of the largest type `qtype`, and how many
-// unpacking warps have to arrive, beside the summing ones, before one is loaded again.
-HE_API int he_rows_tc_ring(int R, int qtype, int* arrivals) {
-  const int s = ring_stages(tc_rows(R), TILE * rows_block_bytes(qtype));
-  *arrivals = tc_empty_arrivals(s) - TC_SUM_WARPS;
-  return s;
+// The way of blocks 0 .. n through the ring of a product of R rows (blocks of the largest type `qtype`): stage and parity of the
+// arrival of each.  Returns the stages.
+HE_API int he_rows_tc_walk(int R, int qtype, int n, int* stage, int* parity) {
+  const int stages = ring_stages(tc_rows(R), TILE * rows_block_bytes(qtype));
+  TcWalk w;
+  for (int j = 0; j < n; ++j, w.next(stages)) {
+    stage[j] = w.s;
+    parity[j] = (int)w.ph;
+  }
+  return stages;
 }
 
 // Bytes of the images of `jobs` jobs of up to 64 rows of K columns.

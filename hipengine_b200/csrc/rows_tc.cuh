@@ -12,20 +12,27 @@ constexpr int TC_MAX_STAGES = 8;
 constexpr int TC_SMEM = 227 * 1024;                 // dynamic shared memory of a block
 constexpr int TC_HALF = 64;                         // rows of each weight of a gate/up pair in a tile
 constexpr int TC_MIN_BYTES = 128 * 32;              // operand of the minima: 128 rows x 16 fp16
-// Arrivals that give a stage back: the summing warps, the last to read it.  Blocks go to the two groups of unpacking warps in turn: in an
-// even ring a group has stages of its own; in an odd one it has to see the other group's blocks land as well (a phase bit tells only
-// neighbours apart), so no stage is loaded again before that group's warps have looked at it.
-__host__ __device__ constexpr bool tc_own_stages(int stages) { return (stages & 1) == 0; }
-__host__ __device__ constexpr int tc_empty_arrivals(int stages) {
-  return TC_SUM_WARPS + (tc_own_stages(stages) ? 0 : TC_UNPACK_WARPS / 2);
-}
+// The way of a group of unpacking warps through the ring: a block's stage and the parity of its arrival.  Blocks go to the two groups in
+// turn, and an arrival is signalled to the group that takes the block alone: a phase bit tells only neighbours apart, and in an odd ring
+// a stage holds a block of each group in turn.  A group comes by all its barriers in one lap of an even ring, in two of an odd one.
+struct TcWalk {
+  int s = 0;
+  uint32_t ph = 0, lap = 0;
+  __host__ __device__ __forceinline__ void next(int stages) {
+    if (++s == stages) {
+      s = 0;
+      lap ^= 1u;
+      ph ^= (stages & 1) != 0 ? lap ^ 1u : 1u;
+    }
+  }
+};
 
 // Does a block of this type take a second operand for what the first one's rounding to 11 bits leaves?
 __host__ __device__ constexpr bool tc_two(int qtype) { return qtype == HE_Q8_0; }
 
 struct TcBars {
-  uint64_t full[TC_MAX_STAGES];     // blocks and image have landed
-  uint64_t empty[TC_MAX_STAGES];    // ... and are read (tc_empty_arrivals)
+  uint64_t full[2][TC_MAX_STAGES];  // blocks and image have landed, for the group of unpacking warps that takes them
+  uint64_t empty[TC_MAX_STAGES];    // ... and are read (by the summing warps, the last to do so)
   uint64_t ready[4];                // [2 slot + half]: the operand is stored
   uint64_t done[4];                 // the products of this half are complete
   uint64_t filled[2];               // the products of the block in this slot are complete

@@ -7,42 +7,39 @@ import pytest
 from hipengine_b200.core import native
 from hipengine_b200.quant.ggml import GGMLType as T
 
-BLOCKS = 9
+BLOCKS = 13
 
 
-def _lost(stages: int, arrivals: int) -> bool:
-    """Can the pipeline stop short of the last block?  All orders of: a producer that loads block j into stage j % stages, two groups
-    of expanding warps (one of each stands for the group's last) that take blocks in turn and, in an odd ring, look at the other
-    group's too, arriving on the stage's `empty` if it counts them (`arrivals`); a summer that follows the expanded blocks.
-    A barrier is the number of its completed phases; a wait for parity p passes while the last completed one has it."""
+def _lost(stages: int, parity, shared: bool) -> bool:
+    """Can the pipeline stop short of the last block, or a group take a block that has not landed?  All orders of: a producer that
+    loads block j into stage j % stages, two groups of expanding warps (one of each stands for the group's last) that take blocks in turn,
+    waiting for the arrival of block j with parity[j], and a summer that follows the expanded blocks and gives their stages back.
+    An arrival is signalled to the group that takes the block, or (`shared`) to both, which in an odd ring have to look at each
+    other's blocks then.  A barrier is the number of its completed phases; a wait for a parity passes while the last one has it."""
     passes = lambda phases, p: phases & 1 != p
-    own = stages % 2 == 0
-    start = (0, (0, 0), 0, (0,) * stages)                 # loaded, next block of each group, summed, group arrivals at `empty`
+    look = shared and stages % 2 == 1
+    start = (0, (0, 0), 0)                                # loaded, next block of each group, summed
     todo, seen = [start], {start}
     while todo:
-        loaded, at, summed, come = state = todo.pop()
+        loaded, at, summed = state = todo.pop()
         after = []
-        full = [(loaded - s + stages - 1) // stages for s in range(stages)]
-        # a stage is given back once its block is summed and, where they are counted, the other group's warps have come by
-        given = [min((summed - s + stages - 1) // stages, come[s] if arrivals else BLOCKS) for s in range(stages)]
         s = loaded % stages
-        if loaded < BLOCKS and (loaded < stages or passes(given[s], loaded // stages - 1 & 1)):
-            after.append((loaded + 1, at, summed, come))
+        if loaded < BLOCKS and (loaded < stages or passes((summed - s + stages - 1) // stages, loaded // stages - 1 & 1)):
+            after.append((loaded + 1, at, summed))
         for g in range(2):
             j = at[g]
             if j == BLOCKS:
                 continue
-            mine, s = j % 2 == g, j % stages
-            if (mine or not own) and not passes(full[s], j // stages & 1):
-                continue
-            nxt = (j + 1, at[1]) if g == 0 else (at[0], j + 1)
-            here = list(come)
-            if not mine and not own:
-                here[s] += 1
-            after.append((loaded, nxt, summed, tuple(here)))
+            phases = sum(i % stages == j % stages and (shared or i % 2 == j % 2) for i in range(loaded))
+            if j % 2 == g or look:
+                if not passes(phases, parity[j]):
+                    continue
+                if j >= loaded:
+                    return True
+            after.append((loaded, (j + 1, at[1]) if g == 0 else (at[0], j + 1), summed))
         if summed < BLOCKS and at[summed % 2] > summed:
-            after.append((loaded, at, summed + 1, come))
-        if not after and state[:3] != (BLOCKS, (BLOCKS, BLOCKS), BLOCKS):
+            after.append((loaded, at, summed + 1))
+        if not after and state != (BLOCKS, (BLOCKS, BLOCKS), BLOCKS):
             return True
         for x in after:
             if x not in seen:
@@ -52,13 +49,14 @@ def _lost(stages: int, arrivals: int) -> bool:
 
 
 @pytest.mark.skipif(not native.lib_available(), reason="native library not built")
-def test_no_stage_is_loaded_again_before_both_groups_have_seen_it():
-    assert _lost(3, 0) and not _lost(3, 1) and not _lost(4, 0) and not _lost(2, 0)
-    odd = 0
+def test_no_group_misses_the_arrival_of_a_block():
+    per_lap = lambda n: [j // n & 1 for j in range(BLOCKS)]
+    assert _lost(3, per_lap(3), True) and not _lost(4, per_lap(4), True) and _lost(3, per_lap(3), False)
+    stage, parity, odd = (C.c_int * BLOCKS)(), (C.c_int * BLOCKS)(), 0
     for rows in (17, 32, 33, 48, 49, 64):
         for t in (T.Q4_K, T.Q6_K, T.Q8_0):
-            n = C.c_int(-1)
-            stages = native.lib().he_rows_tc_ring(C.c_int(rows), C.c_int(int(t)), C.byref(n))
-            assert stages >= 2 and not _lost(stages, n.value), (rows, t, stages, n.value)
+            stages = native.lib().he_rows_tc_walk(C.c_int(rows), C.c_int(int(t)), C.c_int(BLOCKS), stage, parity)
+            assert stages >= 2 and list(stage) == [j % stages for j in range(BLOCKS)]
+            assert not _lost(stages, list(parity), False), (rows, t, stages, list(parity))
             odd += stages % 2
     assert odd > 0
