@@ -4,24 +4,26 @@
 //   operands : as in the mma.sync form: sc * q of a k-quant exactly in fp16 (one packed FMA makes two), fp32 sums of a 256-column
 //              block, d / dmin / the rows' powers of two once per block, the minima as one more MMA (16 columns, from shared memory)
 //              against the rows' sums.  Q8_0 (integer * fp16 scale: 19 bits) takes a second operand for what the first one's
-//              rounding leaves, into the accumulator of the minima (64 columns of both in half a slot): exact.  Q6_K: scale * (q - 32), 13 bits rounded to 11.
+//              rounding leaves, into the accumulator of the minima (64 columns of both in half a slot): exact down to 2^-22 of a
+//              block's largest scale.  Q6_K: scale * (q - 32), 13 bits rounded to 11.
 //   split    : (tile of 128 weight rows) x (block) units in one contiguous range per SM, shared tiles summed in CTA order by whoever
 //              arrives last, as in gemm_rows.cu
 //   roles    : eight unpacking warps in two groups, a slot of the tensor memory each: a thread expands a weight row (64 columns at a
 //              time, two k-blocks to a barrier).  Two issuers, one for each slot.  Eight summing warps: accumulators -> registers,
 //              scaled, over all blocks of the tile.  Producer and signal warp.
 //
-// What bounds it: chains of instructions in the warps that expand (a block costs a warp 2500 cycles at 1.9 GHz, half of them waits that
+// What bounds it (counters in profiles/few_row_products_and_expert_jobs.md: issue slots 33 %, tensor pipe 10-16 %, DRAM 18-22 %): chains of instructions in the warps that expand (a block costs a warp 2500 cycles at 1.9 GHz, half of them waits that
 // are over, branches and the hand-over; the two groups take turns), above 48 rows also the image, 35 KB from L2 for 18 KB of weights.
 // Tried: 16 unpacking warps (22.9 / 25.3 / 27.8 us at 32 / 48 / 64 rows where eight took 21.3 / 22.9 / 26.3), one issuer (23.3 / 24.3 /
 // 27.1), tiles of 256 rows that share an image (22.3 / 25.0 / 29.0: 19 % off a block, twice the partial tiles to sum).
 // Against mma.sync, whose warps each read the whole image for 16 weight rows (17408 x 5120, 32 / 48 / 64 rows, us in a graph):
-// Q4_K 30.7 / 37.9 / 46.8 -> 20.7 / 22.4 / 25.4, Q8_0 44.5 / 42.5 / 54.4 -> 36.3 / 38.0 / 40.3, Q6_K (5120 x 17408) 35.2 / 37.7 / 45.8
-// -> 27.0 / 29.4 / 32.6; a step of 64 rows, 8 layers of the 27B, 3295 -> 2315 us.
+// Q4_K 30.7 / 37.9 / 46.8 -> 20.0 / 21.7 / 24.8, Q8_0 44.5 / 42.5 / 54.4 -> 34.3 / 36.5 / 39.2, Q6_K (5120 x 17408) 35.2 / 37.7 / 45.8
+// -> 26.1 / 27.8 / 31.9; a step of 64 rows after 1000 tokens, 8 layers of the 27B, 3279 -> 2354 us.
 // Experts of prompts: the same pipeline over (job of up to 64 rows of an expert, tile) items.  A job's rows are first gathered into an
 // image of their own (43 us for 16384 rows of 2048 columns), which its tiles read from L2.  2048 rows, 256 experts, 8 used, hidden 2048,
-// width 512: gate/up 180-215 us and down 163 us a layer; the grouped GEMM took 130 + 124 + 52 (activation) and 190, with 128-row tiles
-// half padding, and rounds its weights to bf16, which these do not.
+// width 512 (Q4_K, Q6_K): gate/up 180-215 us and down 163 us a layer; the grouped GEMM took 130 + 124 + 52 (activation) and 190, with
+// 128-row tiles half padding, and rounds its weights to bf16, which these do not.  With Q8_0 experts it is the faster one above 64 pairs an
+// expert (models/moe.py).
 #include "rows_tc.cuh"
 
 using namespace he;
@@ -219,7 +221,7 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
         const uint32_t row = ring + (uint32_t)at_stage.s * stage_bytes + IMG_PAD + at_row.off;
         if (mine && qtype == HE_Q8_0) {
           // 64 columns at a time: first and second operands in a half of the slot
-          const float inv = __uint_as_float(0x7F000000u - __float_as_uint(tc_q80_pow(row, at_row)));
+          const float inv = tc_q80_inv(tc_q80_pow(row, at_row));
 #pragma unroll 2
           for (int c = 0; c < 4; ++c) {
             uint32_t x[32], f[2], r[32];
@@ -296,7 +298,7 @@ rows_gemm_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ 
             const float2 dv = __half22float2(*reinterpret_cast<const __half2*>(&dm));
             tc_add<NC, true>(t, N, xs, dv.x, -dv.y, sum);
           } else {
-            const float d = qtype == HE_Q6_K ? half_bits_to_f32((uint16_t)lds32(row + 208)) : tc_q80_pow(row, at_row);
+            const float d = qtype == HE_Q6_K ? half_bits_to_f32((uint16_t)lds32(row + 208)) : tc_q80_pow(row, at_row) * TC_Q80_SCALE;
             if (tc_two(qtype)) tc_add<NC, true>(t, N, xs, d, d, sum);
             else tc_add<NC, false>(t, N, xs, d, 0.f, sum);
           }

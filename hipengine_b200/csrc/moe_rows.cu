@@ -318,7 +318,8 @@ HE_API long long he_moe_jobs_bound(long long P, int E, int cols) {
   return full < P ? full : P;
 }
 
-// ids[P] (0 <= id < E <= 512; pairs with others are in no job) -> entries[P], jobs (4 ints each), meta[0].  cols: 8, 16 or 32.
+// ids[P] (0 <= id < E <= 512; pairs with others are in no job) -> entries[P], jobs (4 ints each), meta[0].  cols: 8, 16 or 32 for
+// he_rows_experts, 64 for he_tc_experts.
 HE_API int he_moe_jobs(const int* ids, int P, int E, int cols, int* entries, void* jobs, int max_jobs, int* meta,
                        cudaStream_t stream) {
   if (P <= 0) return 0;

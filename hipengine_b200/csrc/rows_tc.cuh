@@ -125,8 +125,8 @@ __device__ __forceinline__ void tc_q6k(uint32_t row, int c, uint32_t mg, uint32_
     }
   }
 }
-// Q8_0: the power of two that a row's block is held under, 2^-8 of that of its largest scale (511.75, the largest then, times -128 is
-// fp16's largest number); integers, and the scales under it (`inv`) of 32 columns each.  x * f rounds to 11 bits; what that leaves of the
+// Q8_0: the power of two of the largest scale of a row's block; integers, and the scales under 2^-8 of it (`inv`: 511.75, the largest then,
+// times -128 is fp16's largest number) of 32 columns each.  x * f rounds to 11 bits; what that leaves of the
 // 19, fma(x, f, -that), is exact down to 2^-24.  So scales down to 2^-22 of the block's largest are exact; smaller ones become multiples
 // of 2^-32 of its power of two.
 __device__ __forceinline__ float tc_q80_pow(uint32_t plane, const TcRow& at) {
@@ -135,8 +135,10 @@ __device__ __forceinline__ float tc_q80_pow(uint32_t plane, const TcRow& at) {
   const uint32_t v = __vmaxu2(__vmaxu2(s.x & m, s.y & m), __vmaxu2(s.z & m, s.w & m));
   const uint16_t top = (uint16_t)max(v & 0xFFFFu, v >> 16);
   const uint32_t e = __float_as_uint(half_bits_to_f32(top)) & 0x7F800000u;
-  return e == 0 ? 1.f : __uint_as_float(min(e, 143u << 23) - (8u << 23));        // (a scale that is not finite stays so)
+  return e == 0 ? 1.f : __uint_as_float(min(e, 143u << 23));        // (a scale that is not finite stays so)
 }
+constexpr float TC_Q80_SCALE = 1.f / 256.f;
+__device__ __forceinline__ float tc_q80_inv(float pow) { return __uint_as_float(0x7F000000u + (8u << 23) - __float_as_uint(pow)); }
 __device__ __forceinline__ void tc_q80(uint32_t plane, const TcRow& at, int c, float inv, uint32_t mg, uint32_t (&x)[32],
                                        uint32_t (&f)[2]) {
   const uint32_t scw = lds32(plane + at.rows * 256 + at.i * 16 + 4 * c);
