@@ -8,7 +8,7 @@ Three routes, chosen by the number of packed rows:
   sorted by expert and run as jobs (``csrc/moe_rows.cu``).  No expert id is ever read by the host,
   so the whole block is CUDA-graph capturable.
 * larger ``T`` with few pairs per expert (``JOBS_MAX_LOAD``): the same jobs, with the shared expert on the GEMM; up to
-  ``JOBS_TC_LOAD`` jobs of 64 rows on tcgen05.
+  ``JOBS_TC_LOAD`` jobs of 64 rows on tcgen05.  (Lines of their own with Q8_0 experts.)
 * larger ``T``: *grouped tensor-core GEMM*.  Pairs are bucketed by expert (128-row padded segments), rows are
   gathered and the tcgen05 GEMM runs in grouped mode over the experts' quantised blocks (each 128-row tile
   carries its expert id; the blocks are expanded to bf16 inside the GEMM pipeline), followed by a combine kernel that applies the routing weights, the

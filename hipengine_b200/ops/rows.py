@@ -1,5 +1,5 @@
-"""Launchers of the few-row products with quantised weights (``csrc/gemm_rows.cu``): 1..64 activation rows, written once
-per product as an image of MMA fragments, times any number of weight rows streamed once."""
+"""Launchers of the few-row products with quantised weights (``csrc/gemm_rows.cu``, on tcgen05 ``csrc/gemm_rows_tc.cu``): 1..64
+activation rows, written once per product as an image of MMA operands, times any number of weight rows streamed once."""
 from __future__ import annotations
 
 import ctypes as C
